@@ -60,8 +60,9 @@ __device__ __forceinline__ void st_dsmem_f32(float* local, unsigned rank, float 
 
 struct AttnArgs {
     const float* q;             // [n_head * hd], RoPE applied
-    const unsigned short* kc;   // layer base, [max_seq][n_kv * hd] f16 bits
+    const unsigned short* kc;   // layer base, [max_seq][n_kv * hd] f16 bits; with a TokenState: its cache + kv_off
     const unsigned short* vc;
+    size_t kv_off;
     float* partial;             // [n_head][S][2 + hd]: per-cluster partials (contexts of more than 8 splits)
     unsigned int* counters;     // [n_kv][8] (KV head, output slice), zero between launches
     float* out;                 // [n_head * hd]
@@ -142,6 +143,8 @@ __global__ void __launch_bounds__(attn_threads(STAGED, HD)) k_attn_decode(AttnAr
     // completes only after its predecessor: position and stop flag are final here, before the wait.
     const int done = st ? st->done : 0;
     const int T = (st ? st->pos : a.pos) + 1;
+    const unsigned short* const kc = st ? st->kv_k + a.kv_off : a.kc;
+    const unsigned short* const vc = st ? st->kv_v + a.kv_off : a.vc;
     int S_eff = (T + a.min_keys - 1) / a.min_keys;
     S_eff = S_eff < 1 ? 1 : (S_eff > a.S ? a.S : S_eff);
     // up to CL splits: the first cluster of the KV head merges on chip; its idle members
@@ -165,7 +168,7 @@ __global__ void __launch_bounds__(attn_threads(STAGED, HD)) k_attn_decode(AttnAr
             const int t = tt + kg + 4 * i;
             if (!fresh) vraw[i] = make_uint2(0u, 0u);
             if (fresh ? (t == T - 1 && t < t1) : t < limit) {
-                const unsigned short* vr = a.vc + (size_t)t * kvdim + g * HD + dp * DPT;
+                const unsigned short* vr = vc + (size_t)t * kvdim + g * HD + dp * DPT;
                 if constexpr (DPT == 4) vraw[i] = *reinterpret_cast<const uint2*>(vr);
                 else if constexpr (DPT == 2) vraw[i].x = *reinterpret_cast<const unsigned int*>(vr);
                 else vraw[i].x = *vr;
@@ -180,7 +183,7 @@ __global__ void __launch_bounds__(attn_threads(STAGED, HD)) k_attn_decode(AttnAr
                 const int t = tt + (bt * 8 + warp) * 4 + kk;
                 if (!fresh) kraw[bt][kk] = KRaw{};
                 if (fresh ? (t == T - 1 && t < t1) : t < limit) {
-                    const unsigned short* kr = a.kc + (size_t)t * kvdim + g * HD + lane * DL;
+                    const unsigned short* kr = kc + (size_t)t * kvdim + g * HD + lane * DL;
                     if constexpr (DL == 1) kraw[bt][kk] = *kr;
                     else kraw[bt][kk] = *reinterpret_cast<const KRaw*>(kr);
                 }
@@ -212,8 +215,8 @@ __global__ void __launch_bounds__(attn_threads(STAGED, HD)) k_attn_decode(AttnAr
                 const bool in = tt + row < t1;
                 if (tt + row == skip_row) continue;
                 const size_t off = (size_t)(in ? tt + row : t1 - 1) * kvdim + (size_t)g * HD + c8 * 8;
-                cp_async16(ks + row * KROW + c8 * 8, a.kc + off, in ? 16 : 0);
-                cp_async16(vs + row * KROW + c8 * 8, a.vc + off, in ? 16 : 0);
+                cp_async16(ks + row * KROW + c8 * 8, kc + off, in ? 16 : 0);
+                cp_async16(vs + row * KROW + c8 * 8, vc + off, in ? 16 : 0);
             }
         cp_async_commit();  // a group per tile slot, empty past the end: the wait in the tile loop counts groups
     };
@@ -399,8 +402,8 @@ __global__ void __launch_bounds__(attn_threads(STAGED, HD)) k_attn_decode(AttnAr
             if (T - 1 < t1 && row < (NST - 1) * ATTN_TILE && tid < 2 * CPR) {
                 const int st_ = row / ATTN_TILE, r = row % ATTN_TILE, c8 = tid % CPR;
                 const size_t off = (size_t)(T - 1) * kvdim + (size_t)g * HD + c8 * 8;
-                if (tid < CPR) *reinterpret_cast<int4*>(k_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(a.kc + off);
-                else *reinterpret_cast<int4*>(v_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(a.vc + off);
+                if (tid < CPR) *reinterpret_cast<int4*>(k_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(kc + off);
+                else *reinterpret_cast<int4*>(v_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(vc + off);
             }
         }
         constexpr int KS = HD / 16;  // 16-dim steps of the score product = 16-dim blocks of the value product
@@ -588,8 +591,8 @@ __global__ void __launch_bounds__(attn_threads(STAGED, HD)) k_attn_decode(AttnAr
             if (T - 1 < t1 && row < (NST - 1) * ATTN_TILE && tid < 2 * CPR) {
                 const int st_ = row / ATTN_TILE, r = row % ATTN_TILE, c8 = tid % CPR;
                 const size_t off = (size_t)(T - 1) * kvdim + (size_t)g * HD + c8 * 8;
-                if (tid < CPR) *reinterpret_cast<int4*>(k_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(a.kc + off);
-                else *reinterpret_cast<int4*>(v_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(a.vc + off);
+                if (tid < CPR) *reinterpret_cast<int4*>(k_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(kc + off);
+                else *reinterpret_cast<int4*>(v_stage(st_) + r * KROW + c8 * 8) = *reinterpret_cast<const int4*>(vc + off);
             }
         }
         // Both phases are register-blocked so that shared-memory reads stay well below the FMA count (a 16-byte read

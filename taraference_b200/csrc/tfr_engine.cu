@@ -113,6 +113,17 @@ struct TpPlan {
     int v0 = 0, v1 = 0;                         // vocabulary rows of the head
 };
 
+// Captured decode steps.  Kernels find the cache through TokenState, so what a graph depends on is the cache's capacity
+// alone (layer stride, attention route): conversations of one capacity share it.
+struct TokenGraphs {
+    int max_seq = 0;
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};  // [0] with the vocabulary head, [1] without
+    int nodes[2] = {0, 0};
+};
+constexpr size_t TFR_MAX_GRAPHS = 4;
+constexpr size_t STATE_STRIDE = 256;  // bytes of the state block in front of the emitted tokens
+static_assert(sizeof(TokenState) <= STATE_STRIDE, "the emitted tokens follow the state");
+
 constexpr int TFR_MAX_BURST = 8192;
 constexpr int TFR_MAX_PROMPT = 65536;
 
@@ -146,17 +157,14 @@ struct tfr_engine {
     unsigned int* counters = nullptr;
     TokenState* st = nullptr;
     TokenState* st_host = nullptr;  // pinned
-    int *out_tokens = nullptr, *out_host = nullptr, *prompt = nullptr;
-    int *args_dev = nullptr, *args_host = nullptr;  // per-call scalars: pinned host -> device
+    int *out_tokens = nullptr, *out_host = nullptr, *prompt = nullptr;  // the tokens lie behind the state: one copy fetches both
     int attn_S = 1, attn_S_staged = 1, attn_min_keys = 64;  // splits per KV head of the two attention instances
     float* layer_taps = nullptr;  // [n_layer][n_embd] residual stream after each layer (test aid)
     // [n_layer][...] the other vectors a dense layer quantises: attention output, residual after o-proj, SiLU*mul (test aid)
     float *tap_attn = nullptr, *tap_mid = nullptr, *tap_h = nullptr;
     // graphs
     bool use_graph = true;
-    cudaGraphExec_t g_decode = nullptr, g_body = nullptr;
-    const tfr_kv* graph_kv = nullptr;
-    int nodes_decode = 0, nodes_body = 0;
+    std::vector<TokenGraphs> graphs;  // one entry per KV capacity in use, the one used last in front
     int64_t launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
@@ -205,8 +213,9 @@ struct tfr_kv {
 };
 
 static bool is_hybrid(const tfr_engine* e) { return e->cfg.hybrid != 0; }
-static unsigned short* kv_k(const tfr_kv* kv, int li) { return kv->k + (size_t)(kv->kv_slot[li] < 0 ? 0 : kv->kv_slot[li]) * kv->layer_stride; }
-static unsigned short* kv_v(const tfr_kv* kv, int li) { return kv->v + (size_t)(kv->kv_slot[li] < 0 ? 0 : kv->kv_slot[li]) * kv->layer_stride; }
+static size_t kv_layer_off(const tfr_kv* kv, int li) { return (size_t)(kv->kv_slot[li] < 0 ? 0 : kv->kv_slot[li]) * kv->layer_stride; }
+static unsigned short* kv_k(const tfr_kv* kv, int li) { return kv->k + kv_layer_off(kv, li); }
+static unsigned short* kv_v(const tfr_kv* kv, int li) { return kv->v + kv_layer_off(kv, li); }
 // A forward call may run: the exchange the engine is set to use has everything it needs.
 static bool tp_ready(const tfr_engine* e) { return e->use_nccl ? e->nccl_ready : e->peers_wired; }
 static int gdn_channels(const tfr_model_config& c) { return (2 * c.ssm_group_count + c.ssm_time_step_rank) * c.ssm_state_size; }
@@ -592,11 +601,13 @@ extern "C" int tfr_create(int device, tfr_engine** out) {
     return TFR_OK;
 }
 
+static void drop_graph(TokenGraphs& g) {
+    for (cudaGraphExec_t x : g.exec)
+        if (x) cudaGraphExecDestroy(x);
+}
 static void drop_graphs(tfr_engine* e) {
-    if (e->g_decode) cudaGraphExecDestroy(e->g_decode);
-    if (e->g_body) cudaGraphExecDestroy(e->g_body);
-    e->g_decode = e->g_body = nullptr;
-    e->graph_kv = nullptr;
+    for (TokenGraphs& g : e->graphs) drop_graph(g);
+    e->graphs.clear();
 }
 
 extern "C" void tfr_destroy(tfr_engine* e) {
@@ -614,13 +625,10 @@ extern "C" void tfr_destroy(tfr_engine* e) {
     for (auto& kv : e->mats) tfr_mat_free(kv.second);
     for (auto& kv : e->vecs) cudaFree(kv.second.dev);
     for (auto& L : e->layers) cudaFree(L.bias_qkv);
-    void* ws[] = {e->x, e->q, e->attn, e->h, e->logits, e->partial, e->counters, e->st, e->out_tokens, e->prompt,
+    void* ws[] = {e->x, e->q, e->attn, e->h, e->logits, e->partial, e->counters, e->st, e->prompt,
                   e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
     for (void* p : ws) cudaFree(p);
     if (e->st_host) cudaFreeHost(e->st_host);
-    if (e->out_host) cudaFreeHost(e->out_host);
-    if (e->args_host) cudaFreeHost(e->args_host);
-    cudaFree(e->args_dev);
     cudaEventDestroy(e->ev0);
     cudaEventDestroy(e->ev1);
     cudaStreamDestroy(e->stream);
@@ -1200,13 +1208,11 @@ extern "C" int tfr_finalize_load(tfr_engine* e) {
         CU(e, cudaMalloc(&e->comm_local, e->comm.lay.total));
         CU(e, cudaMemsetAsync(e->comm_local, 0, e->comm.lay.total, e->stream));
     }
-    CU(e, cudaMalloc(&e->st, sizeof(TokenState)));
-    CU(e, cudaMalloc(&e->out_tokens, (size_t)TFR_MAX_BURST * 4));
+    CU(e, cudaMalloc(&e->st, STATE_STRIDE + (size_t)TFR_MAX_BURST * 4));
+    e->out_tokens = reinterpret_cast<int*>(reinterpret_cast<char*>(e->st) + STATE_STRIDE);
     CU(e, cudaMalloc(&e->prompt, (size_t)TFR_MAX_PROMPT * 4));
-    CU(e, cudaMallocHost(&e->st_host, sizeof(TokenState)));
-    CU(e, cudaMallocHost(&e->out_host, (size_t)TFR_MAX_BURST * 4));
-    CU(e, cudaMalloc(&e->args_dev, 16 * sizeof(int)));  // k_state_begin reads [0..14]
-    CU(e, cudaMallocHost(&e->args_host, 16 * sizeof(int)));
+    CU(e, cudaMallocHost(&e->st_host, STATE_STRIDE + (size_t)TFR_MAX_BURST * 4));
+    e->out_host = reinterpret_cast<int*>(reinterpret_cast<char*>(e->st_host) + STATE_STRIDE);
     CU(e, cudaMemsetAsync(e->counters, 0, (size_t)P.n_kv * ATTN_CLUSTER * 4, e->stream));
     CU(e, cudaMemsetAsync(e->st, 0, sizeof(TokenState), e->stream));
     CU(e, cudaMemsetAsync(e->logits, 0, (size_t)Vl * 4, e->stream));
@@ -1259,7 +1265,6 @@ extern "C" int tfr_alloc_kv(tfr_engine* e, int max_seq, tfr_kv** out) {
 }
 extern "C" void tfr_free_kv(tfr_kv* kv) {
     if (!kv) return;
-    if (kv->e && kv->e->graph_kv == kv) drop_graphs(kv->e);
     cudaFree(kv->k);
     cudaFree(kv->v);
     cudaFree(kv->ssm);
@@ -1372,9 +1377,9 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
         pn.raw_out = e->x;
         pn.prof_id = n;
         AttnArgs a{};
+        const size_t kv_off = kv_layer_off(kv, li);
         a.q = e->q;
-        a.kc = kv_k(kv, li);
-        a.vc = kv_v(kv, li);
+        a.kv_off = kv_off;
         a.partial = e->partial;
         a.counters = e->counters;
         a.out = e->attn + P.attn_off;
@@ -1418,8 +1423,8 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             GdnArgs g{};
             g.proj = e->proj;
             g.conv_w = L.conv_w;
-            g.conv_ring = kv->conv + (size_t)li * kv->conv_stride;
-            g.state = kv->ssm + (size_t)li * kv->ssm_stride;
+            g.conv_off = (size_t)li * kv->conv_stride;
+            g.state_off = (size_t)li * kv->ssm_stride;
             g.ssm_a = L.ssm_a;
             g.ssm_dt = L.ssm_dt;
             g.norm_w = L.ssm_norm;
@@ -1449,8 +1454,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             qa.k_norm = L.k_norm;
             qa.q_out = e->q;
             qa.gate_out = e->qgate;
-            qa.kc = kv_k(kv, li);
-            qa.vc = kv_v(kv, li);
+            qa.kv_off = kv_off;
             qa.n_head = P.n_head;
             qa.n_kv = P.n_kv;
             qa.hd = hd;
@@ -1472,13 +1476,11 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             fseg.m = L.wv->m;
             fseg.sh = make_share(nkv / 2, cap);
             fseg.id_base = (nq + nkv) / 2;
-            pn.l2_rows_a = (const unsigned char*)(kv_k(kv, li));
-            pn.l2_rows_b = (const unsigned char*)(kv_v(kv, li));
-            pn.l2_row_bytes = nkv * 2;
+            pn.l2_kv_off = kv_off;
+            pn.l2_row_bytes = li > 0 ? nkv * 2 : 0;
             EpiQkv epi{};
             epi.q_out = e->q;
-            epi.kc = kv_k(kv, li);
-            epi.vc = kv_v(kv, li);
+            epi.kv_off = kv_off;
             epi.bias = L.bias_qkv;
             epi.nq = nq;
             epi.nk = nkv;
@@ -1559,39 +1561,59 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
     return n;
 }
 
-static int ensure_graphs(tfr_engine* e, const tfr_kv* kv) {
-    if (e->graph_kv == kv && e->g_decode && e->g_body) return TFR_OK;
-    drop_graphs(e);
-    for (int which = 0; which < 2; which++) {
-        cudaGraph_t g = nullptr;
-        CU(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
-        int n = record_token(e, kv, which == 0);
-        cudaError_t r = cudaStreamEndCapture(e->stream, &g);
-        if (n < 0 || r != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            cudaGetLastError();
-            return fail(e, TFR_E_CUDA, "graph capture failed: %s", cudaGetErrorString(r));
+// The graph of a decode step with / without the vocabulary head on caches of kv's capacity, captured on first use.
+static int token_graph(tfr_engine* e, const tfr_kv* kv, bool with_head, TokenGraphs*& out) {
+    size_t at = 0;
+    while (at < e->graphs.size() && e->graphs[at].max_seq != kv->max_seq) at++;
+    if (at == e->graphs.size()) {
+        if (at == TFR_MAX_GRAPHS) {
+            CU(e, cudaStreamSynchronize(e->stream));  // the one given up may still run
+            drop_graph(e->graphs.back());
+            e->graphs.pop_back();
+            at--;
         }
-        cudaGraphExec_t ex = nullptr;
-        r = cudaGraphInstantiate(&ex, g, 0);
-        cudaGraphDestroy(g);
-        if (r != cudaSuccess) return fail(e, TFR_E_CUDA, "graph instantiate: %s", cudaGetErrorString(r));
-        if (which == 0) {
-            e->g_decode = ex;
-            e->nodes_decode = n;
-        } else {
-            e->g_body = ex;
-            e->nodes_body = n;
-        }
+        e->graphs.emplace_back();
+        e->graphs.back().max_seq = kv->max_seq;
     }
-    e->graph_kv = kv;
+    if (at) std::rotate(e->graphs.begin(), e->graphs.begin() + at, e->graphs.begin() + at + 1);
+    TokenGraphs& t = e->graphs.front();
+    out = &t;
+    const int which = with_head ? 0 : 1;
+    if (t.exec[which]) return TFR_OK;
+    cudaGraph_t g = nullptr;
+    CU(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
+    const int n = record_token(e, kv, with_head);
+    cudaError_t r = cudaStreamEndCapture(e->stream, &g);
+    if (n < 0 || r != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        cudaGetLastError();
+        return fail(e, TFR_E_CUDA, "graph capture failed: %s", cudaGetErrorString(r));
+    }
+    r = cudaGraphInstantiate(&t.exec[which], g, 0);
+    cudaGraphDestroy(g);
+    if (r != cudaSuccess) {
+        t.exec[which] = nullptr;
+        return fail(e, TFR_E_CUDA, "graph instantiate: %s", cudaGetErrorString(r));
+    }
+    t.nodes[which] = n;
     return TFR_OK;
+}
+
+// Captures what a call is about to replay, ahead of its timed region.
+static int ready_graphs(tfr_engine* e, const tfr_kv* kv, bool body) {
+    if (!e->use_graph || use_loop(e)) return TFR_OK;
+    TokenGraphs* t = nullptr;
+    const int rc = token_graph(e, kv, true, t);
+    return rc || !body ? rc : token_graph(e, kv, false, t);
 }
 
 static int run_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
     if (e->use_graph) {
-        CU(e, cudaGraphLaunch(with_head ? e->g_decode : e->g_body, e->stream));
-        e->launches += with_head ? e->nodes_decode : e->nodes_body;
+        TokenGraphs* t = nullptr;
+        const int rc = token_graph(e, kv, with_head, t);
+        if (rc) return rc;
+        CU(e, cudaGraphLaunch(t->exec[with_head ? 0 : 1], e->stream));
+        e->launches += t->nodes[with_head ? 0 : 1];
         return TFR_OK;
     }
     int n = record_token(e, kv, with_head);
@@ -1599,7 +1621,6 @@ static int run_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
     e->launches += n;
     return TFR_OK;
 }
-
 
 // ------------------------------------------------------------------ multi-token chunks
 
@@ -1784,29 +1805,31 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
 
 static int begin_state(tfr_engine* e, const tfr_kv* kv, int token, int pos, int max_steps, int max_seq, const uint32_t* stops,
                        int n_stop, int force_prompt = 0) {
-    int* a = e->args_host;
+    BeginArgs a{};
     // the conv ring's write slot follows the position; the offset keeps it continuous when the
     // caller moved the KV length between calls
     const int ck = is_hybrid(e) ? e->cfg.ssm_conv_kernel : 1;
-    a[13] = (int)(((kv->rec_steps - pos) % ck + ck) % ck);
-    a[14] = force_prompt;
-    a[0] = token;
-    a[1] = pos;
-    a[2] = max_steps;
-    a[3] = max_seq;
-    a[4] = n_stop;
-    for (int i = 0; i < 8; i++) a[5 + i] = i < n_stop ? (int)stops[i] : -1;
-    CU(e, cudaMemcpyAsync(e->args_dev, a, 16 * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    k_state_begin<<<1, 1, 0, e->stream>>>(e->st, e->args_dev);
+    a.ring_off = (int)(((kv->rec_steps - pos) % ck + ck) % ck);
+    a.force_prompt = force_prompt;
+    a.token = token;
+    a.pos = pos;
+    a.max_steps = max_steps;
+    a.max_seq = max_seq;
+    a.n_stop = n_stop;
+    for (int i = 0; i < 8; i++) a.stop_ids[i] = i < n_stop ? (int)stops[i] : -1;
+    a.kv_k = kv->k;
+    a.kv_v = kv->v;
+    a.kv_ssm = kv->ssm;
+    a.kv_conv = kv->conv;
+    k_state_begin<<<1, 1, 0, e->stream>>>(e->st, a);
     CU(e, cudaGetLastError());
     e->launches += 1;
     return TFR_OK;
 }
 
 static int finish_state(tfr_engine* e, int n_tokens_out) {
-    CU(e, cudaMemcpyAsync(e->st_host, e->st, sizeof(TokenState), cudaMemcpyDeviceToHost, e->stream));
-    if (n_tokens_out > 0)
-        CU(e, cudaMemcpyAsync(e->out_host, e->out_tokens, (size_t)n_tokens_out * 4, cudaMemcpyDeviceToHost, e->stream));
+    const size_t bytes = n_tokens_out > 0 ? STATE_STRIDE + (size_t)n_tokens_out * 4 : sizeof(TokenState);
+    CU(e, cudaMemcpyAsync(e->st_host, e->st, bytes, cudaMemcpyDeviceToHost, e->stream));
     CU(e, cudaStreamSynchronize(e->stream));
     cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1);
     if (e->st_host->err == 3) return fail(e, TFR_E_CUDA, "tensor parallelism: a peer rank did not deliver within the wait limit");
@@ -1826,15 +1849,11 @@ extern "C" int tfr_forward_greedy(tfr_engine* e, tfr_kv* kv, const uint32_t* tok
         if (tokens[i] >= (uint32_t)e->token_embd->m.N) return fail(e, TFR_E_INVALID, "token id %u out of range", tokens[i]);
     cudaSetDevice(e->device);
     const bool loop = use_loop(e);
-    if (e->use_graph && !loop) {
-        int rc = ensure_graphs(e, kv);
-        if (rc) return rc;
-    }
-    CU(e, cudaMemcpyAsync(e->prompt, tokens, (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
+    if (n > 1) CU(e, cudaMemcpyAsync(e->prompt, tokens, (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
     // all but the last token go through the chunk kernels (weights read once per chunk); the last is a decode step
     const bool chunked = !loop && e->chunk_ok && e->chunk_tokens > 0 && n > 1;
-    int rc = TFR_OK;
-    if (chunked) rc = chunk_buffers(e);
+    int rc = ready_graphs(e, kv, n > 1 && !chunked);
+    if (!rc && chunked) rc = chunk_buffers(e);
     if (rc) return rc;
     rc = begin_state(e, kv, (int)tokens[chunked ? n - 1 : 0], kv->len + (chunked ? n - 1 : 0), 1, kv->max_seq + 1, nullptr, 0);
     if (rc) return rc;
@@ -1873,10 +1892,6 @@ extern "C" int tfr_forward_greedy_all(tfr_engine* e, tfr_kv* kv, const uint32_t*
         if (tokens[i] >= (uint32_t)e->token_embd->m.N) return fail(e, TFR_E_INVALID, "token id %u out of range", tokens[i]);
     cudaSetDevice(e->device);
     const bool loop = use_loop(e);
-    if (e->use_graph && !loop) {
-        int rc = ensure_graphs(e, kv);
-        if (rc) return rc;
-    }
     CU(e, cudaMemcpyAsync(e->prompt, tokens, (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
     const bool chunked = !loop && e->chunk_ok && e->chunk_tokens > 0 && n > 1 && !e->vocab_limit;
     int rc = TFR_OK;
@@ -1901,7 +1916,8 @@ extern "C" int tfr_forward_greedy_all(tfr_engine* e, tfr_kv* kv, const uint32_t*
         kv->rec_steps += n;
         return TFR_OK;
     }
-    rc = begin_state(e, kv, (int)tokens[0], kv->len, n, kv->max_seq + 1, nullptr, 0, 1);
+    rc = ready_graphs(e, kv, false);
+    if (!rc) rc = begin_state(e, kv, (int)tokens[0], kv->len, n, kv->max_seq + 1, nullptr, 0, 1);
     if (rc) return rc;
     CU(e, cudaEventRecord(e->ev0, e->stream));
     if (loop) rc = run_loop(e, kv, 0);
@@ -1930,11 +1946,8 @@ extern "C" int tfr_decode_burst(tfr_engine* e, tfr_kv* kv, uint32_t first_token,
     int n_run = max_n < TFR_MAX_BURST ? max_n : TFR_MAX_BURST;
     if (n_run > kv->max_seq - kv->len) n_run = kv->max_seq - kv->len;
     const bool loop = use_loop(e);
-    if (e->use_graph && !loop) {
-        int rc = ensure_graphs(e, kv);
-        if (rc) return rc;
-    }
-    int rc = begin_state(e, kv, (int)first_token, kv->len, n_run, kv->max_seq + 1, stop_ids, n_stop);
+    int rc = ready_graphs(e, kv, false);
+    if (!rc) rc = begin_state(e, kv, (int)first_token, kv->len, n_run, kv->max_seq + 1, stop_ids, n_stop);
     if (rc) return rc;
     CU(e, cudaEventRecord(e->ev0, e->stream));
     if (loop) rc = run_loop(e, kv, 0);
@@ -2092,7 +2105,7 @@ extern "C" int tfr_set_cuda_graph(tfr_engine* e, int enabled) {
     if (!e->use_graph) drop_graphs(e);
     return TFR_OK;
 }
-extern "C" int tfr_graph_active(const tfr_engine* e) { return e && e->use_graph && e->g_decode ? 1 : 0; }
+extern "C" int tfr_graph_active(const tfr_engine* e) { return e && e->use_graph && !e->graphs.empty() && e->graphs.front().exec[0] ? 1 : 0; }
 extern "C" int64_t tfr_launch_count(const tfr_engine* e) { return e ? e->launches : 0; }
 extern "C" float tfr_last_device_ms(const tfr_engine* e) { return e ? e->last_ms : 0.f; }
 

@@ -21,7 +21,8 @@ struct GdnArgs {
     const float* proj;     // [channels | val_dim | n_v | n_v]: raw qkv, z gate, beta, alpha projections
     const float* conv_w;   // [channels][kernel], tap k of channel c at k + c * kernel (GGUF dims [kernel, channels])
     float* conv_ring;      // [kernel][channels]: slot (pos + ring_off) % kernel takes the current input
-    float* state;          // [n_v][128][128] fp32
+    float* state;          // [n_v][128][128] fp32; with a TokenState: its cache's arrays + the two offsets
+    size_t conv_off, state_off;
     const float* ssm_a;    // [n_v], already -exp(A_log)
     const float* ssm_dt;   // [n_v]
     const float* norm_w;   // [128]
@@ -55,6 +56,10 @@ __global__ void __launch_bounds__(GDN_THREADS, 1) k_gdn_step(GdnArgs a, const To
     griddep_wait();  // the projections come from the previous kernel
     griddep_launch_dependents();
     if (st && st->done) return;
+    if (st) {
+        a.conv_ring = st->kv_conv + a.conv_off;
+        a.state = st->kv_ssm + a.state_off;
+    }
     constexpr int D = GDN_D, R = D / GDN_PARTS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.x, hk = h % a.n_k;
@@ -145,8 +150,9 @@ struct QkNormArgs {
     const float* k_norm;
     float* q_out;             // [n_head * hd]
     float* gate_out;          // [n_head * hd]
-    unsigned short* kc;       // layer base [max_seq][n_kv * hd]
+    unsigned short* kc;       // layer base [max_seq][n_kv * hd]; with a TokenState: its cache + kv_off
     unsigned short* vc;
+    size_t kv_off;
     int n_head, n_kv, hd, n_rot;
     float theta, eps;
     int pos;                  // used when st == nullptr
@@ -156,6 +162,10 @@ __global__ void __launch_bounds__(256) k_qk_norm_rope_store(QkNormArgs a, const 
     griddep_wait();
     griddep_launch_dependents();
     if (st && st->done) return;
+    if (st) {
+        a.kc = st->kv_k + a.kv_off;
+        a.vc = st->kv_v + a.kv_off;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int head = blockIdx.x, hd = a.hd;
     const bool isq = head < a.n_head;

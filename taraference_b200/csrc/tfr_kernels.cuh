@@ -61,14 +61,19 @@ struct EpiSilu {
 struct EpiQkv {
     static constexpr int MODE = EPI_PAIRS;
     float* q_out;            // [n_head * hd] natural order
-    unsigned short* kc;      // layer base [max_seq][kvdim]
+    unsigned short* kc;      // layer base [max_seq][kvdim]; with a TokenState: its cache + kv_off
     unsigned short* vc;
     const float* bias;       // [nq + nk + nv] in stored-row order, or nullptr
     int nq, nk, hd, kvdim;
     float theta;
     int pos;
+    size_t kv_off;
     __device__ void begin(const TokenState* st) {
-        if (st) pos = st->pos;
+        if (st) {
+            pos = st->pos;
+            kc = st->kv_k + kv_off;
+            vc = st->kv_v + kv_off;
+        }
     }
     __device__ __forceinline__ bool wants_residual() const { return false; }
     __device__ __forceinline__ float residual(int) const { return 0.f; }
@@ -211,10 +216,9 @@ struct PrepArgs {
     float* raw_out;       // embedding source only: CTA 0 stores the decoded row here (residual stream)
     int token;            // embedding source without TokenState
     int prof_id;          // timeline probe: which launch of the token this is (test aid)
-    // rows [0, pos] of these two arrays (row_bytes each) are pulled into L2 for the kernel that follows
-    // (the layer's K and V cache before flash-decode); nullptr: none
-    const unsigned char* l2_rows_a;
-    const unsigned char* l2_rows_b;
+    // rows [0, pos] of the layer's K and V cache (l2_row_bytes each, at element kv_off of the call's cache) are pulled
+    // into L2 for the flash-decode kernel that follows; l2_row_bytes 0: none
+    size_t l2_kv_off;
     int l2_row_bytes;
 };
 
@@ -383,17 +387,16 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             wreg[k] = i4 < (K >> 2) ? reinterpret_cast<const float4*>(pa.normw)[i4] : make_float4(1.f, 1.f, 1.f, 1.f);
         }
     }
-    if (pa.l2_rows_a && st && tid == GEMV_THREADS - 32) {
-        // A hint only: the position may still be the previous token's if the kernel before this one is the
-        // vocabulary head; a row more or less in L2 changes nothing but timing.
+    if (pa.l2_row_bytes && st && tid == GEMV_THREADS - 32) {
+        // Never in a layer 0: behind the kernel that begins a call the state may not have landed yet.
         const int rows = st->pos + 1, per = (rows + (int)gridDim.x - 1) / (int)gridDim.x;
         const int r0 = cta * per, r1 = min(rows, r0 + per);
         if (r1 > r0) {
             const size_t off = (size_t)r0 * pa.l2_row_bytes;
             const unsigned bytes = (unsigned)((r1 - r0) * pa.l2_row_bytes) & ~15u;
             if (bytes) {
-                bulk_prefetch_l2(pa.l2_rows_a + off, bytes);
-                bulk_prefetch_l2(pa.l2_rows_b + off, bytes);
+                bulk_prefetch_l2(reinterpret_cast<const unsigned char*>(st->kv_k + pa.l2_kv_off) + off, bytes);
+                bulk_prefetch_l2(reinterpret_cast<const unsigned char*>(st->kv_v + pa.l2_kv_off) + off, bytes);
             }
         }
     }
@@ -807,24 +810,33 @@ __global__ void k_permute_f32(const float* __restrict__ src, float* __restrict__
     if (v < n) dst[v] = src[perm_src_row(v, perm_hd)];
 }
 
-// Decode-state control (single thread each).  args (device memory, copied from the host per call):
-// [0] token, [1] pos, [2] max_steps, [3] max_seq, [4] n_stop, [5..12] stop ids, [13] conv ring offset,
-// [14] forced-input (verification) flag.
-__global__ void k_state_begin(TokenState* st, const int* __restrict__ args) {
-    st->token = args[0];
-    st->pos = args[1];
+// Decode-state control (single thread each).  What a call starts from travels as the kernel's parameter: no copy.
+struct BeginArgs {
+    int token, pos, max_steps, max_seq, n_stop;
+    int stop_ids[8];
+    int ring_off, force_prompt;
+    unsigned short *kv_k, *kv_v;
+    float *kv_ssm, *kv_conv;
+};
+__global__ void k_state_begin(TokenState* st, const BeginArgs a) {
+    st->token = a.token;
+    st->pos = a.pos;
     st->step = 0;
-    st->max_steps = args[2];
-    st->max_seq = args[3];
+    st->max_steps = a.max_steps;
+    st->max_seq = a.max_seq;
     st->done = 0;
-    st->n_stop = args[4];
-    for (int i = 0; i < 8; i++) st->stop_ids[i] = args[5 + i];
+    st->n_stop = a.n_stop;
+    for (int i = 0; i < 8; i++) st->stop_ids[i] = a.stop_ids[i];
     st->best = 0ull;
     st->head_done = 0u;
     st->prompt_idx = 0;
     st->err = 0;
-    st->ring_off = args[13];
-    st->force_prompt = args[14];
+    st->ring_off = a.ring_off;
+    st->force_prompt = a.force_prompt;
+    st->kv_k = a.kv_k;
+    st->kv_v = a.kv_v;
+    st->kv_ssm = a.kv_ssm;
+    st->kv_conv = a.kv_conv;
 }
 
 // Second half of the vocabulary head when the (max, argmax) exchange is done by a library all-reduce:
