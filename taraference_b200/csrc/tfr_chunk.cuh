@@ -9,9 +9,9 @@
 //   k_prep_rows      per token: RMSNorm (kernels/ops.cu:4-34) + Q8 quantiser (kernels/gemv.cu:16-65) -> global
 //   k_gemm_q8        every weight tile is brought on chip once per launch and dotted with the activations of up
 //                    to Mt tokens at a time; same block dots, row sums and epilogues as the batch-1 kernels
-//                    (K rows, fp32-route V rows, Q8_0 matrices, batches of fewer than five tokens)
-//   k_gemm_mma_q4 / k_gemm_mma_q6   the other projections: the same integer sub-block dots as int8 tensor-core MMAs
-//                    over CTA tiles of rows x tokens, scale arithmetic on the accumulator fragments
+//                    (Q8_0 matrices, batches of fewer than five tokens)
+//   k_gemm_tc        the other projections, on the tensor cores (tfr_gemm_tc.cuh, with a k_prep_tc of its own; the
+//                    fp32-route V rows beside it are k_rows_f32)
 //   k_attn_chunk / k_attn_chunk_mma   causal attention of a tile of query tokens x the query heads of one KV head
 //                    over the f16 cache, on CUDA cores / on the tensor cores (head sizes up to 128)
 //   k_argmax_rows    greedy token of every row                                        (kernels/ops.cu:601-629)
@@ -26,8 +26,9 @@
 
 namespace tfr {
 
-constexpr int CHUNK_MAX_TOKENS = 64;   // tokens per chunk forward
+constexpr int CHUNK_MAX_TOKENS = 2048; // tokens per chunk forward: enough that the weights' share of a chunk's time is small
 constexpr int CHUNK_VERIFY_MAX = 16;   // tokens per chunk when every row's greedy token is wanted (logits [M][V])
+constexpr int GEMM_TC_MIN_TOKENS = 5;  // smaller batches keep the dp4a projections
 constexpr int CHUNK_ATTN_SPLITS_MAX = 32;  // most key splits of the chunk attention
 
 // ------------------------------------------------------------------ embedding rows
@@ -230,12 +231,10 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
     unsigned long long* full = reinterpret_cast<unsigned long long*>(pbuf + (size_t)Mt * g.pbuf_floats);
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(full + wa * nsw) + 127) & ~(uintptr_t)127);
 
-    const int rows_a0 = ja.sh.begin(cta) * ja.rows_per_item;
-    const int rows_a = max(0, min(ja.sh.count(cta) * ja.rows_per_item, ja.m.N - rows_a0));
-    const int rows_b0 = jb.m.data ? jb.sh.begin(cta) * jb.rows_per_item : 0;
-    const int rows_b = jb.m.data ? max(0, min(jb.sh.count(cta) * jb.rows_per_item, jb.m.N - rows_b0)) : 0;
-    const long long fa0 = (long long)rows_a0 * nb, fa1 = fa0 + (long long)rows_a * nb;
-    const long long fb0 = (long long)rows_b0 * nb, fb1 = fb0 + (long long)rows_b * nb;
+    const int rows_a0 = ja.row0(cta), rows_a = max(0, ja.rows(cta)), blocks_a = group_rows(rows_a) * nb;
+    const int rows_b0 = jb.m.data ? jb.row0(cta) : 0, rows_b = jb.m.data ? max(0, jb.rows(cta)) : 0, blocks_b = group_rows(rows_b) * nb;
+    const long long fa0 = (long long)rows_a0 * nb, fa1 = fa0 + blocks_a;
+    const long long fb0 = (long long)rows_b0 * nb, fb1 = fb0 + blocks_b;
     const int ta0 = (int)(fa0 >> 5), tiles_a = rows_a > 0 ? (int)((fa1 + 31) >> 5) - ta0 : 0;
     const int tb0 = (int)(fb0 >> 5), tiles_b = rows_b > 0 ? (int)((fb1 + 31) >> 5) - tb0 : 0;
     const int n_jobs = tiles_a + tiles_b;
@@ -283,7 +282,7 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
                 float w[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) w[i] = 0.f;
-                if (on && row_g < fseg.m.N) q6k_run_weights_f32(fseg.m, (long long)row_g * nb + (rem >> 4), rem & 15, w);
+                if (on && row_g < fseg.m.N) q6k_run_weights_f32(fseg.m, mat_flat(nb, row_g, rem >> 4), rem & 15, w);
                 for (int m0 = 0; m0 < g.M; m0 += Mt) {
                     const int mt = min(Mt, g.M - m0);
                     if (on)
@@ -334,7 +333,7 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
                     const int row_g = 2 * (pbase + p0) + row_l;
                     float v = 0.f;
                     if (row_g < fseg.m.N)
-                        v = q6k_run_dot_f32_g(fseg.m, (long long)row_g * nb + (rem >> 4), rem >> 4, rem & 15, xn + (size_t)(m0 + m) * K);
+                        v = q6k_run_dot_f32_g(fseg.m, mat_flat(nb, row_g, rem >> 4), rem >> 4, rem & 15, xn + (size_t)(m0 + m) * K);
                     pbuf[(size_t)m * g.pbuf_floats + t] = v;
                 }
                 __syncthreads();
@@ -373,8 +372,9 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
                     if (q == 0) late_slot = s, late_parity = 0u;
                 }
                 if (mine) {
-                    const int off = is_b ? rows_a * nb + (int)(f - fb0) : (int)(f - fa0);
-                    const int b = (int)(f % nb);
+                    int row, b;
+                    flat_row_block((int)(f - (is_b ? fb0 : fa0)), nb, row, b);
+                    const int off = (is_b ? blocks_a : 0) + row * nb + b;
                     const unsigned char* tile = ring + (size_t)(j * nsw + s) * TB;
                     for (int m = q; m < mt; m += H) {
                         const Act act = act_carve(act_s + (size_t)m * g.act_b16, K, false, false);
@@ -397,8 +397,9 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
                 late_parity = (unsigned)((k / nsw) & 1);
             }
             if (mine) {
-                const int off = is_b ? rows_a * nb + (int)(f - fb0) : (int)(f - fa0);
-                const int b = (int)(f % nb);
+                int row, b;
+                flat_row_block((int)(f - (is_b ? fb0 : fa0)), nb, row, b);
+                const int off = (is_b ? blocks_a : 0) + row * nb + b;
                 // (Sharing the nibble masks / 6-bit assembly of a block across four tokens was measured: at the 64
                 // registers a 1024-thread CTA allows it spills and runs 13 % slower than one block_dot per token.)
                 for (int m = 0; m < mt; m++) {
@@ -421,7 +422,7 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
         for (int m = grp; m < mt; m += G) {
             const ChunkEpiTok et{&epi, m0 + m};
             const float* part_a = pbuf + (size_t)m * g.pbuf_floats;
-            const float* part_b = part_a + rows_a * nb;
+            const float* part_b = part_a + blocks_a;
             if (epi.kind == CEPI_SILU) {
                 reduce_rows_group<EPI_ZIP>(part_a, part_b, rows_a, nb, ja.id_base + rows_a0, et, wig, gw);
             } else {
@@ -445,7 +446,7 @@ struct GemmLaunch {
 inline GemmLaunch gemm_plan(int tile_bytes, int M, int K, const RowJob& ja, const RowJob& jb, bool with_f32) {
     GemmLaunch L{};
     const int nb = K / 256;
-    const int ra = (ja.sh.quot + 1) * ja.rows_per_item, rb = jb.m.data ? (jb.sh.quot + 1) * jb.rows_per_item : 0;
+    const int ra = ja.rows_max(), rb = jb.m.data ? jb.rows_max() : 0;
     int pf = ((ra + rb) * nb + 3) & ~3;
     if (with_f32 && pf < 2 * 16 * nb) pf = 2 * 16 * nb;
     const size_t act_b16 = (act_smem_bytes(K, false, false) + 15) & ~(size_t)15;
@@ -476,449 +477,6 @@ inline cudaError_t launch_gemm(cudaStream_t stream, int grid, const unsigned cha
     if (!L.fits) return cudaErrorInvalidValue;
     L.g.act_stride = act_stride;
     return launch_pdl(k_gemm_q8<BLK>, dim3(grid), dim3(GEMV_THREADS), L.smem, stream, act_g, xn, ja, jb, fseg, epi, L.g, st);
-}
-
-// ------------------------------------------------------------------ the chunk GEMM on the tensor cores (Q4_K)
-
-// CTA tile = 16 * RG rows x 64 tokens, k-loop over the 256-weight blocks, both operands staged in shared memory three
-// or four k steps deep by 16-byte asynchronous copies: the 144-byte block of (row r, block b) is nine pieces of the tiled layout, the
-// tokens' int8 groups of block b are sixteen pieces of their activation record, their group scales and scaled sums four
-// more.  A warp owns 16 rows and NBW blocks of eight tokens.  The sub-block dots I_j = sum nibble * q8 (kernels/gemv.cu:
-// 71-130) run as m16n8k32 u8 x s8 MMAs — the low nibbles of a 32-byte stretch are sub-block 2 t, the high nibbles, left
-// in place and shifted out of the sum afterwards, sub-block 2 t + 1 — and are the exact integers of block_dot; the scale
-// arithmetic runs on the accumulator fragments (a lane holds two rows x two tokens), block partials d * acc - dmin *
-// accm are summed along k in registers.  That order of a row's sum differs from reduce_rows' butterfly: results agree
-// with the decode kernels' to fp32 rounding, not bit for bit.
-constexpr int GM_MT = 64;         // tokens per CTA tile (16 for batches of up to 16 tokens)
-constexpr int GM_ASTRIDE = 160;   // bytes per staged Q4_K block (144 + 16): 8 words modulo 32, four rows' 8-byte reads of four lanes each fill the banks
-constexpr int GM4_BSTRIDE = 288;  // bytes per staged token in the Q4_K kernel (256 int8 + 32): 8 words modulo 32 as well
-constexpr int GM_BSTRIDE = 272;   // bytes per staged token in the Q6_K kernel (256 int8 + 16): 4 words modulo 32 for its 4-byte reads
-constexpr int GM_THREADS = 256;
-constexpr int GEMM_MMA_MIN_TOKENS = 5;   // smaller batches keep the dp4a kernel
-inline size_t gemm_mma_stage_bytes(int rg, bool zip, int mt) { return (size_t)rg * 16 * GM_ASTRIDE * (zip ? 2 : 1) + (size_t)mt * GM4_BSTRIDE + (size_t)mt * 64; }
-// Stages of the copy pipeline: the 16-row tiles do little per k step and need the copies of three steps in flight to hide
-// a trip to L2; the others take three stages (one barrier per k step).
-__host__ __device__ constexpr int gemm_mma_stages(int rg) { return rg == 1 ? 4 : 3; }
-inline size_t gemm_mma_smem(int rg, bool zip, int mt) { return gemm_mma_stages(rg) * gemm_mma_stage_bytes(rg, zip, mt); }
-
-__device__ __forceinline__ void mma_16832_u8s8(int (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// ZIP: two matrices of the same shape (gate, up), epilogue apply(row, gate, up); otherwise one matrix and the
-// pair-ordered epilogues (store / Q, K rows with RoPE), whose two rows meet by a shuffle.
-template <int RG, bool ZIP, int MT>
-__global__ void __launch_bounds__(GM_THREADS, 2)
-k_gemm_mma_q4(const unsigned char* act_g, size_t act_stride, Mat A1, Mat B2, int id_base1, int id_base2, ChunkEpi epi, int M, int m_base) {
-    constexpr int NBW = MT * RG / 64;            // 8-token blocks per warp: 8 warps = RG row groups x (8 / RG) token parts of MT * RG / 8 tokens
-    static_assert(NBW >= 1, "a token part holds at least one block of eight tokens");
-    constexpr int NMAT = ZIP ? 2 : 1;
-    constexpr int TB = Q4_TILE_BYTES;
-    extern __shared__ __align__(128) unsigned char gm_smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
-    // Without ZIP a second matrix of the same K may follow the first in the grid (the K rows behind the Q rows: one launch
-    // instead of two): a CTA's rows lie in one of them.
-    const int tiles1 = (A1.N + RG * 16 - 1) / (RG * 16);
-    const bool second = !ZIP && B2.data != nullptr && (int)blockIdx.x >= tiles1;
-    const Mat A = second ? B2 : A1;
-    const int id_base = second ? id_base2 : id_base1;
-    const int K = A.K, nb = A.nb;
-    const int row0 = (second ? (int)blockIdx.x - tiles1 : (int)blockIdx.x) * RG * 16;
-    const size_t a_bytes = (size_t)RG * 16 * GM_ASTRIDE, stage_b = a_bytes * NMAT + (size_t)MT * GM4_BSTRIDE + (size_t)MT * 64;
-    const int mt = min(MT, M - m_base);       // tokens of this launch's token tile
-    const unsigned char* act_t = act_g + (size_t)m_base * act_stride;
-    auto stage_a = [&](int st_, int mat) { return gm_smem + (size_t)st_ * stage_b + (size_t)mat * a_bytes; };
-    auto stage_q = [&](int st_) { return gm_smem + (size_t)st_ * stage_b + a_bytes * NMAT; };
-    auto stage_s = [&](int st_) { return reinterpret_cast<float*>(gm_smem + (size_t)st_ * stage_b + a_bytes * NMAT + (size_t)MT * GM4_BSTRIDE); };
-    constexpr int NST = gemm_mma_stages(RG);
-    auto issue = [&](int b, int st_) {
-        if (b >= nb) {
-            cp_async_commit();  // an empty group keeps the count of the wait below
-            return;
-        }
-#pragma unroll
-        for (int mat = 0; mat < NMAT; mat++) {
-            const uint8_t* data = mat ? B2.data : A.data;
-            unsigned char* dst = stage_a(st_, mat);
-            for (int i = tid; i < RG * 16 * 9; i += GM_THREADS) {
-                const int r = i / 9, piece = i - r * 9;
-                const long long f = (long long)min(row0 + r, A.N - 1) * nb + b;  // rows past the matrix repeat its last row
-                cp_async16(dst + r * GM_ASTRIDE + piece * 16, data + (f >> 5) * TB + piece * 512 + (f & 31) * 16, 16);
-            }
-        }
-        unsigned char* q = stage_q(st_);
-        for (int i = tid; i < MT * 16; i += GM_THREADS) {
-            const int t = i >> 4, c = i & 15;
-            const bool in = t < mt;
-            cp_async16(q + t * GM4_BSTRIDE + c * 16, act_t + (size_t)(in ? t : 0) * act_stride + ((size_t)c * nb + b) * 16, in ? 16 : 0);
-        }
-        float* sc = stage_s(st_);
-        for (int i = tid; i < MT * 4; i += GM_THREADS) {
-            const int t = i >> 2, part = i & 3;  // parts 0, 1: group scales d8[8 b ..]; 2, 3: scaled sums ds[8 b ..]
-            const bool in = t < mt;
-            const unsigned char* rec = act_t + (size_t)(in ? t : 0) * act_stride + K + (part >> 1) * (K / 32) * 4;
-            cp_async16(sc + t * 16 + part * 4, rec + (size_t)(8 * b + 4 * (part & 1)) * 4, in ? 16 : 0);
-        }
-        cp_async_commit();
-    };
-    griddep_wait();
-    griddep_launch_dependents();
-    const int rg = warp % RG, tpart = warp / RG;  // row group and token part of this warp
-    float total[NMAT][NBW][4];
-#pragma unroll
-    for (int mat = 0; mat < NMAT; mat++)
-#pragma unroll
-        for (int n = 0; n < NBW; n++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) total[mat][n][i] = 0.f;
-#pragma unroll
-    for (int p = 0; p < NST - 1; p++) issue(p, p);
-    for (int b = 0; b < nb; b++) {
-        const int st_ = b % NST;
-        cp_async_wait_group<NST - 2>();  // this thread's pieces of step b
-        __syncthreads();                 // everybody's pieces, and everybody is done with step b - 1
-        issue(b + NST - 1, (b + NST - 1) % NST);  // into the stage step b - 1 has just left
-        const unsigned char* qs = stage_q(st_);
-        const float* scs = stage_s(st_);
-#pragma unroll
-        for (int mat = 0; mat < NMAT; mat++) {
-            const unsigned char* ar = stage_a(st_, mat) + (size_t)(rg * 16 + gq) * GM_ASTRIDE;  // row gq of the group; row gq + 8 is 8 strides on
-            // d, dmin and the 6-bit scales and mins of the two rows (kernels/common.cu:40-50, as in block_dot)
-            unsigned sc_lo[2], sc_hi[2], m_lo[2], m_hi[2];
-            float2 dd[2];
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const int4 wh = *reinterpret_cast<const int4*>(ar + r * 8 * GM_ASTRIDE);
-                const unsigned s0 = (unsigned)wh.y, s1 = (unsigned)wh.z, s2 = (unsigned)wh.w;
-                sc_lo[r] = s0 & 0x3f3f3f3fu, sc_hi[r] = (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
-                m_lo[r] = s1 & 0x3f3f3f3fu, m_hi[r] = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
-                dd[r] = __half22float2(*reinterpret_cast<const __half2*>(&wh.x));
-            }
-#pragma unroll
-            for (int n = 0; n < NBW; n++) {
-                const int tok0 = (tpart * NBW + n) * 8;
-                if (tok0 >= mt) continue;  // the same for the whole warp
-                // group scales (d8) and scaled sums (ds) of tokens tok0 + 2 tq, + 1 for the eight sub-blocks
-                float d8[2][8], ds[2][8];
-#pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    const float4* sp = reinterpret_cast<const float4*>(scs + (tok0 + 2 * tq + c) * 16);
-                    const float4 x0 = sp[0], x1 = sp[1], y0 = sp[2], y1 = sp[3];
-                    d8[c][0] = x0.x, d8[c][1] = x0.y, d8[c][2] = x0.z, d8[c][3] = x0.w, d8[c][4] = x1.x, d8[c][5] = x1.y, d8[c][6] = x1.z, d8[c][7] = x1.w;
-                    ds[c][0] = y0.x, ds[c][1] = y0.y, ds[c][2] = y0.z, ds[c][3] = y0.w, ds[c][4] = y1.x, ds[c][5] = y1.y, ds[c][6] = y1.z, ds[c][7] = y1.w;
-                }
-                // The order of a sub-block's 32 products is free: MMA k slots 4 tq .. and 16 + 4 tq .. take elements
-                // 8 tq .. 8 tq + 3 and 8 tq + 4 .. 8 tq + 7, so a lane's two weight words and two activation words are
-                // one 8-byte read each.
-                const unsigned char* qt = qs + (size_t)(tok0 + gq) * GM4_BSTRIDE + 8 * tq;  // B operand: token tok0 + gq
-                float acc[4] = {0.f, 0.f, 0.f, 0.f}, accm[4] = {0.f, 0.f, 0.f, 0.f};  // [0], [1]: row gq, tokens 2 tq, + 1; [2], [3]: row gq + 8
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    const uint2 wa = *reinterpret_cast<const uint2*>(ar + (1 + 2 * t) * 16 + tq * 8);                   // row gq
-                    const uint2 wb = *reinterpret_cast<const uint2*>(ar + 8 * GM_ASTRIDE + (1 + 2 * t) * 16 + tq * 8);  // row gq + 8
-                    const unsigned w[4] = {wa.x, wb.x, wa.y, wb.y};
-#pragma unroll
-                    for (int half = 0; half < 2; half++) {
-                        const int j = 2 * t + half;
-                        const unsigned mask = half ? 0xf0f0f0f0u : 0x0f0f0f0fu;
-                        const unsigned af[4] = {w[0] & mask, w[1] & mask, w[2] & mask, w[3] & mask};
-                        const uint2 bw = *reinterpret_cast<const uint2*>(qt + j * 32);
-                        const unsigned b0 = bw.x, b1 = bw.y;
-                        int c[4] = {0, 0, 0, 0};
-                        mma_16832_u8s8(c, af, b0, b1);
-                        if (half) {
-#pragma unroll
-                            for (int i = 0; i < 4; i++) c[i] >>= 4;  // the high nibbles were multiplied as nibble * 16
-                        }
-#pragma unroll
-                        for (int r = 0; r < 2; r++) {
-                            const int scj = ((j < 4 ? sc_lo[r] : sc_hi[r]) >> (8 * (j & 3))) & 0xff;
-                            const float mj = i2f_small((int)(((j < 4 ? m_lo[r] : m_hi[r]) >> (8 * (j & 3))) & 0xff));
-#pragma unroll
-                            for (int cc = 0; cc < 2; cc++) {
-                                acc[2 * r + cc] = fmaf(d8[cc][j], i2f_small(c[2 * r + cc] * scj), acc[2 * r + cc]);
-                                accm[2 * r + cc] = fmaf(ds[cc][j], mj, accm[2 * r + cc]);
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < 2; r++)
-#pragma unroll
-                    for (int cc = 0; cc < 2; cc++) total[mat][n][2 * r + cc] += dd[r].x * acc[2 * r + cc] - dd[r].y * accm[2 * r + cc];
-            }
-        }
-    }
-    cp_async_wait_all();
-    // ---- epilogue: a lane holds rows gq, gq + 8 of its group x tokens 2 tq, 2 tq + 1 of its token blocks
-#pragma unroll
-    for (int n = 0; n < NBW; n++) {
-        const int tok0 = (tpart * NBW + n) * 8;
-        if (tok0 >= mt) continue;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int row = row0 + rg * 16 + gq + 8 * r;
-            if (ZIP) {
-#pragma unroll
-                for (int cc = 0; cc < 2; cc++) {
-                    const int t = tok0 + 2 * tq + cc;
-                    if (row < A.N && t < mt) ChunkEpiTok{&epi, m_base + t}.apply(id_base + row, total[0][n][2 * r + cc], total[NMAT - 1][n][2 * r + cc]);
-                }
-            } else {
-                // rows 2 p and 2 p + 1 sit in lanes gq and gq ^ 1: the even lane takes token 2 tq, the odd one 2 tq + 1
-                const float mine0 = total[0][n][2 * r], mine1 = total[0][n][2 * r + 1];
-                const float other0 = __shfl_xor_sync(TFR_FULL_MASK, mine0, 4), other1 = __shfl_xor_sync(TFR_FULL_MASK, mine1, 4);
-                const bool odd = gq & 1;
-                const int t = tok0 + 2 * tq + (odd ? 1 : 0), row_even = row & ~1;
-                const float x0 = odd ? other1 : mine0, x1 = odd ? mine1 : other0;
-                if (row_even < A.N && t < mt) ChunkEpiTok{&epi, m_base + t}.apply(id_base + (row_even >> 1), x0, x1);
-            }
-        }
-    }
-}
-
-// Launches k_gemm_mma_q4 for one matrix or two in a row (pair-ordered epilogues) or a gate / up pair (ZIP).  Row tiles of 64 when
-// that still gives every SM a CTA, of 16 otherwise (the output and down projections have 2 048 rows).
-inline cudaError_t launch_gemm_mma_q4(cudaStream_t stream, int sms, const unsigned char* act_g, size_t act_stride, int M, const RowJob& ja,
-                                      const RowJob& jb, const ChunkEpi& epi) {
-    const bool zip = epi.kind == CEPI_SILU;
-    const bool two = !zip && jb.m.data != nullptr;  // a second matrix behind the first (Q rows, then K rows)
-    const int rows = ja.m.N + (two ? jb.m.N : 0);
-    const bool big = (rows + 63) / 64 >= sms;
-    const bool few = M <= 16 && big;  // a token tile of 16: every warp of a 64-row CTA has a token block
-    // 64-row tiles that do not divide evenly over the SMs leave some SMs twice the rows of the others (11 008 rows: 172
-    // tiles on 148 SMs): 32-row tiles then even the load out at a little more unpacking per MMA
-    const int t64 = (rows + 63) / 64, t32 = (rows + 31) / 32;
-    const bool mid = big && !few && ((t32 + sms - 1) / sms) * 32 < ((t64 + sms - 1) / sms) * 64;
-    const int rg = mid ? 2 : big ? 4 : 1, mt_tile = few ? 16 : GM_MT;
-    const int tile_rows = 16 * rg;
-    const dim3 grid((ja.m.N + tile_rows - 1) / tile_rows + (two ? (jb.m.N + tile_rows - 1) / tile_rows : 0)), block(GM_THREADS);
-    const size_t smem = gemm_mma_smem(rg, zip, mt_tile);
-    const Mat m2 = (zip || two) ? jb.m : Mat{};
-    const int id1 = ja.id_base, id2 = two ? jb.id_base : 0;
-    for (int m_base = 0; m_base < M; m_base += mt_tile) {
-        cudaError_t r;
-        if (zip) r = few   ? launch_pdl(k_gemm_mma_q4<4, true, 16>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base)
-                     : mid ? launch_pdl(k_gemm_mma_q4<2, true, 64>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base)
-                     : big ? launch_pdl(k_gemm_mma_q4<4, true, 64>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base)
-                           : launch_pdl(k_gemm_mma_q4<1, true, 64>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base);
-        else r = few   ? launch_pdl(k_gemm_mma_q4<4, false, 16>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base)
-                 : mid ? launch_pdl(k_gemm_mma_q4<2, false, 64>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base)
-                 : big ? launch_pdl(k_gemm_mma_q4<4, false, 64>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base)
-                       : launch_pdl(k_gemm_mma_q4<1, false, 64>, grid, block, smem, stream, act_g, act_stride, ja.m, m2, id1, id2, epi, M, m_base);
-        if (r != cudaSuccess) return r;
-    }
-    return cudaSuccess;
-}
-
-// ------------------------------------------------------------------ the chunk GEMM on the tensor cores (Q6_K)
-
-// The same frame for Q6_K matrices (down, the head): 64 rows x 64 tokens per CTA, eight warps = four row groups x two
-// token halves, and optionally a part of the k range (grid.y parts: a matrix of 2 048 rows has only 32 row tiles).
-// A block's sixteen scale groups are one m16n8k16 s8 x s8 MMA each: the 6-bit values are assembled from the ql nibbles
-// and qh bit pairs as in block_dot(BlockQ6) (kernels/gemv.cu:302-337), the accumulators start at -32 * sum(q8) of the
-// group, so the MMA leaves the exact J = sum (q6 - 32) * q8.  With k parts the CTA stores its partial sums and
-// k_gemm_splitk_finish adds the parts in a fixed order and runs the epilogue.
-constexpr int GM6_ASTRIDE = 240;  // 13 pieces + the d pair + padding: eight rows' words hit 32 different banks
-inline size_t gemm_mma_q6_smem(int mt) { return 2 * ((size_t)64 * GM6_ASTRIDE + (size_t)mt * GM_BSTRIDE + (size_t)mt * 96); }
-
-__device__ __forceinline__ void mma_16816_s8(int (&c)[4], unsigned a0, unsigned a1, unsigned b0) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(b0));
-}
-
-template <int MT>
-__global__ void __launch_bounds__(GM_THREADS, 2)
-k_gemm_mma_q6(const unsigned char* act_g, size_t act_stride, Mat A, int id_base, ChunkEpi epi, int M, float* partial) {
-    constexpr int RG = 4, NBW = MT / 16, TB = Q6_TILE_BYTES;  // eight warps = four row groups x two token halves of MT / 2 tokens
-    extern __shared__ __align__(128) unsigned char gm_smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
-    const int K = A.K, nb = A.nb;
-    const int row0 = blockIdx.x * RG * 16;
-    const int kparts = gridDim.y, kp = blockIdx.y;
-    const int b_begin = (int)((long long)nb * kp / kparts), b_end = (int)((long long)nb * (kp + 1) / kparts);
-    constexpr size_t a_bytes = (size_t)RG * 16 * GM6_ASTRIDE, q_bytes = (size_t)MT * GM_BSTRIDE, stage_b = a_bytes + q_bytes + (size_t)MT * 96;
-    const int mt = min(MT, M);
-    auto stage_a = [&](int st_) { return gm_smem + (size_t)st_ * stage_b; };
-    auto stage_q = [&](int st_) { return gm_smem + (size_t)st_ * stage_b + a_bytes; };
-    auto stage_x = [&](int st_) { return gm_smem + (size_t)st_ * stage_b + a_bytes + q_bytes; };  // per token: 8 floats d8, 16 ints -32 * S16
-    auto issue = [&](int b, int st_) {
-        unsigned char* dst = stage_a(st_);
-        for (int i = tid; i < RG * 16 * 14; i += GM_THREADS) {
-            const int r = i / 14, piece = i - r * 14;
-            const long long f = (long long)min(row0 + r, A.N - 1) * nb + b;  // rows past the matrix repeat its last row
-            const uint8_t* tile = A.data + (f >> 5) * TB;
-            if (piece < 13) cp_async16(dst + r * GM6_ASTRIDE + piece * 16, tile + piece * 512 + (f & 31) * 16, 16);
-            else cp_async4(dst + r * GM6_ASTRIDE + 208, tile + Q6_PIECES * 512 + ((f & 31) & ~1) * 2);  // d of this block and its neighbour
-        }
-        unsigned char* q = stage_q(st_);
-        for (int i = tid; i < MT * 16; i += GM_THREADS) {
-            const int t = i >> 4, c = i & 15;
-            const bool in = t < mt;
-            cp_async16(q + t * GM_BSTRIDE + c * 16, act_g + (size_t)(in ? t : 0) * act_stride + ((size_t)c * nb + b) * 16, in ? 16 : 0);
-        }
-        unsigned char* x = stage_x(st_);
-        for (int i = tid; i < MT * 6; i += GM_THREADS) {
-            const int t = i / 6, part = i - t * 6;  // parts 0, 1: d8[8 b ..]; 2 .. 5: s16n[16 b ..]
-            const bool in = t < mt;
-            const unsigned char* rec = act_g + (size_t)(in ? t : 0) * act_stride + K;
-            const unsigned char* src = part < 2 ? rec + (size_t)(8 * b + 4 * part) * 4 : rec + (size_t)(K / 32) * 8 + (size_t)(16 * b + 4 * (part - 2)) * 4;
-            cp_async16(x + t * 96 + part * 16, src, in ? 16 : 0);
-        }
-        cp_async_commit();
-    };
-    griddep_wait();
-    griddep_launch_dependents();
-    const int rg = warp & 3, tpart = warp >> 2;
-    float total[NBW][4];
-#pragma unroll
-    for (int n = 0; n < NBW; n++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) total[n][i] = 0.f;
-    if (b_begin < b_end) issue(b_begin, 0);
-    for (int b = b_begin; b < b_end; b++) {
-        const int st_ = (b - b_begin) & 1;
-        if (b + 1 < b_end) {
-            issue(b + 1, st_ ^ 1);
-            cp_async_wait_group<1>();
-        } else {
-            cp_async_wait_all();
-        }
-        __syncthreads();
-        const unsigned char* qs = stage_q(st_);
-        const unsigned char* xs = stage_x(st_);
-        const unsigned char* ar = stage_a(st_) + (size_t)(rg * 16 + gq) * GM6_ASTRIDE;  // row gq of the group; row gq + 8 is 8 strides on
-        int4 wsc[2];
-        float dw[2];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            wsc[r] = *reinterpret_cast<const int4*>(ar + r * 8 * GM6_ASTRIDE + 12 * 16);
-            const unsigned dpair = *reinterpret_cast<const unsigned*>(ar + r * 8 * GM6_ASTRIDE + 208);
-            const long long f = (long long)min(row0 + rg * 16 + gq + 8 * r, A.N - 1) * nb + b;
-            dw[r] = f16_to_f32((unsigned short)((f & 1) ? dpair >> 16 : dpair & 0xffffu));
-        }
-#pragma unroll
-        for (int n = 0; n < NBW; n++) {
-            const int tok0 = (tpart * NBW + n) * 8;
-            if (tok0 >= mt) continue;  // the same for the whole warp
-            float d8[2][8];
-            int s16[2][16];
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const int4* xp = reinterpret_cast<const int4*>(xs + (size_t)(tok0 + 2 * tq + c) * 96);
-                const int4 x0 = xp[0], x1 = xp[1];
-                d8[c][0] = __int_as_float(x0.x), d8[c][1] = __int_as_float(x0.y), d8[c][2] = __int_as_float(x0.z), d8[c][3] = __int_as_float(x0.w);
-                d8[c][4] = __int_as_float(x1.x), d8[c][5] = __int_as_float(x1.y), d8[c][6] = __int_as_float(x1.z), d8[c][7] = __int_as_float(x1.w);
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int4 y = xp[2 + k];
-                    s16[c][4 * k] = y.x, s16[c][4 * k + 1] = y.y, s16[c][4 * k + 2] = y.z, s16[c][4 * k + 3] = y.w;
-                }
-            }
-            const unsigned char* qt = qs + (size_t)(tok0 + gq) * GM_BSTRIDE + 4 * tq;  // B operand: token tok0 + gq
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};  // [0], [1]: row gq, tokens 2 tq, + 1; [2], [3]: row gq + 8
-#pragma unroll
-            for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-                for (int is = 0; is < 2; is++) {
-                    unsigned la[2], lb[2], hw[2];
-#pragma unroll
-                    for (int r = 0; r < 2; r++) {
-                        const unsigned char* rowp = ar + r * 8 * GM6_ASTRIDE + tq * 4;
-                        la[r] = *reinterpret_cast<const unsigned*>(rowp + (4 * nn + is) * 16);
-                        lb[r] = *reinterpret_cast<const unsigned*>(rowp + (4 * nn + 2 + is) * 16);
-                        hw[r] = *reinterpret_cast<const unsigned*>(rowp + (8 + 2 * nn + is) * 16);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int c = 8 * nn + 2 * j + is;  // the scale group: elements 16 c .. 16 c + 15 of the block
-                        unsigned af[2];
-#pragma unroll
-                        for (int r = 0; r < 2; r++) {
-                            const unsigned nibw = (j & 1) ? lb[r] : la[r];
-                            af[r] = ((nibw >> (4 * (j >> 1))) & 0x0f0f0f0fu) | (((hw[r] >> (2 * j)) << 4) & 0x30303030u);
-                        }
-                        const unsigned b0 = *reinterpret_cast<const unsigned*>(qt + c * 16);
-                        int cj[4] = {s16[0][c], s16[1][c], s16[0][c], s16[1][c]};
-                        mma_16816_s8(cj, af[0], af[1], b0);
-#pragma unroll
-                        for (int r = 0; r < 2; r++) {
-                            const int w = r ? (c < 4 ? wsc[1].x : c < 8 ? wsc[1].y : c < 12 ? wsc[1].z : wsc[1].w)
-                                            : (c < 4 ? wsc[0].x : c < 8 ? wsc[0].y : c < 12 ? wsc[0].z : wsc[0].w);
-                            const float cf = i2f_small((int)(signed char)((w >> (8 * (c & 3))) & 0xff));
-#pragma unroll
-                            for (int cc = 0; cc < 2; cc++) acc[2 * r + cc] = fmaf(cf * d8[cc][c >> 1], i2f_small(cj[2 * r + cc]), acc[2 * r + cc]);
-                        }
-                    }
-                }
-#pragma unroll
-            for (int r = 0; r < 2; r++)
-#pragma unroll
-                for (int cc = 0; cc < 2; cc++) total[n][2 * r + cc] += dw[r] * acc[2 * r + cc];
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int n = 0; n < NBW; n++) {
-        const int tok0 = (tpart * NBW + n) * 8;
-        if (tok0 >= mt) continue;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int row = row0 + rg * 16 + gq + 8 * r;
-            if (kparts > 1) {
-#pragma unroll
-                for (int cc = 0; cc < 2; cc++) {
-                    const int t = tok0 + 2 * tq + cc;
-                    if (row < A.N && t < mt) partial[((size_t)kp * M + t) * A.N + row] = total[n][2 * r + cc];
-                }
-            } else {
-                const float mine0 = total[n][2 * r], mine1 = total[n][2 * r + 1];
-                const float other0 = __shfl_xor_sync(TFR_FULL_MASK, mine0, 4), other1 = __shfl_xor_sync(TFR_FULL_MASK, mine1, 4);
-                const bool odd = gq & 1;
-                const int t = tok0 + 2 * tq + (odd ? 1 : 0), row_even = row & ~1;
-                const float x0 = odd ? other1 : mine0, x1 = odd ? mine1 : other0;
-                if (row_even < A.N && t < mt) ChunkEpiTok{&epi, t}.apply(id_base + (row_even >> 1), x0, x1);
-            }
-        }
-    }
-}
-
-// Adds the k parts of k_gemm_mma_q6 in their order and runs the pair-ordered epilogue: one thread per (token, row pair).
-__global__ void k_gemm_splitk_finish(const float* partial, int kparts, int M, int N, int id_base, ChunkEpi epi) {
-    griddep_wait();
-    griddep_launch_dependents();
-    const int pairs = (N + 1) >> 1;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * pairs) return;
-    const int t = i / pairs, p = i - t * pairs;
-    float x0 = 0.f, x1 = 0.f;
-    for (int k = 0; k < kparts; k++) {
-        const float* src = partial + ((size_t)k * M + t) * N + 2 * p;
-        x0 += src[0];
-        if (2 * p + 1 < N) x1 += src[1];
-    }
-    ChunkEpiTok{&epi, t}.apply(id_base + p, x0, x1);
-}
-
-// ws: scratch for the k parts (ws_floats floats; nullptr: no split).
-inline cudaError_t launch_gemm_mma_q6(cudaStream_t stream, int sms, const unsigned char* act_g, size_t act_stride, int M, const RowJob& ja,
-                                      const ChunkEpi& epi, float* ws, size_t ws_floats) {
-    const int rows = ja.m.N, tiles = (rows + 63) / 64;
-    int kparts = 1;
-    if (ws && tiles < sms) {
-        kparts = std::min(std::min(4, ja.m.nb), std::max(1, sms / tiles));
-        if ((size_t)kparts * M * rows > ws_floats) kparts = 1;
-    }
-    cudaError_t r = M <= 16 ? launch_pdl(k_gemm_mma_q6<16>, dim3(tiles, kparts), dim3(GM_THREADS), gemm_mma_q6_smem(16), stream, act_g, act_stride,
-                                         ja.m, ja.id_base, epi, M, ws)
-                            : launch_pdl(k_gemm_mma_q6<64>, dim3(tiles, kparts), dim3(GM_THREADS), gemm_mma_q6_smem(64), stream, act_g, act_stride,
-                                         ja.m, ja.id_base, epi, M, ws);
-    if (r != cudaSuccess || kparts == 1) return r;
-    const int items = M * ((rows + 1) / 2);
-    return launch_pdl(k_gemm_splitk_finish, dim3((items + 255) / 256), dim3(256), (size_t)0, stream, (const float*)ws, kparts, M, rows, ja.id_base, epi);
 }
 
 // ------------------------------------------------------------------ causal attention of a chunk

@@ -28,6 +28,7 @@
 #include "../../include/tarafer_b200.h"
 #include "tfr_kernels.cuh"
 #include "tfr_chunk.cuh"
+#include "tfr_gemm_tc.cuh"
 #include "tfr_loop.cuh"
 
 using namespace tfr;
@@ -190,7 +191,10 @@ struct tfr_engine {
     std::string chunk_why;
     float *cx = nullptr, *cq = nullptr, *cattn = nullptr, *ch = nullptr, *cxn = nullptr, *clogits = nullptr, *cpart = nullptr;
     size_t cpart_floats = 0;
+    int chunk_cap = 0;  // tokens the chunk buffers have room for
     unsigned char* cact = nullptr;
+    unsigned char* cimage = nullptr;  // operand image of the tensor-core projections (tfr_gemm_tc.cuh), its token scales
+    float* ctscale = nullptr;
     size_t cact_stride = 0;
     unsigned long long* ckeys = nullptr;  // per-row, per-slice argmax keys of a verification pass
     unsigned int* ccount = nullptr;       // per-row arrival counters, zero between launches
@@ -293,23 +297,20 @@ static void configure_kernels_once() {
     configure_kernel(k_gemm_q8<BlockQ4>, true);
     configure_kernel(k_gemm_q8<BlockQ6>, true);
     configure_kernel(k_gemm_q8<BlockQ8>, true);
-    configure_kernel(k_gemm_mma_q6<64>, true);
-    configure_kernel(k_gemm_mma_q6<16>, true);
-    configure_kernel(k_gemm_splitk_finish, false);
-    configure_kernel(k_gemm_mma_q4<4, true, 64>, true);
-    configure_kernel(k_gemm_mma_q4<1, true, 64>, true);
-    configure_kernel(k_gemm_mma_q4<4, false, 64>, true);
-    configure_kernel(k_gemm_mma_q4<1, false, 64>, true);
-    configure_kernel(k_gemm_mma_q4<4, true, 16>, true);
-    configure_kernel(k_gemm_mma_q4<2, true, 64>, true);
-    configure_kernel(k_gemm_mma_q4<2, false, 64>, true);
-    configure_kernel(k_gemm_mma_q4<4, false, 16>, true);
     configure_kernel(k_attn_chunk<64>, true);
     configure_kernel(k_attn_chunk<128>, true);
     configure_kernel(k_attn_chunk<256>, true);
     configure_kernel(k_attn_chunk_mma<64>, true);
     configure_kernel(k_attn_chunk_mma<128>, true);
     configure_kernel(k_prep_rows, false);
+    configure_kernel(k_prep_tc, true);
+    configure_kernel(k_rows_f32, true);
+    configure_kernel(k_gemm_tc<RawQ4, true, 64, 1>, true);
+    configure_kernel(k_gemm_tc<RawQ6, true, 128, 1>, true);
+    configure_kernel(k_gemm_tc<RawQ4, false, 32, 1>, true);
+    configure_kernel(k_gemm_tc<RawQ4, false, 8, 4>, true);
+    configure_kernel(k_gemm_tc<RawQ6, false, 32, 1>, true);
+    configure_kernel(k_gemm_tc<RawQ6, false, 8, 2>, true);
     configure_kernel(k_attn_chunk_merge, false);
     // the attention kernel also has static shared memory: ask for exactly the dynamic part it uses
     configure_kernel(k_attn_decode<64>, false);
@@ -553,8 +554,6 @@ static int mat_create_impl(tfr_engine* e, int type, int64_t K, int64_t N, const 
     if (r == cudaSuccess) r = cudaMemcpyAsync(staging, bytes, nbytes, cudaMemcpyDefault, stream);
     if (r == cudaSuccess) {
         const int grid = sm_count_cached() * 8;
-        const size_t last_tile = (size_t)tile_bytes(type);  // zero the tail tile's unused lanes
-        cudaMemsetAsync((uint8_t*)m->dev + m->bytes - last_tile, 0, last_tile, stream);
         k_repack_tiled<<<grid, 256, 0, stream>>>((const uint8_t*)staging, (uint8_t*)m->dev, type, (int)N, m->m.nb, perm_hd);
         r = cudaGetLastError();
     }
@@ -626,7 +625,7 @@ extern "C" void tfr_destroy(tfr_engine* e) {
     for (auto& kv : e->vecs) cudaFree(kv.second.dev);
     for (auto& L : e->layers) cudaFree(L.bias_qkv);
     void* ws[] = {e->x, e->q, e->attn, e->h, e->logits, e->partial, e->counters, e->st, e->prompt,
-                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
+                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->ctscale, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
     for (void* p : ws) cudaFree(p);
     if (e->st_host) cudaFreeHost(e->st_host);
     cudaEventDestroy(e->ev0);
@@ -932,19 +931,19 @@ static int loop_setup(tfr_engine* e) {
         used[1 + (L.wo->m.type == TFR_Q6_K)] = true;
         used[4 + (L.down->m.type == TFR_Q6_K)] = true;
     }
-    ph[0].job[0] = loop_job(TFR_Q4_K, P.nq, 2, 0, 0, G);
-    ph[0].job[1] = loop_job(TFR_Q4_K, P.nkv, 2, P.nq / 2, 0, G);
-    ph[0].job[2] = loop_job(TFR_Q6_K, P.nkv, 2, (P.nq + P.nkv) / 2, 1, G);
+    ph[0].job[0] = loop_job(TFR_Q4_K, P.nq, 0, 0, G);
+    ph[0].job[1] = loop_job(TFR_Q4_K, P.nkv, P.nq / 2, 0, G);
+    ph[0].job[2] = loop_job(TFR_Q6_K, P.nkv, (P.nq + P.nkv) / 2, 1, G);
     for (int t = 0; t < 2; t++) {
         const int type = t ? TFR_Q6_K : TFR_Q4_K;
-        ph[1 + t].job[0] = loop_job(type, K, 2, 0, 0, G);
-        ph[4 + t].job[0] = loop_job(type, K, 2, 0, 0, G);
+        ph[1 + t].job[0] = loop_job(type, K, 0, 0, G);
+        ph[4 + t].job[0] = loop_job(type, K, 0, 0, G);
     }
-    ph[3].job[0] = loop_job(TFR_Q4_K, P.ff, 1, 0, 0, G);
-    ph[3].job[1] = loop_job(TFR_Q4_K, P.ff, 1, 0, 0, G);
+    ph[3].job[0] = loop_job(TFR_Q4_K, P.ff, 0, 0, G);
+    ph[3].job[1] = loop_job(TFR_Q4_K, P.ff, 0, 0, G);
     ph[3].zip = 1;
     const int V = e->head->m.N;
-    ph[6].job[0] = loop_job(e->head->m.type, V, 2, 0, 0, G);
+    ph[6].job[0] = loop_job(e->head->m.type, V, 0, 0, G);
     const int sec_k[SCHED_SECTIONS] = {K, P.attn_width, P.attn_width, K, P.ff, P.ff, K};
     const int sec_lpb[SCHED_SECTIONS] = {lpb[0], lpb[1], lpb[1], lpb[2], lpb[3], lpb[3], lpb[4]};
     bool fits = true;
@@ -967,9 +966,9 @@ static int loop_setup(tfr_engine* e) {
     if (work < attn_need) work = attn_need;
     a.off_blob = LOOP_CTX_OFFSET + 256;  // barriers, control words, reduction scratch, then the context struct
     a.off_layers = (int)((a.off_blob + (size_t)plan.blob_stride * 4 + 15) & ~(size_t)15);
-    a.sh_x = make_share((K + 1) / 2, G);
+    a.sh_x = make_share(group_rows(K) / ROW_GROUP, G);
     a.off_own = (int)((a.off_layers + (size_t)c.n_layer * sizeof(LoopLayer) + 15) & ~(size_t)15);
-    a.off_act = (int)((a.off_own + (size_t)4 * 2 * (a.sh_x.quot + 1) + 127) & ~(size_t)127);
+    a.off_act = (int)((a.off_own + (size_t)4 * ROW_GROUP * (a.sh_x.quot + 1) + 127) & ~(size_t)127);
     a.off_xf = a.off_act + (int)act_b;
     a.off_pbuf = a.off_xf + (int)xf_b;
     a.off_ring = (int)((a.off_act + work + 127) & ~(size_t)127);
@@ -1077,6 +1076,17 @@ static int run_loop(tfr_engine* e, const tfr_kv* kv, int n_headless) {
 
 static void chunk_setup(tfr_engine* e);
 
+// Gives `out` (type, K, N set) a copy of rows row0 .. row0 + N - 1 of `from`.
+static int slice_rows(tfr_engine* e, const tfr_mat* from, int row0, tfr_mat* out) {
+    const Mat& m = out->m;
+    out->bytes = (size_t)mat_device_bytes(m.type, m.K, m.N);
+    CU(e, cudaMalloc(&out->dev, out->bytes));
+    k_slice_rows<<<sm_count_cached() * 4, 256, 0, e->stream>>>(from->m.data, (uint8_t*)out->dev, m.type, row0, m.N, m.nb);
+    CU(e, cudaGetLastError());
+    out->m.data = (const uint8_t*)out->dev;
+    return TFR_OK;
+}
+
 extern "C" int tfr_finalize_load(tfr_engine* e) {
     if (!e || !e->has_cfg) return TFR_E_INVALID;
     if (e->finalized) return TFR_OK;
@@ -1093,14 +1103,17 @@ extern "C" int tfr_finalize_load(tfr_engine* e) {
     } else if (P.tp == 1) {
         e->head = e->token_embd;
     } else {
-        // tied head: this rank's vocabulary rows are a run of whole tiles of the embedding matrix
+        // tied head: this rank's vocabulary rows of the embedding matrix, where they start on a tile as a view of it
         const long long f0 = (long long)P.v0 * (K / 256);
-        if (f0 % 32) return fail(e, TFR_E_UNSUPPORTED, "tied vocabulary head: slice of rank %d does not start on a tile", P.rank);
         tfr_mat* view = new tfr_mat();
         view->m = e->token_embd->m;
         view->m.N = Vl;
-        view->m.data = e->token_embd->m.data + (f0 / 32) * tile_bytes(view->m.type);
         e->mats["output.weight(view)"] = view;
+        if (P.v0 % ROW_GROUP == 0 && f0 % 32 == 0) {
+            view->m.data = e->token_embd->m.data + (f0 / 32) * tile_bytes(view->m.type);
+        } else if (int r = slice_rows(e, e->token_embd, P.v0, view)) {
+            return r;
+        }
         e->head = view;
     }
     if (e->vocab_limit) {
@@ -1118,14 +1131,8 @@ extern "C" int tfr_finalize_load(tfr_engine* e) {
             tfr_mat* one = new tfr_mat();
             one->m = full->m;
             one->m.N = 1;
-            one->bytes = (size_t)tile_bytes(full->m.type);
-            CU(e, cudaMalloc(&one->dev, one->bytes));
-            CU(e, cudaMemsetAsync(one->dev, 0, one->bytes, e->stream));
-            const int work = full->m.nb * 18;
-            k_extract_row<<<(work + 127) / 128, 128, 0, e->stream>>>(full->m.data, (uint8_t*)one->dev, full->m.type, e->special_id, full->m.nb);
-            CU(e, cudaGetLastError());
-            one->m.data = (const uint8_t*)one->dev;
             e->mats["output(shortlist extra row)"] = one;
+            if (int r = slice_rows(e, full, e->special_id, one)) return r;
             e->head_special = one;
         }
     }
@@ -1331,6 +1338,43 @@ static cudaError_t launch_typed(cudaStream_t s, int grid, int type, const PrepAr
     return launch_gemv<BlockQ6, Epi>(s, grid, pa, ja, jb, fseg, epi, K, st);
 }
 
+// Final norm + vocabulary head + argmax + state advance over the residual stream x; returns the launches or -1.
+static int record_head(tfr_engine* e, const float* x, int prof_id) {
+    const tfr_model_config& c = e->cfg;
+    const TpPlan& P = e->plan;
+    const int K = c.n_embd, V = P.v1 - P.v0, cap = e->prop.multiProcessorCount;
+    cudaStream_t s = e->stream;
+    PrepArgs pa{};
+    pa.vec = x;
+    pa.normw = e->output_norm;
+    pa.eps = c.rms_eps;
+    pa.prof_id = prof_id;
+    EpiLogits epi{};
+    epi.logits = e->logits;
+    epi.out_tokens = e->out_tokens;
+    epi.prompt = e->prompt;
+    epi.n_rows = e->vocab_limit ? e->vocab_limit + (e->head_special ? 1 : 0) : V;
+    epi.special_row = e->vocab_limit;
+    epi.special_id = e->head_special ? e->special_id : -1;
+    epi.row_offset = P.v0;
+    epi.use_tp = P.tp > 1 && !e->use_nccl;
+    epi.c = e->comm;
+    epi.defer_best = P.tp > 1 && e->use_nccl ? e->best_buf : nullptr;
+    const RowJob extra = e->head_special ? make_job(e->head_special->m, cap, e->vocab_limit / 2) : RowJob{};
+    if (launch_typed(s, cap, e->head->m.type, pa, make_job(e->head->m, cap), extra, F32Seg{}, epi, K, e->st) !=
+        cudaSuccess)
+        return -1;
+    if (epi.defer_best) {
+        if (nccl_api()->AllReduce(e->best_buf, e->best_buf, 1, NCCL_UINT64, NCCL_MAX, e->nccl_comm, s) != 0) return -1;
+        if (launch_pdl(k_state_advance, dim3(1), dim3(1), 0, s, e->st, (const unsigned long long*)e->best_buf, e->out_tokens,
+                       (const int*)e->prompt) !=
+            cudaSuccess)
+            return -1;
+        return 3;
+    }
+    return 1;
+}
+
 // Enqueues the kernels of one decode step; returns the number of launches or a negative error.
 static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
     const tfr_model_config& c = e->cfg;
@@ -1344,7 +1388,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
         PrepArgs pa{};
         pa.vec = vec;
         pa.prof_id = n;
-        const RowJob job = make_job(w->m, 2, cap);
+        const RowJob job = make_job(w->m, cap);
         if (P.tp == 1) {
             EpiStore epi{e->x, nullptr, 2, K};
             return launch_typed(s, cap, w->m.type, pa, job, RowJob{}, F32Seg{}, epi, width, e->st);
@@ -1396,7 +1440,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             // 1. norm + quant + [qkv | z | beta | alpha] projections (layer.rs:736-798)
             if (L.gdn_proj) {
                 EpiStore ep{e->proj, nullptr, 0, L.gdn_proj->m.N};
-                if (launch_typed(s, cap, L.gdn_proj->m.type, pn, make_job(L.gdn_proj->m, 2, cap), RowJob{}, F32Seg{}, ep, K, e->st) !=
+                if (launch_typed(s, cap, L.gdn_proj->m.type, pn, make_job(L.gdn_proj->m, cap), RowJob{}, F32Seg{}, ep, K, e->st) !=
                     cudaSuccess)
                     return -1;
                 n++;
@@ -1413,7 +1457,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
                     }
                     pk.prof_id = n;
                     EpiStore ep{e->proj + off, nullptr, 0, w->m.N};
-                    if (launch_typed(s, cap, w->m.type, pk, make_job(w->m, 2, cap), RowJob{}, F32Seg{}, ep, K, e->st) != cudaSuccess)
+                    if (launch_typed(s, cap, w->m.type, pk, make_job(w->m, cap), RowJob{}, F32Seg{}, ep, K, e->st) != cudaSuccess)
                         return -1;
                     off += w->m.N;
                     n++;
@@ -1439,7 +1483,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             wout = L.ssm_out;
         } else if (L.kind == LAYER_FULL_GATED) {
             // 1. norm + quant + raw [Q|gate, K, V] (+bias)
-            const RowJob jq = make_job(L.wq->m, 2, cap, 0), jk = make_job(L.wk->m, 2, cap, nq);
+            const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, nq);
             F32Seg fseg{};
             fseg.m = L.wv->m;
             fseg.sh = make_share(nkv / 2, cap);
@@ -1471,7 +1515,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             n++;
         } else {
             // 1. norm + quant + QKV + rope + KV store
-            const RowJob jq = make_job(L.wq->m, 2, cap, 0), jk = make_job(L.wk->m, 2, cap, nq / 2);
+            const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, nq / 2);
             F32Seg fseg{};
             fseg.m = L.wv->m;
             fseg.sh = make_share(nkv / 2, cap);
@@ -1509,7 +1553,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             pa.eps = c.rms_eps;
             pa.prof_id = n;
             EpiSilu epi{e->h};
-            if (launch_gemv<BlockQ4, EpiSilu>(s, cap, pa, make_job(L.gate->m, 1, cap), make_job(L.up->m, 1, cap), F32Seg{}, epi,
+            if (launch_gemv<BlockQ4, EpiSilu>(s, cap, pa, make_job(L.gate->m, cap), make_job(L.up->m, cap), F32Seg{}, epi,
                                               K, e->st) != cudaSuccess)
                 return -1;
             n++;
@@ -1523,35 +1567,9 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             return -1;
     }
     if (with_head) {
-        PrepArgs pa{};
-        pa.vec = e->x;
-        pa.normw = e->output_norm;
-        pa.eps = c.rms_eps;
-        pa.prof_id = n;
-        EpiLogits epi{};
-        epi.logits = e->logits;
-        epi.out_tokens = e->out_tokens;
-        epi.prompt = e->prompt;
-        epi.n_rows = e->vocab_limit ? e->vocab_limit + (e->head_special ? 1 : 0) : V;
-        epi.special_row = e->vocab_limit;
-        epi.special_id = e->head_special ? e->special_id : -1;
-        epi.row_offset = P.v0;
-        epi.use_tp = P.tp > 1 && !e->use_nccl;
-        epi.c = e->comm;
-        epi.defer_best = P.tp > 1 && e->use_nccl ? e->best_buf : nullptr;
-        const RowJob extra = e->head_special ? make_job(e->head_special->m, 2, cap, e->vocab_limit / 2) : RowJob{};
-        if (launch_typed(s, cap, e->head->m.type, pa, make_job(e->head->m, 2, cap), extra, F32Seg{}, epi, K, e->st) !=
-            cudaSuccess)
-            return -1;
-        n++;
-        if (epi.defer_best) {
-            if (nccl_api()->AllReduce(e->best_buf, e->best_buf, 1, NCCL_UINT64, NCCL_MAX, e->nccl_comm, s) != 0) return -1;
-            if (launch_pdl(k_state_advance, dim3(1), dim3(1), 0, s, e->st, (const unsigned long long*)e->best_buf, e->out_tokens,
-                           (const int*)e->prompt) !=
-                cudaSuccess)
-                return -1;
-            n += 2;
-        }
+        const int nh = record_head(e, e->x, n);
+        if (nh < 0) return -1;
+        n += nh;
     } else {
         if (launch_pdl(k_state_next_prompt, dim3(1), dim3(1), 0, s, e->st, (const int*)e->prompt,
                        P.tp > 1 ? e->comm.ops_per_token : 0) != cudaSuccess)
@@ -1643,38 +1661,51 @@ static void chunk_setup(tfr_engine* e) {
     e->chunk_why.clear();
 }
 
-static int chunk_buffers(tfr_engine* e) {
-    if (e->cx) return TFR_OK;
+// Buffers for chunks of M tokens: grown to the next of a few sizes, kept.
+static int chunk_buffers(tfr_engine* e, int M) {
+    if (M <= e->chunk_cap) return TFR_OK;
+    int cap = 64;
+    while (cap < M) cap *= 4;
+    cap = std::min(cap, std::max(CHUNK_MAX_TOKENS, CHUNK_VERIFY_MAX));
     const TpPlan& P = e->plan;
-    const int K = e->cfg.n_embd, M = CHUNK_MAX_TOKENS;
+    const int K = e->cfg.n_embd, hd = e->cfg.head_dim;
     const int kmax = std::max(std::max(K, P.ff), P.attn_width);
+    CU(e, cudaStreamSynchronize(e->stream));
+    void** grown[] = {(void**)&e->cx, (void**)&e->cxn, (void**)&e->cq, (void**)&e->cattn, (void**)&e->ch, (void**)&e->cact, (void**)&e->cpart,
+                      (void**)&e->cimage, (void**)&e->ctscale};
+    e->chunk_cap = 0;
+    for (void** p : grown) {
+        cudaFree(*p);
+        *p = nullptr;
+    }
     e->cact_stride = (act_smem_bytes(kmax, false, false) + 255) & ~(size_t)255;
-    CU(e, cudaMalloc(&e->cx, (size_t)M * K * 4));
-    CU(e, cudaMalloc(&e->cxn, (size_t)M * K * 4));
-    CU(e, cudaMalloc(&e->cq, (size_t)M * P.nq * 4));
-    CU(e, cudaMalloc(&e->cattn, (size_t)M * P.attn_width * 4));
-    CU(e, cudaMalloc(&e->ch, (size_t)M * P.ff * 4));
-    CU(e, cudaMalloc(&e->cact, (size_t)M * e->cact_stride));
-    CU(e, cudaMalloc(&e->clogits, (size_t)CHUNK_VERIFY_MAX * e->head->m.N * 4));
-    CU(e, cudaMalloc(&e->ckeys, (size_t)CHUNK_VERIFY_MAX * ARGMAX_SLICES * 8));
-    CU(e, cudaMalloc(&e->ccount, CHUNK_VERIFY_MAX * 4));
-    CU(e, cudaMemset(e->ccount, 0, CHUNK_VERIFY_MAX * 4));
-    e->cpart_floats = (size_t)M * P.n_head * CHUNK_ATTN_SPLITS_MAX * (2 + e->cfg.head_dim);
+    CU(e, cudaMalloc(&e->cx, (size_t)cap * K * 4));
+    CU(e, cudaMalloc(&e->cxn, (size_t)cap * K * 4));
+    CU(e, cudaMalloc(&e->cq, (size_t)cap * P.nq * 4));
+    CU(e, cudaMalloc(&e->cattn, (size_t)cap * P.attn_width * 4));
+    CU(e, cudaMalloc(&e->ch, (size_t)cap * P.ff * 4));
+    CU(e, cudaMalloc(&e->cact, (size_t)cap * e->cact_stride));
+    CU(e, cudaMalloc(&e->cimage, tc_image_bytes(kmax, cap)));
+    CU(e, cudaMalloc(&e->ctscale, (size_t)tc_pad_tokens(cap) * 4));
+    // attention partials: the key splits of few query tiles, or two per token of a full chunk
+    e->cpart_floats = (size_t)P.n_head * (2 + hd) * std::max(64 * CHUNK_ATTN_SPLITS_MAX, 2 * cap);
     CU(e, cudaMalloc(&e->cpart, e->cpart_floats * 4));
+    if (!e->clogits) {
+        CU(e, cudaMalloc(&e->clogits, (size_t)CHUNK_VERIFY_MAX * e->head->m.N * 4));
+        CU(e, cudaMalloc(&e->ckeys, (size_t)CHUNK_VERIFY_MAX * ARGMAX_SLICES * 8));
+        CU(e, cudaMalloc(&e->ccount, CHUNK_VERIFY_MAX * 4));
+        CU(e, cudaMemset(e->ccount, 0, CHUNK_VERIFY_MAX * 4));
+    }
+    e->chunk_cap = cap;
     return TFR_OK;
 }
 
-// ws / ws_floats: scratch a launch may use for partial sums (the attention partials' buffer: free between the attention
-// of a layer and the next one's).
+// Batches from five tokens on: projections of Q4_K and Q6_K matrices on the tensor cores.  Fewer tokens leave those idle
+// and keep the dp4a kernel, as Q8_0 matrices do; TFR_GEMM_DP4A=1 in the environment keeps everything there (a test aid).
+static bool gemm_on_tc(int type, int M) { return M >= GEMM_TC_MIN_TOKENS && tc_type(type) && !getenv("TFR_GEMM_DP4A"); }
+
 static cudaError_t launch_gemm_typed(cudaStream_t s, int grid, int type, const unsigned char* act, size_t stride, const float* xn, int M,
-                                     const RowJob& ja, const RowJob& jb, const F32Seg& fseg, const ChunkEpi& epi, int K, TokenState* st,
-                                     float* ws = nullptr, size_t ws_floats = 0) {
-    // Q4_K projections of prompt chunks run their sub-block dots on the tensor cores (one matrix with a pair-ordered
-    // epilogue, or the gate / up pair); TFR_GEMM_DP4A=1 in the environment keeps them on the dp4a kernel (a test aid)
-    if (type == TFR_Q4_K && M >= GEMM_MMA_MIN_TOKENS && !fseg.m.data && (!jb.m.data || epi.kind == CEPI_SILU) && !getenv("TFR_GEMM_DP4A"))
-        return launch_gemm_mma_q4(s, grid, act, stride, M, ja, jb, epi);
-    if (type == TFR_Q6_K && M >= GEMM_MMA_MIN_TOKENS && !fseg.m.data && !jb.m.data && epi.kind != CEPI_SILU && !getenv("TFR_GEMM_DP4A"))
-        return launch_gemm_mma_q6(s, grid, act, stride, M, ja, epi, ws, ws_floats);
+                                     const RowJob& ja, const RowJob& jb, const F32Seg& fseg, const ChunkEpi& epi, int K, TokenState* st) {
     if (type == TFR_Q4_K) return launch_gemm<BlockQ4>(s, grid, act, stride, xn, M, ja, jb, fseg, epi, K, st);
     if (type == TFR_Q8_0) return launch_gemm<BlockQ8>(s, grid, act, stride, xn, M, ja, jb, fseg, epi, K, st);
     return launch_gemm<BlockQ6>(s, grid, act, stride, xn, M, ja, jb, fseg, epi, K, st);
@@ -1690,11 +1721,25 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     const int cap = e->prop.multiProcessorCount;
     cudaStream_t s = e->stream;
     int n = 0;
-    auto prep = [&](const float* x, int ldx, int width, const float* normw, float* xn) -> cudaError_t {
+    // x -> RMSNorm (optional) -> Q8, in the form the projections that follow read
+    auto prep = [&](bool tc, const float* x, int ldx, int width, const float* normw, float* xn) -> cudaError_t {
+        n++;
+        if (tc) {
+            PrepTcArgs a{x, ldx, width, M, normw, c.rms_eps, e->cimage, e->ctscale, xn};
+            return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(TC_PREP_THREADS), tc_prep_smem(width), s, a);
+        }
         PrepRowsArgs a{x, ldx, width, normw, c.rms_eps, e->cact, e->cact_stride, xn};
         const size_t smem = normw ? (xs_floats(width) + 272) * sizeof(float) : 0;
-        n++;
         return launch_pdl(k_prep_rows, dim3(M), dim3(GEMV_THREADS), smem, s, a);
+    };
+    // RMSNorm + Q8 + W x + epilogue
+    auto project = [&](const float* x, int width, const float* normw, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep) -> cudaError_t {
+        const bool tc = gemm_on_tc(ja.m.type, M);
+        cudaError_t r = prep(tc, x, width, width, normw, nullptr);
+        if (r != cudaSuccess) return r;
+        n++;
+        if (tc) return launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, ja, jb, ep, e->st);
+        return launch_gemm_typed(s, cap, ja.m.type, e->cact, e->cact_stride, nullptr, M, ja, jb, F32Seg{}, ep, width, e->st);
     };
     auto store_epi = [&](float* out, int ldo, int rows, int use_res) {
         ChunkEpi ep{};
@@ -1708,9 +1753,10 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     for (int li = 0; li < c.n_layer; li++) {
         const LayerW& L = e->layers[li];
         // 1. RMSNorm + Q8, Q/K/V (+bias) + RoPE + f16 KV rows
-        if (prep(e->cx, K, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
+        const bool tc_qk = gemm_on_tc(TFR_Q4_K, M);
+        if (prep(tc_qk, e->cx, K, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
         {
-            const RowJob jq = make_job(L.wq->m, 2, cap, 0), jk = make_job(L.wk->m, 2, cap, nq / 2);
+            const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, nq / 2);
             F32Seg fseg{};
             fseg.m = L.wv->m;
             fseg.sh = make_share(nkv / 2, cap);
@@ -1720,12 +1766,11 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             ep.out = e->cq, ep.ldo = nq, ep.bias = L.bias_qkv;
             ep.kc = kv_k(kv, li), ep.vc = kv_v(kv, li);
             ep.nq = nq, ep.nk = nkv, ep.hd = hd, ep.kvdim = nkv, ep.pos0 = pos0, ep.theta = c.rope_theta;
-            if (M >= GEMM_MMA_MIN_TOKENS && !getenv("TFR_GEMM_DP4A")) {
-                // batches from five tokens on: the Q and K rows on the tensor cores (same integer sub-block sums, row sums
-                // along k); the fp32-route V rows keep the decode kernels' arithmetic bit for bit
-                if (launch_gemm_mma_q4(s, cap, e->cact, e->cact_stride, M, jq, jk, ep) != cudaSuccess) return -1;
+            if (tc_qk) {
+                // the fp32-route V rows keep the decode kernels' arithmetic bit for bit
+                if (launch_rows_f32(s, fseg.m, fseg.id_base, e->cxn, M, ep) != cudaSuccess) return -1;
                 n++;
-                if (launch_gemm<BlockQ4>(s, cap, e->cact, e->cact_stride, e->cxn, M, RowJob{}, RowJob{}, fseg, ep, K, e->st) != cudaSuccess) return -1;
+                if (launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, jq, jk, ep, e->st) != cudaSuccess) return -1;
             } else if (launch_gemm<BlockQ4>(s, cap, e->cact, e->cact_stride, e->cxn, M, jq, jk, fseg, ep, K, e->st) != cudaSuccess) {
                 return -1;
             }
@@ -1741,12 +1786,13 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             // few tokens (verification batches): one query token per CTA, so that a row's serial walk over the keys is
             // a warp's only work; prompts: four tokens share every K/V tile
             // batches from five tokens on with head sizes up to 128 run on the tensor cores: 128 (token, head) rows per CTA
-            const bool mma = M >= GEMM_MMA_MIN_TOKENS && attn_staged_mma(hd) && !getenv("TFR_ATTN_REGISTER_ROUTE");
+            const bool mma = M >= GEMM_TC_MIN_TOKENS && attn_staged_mma(hd) && !getenv("TFR_ATTN_REGISTER_ROUTE");
             a.QT = mma ? std::max(1, ATTM_ROWS / rep) : M <= CHUNK_VERIFY_MAX ? 1 : std::max(1, ATTC_ROWS_MAX / rep);
             const int q_tiles = (M + a.QT - 1) / a.QT;
             // key splits: enough CTAs for every SM, never less than 256 keys per split
             const int blocks256 = (pos0 + M + 255) / 256;
             a.S = std::max(1, std::min(std::min(CHUNK_ATTN_SPLITS_MAX, blocks256), (2 * cap + P.n_kv * q_tiles - 1) / (P.n_kv * q_tiles)));
+            a.S = std::max(1, std::min(a.S, (int)(e->cpart_floats / ((size_t)M * P.n_head * (2 + hd)))));
             a.partial = e->cpart;
             const dim3 grid(P.n_kv, q_tiles, a.S);
             const size_t smem = mma ? attn_chunk_mma_smem(hd) : attn_chunk_smem(hd);
@@ -1765,34 +1811,17 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             }
         }
         // 3. Q8 + o-proj + residual
-        if (prep(e->cattn, P.attn_width, P.attn_width, nullptr, nullptr) != cudaSuccess) return -1;
-        if (launch_gemm_typed(s, cap, L.wo->m.type, e->cact, e->cact_stride, nullptr, M, make_job(L.wo->m, 2, cap), RowJob{}, F32Seg{},
-                              store_epi(e->cx, K, K, 2), P.attn_width, e->st) != cudaSuccess)
-            return -1;
-        n++;
+        if (project(e->cattn, P.attn_width, nullptr, make_job(L.wo->m, cap), RowJob{}, store_epi(e->cx, K, K, 2)) != cudaSuccess) return -1;
         // 4. RMSNorm + Q8 + gate/up + SiLU*mul
-        if (prep(e->cx, K, K, L.ffn_norm, nullptr) != cudaSuccess) return -1;
-        {
-            ChunkEpi ep{};
-            ep.kind = CEPI_SILU;
-            ep.out = e->ch, ep.ldo = FF;
-            if (launch_gemm_typed(s, cap, L.gate->m.type, e->cact, e->cact_stride, nullptr, M, make_job(L.gate->m, 1, cap), make_job(L.up->m, 1, cap),
-                                  F32Seg{}, ep, K, e->st) != cudaSuccess)
-                return -1;
-            n++;
-        }
+        ChunkEpi ep{};
+        ep.kind = CEPI_SILU;
+        ep.out = e->ch, ep.ldo = FF;
+        if (project(e->cx, K, L.ffn_norm, make_job(L.gate->m, cap), make_job(L.up->m, cap), ep) != cudaSuccess) return -1;
         // 5. Q8 + down + residual
-        if (prep(e->ch, FF, FF, nullptr, nullptr) != cudaSuccess) return -1;
-        if (launch_gemm_typed(s, cap, L.down->m.type, e->cact, e->cact_stride, nullptr, M, make_job(L.down->m, 2, cap), RowJob{}, F32Seg{},
-                              store_epi(e->cx, K, K, 2), FF, e->st, e->cpart, e->cpart_floats) != cudaSuccess)
-            return -1;
-        n++;
+        if (project(e->ch, FF, nullptr, make_job(L.down->m, cap), RowJob{}, store_epi(e->cx, K, K, 2)) != cudaSuccess) return -1;
     }
     if (all_rows) {
-        if (prep(e->cx, K, K, e->output_norm, nullptr) != cudaSuccess) return -1;
-        if (launch_gemm_typed(s, cap, e->head->m.type, e->cact, e->cact_stride, nullptr, M, make_job(e->head->m, 2, cap), RowJob{},
-                              F32Seg{}, store_epi(e->clogits, V, V, 0), K, e->st) != cudaSuccess)
-            return -1;
+        if (project(e->cx, K, e->output_norm, make_job(e->head->m, cap), RowJob{}, store_epi(e->clogits, V, V, 0)) != cudaSuccess) return -1;
         k_argmax_rows<<<dim3(M, ARGMAX_SLICES), 256, 0, s>>>(e->clogits, V, e->out_tokens, e->ckeys, e->ccount);
         if (cudaGetLastError() != cudaSuccess) return -1;
         // tfr_current_logits reports the last position's row
@@ -1850,10 +1879,10 @@ extern "C" int tfr_forward_greedy(tfr_engine* e, tfr_kv* kv, const uint32_t* tok
     cudaSetDevice(e->device);
     const bool loop = use_loop(e);
     if (n > 1) CU(e, cudaMemcpyAsync(e->prompt, tokens, (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
-    // all but the last token go through the chunk kernels (weights read once per chunk); the last is a decode step
+    // the prompt goes through the chunk kernels (weights read once per chunk), the head reads the last token's row
     const bool chunked = !loop && e->chunk_ok && e->chunk_tokens > 0 && n > 1;
-    int rc = ready_graphs(e, kv, n > 1 && !chunked);
-    if (!rc && chunked) rc = chunk_buffers(e);
+    int rc = chunked ? TFR_OK : ready_graphs(e, kv, n > 1);
+    if (!rc && chunked) rc = chunk_buffers(e, std::min(n, e->chunk_tokens));
     if (rc) return rc;
     rc = begin_state(e, kv, (int)tokens[chunked ? n - 1 : 0], kv->len + (chunked ? n - 1 : 0), 1, kv->max_seq + 1, nullptr, 0);
     if (rc) return rc;
@@ -1861,12 +1890,12 @@ extern "C" int tfr_forward_greedy(tfr_engine* e, tfr_kv* kv, const uint32_t* tok
     if (loop) {
         rc = run_loop(e, kv, n - 1);
     } else if (chunked) {
-        for (int i = 0; i < n - 1 && !rc; i += e->chunk_tokens) {
-            const int M = std::min(e->chunk_tokens, n - 1 - i);
-            if (forward_chunk(e, kv, e->prompt + i, M, kv->len + i, false) != TFR_OK)
-                rc = fail(e, TFR_E_CUDA, "chunk kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+        for (int i = 0; i < n; i += e->chunk_tokens) {
+            const int M = std::min(e->chunk_tokens, n - i);
+            if (forward_chunk(e, kv, e->prompt + i, M, kv->len + i, false) != TFR_OK || (i + M == n && record_head(e, e->cx + (size_t)(M - 1) * e->cfg.n_embd, 0) < 0))
+                return fail(e, TFR_E_CUDA, "chunk kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         }
-        if (!rc) rc = run_token(e, kv, true);
+        e->launches += 1;
     } else {
         for (int i = 0; i < n && !rc; i++) rc = run_token(e, kv, i == n - 1);
     }
@@ -1897,7 +1926,7 @@ extern "C" int tfr_forward_greedy_all(tfr_engine* e, tfr_kv* kv, const uint32_t*
     int rc = TFR_OK;
     if (chunked) {
         // one weight pass per chunk of up to CHUNK_VERIFY_MAX tokens (the reference: MAX_VERIFY_TOKENS = 9 per pass)
-        rc = chunk_buffers(e);
+        rc = chunk_buffers(e, std::min(n, CHUNK_VERIFY_MAX));
         if (rc) return rc;
         rc = begin_state(e, kv, (int)tokens[0], kv->len, n, kv->max_seq + 1, nullptr, 0, 1);  // resets the error word
         if (rc) return rc;
@@ -2256,7 +2285,7 @@ extern "C" int tfr_op_gemv(const tfr_mat* w, const float* x, float* out, const f
     pa.normw = norm_w;
     pa.eps = eps;
     const int C = sm_count_cached();
-    RowJob ja = make_job(w->m, 2, C);
+    RowJob ja = make_job(w->m, C);
     F32Seg fseg{};
     if (act_mode == 1) {
         ja.sh = make_share(0, C);  // every row goes through the fp32-activation route
@@ -2279,7 +2308,7 @@ extern "C" int tfr_op_ffn_gate_up(const tfr_mat* gate, const tfr_mat* up, const 
     pa.eps = eps;
     const int C = sm_count_cached();
     EpiSilu epi{h};
-    return check(launch_gemv<BlockQ4, EpiSilu>((cudaStream_t)stream, C, pa, make_job(gate->m, 1, C), make_job(up->m, 1, C),
+    return check(launch_gemv<BlockQ4, EpiSilu>((cudaStream_t)stream, C, pa, make_job(gate->m, C), make_job(up->m, C),
                                                F32Seg{}, epi, gate->m.K, nullptr));
 }
 
@@ -2533,7 +2562,7 @@ extern "C" int tfr_op_qkv_rope_store(const tfr_mat* wq, const tfr_mat* wk, const
     pa.normw = norm_w;
     pa.eps = eps;
     const int C = sm_count_cached();
-    const RowJob jq = make_job(wq->m, 2, C, 0), jk = make_job(wk->m, 2, C, nq / 2);
+    const RowJob jq = make_job(wq->m, C, 0), jk = make_job(wk->m, C, nq / 2);
     F32Seg fseg{};
     fseg.m = wv->m;
     fseg.sh = make_share(nkv / 2, C);

@@ -1,11 +1,14 @@
 // Packed-weight x Q8-activation matrix-vector machinery for batch-1 decode.
 //
 // Data layout in HBM ("warp tiles")
-//   A matrix is a flat sequence of K-quant blocks, f = row * (K/256) + block.  At upload the
+//   A matrix is a flat sequence of K-quant blocks in groups of four rows, the rows of a group
+//   interleaved block by block: f = (row / 4) * 4 * (K/256) + 4 * block + row % 4.  At upload the
 //   blocks are regrouped into tiles of 32 consecutive blocks, stored piece-major: the j-th
 //   16-byte piece of all 32 blocks is one contiguous 512-byte slab.  A warp that gives lane l
 //   the block 32*t + l therefore reads every slab with one fully coalesced 512-byte request,
-//   and each lane ends up holding one whole block (Q4_K: 9 pieces = 144 B; Q6_K: 13 pieces +
+//   a warp that gives lane l row l of one and the same block reads runs of 64 bytes (the batched
+//   projections; row after row, the order before, left them 16-byte runs and a miss per lane:
+//   12 000 cycles for the blocks of 256 rows), and each lane ends up holding one whole block (Q4_K: 9 pieces = 144 B; Q6_K: 13 pieces +
 //   the fp16 d = 210 B).  Block CONTENTS are the GGUF bytes, untouched; density is exactly
 //   144 B / 210 B per 256 weights.  (The reference keeps GGUF order and pads Q6_K blocks to
 //   212 B for 4-byte alignment, crates/core/src/cuda/load.rs:145-159.)
@@ -15,8 +18,7 @@
 //   against the block's int8 activations held in shared memory and produces one fp32 partial.
 //   Owning a whole block keeps the instruction count per weight byte low enough for an SM to
 //   keep up with its share of HBM bandwidth — with smaller units the kernel is issue-bound.
-//   K = 2048 puts a row in 8 adjacent lanes: three shuffles finish it.  Other K write the
-//   partials to shared memory and rows are summed in a fixed order after one barrier.
+//   The partials go to shared memory and rows are summed in a fixed order after one barrier.
 //   Results never depend on grid size and are run-to-run deterministic.
 //
 // Integer contract (what must match the reference bit for bit)
@@ -49,7 +51,21 @@ __host__ __device__ inline int tile_bytes(int type) {
     return type == TFR_Q4_K ? Q4_TILE_BYTES : type == TFR_Q8_0 ? Q8_TILE_BYTES : Q6_TILE_BYTES;
 }
 __host__ __device__ inline int block_bytes_256(int type) { return type == TFR_Q4_K ? 144 : type == TFR_Q8_0 ? Q8_SUPER_BYTES : 210; }
-__host__ __device__ inline long long mat_tiles(int K, long long N) { return (N * (K / 256) + 31) / 32; }
+constexpr int ROW_GROUP = 4;  // rows whose blocks are interleaved; CTAs share a matrix out in whole groups
+__host__ __device__ inline int group_rows(int n) { return (n + ROW_GROUP - 1) & ~(ROW_GROUP - 1); }
+// Flat index of block b of a row.
+__host__ __device__ __forceinline__ long long mat_flat(int nb, int row, int b) {
+    return (long long)(row / ROW_GROUP) * (ROW_GROUP * nb) + ROW_GROUP * b + row % ROW_GROUP;
+}
+// Row and block of flat index f, counted from the start of a row group.
+__host__ __device__ __forceinline__ void flat_row_block(int f, int nb, int& row, int& b) {
+    const int g = f / (ROW_GROUP * nb), rem = f - g * (ROW_GROUP * nb);
+    row = g * ROW_GROUP + rem % ROW_GROUP;
+    b = rem / ROW_GROUP;
+}
+__host__ __device__ inline long long mat_tiles(int K, long long N) {
+    return ((N + ROW_GROUP - 1) / ROW_GROUP * ROW_GROUP * (K / 256) + 31) / 32;
+}
 __host__ __device__ inline long long mat_device_bytes(int type, int K, long long N) {
     return mat_tiles(K, N) * tile_bytes(type);
 }
@@ -123,7 +139,7 @@ struct SrcEmbed {
     Mat E;
     int token;
     __device__ __forceinline__ float get(int i) const {
-        const long long f = (long long)token * E.nb + (i >> 8);
+        const long long f = mat_flat(E.nb, token, i >> 8);
         const int e = i & 255;
         if (E.type == TFR_Q4_K) {
             const float d = f16_to_f32(*reinterpret_cast<const unsigned short*>(block_byte(E, f, 0)));

@@ -222,13 +222,18 @@ struct PrepArgs {
     int l2_row_bytes;
 };
 
-// A matrix whose rows are spread over the CTAs in contiguous shares of `rows_per_item` rows.
+// A matrix whose rows are spread over the CTAs in contiguous shares of row groups.
 // data == nullptr: absent.
 struct RowJob {
     Mat m;
     Share sh;
-    int rows_per_item;  // 2: the share counts row pairs; 1: rows
-    int id_base;        // epilogue id of the matrix's first item
+    int id_base;  // epilogue id of the matrix's first item (row pair, or row with EPI_ZIP)
+    __host__ __device__ __forceinline__ int row0(int cta) const { return sh.begin(cta) * ROW_GROUP; }
+    __host__ __device__ __forceinline__ int rows(int cta) const {
+        const int r0 = row0(cta), r1 = r0 + sh.count(cta) * ROW_GROUP;
+        return (r1 < m.N ? r1 : m.N) - r0;
+    }
+    __host__ __device__ __forceinline__ int rows_max() const { return (sh.quot + 1) * ROW_GROUP; }
 };
 
 // Rows that take the fp32 activation instead (Q6_K attn_v); m.data == nullptr: none.
@@ -330,17 +335,15 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         (reinterpret_cast<uintptr_t>(full + slots) + 127) & ~(uintptr_t)127);
 
     // flat block ranges of this CTA in A and B, and the tiles that cover them
-    const int rows_a0 = ja.sh.begin(cta) * ja.rows_per_item;
-    const int rows_a = max(0, min(ja.sh.count(cta) * ja.rows_per_item, ja.m.N - rows_a0));
-    const int rows_b0 = jb.m.data ? jb.sh.begin(cta) * jb.rows_per_item : 0;
-    const int rows_b = jb.m.data ? max(0, min(jb.sh.count(cta) * jb.rows_per_item, jb.m.N - rows_b0)) : 0;
-    const long long fa0 = (long long)rows_a0 * nb, fa1 = fa0 + (long long)rows_a * nb;
-    const long long fb0 = (long long)rows_b0 * nb, fb1 = fb0 + (long long)rows_b * nb;
+    const int rows_a0 = ja.row0(cta), rows_a = max(0, ja.rows(cta)), blocks_a = group_rows(rows_a) * nb;
+    const int rows_b0 = jb.m.data ? jb.row0(cta) : 0, rows_b = jb.m.data ? max(0, jb.rows(cta)) : 0, blocks_b = group_rows(rows_b) * nb;
+    const long long fa0 = (long long)rows_a0 * nb, fa1 = fa0 + blocks_a;
+    const long long fb0 = (long long)rows_b0 * nb, fb1 = fb0 + blocks_b;
     const int ta0 = (int)(fa0 >> 5), tiles_a = rows_a > 0 ? (int)((fa1 + 31) >> 5) - ta0 : 0;
     const int tb0 = (int)(fb0 >> 5), tiles_b = rows_b > 0 ? (int)((fb1 + 31) >> 5) - tb0 : 0;
     const int n_jobs = tiles_a + tiles_b;
     float* part_a = pbuf;
-    float* part_b = pbuf + rows_a * nb;
+    float* part_b = pbuf + blocks_a;
     auto job_src = [&](int j) -> const uint8_t* {
         return j < tiles_a ? ja.m.data + (long long)(ta0 + j) * TB : jb.m.data + (long long)(tb0 + j - tiles_a) * TB;
     };
@@ -371,8 +374,9 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     }
     if (fseg.m.data && tid == GEMV_THREADS - 1) {
         // the fp32-route rows are read with plain loads later: have their tiles in L2 by then
-        const long long f0 = 2ll * fseg.sh.begin(cta) * nb, f1 = f0 + 2ll * fseg.sh.count(cta) * nb;
-        if (f1 > f0) {
+        const int r0 = 2 * fseg.sh.begin(cta), r1 = r0 + 2 * fseg.sh.count(cta);
+        if (r1 > r0) {
+            const long long f0 = (long long)(r0 / ROW_GROUP * ROW_GROUP) * nb, f1 = (long long)group_rows(r1) * nb;
             const long long t0 = f0 >> 5, t1 = (f1 + 31) >> 5;
             bulk_prefetch_l2(fseg.m.data + t0 * Q6_TILE_BYTES, (unsigned)((t1 - t0) * Q6_TILE_BYTES));
         }
@@ -506,7 +510,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     // with the tile dots — taken from the last thread downwards, so the few warps that own tiles keep to their tiles —
     // and share the tile dots' barrier; otherwise they run first, chunk by chunk, with barriers of their own.
     const int f32_tasks = fseg.m.data ? 2 * fseg.sh.count(cta) * 16 * nb : 0;
-    const int f32_off = ((rows_a + rows_b) * nb + 3) & ~3;
+    const int f32_off = blocks_a + blocks_b;
     const bool f32_fused = f32_tasks > 0 && f32_off + f32_tasks <= pbuf_floats;
     if (fseg.m.data && !f32_fused) {
         const int np = fseg.sh.count(cta), pbase = fseg.sh.begin(cta);
@@ -519,7 +523,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                 const int row_l = task / per_row, rem = task - row_l * per_row;
                 const int row_g = 2 * pbase + row_l;
                 float v = 0.f;
-                if (row_g < fseg.m.N) v = q6k_run_dot_f32(fseg.m, (long long)row_g * nb + (rem >> 4), rem >> 4, rem & 15, xs);
+                if (row_g < fseg.m.N) v = q6k_run_dot_f32(fseg.m, mat_flat(nb, row_g, rem >> 4), rem >> 4, rem & 15, xs);
                 pbuf[t] = v;
             }
             __syncthreads();
@@ -560,8 +564,9 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                 late_parity = reuse ? (it & 1) : 0;
             }
             if (mine) {
-                float* dst = is_b ? part_b + (f - fb0) : part_a + (f - fa0);
-                *dst = landed ? block_dot<true>(BLK{}, ring + (size_t)s * TB, lane, act, (int)(f % nb), nb, nullptr) : 0.f;
+                int row, b;
+                flat_row_block((int)(f - (is_b ? fb0 : fa0)), nb, row, b);
+                (is_b ? part_b : part_a)[row * nb + b] = landed ? block_dot<true>(BLK{}, ring + (size_t)s * TB, lane, act, b, nb, nullptr) : 0.f;
             }
             __syncwarp();
             if (!landed) {
@@ -583,7 +588,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             const int row_l = t / per_row, rem = t - row_l * per_row;
             const int row_g = 2 * pbase + row_l;
             float v = 0.f;
-            if (row_g < fseg.m.N) v = q6k_run_dot_f32(fseg.m, (long long)row_g * nb + (rem >> 4), rem >> 4, rem & 15, xs);
+            if (row_g < fseg.m.N) v = q6k_run_dot_f32(fseg.m, mat_flat(nb, row_g, rem >> 4), rem >> 4, rem & 15, xs);
             pbuf[f32_off + t] = v;
         }
     }
@@ -643,7 +648,7 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
                                const F32Seg& fseg, const Epi& epi, int K, TokenState* st) {
     const int nb = K / 256;
     constexpr int TB = BLK::TILE_BYTES;
-    const int ra = (ja.sh.quot + 1) * ja.rows_per_item, rb = jb.m.data ? (jb.sh.quot + 1) * jb.rows_per_item : 0;
+    const int ra = ja.rows_max(), rb = jb.m.data ? jb.rows_max() : 0;
     int pf = gemv_pbuf_floats(ra, rb, nb);
     if (fseg.m.data && pf < 2 * 16 * nb) pf = 2 * 16 * nb;
     const bool has_norm = pa.normw != nullptr;
@@ -660,11 +665,10 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     return launch_pdl(k_gemv<BLK, Epi>, dim3(grid), dim3(GEMV_THREADS), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
 }
 
-inline RowJob make_job(const Mat& m, int rows_per_item, int C, int id_base = 0) {
+inline RowJob make_job(const Mat& m, int C, int id_base = 0) {
     RowJob j{};
     j.m = m;
-    j.rows_per_item = rows_per_item;
-    j.sh = make_share((m.N + rows_per_item - 1) / rows_per_item, C);
+    j.sh = make_share(group_rows(m.N) / ROW_GROUP, C);
     j.id_base = id_base;
     return j;
 }
@@ -730,13 +734,15 @@ __global__ void k_int_dots(Mat m, const float* x, const signed char* q8, const f
     } else {
         act_from_q8(act, q8, d8, K);
     }
-    const long long total = (long long)m.N * nb;
+    const long long total = (long long)group_rows(m.N) * nb;
     const long long tiles = (total + 31) >> 5;
     const int TB = tile_bytes(m.type);
     for (long long t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < tiles; t += (long long)gridDim.x * (blockDim.x >> 5)) {
         const long long f = t * 32 + lane;
         if (f >= total) continue;
-        const int r = (int)(f / nb), b = (int)(f % nb);
+        int r, b;
+        flat_row_block((int)f, nb, r, b);
+        if (r >= m.N) continue;
         int ints[16];
         block_dot<false>(BLK{}, m.data + t * TB, lane, act, b, nb, ints);
         if (BLK::TILE_BYTES == Q4_TILE_BYTES) {
@@ -764,44 +770,51 @@ __device__ __forceinline__ int perm_src_row(int v, int perm_hd) {
 }
 
 // GGUF block bytes -> warp-tiled layout (see tfr_gemv.cuh).  One thread per (flat block, 16-byte
-// piece); tail tiles are zero-filled by the caller.
+// piece); the padding rows of the last group and the tail tile's unused lanes become zero.
 __global__ void k_repack_tiled(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int type, int N, int nb,
                                int perm_hd) {
     const int pieces = type == TFR_Q4_K ? Q4_PIECES : type == TFR_Q8_0 ? Q8_PIECES : Q6_PIECES + 1;  // Q6_K: 13 pieces + the 2-byte d
     const int blk = block_bytes_256(type), TB = tile_bytes(type);
-    const long long total = (long long)N * nb * pieces;
+    const long long total = mat_tiles(256 * nb, N) * 32 * pieces;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long f = i / pieces;
         const int pc = (int)(i - f * pieces);
-        const int row = (int)(f / nb), b = (int)(f - (long long)row * nb);
-        const uint8_t* sb = src + ((long long)perm_src_row(row, perm_hd) * nb + b) * blk;
+        int row, b;
+        flat_row_block((int)f, nb, row, b);
+        const bool in = row < N;
+        const uint8_t* sb = src + ((long long)(in ? perm_src_row(row, perm_hd) : 0) * nb + b) * blk;
         uint8_t* tile = dst + (f >> 5) * TB;
         const int lane = (int)(f & 31);
         if (type == TFR_Q6_K && pc == Q6_PIECES) {
-            tile[Q6_PIECES * 512 + lane * 2] = sb[208];
-            tile[Q6_PIECES * 512 + lane * 2 + 1] = sb[209];
+            tile[Q6_PIECES * 512 + lane * 2] = in ? sb[208] : 0;
+            tile[Q6_PIECES * 512 + lane * 2 + 1] = in ? sb[209] : 0;
         } else {
-            for (int k = 0; k < 16; k++) tile[pc * 512 + lane * 16 + k] = sb[pc * 16 + k];
+            for (int k = 0; k < 16; k++) tile[pc * 512 + lane * 16 + k] = in ? sb[pc * 16 + k] : 0;
         }
     }
 }
 
-// One row of a tiled matrix as a one-row tiled matrix (a single tile, lanes 0 .. nb-1): the extra
-// vocabulary row of a shortlisted head (load.rs:308-342).  One thread per (block, piece).
-__global__ void k_extract_row(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int type, int row, int nb) {
+// Rows row0 .. row0 + N - 1 of a tiled matrix as a tiled matrix of their own: the extra vocabulary row of a shortlisted
+// head (load.rs:308-342), a rank's slice of a tied head.  One thread per (block, piece).
+__global__ void k_slice_rows(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int type, int row0, int N, int nb) {
     const int pieces = type == TFR_Q4_K ? Q4_PIECES : type == TFR_Q8_0 ? Q8_PIECES : Q6_PIECES + 1;
     const int TB = tile_bytes(type);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nb * pieces) return;
-    const int b = i / pieces, pc = i - b * pieces;
-    const long long f = (long long)row * nb + b;
-    const uint8_t* st = src + (f >> 5) * TB;
-    const int sl = (int)(f & 31);
-    if (type == TFR_Q6_K && pc == Q6_PIECES) {
-        dst[Q6_PIECES * 512 + b * 2] = st[Q6_PIECES * 512 + sl * 2];
-        dst[Q6_PIECES * 512 + b * 2 + 1] = st[Q6_PIECES * 512 + sl * 2 + 1];
-    } else {
-        for (int k = 0; k < 16; k++) dst[pc * 512 + b * 16 + k] = st[pc * 512 + sl * 16 + k];
+    const long long total = mat_tiles(256 * nb, N) * 32 * pieces;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long f = i / pieces;
+        const int pc = (int)(i - f * pieces);
+        int row, b;
+        flat_row_block((int)f, nb, row, b);
+        const bool in = row < N;
+        const long long fs = mat_flat(nb, row0 + (in ? row : 0), in ? b : 0);
+        const uint8_t* st = src + (fs >> 5) * TB;
+        uint8_t* dt = dst + (f >> 5) * TB;
+        const int sl = (int)(fs & 31), dl = (int)(f & 31);
+        if (type == TFR_Q6_K && pc == Q6_PIECES) {
+            for (int k = 0; k < 2; k++) dt[Q6_PIECES * 512 + dl * 2 + k] = in ? st[Q6_PIECES * 512 + sl * 2 + k] : 0;
+        } else {
+            for (int k = 0; k < 16; k++) dt[pc * 512 + dl * 16 + k] = in ? st[pc * 512 + sl * 16 + k] : 0;
+        }
     }
 }
 

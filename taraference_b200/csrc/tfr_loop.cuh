@@ -62,11 +62,10 @@ constexpr int LOOP_BAR_STRIDE = 32;          // words between the eight grid-bar
 enum { CTL_STOP = 0, CTL_ABORT = 1, CTL_SNAP = 2, CTL_STOPS = 8, CTL_WORDS = 16 };  // [CTL_STOPS, +8): stop ids
 enum { LEPI_QKV = 0, LEPI_RESIDUAL = 1, LEPI_SILU = 2, LEPI_LOGITS = 3 };
 
-// One matrix of a phase, spread over the CTAs in contiguous shares of `rpi` rows.
+// One matrix of a phase, spread over the CTAs in contiguous shares of row groups.
 struct LoopJob {
     int type;     // TFR_Q4_K / TFR_Q6_K; 0: absent
     int N;        // rows
-    int rpi;      // rows per share item: 2 (row pairs) or 1
     int id_base;  // epilogue id of the matrix's first item
     int f32;      // 1: fp32-activation route (Q6_K attn_v, kernels/gemv.cu:233-264)
     Share sh;
@@ -99,7 +98,7 @@ struct LoopArgs {
     // vectors handed from phase to phase through global memory: residual stream, q, attention output,
     // SiLU*mul output, split-KV partials [n_head][attn_smax][4 + hd] = (m, l, -, -, O); logits for the host
     float *x, *q, *att, *h, *pc, *logits;
-    Share sh_x;              // row pairs of the residual stream per CTA (the shares of o-proj and down)
+    Share sh_x;              // row groups of the residual stream per CTA (the shares of o-proj and down)
     int off_own;             // shared memory: the CTA's own residual rows
     float* layer_taps;       // optional [n_layer][K]
     unsigned int* bar;       // 8 counters, LOOP_BAR_STRIDE words apart, zero at launch
@@ -214,21 +213,22 @@ __host__ __device__ __forceinline__ void cursor_advance(int& slot, int& lap, int
 
 // Flat 256-weight blocks [f0, f1) of one matrix inside one chunk of a phase, for one CTA (f0 == f1: none).
 struct JobSpan {
-    int f0, f1;
+    int f0, f1, rows;
 };
 __host__ __device__ __forceinline__ JobSpan job_span(const LoopJob& j, int nb, int cta, int chunk, int rpc) {
     JobSpan v;
-    v.f0 = v.f1 = 0;
+    v.f0 = v.f1 = v.rows = 0;
     if (!j.type) return v;
     const int i0 = j.sh.begin(cta), cnt = j.sh.count(cta);
-    int ra = i0 * j.rpi, rb = (i0 + cnt) * j.rpi < j.N ? (i0 + cnt) * j.rpi : j.N;
+    int ra = i0 * ROW_GROUP, rb = (i0 + cnt) * ROW_GROUP < j.N ? (i0 + cnt) * ROW_GROUP : j.N;
     if (rpc > 0) {
         ra += chunk * rpc;
         rb = rb < ra + rpc ? rb : ra + rpc;
     }
     if (rb <= ra) return v;
-    v.f0 = ra * nb;
-    v.f1 = rb * nb;
+    v.f0 = ra * nb;              // ra starts a row group
+    v.f1 = group_rows(rb) * nb;  // the padding rows of the last group included
+    v.rows = rb - ra;
     return v;
 }
 __host__ __device__ __forceinline__ int span_t0(const JobSpan& v) { return v.f0 >> 5; }
@@ -247,7 +247,7 @@ __host__ __device__ __forceinline__ int phase_chunks(const LoopPhase& ph, int ct
         const LoopJob& jb = ph.job[j];
         if (!jb.type) continue;
         const int i0 = jb.sh.begin(cta), cnt = jb.sh.count(cta);
-        const int r = ((i0 + cnt) * jb.rpi < jb.N ? (i0 + cnt) * jb.rpi : jb.N) - i0 * jb.rpi;
+        const int r = ((i0 + cnt) * ROW_GROUP < jb.N ? (i0 + cnt) * ROW_GROUP : jb.N) - i0 * ROW_GROUP;
         rows = rows > r ? rows : r;
     }
     return (rows + ph.rpc - 1) / ph.rpc;
@@ -255,21 +255,20 @@ __host__ __device__ __forceinline__ int phase_chunks(const LoopPhase& ph, int ct
 
 // ------------------------------------------------------------------ plan helpers (host)
 
-inline LoopJob loop_job(int type, int N, int rpi, int id_base, int f32, int G) {
+inline LoopJob loop_job(int type, int N, int id_base, int f32, int G) {
     LoopJob j{};
     j.type = type;
     j.N = N;
-    j.rpi = rpi;
     j.id_base = id_base;
     j.f32 = f32;
-    j.sh = make_share((N + rpi - 1) / rpi, G);
+    j.sh = make_share(group_rows(N) / ROW_GROUP, G);
     return j;
 }
 // Finishes a phase descriptor: block-split and, when the CTA's block partials exceed the buffer, a chunk size.
 // Most tiles a CTA's share of the job can touch (a share may straddle a tile at either end).
 inline int loop_job_tiles(const LoopJob& j, int nb) {
     if (!j.type) return 0;
-    const int rows = (j.sh.quot + (j.sh.rem ? 1 : 0)) * j.rpi;
+    const int rows = (j.sh.quot + (j.sh.rem ? 1 : 0)) * ROW_GROUP;
     return rows ? (rows * nb + 31) / 32 + 1 : 0;
 }
 // Lanes per block for a phase.  A warp task costs a fixed part (descriptor, tile wait, partial store, slot release)
@@ -290,16 +289,15 @@ inline int loop_pick_lpb(int q8_tiles, int f32_tiles) {
 inline bool loop_finish_phase(LoopPhase& ph, int K, int pbuf_floats, int lpb_forced) {
     ph.K = K;
     ph.nb = K / 256;
-    int q8_tiles = 0, f32_tiles = 0, need = 0, rows_max = 0, njobs = 0, rpi = 1;
+    int q8_tiles = 0, f32_tiles = 0, need = 0, rows_max = 0, njobs = 0;
     for (int j = 0; j < 3; j++) {
         const LoopJob& jb = ph.job[j];
         if (!jb.type) continue;
         njobs++;
         (jb.f32 ? f32_tiles : q8_tiles) += loop_job_tiles(jb, ph.nb);
-        const int rows = (jb.sh.quot + (jb.sh.rem ? 1 : 0)) * jb.rpi;
+        const int rows = (jb.sh.quot + (jb.sh.rem ? 1 : 0)) * ROW_GROUP;
         need += rows * ph.nb;
         rows_max = (rows_max > rows ? rows_max : rows);
-        rpi = (rpi > jb.rpi ? rpi : jb.rpi);
     }
     ph.lpb = (lpb_forced == 1 || lpb_forced == 2 || lpb_forced == 4) ? lpb_forced : loop_pick_lpb(q8_tiles, f32_tiles);
     ph.rpc = 0;
@@ -313,16 +311,16 @@ inline bool loop_finish_phase(LoopPhase& ph, int K, int pbuf_floats, int lpb_for
         a = t;
     }
     int unit = 32 / g;
-    if (unit % rpi) unit *= rpi;
+    if (unit % ROW_GROUP) unit *= ROW_GROUP;
     const int cap_rows = pbuf_floats / (ph.nb * njobs);
-    if (cap_rows < rpi) return false;
+    if (cap_rows < ROW_GROUP) return false;
     const int n_chunks = (rows_max + cap_rows - 1) / cap_rows;
     int rpc = (rows_max + n_chunks - 1) / n_chunks;
     rpc = (rpc + unit - 1) / unit * unit;
     if (rpc > cap_rows) rpc = cap_rows / unit * unit;
-    if (rpc < rpi) rpc = cap_rows / rpi * rpi;
+    if (rpc < ROW_GROUP) rpc = cap_rows / ROW_GROUP * ROW_GROUP;
     ph.rpc = rpc;
-    return rpc >= rpi;
+    return rpc >= ROW_GROUP;
 }
 
 // ------------------------------------------------------------------ weight streamer (the last warp)
@@ -369,18 +367,16 @@ struct ChunkDesc {
     int rows[3], id0[3];  // rows of every matrix in the chunk and the epilogue id of its first item
 };
 // One warp task (4 ints): a tile part of 32 / lp blocks.
-//   x: flat index of the part's first block      y: partial-sum index of block f is f + y
+//   x: flat index of the part's first block      y: partial-sum index of (row, b) is row * nb + b + y
 //   z: entry inside the chunk (10 bits) | tile offset in the slot / 16 (10) | matrix (2) | kind (2: 0 Q4_K, 1 Q6_K,
 //      2 Q6_K fp32 route) | log2 lanes per block (2) | arrival weight (6)
-//   w: x mod blocks-per-row
-__host__ __device__ __forceinline__ uint4 task_desc(int f_first, int part_rel, int ent, int toff, int job, int kind, int lsh, int weight,
-                                                    int b_first) {
+__host__ __device__ __forceinline__ uint4 task_desc(int f_first, int part_rel, int ent, int toff, int job, int kind, int lsh, int weight) {
     uint4 r;
     r.x = (unsigned)f_first;
     r.y = (unsigned)part_rel;
     r.z = (unsigned)ent | ((unsigned)(toff >> 4) << 10) | ((unsigned)job << 20) | ((unsigned)kind << 22) | ((unsigned)lsh << 24) |
           ((unsigned)weight << 26);
-    r.w = (unsigned)b_first;
+    r.w = 0u;
     return r;
 }
 
@@ -421,7 +417,7 @@ inline bool loop_build_plan(const LoopPhase (&ph)[SCHED_SECTIONS], const bool (&
                         const LoopJob& jb = P.job[j];
                         const JobSpan v = job_span(jb, P.nb, cta, ch, P.rpc);
                         cd.f0[j] = v.f0, cd.f1[j] = v.f1;
-                        cd.rows[j] = (v.f1 - v.f0) / P.nb;
+                        cd.rows[j] = v.rows;
                         const int r0 = v.f0 / P.nb;
                         cd.id0[j] = jb.id_base + (P.zip ? r0 : (r0 >> 1));
                         if (v.f1 > v.f0) {
@@ -434,8 +430,7 @@ inline bool loop_build_plan(const LoopPhase (&ph)[SCHED_SECTIONS], const bool (&
                                 for (int sub = 0; sub < lp; sub++) {
                                     const int f_first = (span_t0(v) + tl) * 32 + sub * per;
                                     if (ebase + el >= 1024 || LOOP_EMPTY % (tiles_here * lp)) return false;
-                                    tl_out.push_back(task_desc(f_first, off - v.f0, ebase + el, ti * TB, j, kind, lsh, LOOP_EMPTY / (tiles_here * lp),
-                                                               f_first % P.nb));
+                                    tl_out.push_back(task_desc(f_first, off - v.f0, ebase + el, ti * TB, j, kind, lsh, LOOP_EMPTY / (tiles_here * lp)));
                                 }
                             }
                             ebase += span_entries(v, jb.type);
@@ -993,10 +988,9 @@ __device__ __noinline__ void loop_dots(LoopCtx& c, const LoopArgs& a, const Chun
         const int bl = f & 31;  // block inside the tile
         const bool mine = f >= cd->f0[job] && f < cd->f1[job];
         float val = 0.f;
+        int row, b;
+        flat_row_block(f, nb, row, b);
         if (mine) {
-            int b = (int)cur.w + dl;
-            b = b >= nb ? b - nb : b;
-            b = b >= nb ? b % nb : b;
             if (kind == 0) {
 #pragma unroll 1
                 for (int t = q0; t < q1; t++) val += q4_quarter(tile, bl, t, act, b, nb);
@@ -1010,7 +1004,7 @@ __device__ __noinline__ void loop_dots(LoopCtx& c, const LoopArgs& a, const Chun
         }
         if (lsh >= 1) val += __shfl_xor_sync(TFR_FULL_MASK, val, 16);
         if (lsh == 2) val += __shfl_xor_sync(TFR_FULL_MASK, val, 8);
-        if (mine && q0 == 0) c.pbuf[f + (int)cur.y] = val;
+        if (mine && q0 == 0) c.pbuf[row * nb + b + (int)cur.y] = val;
         __syncwarp();
         if (lane == 0) mbar_arrive_n(c.empty + s, cur.z >> 26);
     }
@@ -1275,7 +1269,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_decode_loop(const __grid_co
         c.blob = reinterpret_cast<const int*>(smem + a.off_blob);
         c.lay = reinterpret_cast<const LoopLayer*>(smem + a.off_layers);
         c.own = reinterpret_cast<float*>(smem + a.off_own);
-        c.own_row0 = 2 * a.sh_x.begin((int)blockIdx.x);
+        c.own_row0 = ROW_GROUP * a.sh_x.begin((int)blockIdx.x);
         c.bar_k = 0;
         c.slot = 0;
         c.lap = 0;
@@ -1317,7 +1311,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_decode_loop(const __grid_co
     if (ltid() < 8) c.ctl[CTL_STOPS + ltid()] = ltid() < n_stop ? st->stop_ids[ltid()] : -1;
     cbar();
     const int K = a.K;
-    const int n_own = max(0, min(K, c.own_row0 + 2 * a.sh_x.count(c.cta)) - c.own_row0);
+    const int n_own = max(0, min(K, c.own_row0 + ROW_GROUP * a.sh_x.count(c.cta)) - c.own_row0);
     bool done = false;
 #pragma unroll 1
     for (int it = 0; !done; it++) {

@@ -85,7 +85,7 @@ struct EpiAllReduce {
     static constexpr int MODE = EPI_PAIRS;
     float* x;          // [n_rows] replicated residual stream, updated in place
     int n_rows;
-    Share sh;          // row-pair shares of the matrix over the grid (the same on every rank)
+    Share sh;          // shares of row groups (two row pairs each) over the grid (the same on every rank)
     TpComm c;
     int op_index;      // which all-reduce of the token this is
     unsigned epoch;
@@ -102,7 +102,7 @@ struct EpiAllReduce {
     }
     __device__ void end(TokenState* st) {
         const int tid = threadIdx.x, cta = blockIdx.x;
-        const int p0 = sh.begin(cta), np = sh.count(cta);
+        const int p0 = 2 * sh.begin(cta), np = min(2 * sh.count(cta), ((n_rows + 1) >> 1) - p0);
         bool ok = true;
         for (int i = tid; i < np; i += blockDim.x) {
             const int p = p0 + i;
