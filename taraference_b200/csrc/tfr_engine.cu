@@ -158,6 +158,7 @@ struct tfr_engine {
     unsigned int* counters = nullptr;
     TokenState* st = nullptr;
     TokenState* st_host = nullptr;  // pinned
+    float* logits_host = nullptr;   // pinned
     int *out_tokens = nullptr, *out_host = nullptr, *prompt = nullptr;  // the tokens lie behind the state: one copy fetches both
     int attn_S = 1, attn_S_staged = 1, attn_min_keys = 64;  // splits per KV head of the two attention instances
     float* layer_taps = nullptr;  // [n_layer][n_embd] residual stream after each layer (test aid)
@@ -167,7 +168,7 @@ struct tfr_engine {
     bool use_graph = true;
     std::vector<TokenGraphs> graphs;  // one entry per KV capacity in use, the one used last in front
     int64_t launches = 0;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_half = nullptr;
     float last_ms = 0.f;
     // persistent decode loop (tfr_loop.cuh): one cooperative kernel per call instead of a graph per token
     bool loop_ok = false;
@@ -591,7 +592,8 @@ extern "C" int tfr_create(int device, tfr_engine** out) {
     e->device = device;
     if (cudaGetDeviceProperties(&e->prop, device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreate(&e->ev0) != cudaSuccess || cudaEventCreate(&e->ev1) != cudaSuccess) {
+        cudaEventCreate(&e->ev0) != cudaSuccess || cudaEventCreate(&e->ev1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e->ev_half, cudaEventDisableTiming) != cudaSuccess) {
         delete e;
         return TFR_E_CUDA;
     }
@@ -628,8 +630,10 @@ extern "C" void tfr_destroy(tfr_engine* e) {
                   e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->ctscale, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
     for (void* p : ws) cudaFree(p);
     if (e->st_host) cudaFreeHost(e->st_host);
+    if (e->logits_host) cudaFreeHost(e->logits_host);
     cudaEventDestroy(e->ev0);
     cudaEventDestroy(e->ev1);
+    cudaEventDestroy(e->ev_half);
     cudaStreamDestroy(e->stream);
     delete e;
 }
@@ -1220,6 +1224,7 @@ extern "C" int tfr_finalize_load(tfr_engine* e) {
     CU(e, cudaMalloc(&e->prompt, (size_t)TFR_MAX_PROMPT * 4));
     CU(e, cudaMallocHost(&e->st_host, STATE_STRIDE + (size_t)TFR_MAX_BURST * 4));
     e->out_host = reinterpret_cast<int*>(reinterpret_cast<char*>(e->st_host) + STATE_STRIDE);
+    CU(e, cudaMallocHost(&e->logits_host, ((size_t)Vl + 4) * 4));
     CU(e, cudaMemsetAsync(e->counters, 0, (size_t)P.n_kv * ATTN_CLUSTER * 4, e->stream));
     CU(e, cudaMemsetAsync(e->st, 0, sizeof(TokenState), e->stream));
     CU(e, cudaMemsetAsync(e->logits, 0, (size_t)Vl * 4, e->stream));
@@ -1999,8 +2004,21 @@ extern "C" int tfr_current_logits(tfr_engine* e, float* out, int n) {
     cudaSetDevice(e->device);
     const int active = e->vocab_limit ? e->vocab_limit + (e->head_special ? 1 : 0) : e->plan.v1;
     const int first = e->plan.v0, end = active < n ? active : n;
-    if (end > first) CU(e, cudaMemcpyAsync(out + first, e->logits, (size_t)(end - first) * 4, cudaMemcpyDeviceToHost, e->stream));
+    if (end <= first) {
+        CU(e, cudaStreamSynchronize(e->stream));
+        return TFR_OK;
+    }
+    // The caller's memory is pageable: copied to directly, the driver stages it piece by piece (300 us for 152 K logits).
+    // Through a pinned buffer of the engine's the first half is copied out while the second one is on its way.
+    const size_t total = (size_t)(end - first), half = std::min(total, (total / 2 + 3) & ~(size_t)3);
+    const float* src = e->logits;
+    CU(e, cudaMemcpyAsync(e->logits_host, src, half * 4, cudaMemcpyDeviceToHost, e->stream));
+    CU(e, cudaEventRecord(e->ev_half, e->stream));
+    if (total > half) CU(e, cudaMemcpyAsync(e->logits_host + half, src + half, (total - half) * 4, cudaMemcpyDeviceToHost, e->stream));
+    CU(e, cudaEventSynchronize(e->ev_half));
+    memcpy(out + first, e->logits_host, half * 4);
     CU(e, cudaStreamSynchronize(e->stream));
+    if (total > half) memcpy(out + first + half, e->logits_host + half, (total - half) * 4);
     return TFR_OK;
 }
 

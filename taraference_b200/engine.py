@@ -315,7 +315,7 @@ class CudaModel:
         rows and zeros elsewhere (taraference_b200.tp.gather_logits merges the ranks).  With a
         vocabulary shortlist only the active entries come back (see active_vocab)."""
         n_active, _ = self.active_vocab()
-        out = np.zeros(self.cfg["n_vocab"], np.float32)
+        out = (np.zeros if int(self.cfg.get("tp_size", 1)) > 1 else np.empty)(self.cfg["n_vocab"], np.float32)
         self._check(_lib.lib().tfr_current_logits(self._h, out.ctypes.data, out.size))
         return out[:n_active] if n_active < out.size else out
 
