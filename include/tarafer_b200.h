@@ -221,7 +221,8 @@ int tfr_decode_path(const tfr_engine* e);
  * the weights once (CudaModel::forward_chunk, crates/core/src/cuda/forward.rs:54-65, 360-407; MAX_BATCH,
  * MAX_VERIFY_TOKENS, crates/core/src/cuda/types.rs:7-9).  tokens = 0 feeds every token of a prompt as a decode step;
  * values above the engine's chunk capacity are clamped.  tfr_prefill_chunk returns the size in effect, 0 for models
- * the chunk kernels do not cover (hybrid layers, tensor parallelism), which keep the step-by-step route. */
+ * the chunk kernels do not cover (tensor parallelism), which keep the step-by-step route, and for hybrid models, whose
+ * recurrent layers step through the tokens inside a chunk. */
 int tfr_set_prefill_chunk(tfr_engine* e, int tokens);
 int tfr_prefill_chunk(const tfr_engine* e);
 /* Kernel launches issued by this engine so far (graph replays count their kernel nodes). */

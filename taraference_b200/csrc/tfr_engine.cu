@@ -197,6 +197,8 @@ struct tfr_engine {
     unsigned char* cimage = nullptr;  // operand image of the tensor-core projections (tfr_gemm_tc.cuh), its token scales
     float* ctscale = nullptr;
     size_t cact_stride = 0;
+    // hybrid layers of a batch: raw projections, the mixer's q / k / v (or the output gates of a full layer), decay and write strength
+    float *cproj = nullptr, *cmix = nullptr, *cgates = nullptr;
     unsigned long long* ckeys = nullptr;  // per-row, per-slice argmax keys of a verification pass
     unsigned int* ccount = nullptr;       // per-row arrival counters, zero between launches
 };
@@ -324,6 +326,10 @@ static void configure_kernels_once() {
     cudaFuncSetAttribute(k_attn_decode<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_dyn_smem(128));
     cudaFuncSetAttribute(k_attn_decode<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_dyn_smem(256));
     configure_kernel(k_gdn_step, false);
+    configure_kernel(k_gdn_chunk_conv, false);
+    configure_kernel(k_gdn_chunk_scan, false);
+    configure_kernel(k_gdn_chunk_norm, false);
+    configure_kernel(k_gate_rows, false);
     configure_kernel(k_qk_norm_rope_store, false);
     configure_kernel(k_state_advance, false);
     configure_kernel(k_add_residual, false);
@@ -627,7 +633,7 @@ extern "C" void tfr_destroy(tfr_engine* e) {
     for (auto& kv : e->vecs) cudaFree(kv.second.dev);
     for (auto& L : e->layers) cudaFree(L.bias_qkv);
     void* ws[] = {e->x, e->q, e->attn, e->h, e->logits, e->partial, e->counters, e->st, e->prompt,
-                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->ctscale, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
+                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->ctscale, e->cproj, e->cmix, e->cgates, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
     for (void* p : ws) cudaFree(p);
     if (e->st_host) cudaFreeHost(e->st_host);
     if (e->logits_host) cudaFreeHost(e->logits_host);
@@ -1652,15 +1658,18 @@ static void chunk_setup(tfr_engine* e) {
     const tfr_model_config& c = e->cfg;
     e->chunk_ok = false;
     auto no = [&](const char* why) { e->chunk_why = why; };
-    if (c.hybrid) return no("hybrid (Gated-DeltaNet) layers");
     if (e->plan.tp > 1) return no("tensor parallelism");
     auto q468 = [](const tfr_mat* m) { return m->m.type == TFR_Q4_K || m->m.type == TFR_Q6_K || m->m.type == TFR_Q8_0; };
     if (!q468(e->head)) return no("head type");
     for (const LayerW& L : e->layers) {
-        if (L.kind != LAYER_DENSE) return no("layer kind");
-        if (L.wq->m.type != TFR_Q4_K || L.wk->m.type != TFR_Q4_K || L.gate->m.type != TFR_Q4_K || L.up->m.type != TFR_Q4_K)
-            return no("attn_q / attn_k / ffn_gate / ffn_up type");
-        if (!q468(L.wo) || !q468(L.down)) return no("attn_output / ffn_down type");
+        if (L.gate->m.type != TFR_Q4_K || L.up->m.type != TFR_Q4_K || !q468(L.down)) return no("ffn_gate / ffn_up / ffn_down type");
+        if (L.kind == LAYER_LINEAR) {
+            if (!q468(L.ssm_out)) return no("ssm_out type");
+            for (int k = 0; k < 4; k++)
+                if (!q468(L.gdn_proj ? L.gdn_proj : L.proj4[k])) return no("type of a linear layer's projections");
+            continue;
+        }
+        if (L.wq->m.type != TFR_Q4_K || L.wk->m.type != TFR_Q4_K || !q468(L.wo)) return no("attn_q / attn_k / attn_output type");
     }
     e->chunk_ok = true;
     e->chunk_why.clear();
@@ -1674,10 +1683,12 @@ static int chunk_buffers(tfr_engine* e, int M) {
     cap = std::min(cap, std::max(CHUNK_MAX_TOKENS, CHUNK_VERIFY_MAX));
     const TpPlan& P = e->plan;
     const int K = e->cfg.n_embd, hd = e->cfg.head_dim;
-    const int kmax = std::max(std::max(K, P.ff), P.attn_width);
+    const tfr_model_config& c = e->cfg;
+    const int vd = c.hybrid ? gdn_val_dim(c) : 0, channels = c.hybrid ? gdn_channels(c) : 0;
+    const int mix_width = std::max(P.attn_width, vd), kmax = std::max(std::max(K, P.ff), mix_width);
     CU(e, cudaStreamSynchronize(e->stream));
     void** grown[] = {(void**)&e->cx, (void**)&e->cxn, (void**)&e->cq, (void**)&e->cattn, (void**)&e->ch, (void**)&e->cact, (void**)&e->cpart,
-                      (void**)&e->cimage, (void**)&e->ctscale};
+                      (void**)&e->cimage, (void**)&e->ctscale, (void**)&e->cproj, (void**)&e->cmix, (void**)&e->cgates};
     e->chunk_cap = 0;
     for (void** p : grown) {
         cudaFree(*p);
@@ -1687,11 +1698,16 @@ static int chunk_buffers(tfr_engine* e, int M) {
     CU(e, cudaMalloc(&e->cx, (size_t)cap * K * 4));
     CU(e, cudaMalloc(&e->cxn, (size_t)cap * K * 4));
     CU(e, cudaMalloc(&e->cq, (size_t)cap * P.nq * 4));
-    CU(e, cudaMalloc(&e->cattn, (size_t)cap * P.attn_width * 4));
+    CU(e, cudaMalloc(&e->cattn, (size_t)cap * mix_width * 4));
     CU(e, cudaMalloc(&e->ch, (size_t)cap * P.ff * 4));
     CU(e, cudaMalloc(&e->cact, (size_t)cap * e->cact_stride));
     CU(e, cudaMalloc(&e->cimage, tc_image_bytes(kmax, cap)));
     CU(e, cudaMalloc(&e->ctscale, (size_t)tc_pad_tokens(cap) * 4));
+    if (c.hybrid) {
+        CU(e, cudaMalloc(&e->cproj, (size_t)cap * std::max(channels + vd + 2 * c.ssm_time_step_rank, 2 * P.nq + 2 * P.nkv) * 4));
+        CU(e, cudaMalloc(&e->cmix, (size_t)cap * std::max(channels, P.nq) * 4));
+        CU(e, cudaMalloc(&e->cgates, (size_t)cap * c.ssm_time_step_rank * 8));
+    }
     // attention partials: the key splits of few query tiles, or two per token of a full chunk
     e->cpart_floats = (size_t)P.n_head * (2 + hd) * std::max(64 * CHUNK_ATTN_SPLITS_MAX, 2 * cap);
     CU(e, cudaMalloc(&e->cpart, e->cpart_floats * 4));
@@ -1717,9 +1733,10 @@ static cudaError_t launch_gemm_typed(cudaStream_t s, int grid, int type, const u
 }
 
 // M tokens (device ids at tok) at positions pos0 .. pos0 + M - 1 through all layers: their K / V rows land in the
-// cache and e->cx holds their residual streams.  all_rows: also the greedy token after every position, to
+// cache and e->cx holds their residual streams.  rec0: tokens the recurrent state (hybrid models) has absorbed before
+// them.  all_rows: also the greedy token after every position, to
 // e->out_tokens[0 .. M).  forward.rs:360-407 (forward_chunk), 292-358 (logits_for_rows).
-static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M, int pos0, bool all_rows) {
+static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M, int pos0, long long rec0, bool all_rows) {
     const tfr_model_config& c = e->cfg;
     const TpPlan& P = e->plan;
     const int K = c.n_embd, hd = c.head_dim, nq = P.nq, nkv = P.nkv, FF = P.ff, V = e->head->m.N;
@@ -1757,20 +1774,52 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     n++;
     for (int li = 0; li < c.n_layer; li++) {
         const LayerW& L = e->layers[li];
-        // 1. RMSNorm + Q8, Q/K/V (+bias) + RoPE + f16 KV rows
-        const bool tc_qk = gemm_on_tc(TFR_Q4_K, M);
+        const tfr_mat* wout = L.wo;
+        int mix_width = P.attn_width;
+        if (L.kind == LAYER_LINEAR) {
+            // 1. RMSNorm + Q8, [qkv | z | beta | alpha]; 2. the mixer
+            GdnChunkArgs g{};
+            g.proj = e->cproj, g.ld = gdn_channels(c) + gdn_val_dim(c) + 2 * c.ssm_time_step_rank;
+            for (int k = 0, off = 0; k < (L.gdn_proj ? 1 : 4); k++) {
+                const tfr_mat* w = L.gdn_proj ? L.gdn_proj : L.proj4[k];
+                if (project(e->cx, K, L.attn_norm, make_job(w->m, cap), RowJob{}, store_epi(e->cproj + off, g.ld, w->m.N, 0)) != cudaSuccess)
+                    return -1;
+                off += w->m.N;
+            }
+            g.conv_w = L.conv_w;
+            g.conv_ring = kv->conv + (size_t)li * kv->conv_stride, g.state = kv->ssm + (size_t)li * kv->ssm_stride;
+            g.ssm_a = L.ssm_a, g.ssm_dt = L.ssm_dt, g.norm_w = L.ssm_norm;
+            g.mixed = e->cmix, g.gates = e->cgates, g.out = e->cattn;
+            g.M = M, g.n_k = c.ssm_group_count, g.n_v = c.ssm_time_step_rank, g.kernel = c.ssm_conv_kernel;
+            g.slot0 = (int)(rec0 % c.ssm_conv_kernel), g.eps = c.rms_eps;
+            if (launch_pdl(k_gdn_chunk_conv, dim3(2 * g.n_k + g.n_v, (M + GDN_CONV_TOKENS - 1) / GDN_CONV_TOKENS), dim3(GDN_D), 0, s, g) != cudaSuccess ||
+                launch_pdl(k_gdn_chunk_scan, dim3(g.n_v, GDN_D / GDN_SCAN_COLS), dim3(GDN_SCAN_THREADS), 0, s, g) != cudaSuccess ||
+                launch_pdl(k_gdn_chunk_norm, dim3(g.n_v, M), dim3(GDN_D), 0, s, g) != cudaSuccess)
+                return -1;
+            n += 3;
+            mix_width = gdn_val_dim(c);
+            wout = L.ssm_out;
+        } else {
+        // 1. RMSNorm + Q8, Q/K/V (+bias); dense layers: RoPE + f16 KV rows
+        const bool gated = L.kind == LAYER_FULL_GATED, tc_qk = gemm_on_tc(TFR_Q4_K, M);
+        const int q_rows = gated ? 2 * nq : nq;
         if (prep(tc_qk, e->cx, K, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
         {
-            const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, nq / 2);
+            const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, q_rows / 2);
             F32Seg fseg{};
             fseg.m = L.wv->m;
             fseg.sh = make_share(nkv / 2, cap);
-            fseg.id_base = (nq + nkv) / 2;
+            fseg.id_base = (q_rows + nkv) / 2;
             ChunkEpi ep{};
-            ep.kind = CEPI_QKV;
-            ep.out = e->cq, ep.ldo = nq, ep.bias = L.bias_qkv;
-            ep.kc = kv_k(kv, li), ep.vc = kv_v(kv, li);
-            ep.nq = nq, ep.nk = nkv, ep.hd = hd, ep.kvdim = nkv, ep.pos0 = pos0, ep.theta = c.rope_theta;
+            if (gated) {
+                ep = store_epi(e->cproj, q_rows + 2 * nkv, q_rows + 2 * nkv, 0);
+            } else {
+                ep.kind = CEPI_QKV;
+                ep.out = e->cq, ep.ldo = nq;
+                ep.kc = kv_k(kv, li), ep.vc = kv_v(kv, li);
+                ep.nq = nq, ep.nk = nkv, ep.hd = hd, ep.kvdim = nkv, ep.pos0 = pos0, ep.theta = c.rope_theta;
+            }
+            ep.bias = L.bias_qkv;
             if (tc_qk) {
                 // the fp32-route V rows keep the decode kernels' arithmetic bit for bit
                 if (launch_rows_f32(s, fseg.m, fseg.id_base, e->cxn, M, ep) != cudaSuccess) return -1;
@@ -1779,6 +1828,16 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             } else if (launch_gemm<BlockQ4>(s, cap, e->cact, e->cact_stride, e->cxn, M, jq, jk, fseg, ep, K, e->st) != cudaSuccess) {
                 return -1;
             }
+            n++;
+        }
+        if (gated) {
+            QkNormArgs qa{};
+            qa.raw = e->cproj, qa.q_norm = L.q_norm, qa.k_norm = L.k_norm;
+            qa.q_out = e->cq, qa.gate_out = e->cmix, qa.kc = kv_k(kv, li), qa.vc = kv_v(kv, li);
+            qa.n_head = P.n_head, qa.n_kv = P.n_kv, qa.hd = hd;
+            qa.n_rot = (c.rope_dim > 0 && c.rope_dim < hd) ? c.rope_dim : hd;
+            qa.theta = c.rope_theta, qa.eps = c.rms_eps, qa.pos = pos0;
+            if (launch_pdl(k_qk_norm_rope_store, dim3(P.n_head + P.n_kv, M), dim3(256), 0, s, qa, (const TokenState*)nullptr) != cudaSuccess) return -1;
             n++;
         }
         // 2. causal attention over the cache (rows of this chunk included)
@@ -1815,8 +1874,15 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
                 n++;
             }
         }
-        // 3. Q8 + o-proj + residual
-        if (project(e->cattn, P.attn_width, nullptr, make_job(L.wo->m, cap), RowJob{}, store_epi(e->cx, K, K, 2)) != cudaSuccess) return -1;
+        if (gated) {
+            const size_t total = (size_t)M * nq;
+            if (launch_pdl(k_gate_rows, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, e->cattn, (const float*)e->cmix, total) != cudaSuccess)
+                return -1;
+            n++;
+        }
+        }
+        // 3. Q8 + output projection + residual
+        if (project(e->cattn, mix_width, nullptr, make_job(wout->m, cap), RowJob{}, store_epi(e->cx, K, K, 2)) != cudaSuccess) return -1;
         // 4. RMSNorm + Q8 + gate/up + SiLU*mul
         ChunkEpi ep{};
         ep.kind = CEPI_SILU;
@@ -1897,7 +1963,7 @@ extern "C" int tfr_forward_greedy(tfr_engine* e, tfr_kv* kv, const uint32_t* tok
     } else if (chunked) {
         for (int i = 0; i < n; i += e->chunk_tokens) {
             const int M = std::min(e->chunk_tokens, n - i);
-            if (forward_chunk(e, kv, e->prompt + i, M, kv->len + i, false) != TFR_OK || (i + M == n && record_head(e, e->cx + (size_t)(M - 1) * e->cfg.n_embd, 0) < 0))
+            if (forward_chunk(e, kv, e->prompt + i, M, kv->len + i, kv->rec_steps + i, false) != TFR_OK || (i + M == n && record_head(e, e->cx + (size_t)(M - 1) * e->cfg.n_embd, 0) < 0))
                 return fail(e, TFR_E_CUDA, "chunk kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         }
         e->launches += 1;
@@ -1938,7 +2004,7 @@ extern "C" int tfr_forward_greedy_all(tfr_engine* e, tfr_kv* kv, const uint32_t*
         CU(e, cudaEventRecord(e->ev0, e->stream));
         for (int i = 0; i < n; i += CHUNK_VERIFY_MAX) {
             const int M = std::min(CHUNK_VERIFY_MAX, n - i);
-            if (forward_chunk(e, kv, e->prompt + i, M, kv->len + i, true) != TFR_OK)
+            if (forward_chunk(e, kv, e->prompt + i, M, kv->len + i, kv->rec_steps + i, true) != TFR_OK)
                 return fail(e, TFR_E_CUDA, "chunk kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
             CU(e, cudaMemcpyAsync(e->out_host + i, e->out_tokens, (size_t)M * 4, cudaMemcpyDeviceToHost, e->stream));
         }
@@ -2169,8 +2235,8 @@ extern "C" int tfr_set_prefill_chunk(tfr_engine* e, int tokens) {
     return TFR_OK;
 }
 // Tokens per chunk in effect: 0 when prompts are fed by decode steps (switched off, or a model the chunk kernels do
-// not cover).
-extern "C" int tfr_prefill_chunk(const tfr_engine* e) { return e && e->finalized && e->chunk_ok ? e->chunk_tokens : 0; }
+// not cover) and, as ever, for hybrid models, whose recurrent layers step through the tokens inside a chunk.
+extern "C" int tfr_prefill_chunk(const tfr_engine* e) { return e && e->finalized && e->chunk_ok && !is_hybrid(e) ? e->chunk_tokens : 0; }
 
 extern "C" int tfr_decode_path(const tfr_engine* e) {
     if (!e) return TFR_E_INVALID;
