@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(ATTC_THREADS) k_attn_chunk_mma(AttnChunkArgs a
     constexpr size_t STAGE_B = 2 * (size_t)ATTM_TK * KROW * 2;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
     const int g = blockIdx.x, rep = a.n_head / a.n_kv, sp = blockIdx.z;
-    const int m_first = blockIdx.y * a.QT, qt = min(a.QT, a.M - m_first);
+    const int m_first = (gridDim.y - 1 - blockIdx.y) * a.QT, qt = min(a.QT, a.M - m_first);  // the tiles that see the most keys start first
     const int n_rows = qt * rep;
     const int T = a.pos0 + m_first + qt;  // keys the tile's last token sees
     const int n_tiles = (T + ATTM_TK - 1) / ATTM_TK, per = (n_tiles + a.S - 1) / a.S;

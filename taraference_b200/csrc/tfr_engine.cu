@@ -307,7 +307,8 @@ static void configure_kernels_once() {
     configure_kernel(k_attn_chunk_mma<128>, true);
     configure_kernel(k_prep_rows, false);
     configure_kernel(k_prep_tc, true);
-    configure_kernel(k_rows_f32, true);
+    configure_kernel(k_rows_f32<4, 4, false>, true);
+    configure_kernel(k_rows_f32<8, 8, true>, true);
     configure_kernel(k_gemm_tc<RawQ4, true, 64, 1>, true);
     configure_kernel(k_gemm_tc<RawQ6, true, 128, 1>, true);
     configure_kernel(k_gemm_tc<RawQ4, false, 32, 1>, true);
@@ -1822,7 +1823,7 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             ep.bias = L.bias_qkv;
             if (tc_qk) {
                 // the fp32-route V rows keep the decode kernels' arithmetic bit for bit
-                if (launch_rows_f32(s, fseg.m, fseg.id_base, e->cxn, M, ep) != cudaSuccess) return -1;
+                if (launch_rows_f32(s, cap, fseg.m, fseg.id_base, e->cxn, M, ep) != cudaSuccess) return -1;
                 n++;
                 if (launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, jq, jk, ep, e->st) != cudaSuccess) return -1;
             } else if (launch_gemm<BlockQ4>(s, cap, e->cact, e->cact_stride, e->cxn, M, jq, jk, fseg, ep, K, e->st) != cudaSuccess) {
@@ -1853,9 +1854,12 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             const bool mma = M >= GEMM_TC_MIN_TOKENS && attn_staged_mma(hd) && !getenv("TFR_ATTN_REGISTER_ROUTE");
             a.QT = mma ? std::max(1, ATTM_ROWS / rep) : M <= CHUNK_VERIFY_MAX ? 1 : std::max(1, ATTC_ROWS_MAX / rep);
             const int q_tiles = (M + a.QT - 1) / a.QT;
-            // key splits: enough CTAs for every SM, never less than 256 keys per split
-            const int blocks256 = (pos0 + M + 255) / 256;
-            a.S = std::max(1, std::min(std::min(CHUNK_ATTN_SPLITS_MAX, blocks256), (2 * cap + P.n_kv * q_tiles - 1) / (P.n_kv * q_tiles)));
+            // key splits.  CUDA cores: two CTAs for every SM, never less than 256 keys per split.  Tensor cores: as many as
+            // fill the SMs once (a CTA has one to itself), down to one 64-key tile each: a tile costs a CTA about 3 us, the
+            // merge of any number of splits 4.
+            const int base = P.n_kv * q_tiles, keys = pos0 + M;
+            a.S = mma ? std::min((keys + ATTM_TK - 1) / ATTM_TK, cap / base) : std::min((keys + 255) / 256, (2 * cap + base - 1) / base);
+            a.S = std::max(1, std::min(a.S, CHUNK_ATTN_SPLITS_MAX));
             a.S = std::max(1, std::min(a.S, (int)(e->cpart_floats / ((size_t)M * P.n_head * (2 + hd)))));
             a.partial = e->cpart;
             const dim3 grid(P.n_kv, q_tiles, a.S);

@@ -227,9 +227,16 @@ __device__ __forceinline__ void tc_ld(float (&v)[W], unsigned addr) {
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
     float2 d;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.ftz.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
         : "=f"(d.x), "=f"(d.y)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.ftz.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return d;
 }
 // Bounded mbarrier wait of a pipeline: once one wait has run out, `dead` lets all others pass at once (the call is then
@@ -391,6 +398,7 @@ struct TcArgs {
     Mat A1, A2;      // ZIP: the pair; otherwise A2 (optional) follows A1 in the grid
     int tiles1;      // row tiles of A1
     int id1, id2, zip, nst;
+    int ahead;       // row tiles between a CTA and the one that takes its place (0: none does)
     ChunkEpi epi;
     TokenState* st;
 };
@@ -433,6 +441,22 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
     // with SUB > 1 one stage holds both
     constexpr int MSTG = SUB > 1 ? 1 : 2;
     const int n_min = Q4 ? tc_min_stages(K) : 0, m0 = n_min * part / S, m1 = n_min * (part + 1) / S;
+    if (warp == 3) {
+        // The tile's weights start towards L2 at once, and so do those of the CTA that will follow on this SM: the registers
+        // of the unpacking warps hold one block ahead, which covers an L2 hit but not a trip to memory.
+        auto ahead = [&](const Mat& m, int group) {
+            if (group * ROW_GROUP >= m.N) return;
+            const size_t f = (size_t)group * ROW_GROUP * nb, t0 = (f + ROW_GROUP * b0) >> 5, t1 = (f + ROW_GROUP * b1 + 31) >> 5;
+            constexpr size_t TB = Q4 ? Q4_TILE_BYTES : Q6_TILE_BYTES;
+            bulk_prefetch_l2(m.data + t0 * TB, (unsigned)((t1 - t0) * TB));
+        };
+        for (int w = 0; w <= 1; w++) {
+            const int row = row0 + w * a.ahead * (a.zip ? 64 : 128);
+            if (w == 1 && a.ahead == 0) break;
+            if (a.zip) ahead(lane & 1 ? a.A2 : A, row / ROW_GROUP + (lane >> 1));
+            else ahead(A, row / ROW_GROUP + lane);
+        }
+    }
     const int min_stages = MSTG * (m1 - m0), stages = min_stages + SPB * (b1 - b0);
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int A_SUB = RAW::PLANES * 16384;            // A of 64 weights: one 16 KB tile per plane
@@ -784,94 +808,148 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
 
 // The Q6_K attn_v rows against the unquantised normalised vectors (kernels/gemv.cu:233-264), bit for bit what the decode
 // kernel computes: a run of 16 products as one chain of multiply-adds, lane l summing runs l, l + 32, ... in order, then
-// the warp's butterfly.  A warp owns four rows and 16 tokens: the weights of two runs per row are unpacked once into
-// registers and serve all tokens, a token's values are read from shared memory once for four rows (the bound: one
-// 16-byte read per 16 multiply-adds), and the 64 sums meet in a halving butterfly, the same tree as warp_sum, which leaves
-// a row pair of one token per lane.
-constexpr int TCV_WARPS = 8, TCV_ROWS = 4, TCV_TOKENS = 16;
+// the warp's butterfly.  A warp unpacks the weights of its rows once, two rows to a packed multiply-add, and walks its
+// tokens; the sums meet in a halving butterfly, the same tree as warp_sum, which leaves one row pair of one token per lane.
+//   staged   more than 16 tokens: eight rows x eight tokens a warp, the warps of a CTA on different rows share the tokens'
+//            vectors in shared memory.  Bound by multiply-adds and the reads that feed them (one 16-byte read per 16 packed
+//            multiply-adds): 256 rows x 2 048 x 2 048 tokens 99 us; 161 with four rows, single multiply-adds and an integer
+//            conversion per weight.
+//   direct   up to 16 tokens: four rows x four tokens a warp, the warps of a CTA on different tokens, vectors straight
+//            from L2: latency is all there is (nine tokens 6.5 us; eight CTAs of a staged form took 21).
+constexpr int TCV_WARPS = 8, TCV_DIRECT_MAX = 16;
 
-// tt: tokens per CTA, as many of the 16 as fit shared memory
+// tt: tokens per CTA (staged: as many of the TOK as fit shared memory)
+template <int ROWS, int TOK, bool STAGED>
 __global__ void __launch_bounds__(TCV_WARPS * 32, 1) k_rows_f32(Mat w, int id_base, const float* xn, int M, int tt, ChunkEpi epi) {
     extern __shared__ __align__(128) unsigned char tcv_smem_raw[];
     float* xs = reinterpret_cast<float*>(tcv_smem_raw);
+    constexpr int U = STAGED ? 1 : 2, RP = ROWS / 2;  // runs per step, row pairs
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = w.K, nb = w.nb, per_row = 16 * nb;
-    const int row0 = (blockIdx.x * TCV_WARPS + warp) * TCV_ROWS, m0 = blockIdx.y * tt, mt = min(tt, M - m0);
+    const int row0 = (STAGED ? blockIdx.x * (blockDim.x >> 5) + warp : blockIdx.x) * ROWS;
+    const int m0 = STAGED ? blockIdx.y * tt : warp * TOK, mt = min(STAGED ? tt : TOK, M - m0);
     const int xf = (int)xs_floats(K);
+    float2 wt[U][RP][16], s[TOK * RP];  // rows 2 r, 2 r + 1; sums [token][row pair]
+    // run 16 of a block's row as in q6k_run_weights_f32: d * scale * (q - 32), four bytes of q at a time
+    auto unpack = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int run = min(i0 + 32 * u, per_row - 1), c = run & 15;
+            const int n = c >> 3, j = (c >> 1) & 3, is = c & 1, nsh = 4 * (j >> 1), hsh = 2 * j;
+#pragma unroll
+            for (int r = 0; r < RP; r++) {
+                unsigned ql[2][4], qh[2][4];
+                float dsc[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const long long f = mat_flat(nb, min(row0 + 2 * r + i, w.N - 1), run >> 4);
+                    const uint8_t* t = w.data + (f >> 5) * Q6_TILE_BYTES;
+                    const uint8_t* p = t + (f & 31) * 16;
+                    const int4 a = __ldg(reinterpret_cast<const int4*>(p + (4 * n + 2 * (j & 1) + is) * 512));
+                    const int4 b = __ldg(reinterpret_cast<const int4*>(p + (8 + 2 * n + is) * 512));
+                    ql[i][0] = a.x, ql[i][1] = a.y, ql[i][2] = a.z, ql[i][3] = a.w;
+                    qh[i][0] = b.x, qh[i][1] = b.y, qh[i][2] = b.z, qh[i][3] = b.w;
+                    const float sc = (float)(int)*reinterpret_cast<const signed char*>(p + 12 * 512 + 8 * n + is + 2 * j);
+                    dsc[i] = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(t + Q6_PIECES * 512 + (f & 31) * 2))) * sc;
+                }
+                const float2 d2 = make_float2(dsc[0], dsc[1]);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    unsigned q[2];
+#pragma unroll
+                    for (int i = 0; i < 2; i++) q[i] = ((ql[i][k] >> nsh) & 0x0f0f0f0fu) | (((qh[i][k] >> hsh) & 0x03030303u) << 4);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        // the byte under the exponent that makes it 2^23 + q, minus 2^23 + 32: exact
+                        const float2 v = make_float2(__uint_as_float(__byte_perm(q[0], 0x4b000000u, 0x7440 + e)) - 8388640.f,
+                                                     __uint_as_float(__byte_perm(q[1], 0x4b000000u, 0x7440 + e)) - 8388640.f);
+                        wt[u][r][4 * k + e] = mul_f32x2(v, d2);
+                    }
+                }
+            }
+        }
+    };
+    unpack(lane);  // weights do not depend on earlier kernels
     griddep_wait();
     griddep_launch_dependents();
-    const int n4 = K >> 2;
-    for (int i = tid; i < mt * n4; i += TCV_WARPS * 32) {
-        const int t = i / n4, i4 = i - t * n4;
-        *reinterpret_cast<float4*>(xs + t * xf + xs_idx(4 * i4)) = reinterpret_cast<const float4*>(xn + (size_t)(m0 + t) * K)[i4];
+    if (STAGED) {
+        const int n4 = K >> 2;
+        for (int t = 0; t < mt; t++)
+            for (int i4 = tid; i4 < n4; i4 += blockDim.x) cp_async16(xs + t * xf + xs_idx(4 * i4), xn + (size_t)(m0 + t) * K + 4 * i4, 16);
+        cp_async_commit();
+        cp_async_wait_all();
+        __syncthreads();
     }
-    __syncthreads();
     if (row0 >= w.N) return;
-    float s[TCV_TOKENS * TCV_ROWS];  // [token][row]
 #pragma unroll
-    for (int i = 0; i < TCV_TOKENS * TCV_ROWS; i++) s[i] = 0.f;
-    for (int i0 = lane; i0 < per_row; i0 += 64) {
-        float wt[TCV_ROWS][2][16];
+    for (int i = 0; i < TOK * RP; i++) s[i] = make_float2(0.f, 0.f);
+    const float2 one = make_float2(1.f, 1.f);
+    for (int i0 = lane; i0 < per_row; i0 += 32 * U) {
+        if (i0 != lane) unpack(i0);
 #pragma unroll
-        for (int r = 0; r < TCV_ROWS; r++)
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int run = min(i0 + 32 * u, per_row - 1);
-                q6k_run_weights_f32(w, mat_flat(nb, min(row0 + r, w.N - 1), run >> 4), run & 15, wt[r][u]);
-            }
-#pragma unroll
-        for (int t = 0; t < TCV_TOKENS; t++) {
+        for (int t = 0; t < TOK; t++) {
             if (t >= mt) break;
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
+            for (int u = 0; u < U; u++) {
                 const int run = i0 + 32 * u;
                 if (run < per_row) {
-                    const float4* x4 = reinterpret_cast<const float4*>(xs + t * xf + xs_idx(16 * run));
-                    float acc[TCV_ROWS] = {0.f, 0.f, 0.f, 0.f};
+                    const float4* x4 = reinterpret_cast<const float4*>(STAGED ? xs + t * xf + xs_idx(16 * run) : xn + (size_t)(m0 + t) * K + 16 * run);
+                    float2 acc[RP];
+#pragma unroll
+                    for (int r = 0; r < RP; r++) acc[r] = make_float2(0.f, 0.f);
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const float4 x = x4[k];
+                        const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-                        for (int r = 0; r < TCV_ROWS; r++) {
-                            acc[r] = fmaf(wt[r][u][4 * k], x.x, acc[r]);
-                            acc[r] = fmaf(wt[r][u][4 * k + 1], x.y, acc[r]);
-                            acc[r] = fmaf(wt[r][u][4 * k + 2], x.z, acc[r]);
-                            acc[r] = fmaf(wt[r][u][4 * k + 3], x.w, acc[r]);
-                        }
+                        for (int e = 0; e < 4; e++)
+#pragma unroll
+                            for (int r = 0; r < RP; r++) acc[r] = fma_f32x2(wt[u][r][4 * k + e], make_float2(xv[e], xv[e]), acc[r]);
                     }
 #pragma unroll
-                    for (int r = 0; r < TCV_ROWS; r++) s[t * TCV_ROWS + r] += acc[r];
+                    for (int r = 0; r < RP; r++) s[t * RP + r] = fma_f32x2(acc[r], one, s[t * RP + r]);
                 }
             }
         }
     }
+    int off = 16;
 #pragma unroll
-    for (int off = 16, n = TCV_TOKENS * TCV_ROWS; off >= 1; off >>= 1, n >>= 1) {
+    for (int n = TOK * RP; n > 1; n >>= 1, off >>= 1) {
         const bool up = (lane & off) != 0;
 #pragma unroll
         for (int i = 0; i < n / 2; i++) {
-            const float send = up ? s[i] : s[i + n / 2];
-            const float keep = up ? s[i + n / 2] : s[i];
-            s[i] = keep + __shfl_xor_sync(TFR_FULL_MASK, send, off);
+            const float2 send = up ? s[i] : s[i + n / 2], keep = up ? s[i + n / 2] : s[i];
+            s[i].x = keep.x + __shfl_xor_sync(TFR_FULL_MASK, send.x, off);
+            s[i].y = keep.y + __shfl_xor_sync(TFR_FULL_MASK, send.y, off);
         }
     }
-    const int t = lane >> 1, row = row0 + 2 * (lane & 1);
-    if (t < mt && row < w.N) ChunkEpiTok{&epi, m0 + t}.apply(id_base + (row >> 1), s[0], s[1]);
+    for (; off > 0; off >>= 1) {
+        s[0].x += __shfl_xor_sync(TFR_FULL_MASK, s[0].x, off);
+        s[0].y += __shfl_xor_sync(TFR_FULL_MASK, s[0].y, off);
+    }
+    constexpr int SHARE = 32 / (TOK * RP);  // lanes with the same sums
+    const int i = lane / SHARE, t = i / RP, row = row0 + 2 * (i % RP);
+    if (lane % SHARE == 0 && t < mt && row < w.N) ChunkEpiTok{&epi, m0 + t}.apply(id_base + (row >> 1), s[0].x, s[0].y);
 }
-inline cudaError_t launch_rows_f32(cudaStream_t stream, const Mat& w, int id_base, const float* xn, int M, const ChunkEpi& epi) {
-    const int rows = TCV_WARPS * TCV_ROWS;
+inline cudaError_t launch_rows_f32(cudaStream_t stream, int sms, const Mat& w, int id_base, const float* xn, int M, const ChunkEpi& epi) {
+    if (M <= TCV_DIRECT_MAX)
+        return launch_pdl(k_rows_f32<4, 4, false>, dim3((w.N + 3) / 4), dim3(32 * ((M + 3) / 4)), 0, stream, w, id_base, xn, M, 4, epi);
     const size_t per = xs_floats(w.K) * sizeof(float);
-    const int tt = std::min(TCV_TOKENS, (int)(GEMV_SMEM_MAX / per));
+    const int tt = std::min(8, (int)(GEMV_SMEM_MAX / per));
     if (tt < 1) return cudaErrorInvalidValue;
-    return launch_pdl(k_rows_f32, dim3((w.N + rows - 1) / rows, (M + tt - 1) / tt), dim3(TCV_WARPS * 32), std::min(tt, M) * per, stream, w, id_base, xn,
-                      M, tt, epi);
+    const int tiles = (M + tt - 1) / tt;
+    int warps = TCV_WARPS;  // fewer per CTA while that brings more SMs to work
+    while (warps > 2 && (w.N + 8 * warps - 1) / (8 * warps) * tiles < sms) warps /= 2;
+    return launch_pdl(k_rows_f32<8, 8, true>, dim3((w.N + 8 * warps - 1) / (8 * warps), tiles), dim3(32 * warps), tt * per, stream, w, id_base, xn, M,
+                      tt, epi);
 }
 
 inline bool tc_type(int type) { return type == TFR_Q4_K || type == TFR_Q6_K; }
 
 template <class RAW, bool PAIR, int NC, int SUB>
-inline cudaError_t launch_tc(cudaStream_t stream, TcArgs& a, int row_tiles, int S) {
+inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_tiles, int S) {
     const int stage = SUB * (RAW::PLANES * 16384 + 2 * (a.NT / (PAIR ? 2 : 1)) * 128);
     a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024) / stage));
+    a.ahead = S == 1 && row_tiles > sms ? sms : 0;
     const size_t sums = S > 1 ? (size_t)a.NT * 512 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(PAIR ? (row_tiles + 1) & ~1 : row_tiles, S, (a.Mp + a.NT - 1) / a.NT);
@@ -922,10 +1000,10 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
     const double single = plan(false, S, a.NT);
     if (M > 128 && plan(true, S2, NT2) < single) {
         a.NT = NT2;
-        return q4 ? launch_tc<RawQ4, true, 64, 1>(stream, a, tiles, S2) : launch_tc<RawQ6, true, 128, 1>(stream, a, tiles, S2);
+        return q4 ? launch_tc<RawQ4, true, 64, 1>(stream, sms, a, tiles, S2) : launch_tc<RawQ6, true, 128, 1>(stream, sms, a, tiles, S2);
     }
-    if (a.NT <= 32) return q4 ? launch_tc<RawQ4, false, 8, 4>(stream, a, tiles, S) : launch_tc<RawQ6, false, 8, 2>(stream, a, tiles, S);
-    return q4 ? launch_tc<RawQ4, false, 32, 1>(stream, a, tiles, S) : launch_tc<RawQ6, false, 32, 1>(stream, a, tiles, S);
+    if (a.NT <= 32) return q4 ? launch_tc<RawQ4, false, 8, 4>(stream, sms, a, tiles, S) : launch_tc<RawQ6, false, 8, 2>(stream, sms, a, tiles, S);
+    return q4 ? launch_tc<RawQ4, false, 32, 1>(stream, sms, a, tiles, S) : launch_tc<RawQ6, false, 32, 1>(stream, sms, a, tiles, S);
 }
 
 }  // namespace tfr
