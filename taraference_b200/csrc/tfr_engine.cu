@@ -309,12 +309,12 @@ static void configure_kernels_once() {
     configure_kernel(k_prep_tc, true);
     configure_kernel(k_rows_f32<4, 4, false>, true);
     configure_kernel(k_rows_f32<8, 8, true>, true);
-    configure_kernel(k_gemm_tc<RawQ4, true, 64, 1>, true);
-    configure_kernel(k_gemm_tc<RawQ6, true, 128, 1>, true);
-    configure_kernel(k_gemm_tc<RawQ4, false, 32, 1>, true);
-    configure_kernel(k_gemm_tc<RawQ4, false, 8, 4>, true);
-    configure_kernel(k_gemm_tc<RawQ6, false, 32, 1>, true);
-    configure_kernel(k_gemm_tc<RawQ6, false, 8, 2>, true);
+    configure_kernel(k_gemm_tc<RawQ4, TC_PAIR>, true);
+    configure_kernel(k_gemm_tc<RawQ6, TC_PAIR>, true);
+    configure_kernel(k_gemm_tc<RawQ4, TC_SINGLE>, true);
+    configure_kernel(k_gemm_tc<RawQ6, TC_SINGLE>, true);
+    configure_kernel(k_gemm_tc<RawQ4, TC_HALF>, true);
+    configure_kernel(k_gemm_tc<RawQ6, TC_HALF>, true);
     configure_kernel(k_attn_chunk_merge, false);
     // the attention kernel also has static shared memory: ask for exactly the dynamic part it uses
     configure_kernel(k_attn_decode<64>, false);

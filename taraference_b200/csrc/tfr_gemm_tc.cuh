@@ -274,15 +274,19 @@ struct RawQ4 {
     static constexpr int WPS = 4, PLANES = 1;
     unsigned s0, s2;  // of the header's three scale words, the two that hold the sub-block scales
     unsigned w[4][WPS];
-    __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
+    // What stage s alone uses; the header with the last one.
+    __device__ __forceinline__ void load_stage(int s, const uint8_t* data, int f, int h) {
         const uint8_t* p = data + (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16;
-        const int4 hdr = ldg_stream(p);
-        s0 = (unsigned)hdr.y, s2 = (unsigned)hdr.w;
-#pragma unroll
-        for (int s = 0; s < 4; s++) {
-            const int4 v = ldg_stream(p + (1 + 2 * s + h) * 512);
-            w[s][0] = v.x, w[s][1] = v.y, w[s][2] = v.z, w[s][3] = v.w;
+        const int4 v = ldg_stream(p + (1 + 2 * s + h) * 512);
+        w[s][0] = v.x, w[s][1] = v.y, w[s][2] = v.z, w[s][3] = v.w;
+        if (s == 3) {
+            const int4 hdr = ldg_stream(p);
+            s0 = (unsigned)hdr.y, s2 = (unsigned)hdr.w;
         }
+    }
+    __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
+#pragma unroll
+        for (int s = 0; s < 4; s++) load_stage(s, data, f, h);
     }
     // 64 weights of stage s: low nibbles = sub-block 2 s, high nibbles = sub-block 2 s + 1 (kernels/common.cu:40-84)
     __device__ __forceinline__ void store(int s, unsigned char* tile, int row, int h, int) const {
@@ -312,16 +316,20 @@ struct RawQ6 {
     static constexpr int WPS = 4, PLANES = 2;
     int4 sc;
     unsigned la[2][WPS], lb[2][WPS], hq[2][WPS];
-    __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
+    // What the stages up to s are the last to use: half n = s >> 1 after its second stage.
+    __device__ __forceinline__ void load_stage(int s, const uint8_t* data, int f, int h) {
+        if (!(s & 1)) return;
         const uint8_t* p = data + (size_t)(f >> 5) * Q6_TILE_BYTES + (f & 31) * 16;
-        sc = ldg_stream(p + 12 * 512);
-#pragma unroll
-        for (int n = 0; n < 2; n++) {
-            const int4 a = ldg_stream(p + (4 * n + h) * 512), b = ldg_stream(p + (4 * n + 2 + h) * 512), c = ldg_stream(p + (8 + 2 * n + h) * 512);
-            la[n][0] = a.x, la[n][1] = a.y, la[n][2] = a.z, la[n][3] = a.w;
-            lb[n][0] = b.x, lb[n][1] = b.y, lb[n][2] = b.z, lb[n][3] = b.w;
-            hq[n][0] = c.x, hq[n][1] = c.y, hq[n][2] = c.z, hq[n][3] = c.w;
-        }
+        const int n = s >> 1;
+        const int4 a = ldg_stream(p + (4 * n + h) * 512), b = ldg_stream(p + (4 * n + 2 + h) * 512), c = ldg_stream(p + (8 + 2 * n + h) * 512);
+        la[n][0] = a.x, la[n][1] = a.y, la[n][2] = a.z, la[n][3] = a.w;
+        lb[n][0] = b.x, lb[n][1] = b.y, lb[n][2] = b.z, lb[n][3] = b.w;
+        hq[n][0] = c.x, hq[n][1] = c.y, hq[n][2] = c.z, hq[n][3] = c.w;
+        if (s == 3) sc = ldg_stream(p + 12 * 512);
+    }
+    __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
+        load_stage(1, data, f, h);
+        load_stage(3, data, f, h);
     }
     // 64 weights of stage s = runs j = 2 (s & 1), + 1 of half n = s >> 1 (kernels/gemv.cu:302-337, as in block_dot):
     // scale * (q - 32) as its f16 rounding and the residual (0 or +-1: |scale * q| <= 4096)
@@ -356,40 +364,47 @@ struct RawQ6 {
 
 // ------------------------------------------------------------------ the kernel
 
-// CTA = 128 weight rows x a tile of tokens x a part of the k range, in stages of SUB x 64 weights: 16 KB of A per 64
-// weights and plane, and the tokens' two planes of B.  Warps 4-11 turn weights into A tiles, lanes of warp 1 request the
-// B planes as bulk copies, lane 0 of warps 0 and 2 issues the MMAs, warps 12-19 drain the accumulators (two buffers in TMEM) into
-// the row sums they hold in registers (TMEM lanes 32 (w & 3) .., one half of the tokens); every role runs ahead of the
-// next as far as the rings allow.  (With all warps doing everything in turn a stage took 4 500 cycles.)  Two forms:
+// CTA = 128 weight rows x a tile of tokens x a part of the k range, in stages of 64 weights: 16 KB of A per plane, and the
+// tokens' two planes of B.  Warps 4-11 turn weights into A tiles, lanes of warp 1 request the B planes as bulk copies, lane
+// 0 of warps 0 and 2 issues the MMAs, the warps behind drain the accumulators (two buffers in TMEM) into the row sums they
+// hold in registers (TMEM lanes 32 (w & 3) .., a share of the tokens); every role runs ahead of the next as far as the
+// rings allow.  (With all warps doing everything in turn a stage took 4 500 cycles.)  Three forms:
 //
 //   pair    batches of more than 128 tokens.  Two CTAs on adjacent row tiles share up to 256 tokens with cta_group::2
 //           MMAs of 256 x 256 x 16: each holds its own rows of A and half of the tokens' B, which halves what B costs in
 //           L2 reads and in shared-memory reads per MMA.  One CTA alone on 2 x 128 rows x 128 tokens ran at a third of it.
-//   single  up to 128 tokens.  The high and the low terms of the tokens are columns of ONE MMA, so A is read once for both;
-//           with up to 32 tokens a stage covers a whole 256-weight block (SUB accumulators side by side), since there a
-//           stage costs its barriers and the MMAs' fixed part, not their columns.
+//   single  up to 128 tokens.  The high and the low terms of the tokens are columns of ONE MMA, so A is read once for both.
+//   half    up to 32 tokens: the same in half an SM.  What a stage costs there is the chain unpack -> MMA -> slot free ->
+//           unpack (about 3 000 cycles, most of it barriers) and a CTA another 9 000 before and after its stages; a second
+//           CTA on the SM, of this or of the next kernel, works through the first one's waits.
 //
 // Gate / up pairs (ZIP) alternate the two matrices' rows in the tile, so that a gate value meets its up value in the
 // neighbouring lane, as the two rows of a RoPE pair do.  The k range is cut over the CTAs of a cluster (grid.y) where a
 // matrix has too few rows to fill the chip: their sums meet through distributed shared memory, each CTA finishing its
 // share of the tokens.
 constexpr int TC_C_WARPS = 4, TC_A_WARPS = 8, TC_MAX_STAGES = 6;
-constexpr size_t TC_SMEM_MAX = 225 * 1024;
+constexpr size_t TC_SMEM_MAX = 225 * 1024, TC_SMEM_HALF = 111 * 1024;
+enum { TC_PAIR, TC_SINGLE, TC_HALF };
 // Draining warps and the registers of a thread of each role (what they add up to is what the launch has).  Draining is a
 // chain of TMEM loads (300 cycles for 16 columns, waited for one by one), so sixteen warps share the columns; the pairs on
 // Q6_K matrices, whose third MMA leaves more time, keep eight and leave the registers to the unpacking.
-template <bool PAIR, bool Q4>
+template <int FORM, bool Q4>
 struct TcRoles {
-    static constexpr int D_WARPS = PAIR && !Q4 ? 8 : 16, THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + D_WARPS);
-    static constexpr int LAUNCH_REGS = D_WARPS == 8 ? 96 : 72;
-    static constexpr int C_REGS = D_WARPS == 8 ? 32 : 24, A_REGS = D_WARPS == 8 ? 64 : PAIR ? 48 : 72, D_REGS = D_WARPS == 8 ? 160 : PAIR ? 96 : 80;
-    static_assert(32 * (TC_C_WARPS * C_REGS + TC_A_WARPS * A_REGS + D_WARPS * D_REGS) <= THREADS * LAUNCH_REGS && THREADS * LAUNCH_REGS <= 65536,
+    static constexpr int D_WARPS = FORM == TC_HALF ? 4 : FORM == TC_PAIR && !Q4 ? 8 : 16, THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + D_WARPS);
+    static constexpr int CTAS = FORM == TC_HALF ? 2 : 1, LAUNCH_REGS = FORM == TC_HALF ? 64 : D_WARPS == 8 ? 96 : 72;
+    static constexpr int C_REGS = D_WARPS == 8 ? 32 : 24, A_REGS = D_WARPS == 8 ? 64 : FORM == TC_PAIR ? 48 : 72,
+                         D_REGS = FORM == TC_HALF ? 88 : D_WARPS == 8 ? 160 : FORM == TC_PAIR ? 96 : 80;
+    static constexpr int NC = FORM == TC_PAIR ? 1024 / D_WARPS : 32;  // tokens of a draining warp
+    static_assert(32 * (TC_C_WARPS * C_REGS + TC_A_WARPS * A_REGS + D_WARPS * D_REGS) <= THREADS * LAUNCH_REGS && CTAS * THREADS * LAUNCH_REGS <= 65536,
                   "more registers than the launch has");
 };
-template <int N>
-__device__ __forceinline__ void tc_regs_less() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void tc_regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+// Registers of a role: N of the LAUNCH a thread has.  Fewer must be given back, more asked for.
+template <int N, int LAUNCH>
+__device__ __forceinline__ void tc_regs() {
+    static_assert(N % 8 == 0, "");
+    if constexpr (N < LAUNCH) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+    else if constexpr (N > LAUNCH) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
 
 struct TcArgs {
     const unsigned char* image;
@@ -412,18 +427,18 @@ struct TcRing {
     }
 };
 
-template <class RAW, bool PAIR, int NC, int SUB>
-__global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k_gemm_tc(const TcArgs a) {
-    constexpr bool Q4 = RAW::PLANES == 1;
-    using Roles = TcRoles<PAIR, Q4>;
-    constexpr int TC_D_WARPS = Roles::D_WARPS, CGS = TC_D_WARPS / 4;  // column groups of NC tokens
-    constexpr int CG = PAIR ? 2 : 1, SPB = 4 / SUB;  // CTAs of an MMA; stages of a 256-weight block
-    constexpr int DR = PAIR ? 2 : 1;                 // stages an accumulator runs over
-    static_assert(!PAIR || SUB == 1, "pairs take 64 weights a stage");
+template <class RAW, int FORM>
+__global__ void __launch_bounds__(TcRoles<FORM, RAW::PLANES == 1>::THREADS, TcRoles<FORM, RAW::PLANES == 1>::CTAS) k_gemm_tc(const TcArgs a) {
+    constexpr bool Q4 = RAW::PLANES == 1, PAIR = FORM == TC_PAIR;
+    using Roles = TcRoles<FORM, Q4>;
+    constexpr int TC_D_WARPS = Roles::D_WARPS, CGS = TC_D_WARPS / 4, NC = Roles::NC;  // column groups of NC tokens
+    constexpr int CG = PAIR ? 2 : 1;  // CTAs of an MMA
+    constexpr int DR = PAIR ? 2 : 1;  // stages an accumulator runs over
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
     __shared__ unsigned long long full[TC_MAX_STAGES], empty[TC_MAX_STAGES], accfull[2], accempty[2];
     __shared__ unsigned tmem_slot;
     __shared__ int dead_s;
+    __shared__ float tscale_s[PAIR ? 256 : 128];
     volatile int* dead = &dead_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = gridDim.y, part = blockIdx.y;           // k parts
@@ -437,9 +452,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
     const int nb = A.nb, K = A.K, N = A.N;
     const int row0 = ((int)blockIdx.x - (second ? a.tiles1 : 0)) * (a.zip ? 64 : 128);
     const int b0 = nb * part / S, b1 = nb * (part + 1) / S;
-    // stages of group sums come in two: the high terms of dmin * m with both of the sums' terms, its low terms with the high ones;
-    // with SUB > 1 one stage holds both
-    constexpr int MSTG = SUB > 1 ? 1 : 2;
+    // stages of group sums come in two: the high terms of dmin * m with both of the sums' terms, its low terms with the high ones
     const int n_min = Q4 ? tc_min_stages(K) : 0, m0 = n_min * part / S, m1 = n_min * (part + 1) / S;
     if (warp == 3) {
         // The tile's weights start towards L2 at once, and so do those of the CTA that will follow on this SM: the registers
@@ -457,12 +470,11 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
             else ahead(A, row / ROW_GROUP + lane);
         }
     }
-    const int min_stages = MSTG * (m1 - m0), stages = min_stages + SPB * (b1 - b0);
+    const int min_stages = 2 * (m1 - m0), stages = min_stages + 4 * (b1 - b0);
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int A_SUB = RAW::PLANES * 16384;            // A of 64 weights: one 16 KB tile per plane
-    const int b_plane = ntc * 128, b_sub = 2 * b_plane, stage_bytes = SUB * (A_SUB + 2 * (a.NT / CG) * 128);
-    constexpr int SUB_COLS = (PAIR ? 1 : 2) * CGS * NC;   // columns of one accumulator: the tokens, single: high then low terms
-    constexpr unsigned ACC_COLS = SUB * SUB_COLS, TMEM_COLS = 2 * ACC_COLS;
+    const int b_plane = ntc * 128, stage_bytes = A_SUB + 2 * (a.NT / CG) * 128;
+    constexpr unsigned ACC_COLS = (PAIR ? 1 : 2) * CGS * NC, TMEM_COLS = 2 * ACC_COLS;  // the tokens; single, half: high then low terms
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
             // every CTA's own A warps and B (with the bytes); the leader's also the word that the peer's are complete
@@ -485,7 +497,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
     float* sums = reinterpret_cast<float*>(smem);  // S > 1: [token][128 rows], over the stages once every MMA has read them
 
     if (warp < TC_C_WARPS) {
-        tc_regs_less<Roles::C_REGS>();
+        tc_regs<Roles::C_REGS, Roles::LAUNCH_REGS>();
         if ((warp & 1) == 0 && pr == 0) {
             // Two issuing threads take turns by accumulator: a wait costs one about 300 cycles even when there is nothing to
             // wait for, and the MMAs of a stage 650.
@@ -501,51 +513,45 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
                     const bool fresh = j % DR == 0;
                     if (fresh && r >= 2) tc_wait<PAIR>(accempty + buf, ((r >> 1) - 1) & 1, dead);
                     tc_wait<PAIR>(full + ring.slot, ring.lap, dead);
+                    // what the unpacking warps stored becomes visible to the tensor core here, not where they store it: a
+                    // fence there waits for the warp's loads in flight, the next block's words (900 to 2 200 cycles a block)
+                    fence_proxy_async();
                     tc_fence_after();
                     const unsigned acc = tmem + buf * ACC_COLS;
-                    const unsigned long long da = d0 + ((ring.slot * stage_bytes) >> 4), db = da + (SUB * A_SUB >> 4);
+                    const unsigned long long da = d0 + ((ring.slot * stage_bytes) >> 4), db = da + (A_SUB >> 4);
                     if (Q4 && j < min_stages) {
                         const unsigned id = tc_idesc(2, 128 * CG, nt), id2 = tc_idesc(2, 128, 2 * nt);
+                        const bool high = !(j & 1);
+                        if (!PAIR && high) {
 #pragma unroll
-                        for (int u = 0; u < (SUB > 1 ? 2 : 1); u++) {
-                            const bool high = SUB > 1 ? u == 0 : !(j & 1);
-                            const unsigned long long dau = da + (u * A_SUB >> 4), dbu = db + (u * b_sub >> 4);
-                            if (!PAIR && high) {
+                            for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, da + 2 * kk, db + 2 * kk, id2, !fresh || kk > 0);
+                        } else {
+                            // the small products go first: the tensor core truncates as it adds, so what counts is how
+                            // often it adds to the full sum
+                            if (PAIR && high)
 #pragma unroll
-                                for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc + u * SUB_COLS, dau + 2 * kk, dbu + 2 * kk, id2, !fresh || kk > 0);
-                            } else {
-                                // the small products go first: the tensor core truncates as it adds, so what counts is how
-                                // often it adds to the full sum
-                                if (PAIR && high)
+                                for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, da + 2 * kk, db + (b_plane >> 4) + 2 * kk, id, !fresh || kk > 0);
 #pragma unroll
-                                    for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, dau + 2 * kk, dbu + (b_plane >> 4) + 2 * kk, id, !fresh || kk > 0);
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc + u * SUB_COLS, dau + 2 * kk, dbu + 2 * kk, id, !fresh || (PAIR && high) || kk > 0);
-                            }
+                            for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, da + 2 * kk, db + 2 * kk, id, !fresh || (PAIR && high) || kk > 0);
                         }
                     } else {
                         const unsigned id = tc_idesc(0, 128 * CG, nt), id2 = tc_idesc(0, 128, 2 * nt);
+                        if (PAIR) {
 #pragma unroll
-                        for (int u = 0; u < SUB; u++) {
-                            const unsigned accu = acc + u * SUB_COLS;
-                            const unsigned long long dau = da + (u * A_SUB >> 4), dbu = db + (u * b_sub >> 4);
-                            if (PAIR) {
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk++) {
-                                    tc_mma<false, CG>(accu, dau + 2 * kk, dbu + (b_plane >> 4) + 2 * kk, id, !fresh || kk > 0);
-                                    if (!Q4) tc_mma<false, CG>(accu, dau + 1024 + 2 * kk, dbu + 2 * kk, id, 1);
-                                }
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(accu, dau + 2 * kk, dbu + 2 * kk, id, 1);
-                            } else {
-                                // Q6_K: the residuals of A touch the high columns alone and go first as well
-                                if (!Q4) {
-#pragma unroll
-                                    for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(accu, dau + 1024 + 2 * kk, dbu + 2 * kk, id2, !fresh || kk > 0);
-                                }
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(accu, dau + 2 * kk, dbu + 2 * kk, id2, !Q4 || !fresh || kk > 0);
+                            for (int kk = 0; kk < 4; kk++) {
+                                tc_mma<false, CG>(acc, da + 2 * kk, db + (b_plane >> 4) + 2 * kk, id, !fresh || kk > 0);
+                                if (!Q4) tc_mma<false, CG>(acc, da + 1024 + 2 * kk, db + 2 * kk, id, 1);
                             }
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(acc, da + 2 * kk, db + 2 * kk, id, 1);
+                        } else {
+                            // Q6_K: the residuals of A touch the high columns alone and go first as well
+                            if (!Q4) {
+#pragma unroll
+                                for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(acc, da + 1024 + 2 * kk, db + 2 * kk, id2, !fresh || kk > 0);
+                            }
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(acc, da + 2 * kk, db + 2 * kk, id2, !Q4 || !fresh || kk > 0);
                         }
                     }
                     tc_commit<CG>(empty + ring.slot, lead);
@@ -562,6 +568,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
                 if (warp == 0)
                     for (int j = 0; j < stages; j++) {
                         tc_wait<false>(full + ring.slot, ring.lap, dead);
+                        fence_proxy_async();
                         tc_arrive_at(full + ring.slot, lead);
                         ring.next(nst);
                     }
@@ -579,15 +586,14 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
             const unsigned char* src = a.image + (size_t)nc0 * 128 + (lane & 1) * plane;
             for (int j = 0; j < stages; j++) {
                 const bool mins = j < min_stages;
-                // a lane per plane and 64 weights; the low terms of dmin * m meet the high plane alone
-                const int image_stage = mins ? K / TC_STAGE_K + m0 + (SUB > 1 ? j : j >> 1) : 4 * b0 + (j - min_stages) * SUB + (lane >> 1);
-                const bool both = !mins || (SUB == 1 && !(j & 1));
-                const int copies = mins && SUB > 1 ? 3 : both ? 2 * SUB : 1;
+                // a lane per plane; the low terms of dmin * m meet the high plane alone
+                const int image_stage = mins ? K / TC_STAGE_K + m0 + (j >> 1) : 4 * b0 + (j - min_stages);
+                const int copies = mins && (j & 1) ? 1 : 2;
                 if (j >= nst) tc_wait<false>(empty + ring.slot, ring.lap ^ 1, dead);
                 if (lane == 0) mbar_expect_tx(full + ring.slot, copies * b_plane);
                 __syncwarp();
                 if (lane < copies)
-                    bulk_load(smem + ring.slot * stage_bytes + SUB * A_SUB + lane * b_plane, src + (size_t)2 * image_stage * plane, b_plane, full + ring.slot);
+                    bulk_load(smem + ring.slot * stage_bytes + A_SUB + lane * b_plane, src + (size_t)2 * image_stage * plane, b_plane, full + ring.slot);
                 __syncwarp();
                 ring.next(nst);
             }
@@ -602,7 +608,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
     }
 
     if (warp < TC_C_WARPS + TC_A_WARPS) {
-        tc_regs_less<Roles::A_REGS>();
+        tc_regs<Roles::A_REGS, Roles::LAUNCH_REGS>();
         // this thread's row of the tile and its half of the row's blocks; rows past the matrix repeat its last row
         const int wa = warp - TC_C_WARPS, row_l = (wa & 3) * 32 + lane, h = wa >> 2;
         const uint8_t* wdata = (a.zip && (row_l & 1)) ? a.A2.data : A.data;
@@ -617,7 +623,6 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
             return smem + ring.slot * stage_bytes;
         };
         auto publish = [&]() {
-            fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(full + ring.slot);
             ring.next(nst);
@@ -629,7 +634,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
                 unsigned char* t = nullptr;
 #pragma unroll 1
                 for (int p = 0; p < 2; p++) {
-                    if (SUB == 1 || p == 0) t = acquire();
+                    t = acquire();
 #pragma unroll 1
                     for (int i = 0; i < 2; i++) {
                         const int b = 4 * c + 2 * h + i, f = f0 + ROW_GROUP * min(b, nb - 1);
@@ -647,10 +652,10 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
                                 const unsigned top = __float_as_uint(v) & 0xffffe000u;
                                 o[k] = p ? __float_as_uint(v - __uint_as_float(top)) : top;
                             }
-                            *reinterpret_cast<uint4*>(t + (SUB > 1 ? p * A_SUB : 0) + tc_swz(row_l, 2 * (2 * h + i) + half)) = make_uint4(o[0], o[1], o[2], o[3]);
+                            *reinterpret_cast<uint4*>(t + tc_swz(row_l, 2 * (2 * h + i) + half)) = make_uint4(o[0], o[1], o[2], o[3]);
                         }
                     }
-                    if (SUB == 1 || p == 1) publish();
+                    publish();
                 }
             }
         }
@@ -658,10 +663,10 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
             unsigned char* t = nullptr;
 #pragma unroll
             for (int s = 0; s < 4; s++) {
-                if (s % SUB == 0) t = acquire();
-                raw.store(s, t + (s % SUB) * A_SUB, row_l, h, 16384);
-                if (s == 3 && b + 1 < b1) raw.load(wdata, f0 + ROW_GROUP * (b + 1), h);  // arrives under the waits of the next stages
-                if (s % SUB == SUB - 1) publish();
+                t = acquire();
+                raw.store(s, t, row_l, h, 16384);
+                publish();
+                if (b + 1 < b1) raw.load_stage(s, wdata, f0 + ROW_GROUP * (b + 1), h);  // the words just used, of the next block
             }
         }
         if (S > 1) cluster_sync_all();
@@ -669,7 +674,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
         return;
     }
 
-    tc_regs_more<Roles::D_REGS>();
+    tc_regs<Roles::D_REGS, Roles::LAUNCH_REGS>();
     const int quad = warp & 3, cg = (warp - TC_C_WARPS - TC_A_WARPS) >> 2, row_d = quad * 32 + lane;
     float2 tot[NC / 2];  // token pairs: one packed multiply-add joins two accumulators to their sums
 #pragma unroll
@@ -685,41 +690,40 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
         };
         float dnext = load_d(b0), dcur = -1.f;
         griddep_launch_dependents();
+        griddep_wait();  // nothing reaches an accumulator before the image is complete; token scales and residuals are then, too
+        const int td = tid - 32 * (TC_C_WARPS + TC_A_WARPS);
+        if (td < nt) tscale_s[td] = n0 + td < a.M ? a.tscale[n0 + td] : 0.f;
         const int min_rounds = min_stages / DR;
         int left = min_rounds;  // rounds until the factor changes
         for (int r = 0; r < stages / DR; r++) {
             const bool minus = Q4 && r < min_rounds;
             if (left == 0) {
                 dcur = dnext;
-                dnext = load_d(b0 + (r - min_rounds) / (SPB / DR) + 1);
-                left = SPB / DR;
+                dnext = load_d(b0 + (r - min_rounds) / (4 / DR) + 1);
+                left = 4 / DR;
             }
             left--;
             const int buf = r & 1;
             tc_wait<false>(accfull + buf, (r >> 1) & 1, dead);
             tc_fence_after();
             const unsigned at = tmem + ((unsigned)quad << 21) + buf * ACC_COLS + cg * NC;
+            // The truncations cost an accumulator, on average, about half (Q4_K) or three quarters (Q6_K) of a unit in its
+            // last place (measured against float64); raising the factor by one unit in as many stages gives it back.
+            const float f = (r & 3) < (Q4 ? 2 : 3) ? dcur * 1.00000012f : dcur;
+            const float2 ff = make_float2(f, f);
+            const bool low = !PAIR && !(minus && (r & 1));  // there are low columns
 #pragma unroll
-            for (int u = 0; u < SUB; u++) {
-                if (cg * NC >= nt || (minus && u > 1)) break;
-                // The truncations cost an accumulator, on average, about half (Q4_K) or three quarters (Q6_K) of a unit in its
-                // last place (measured against float64); raising the factor by one unit in as many stages gives it back.
-                const float f = ((r * SUB + u) & 3) < (Q4 ? 2 : 3) ? dcur * 1.00000012f : dcur;
-                const float2 ff = make_float2(f, f);
-                const bool low = !PAIR && !(minus && (SUB > 1 ? u == 1 : (r & 1)));  // there are low columns
-                constexpr int W = NC < 16 ? NC : 16;  // columns of a load
+            for (int c = 0; c < NC; c += 16) {  // columns of a load
+                if (cg * NC + c >= nt) break;
+                float v[16], w[16];
+                tc_ld<16>(v, at + c);
+                if (low) tc_ld<16>(w, at + nt + c);
+                tc_ld_wait();
 #pragma unroll
-                for (int c = 0; c < NC; c += W) {
-                    float v[W], w[W];
-                    tc_ld<W>(v, at + u * SUB_COLS + c);
-                    if (low) tc_ld<W>(w, at + u * SUB_COLS + nt + c);
-                    tc_ld_wait();
+                for (int i = 0; i < 8; i++) tot[c / 2 + i] = fma_f32x2(ff, make_float2(v[2 * i], v[2 * i + 1]), tot[c / 2 + i]);
+                if (low) {
 #pragma unroll
-                    for (int i = 0; i < W / 2; i++) tot[c / 2 + i] = fma_f32x2(ff, make_float2(v[2 * i], v[2 * i + 1]), tot[c / 2 + i]);
-                    if (low) {
-#pragma unroll
-                        for (int i = 0; i < W / 2; i++) tot[c / 2 + i] = fma_f32x2(ff, make_float2(w[2 * i], w[2 * i + 1]), tot[c / 2 + i]);
-                    }
+                    for (int i = 0; i < 8; i++) tot[c / 2 + i] = fma_f32x2(ff, make_float2(w[2 * i], w[2 * i + 1]), tot[c / 2 + i]);
                 }
             }
             tc_fence_before();
@@ -728,7 +732,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
         }
     }
     if (!cluster) asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");
-    griddep_wait();  // residuals and token scales come from earlier kernels
+    else asm volatile("bar.sync 1, %0;" ::"n"(32 * TC_D_WARPS) : "memory");  // the token scales
 
     // ---- epilogue
     auto total = [&](int i) { return (i & 1) ? tot[i >> 1].y : tot[i >> 1].x; };
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const bool on = i0 + i < tn;
-                    ts[i] = on ? a.tscale[t0 + i0 + i] : 0.f;
+                    ts[i] = on ? tscale_s[cg * NC + i0 + i] : 0.f;
                     res[i] = on && store && epi.use_res == 2 && row < N ? epi.out[(size_t)(t0 + i0 + i) * epi.ldo + 2 * id_base + row] : 0.f;
                 }
 #pragma unroll
@@ -781,22 +785,43 @@ __global__ void __launch_bounds__(TcRoles<PAIR, RAW::PLANES == 1>::THREADS, 1) k
         }
         cluster_sync_all();
         const int per = (nt + S - 1) / S, c0 = part * per, cn = min(per, min(nt, a.M - n0) - c0);
-        for (int c = c0 + cg; c < c0 + cn; c += CGS) {
-            float v = 0.f;
-            const unsigned at0 = smem_u32(sums + c * 128 + row_d);
-            for (int s = 0; s < S; s++) {
-                unsigned remote;
-                float x;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at0), "r"(PAIR ? 2 * s + pr : s));
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
-                v += x;
+        for (int c4 = c0 + cg; c4 < c0 + cn; c4 += 4 * CGS) {
+            // four tokens' residuals and the parts' sums in flight together
+            float res[4], v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int c = c4 + q * CGS;
+                res[q] = c < c0 + cn && store && epi.use_res == 2 && row < N ? epi.out[(size_t)(n0 + c) * epi.ldo + 2 * id_base + row] : 0.f;
             }
-            v = v * a.tscale[n0 + c] + bias;
-            if (store) {
-                if (row < N) ChunkEpiTok{&epi, n0 + c}.store_one(2 * id_base + row, v);
-            } else {
-                const float got = __shfl_xor_sync(TFR_FULL_MASK, v, 1);
-                if (!odd && item_on) ChunkEpiTok{&epi, n0 + c}.apply(item, v, got);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int c = min(c4 + q * CGS, c0 + cn - 1);
+                const unsigned at0 = smem_u32(sums + c * 128 + row_d);
+                float x[8];
+#pragma unroll
+                for (int p = 0; p < 8; p++) {
+                    x[p] = 0.f;
+                    if (p < S) {
+                        unsigned remote;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at0), "r"(PAIR ? 2 * p + pr : p));
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x[p]) : "r"(remote) : "memory");
+                    }
+                }
+                v[q] = 0.f;
+#pragma unroll
+                for (int p = 0; p < 8; p++) v[q] += x[p];
+                v[q] = v[q] * tscale_s[c] + res[q] + bias;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int c = c4 + q * CGS;
+                if (c >= c0 + cn) break;
+                if (store) {
+                    if (row < N) epi.out[(size_t)(n0 + c) * epi.ldo + 2 * id_base + row] = v[q];
+                } else {
+                    const float got = __shfl_xor_sync(TFR_FULL_MASK, v[q], 1);
+                    if (!odd && item_on) ChunkEpiTok{&epi, n0 + c}.apply(item, v[q], got);
+                }
             }
         }
     }
@@ -945,15 +970,17 @@ inline cudaError_t launch_rows_f32(cudaStream_t stream, int sms, const Mat& w, i
 
 inline bool tc_type(int type) { return type == TFR_Q4_K || type == TFR_Q6_K; }
 
-template <class RAW, bool PAIR, int NC, int SUB>
+template <class RAW, int FORM>
 inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_tiles, int S) {
-    const int stage = SUB * (RAW::PLANES * 16384 + 2 * (a.NT / (PAIR ? 2 : 1)) * 128);
-    a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024) / stage));
-    a.ahead = S == 1 && row_tiles > sms ? sms : 0;
+    using Roles = TcRoles<FORM, RAW::PLANES == 1>;
+    constexpr bool PAIR = FORM == TC_PAIR;
+    const int stage = RAW::PLANES * 16384 + 2 * (a.NT / (PAIR ? 2 : 1)) * 128;
+    a.nst = std::min(TC_MAX_STAGES, (int)(((FORM == TC_HALF ? TC_SMEM_HALF : TC_SMEM_MAX) - 1024) / stage));
+    a.ahead = S == 1 && row_tiles > sms * Roles::CTAS ? sms * Roles::CTAS : 0;
     const size_t sums = S > 1 ? (size_t)a.NT * 512 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(PAIR ? (row_tiles + 1) & ~1 : row_tiles, S, (a.Mp + a.NT - 1) / a.NT);
-    cfg.blockDim = dim3(TcRoles<PAIR, RAW::PLANES == 1>::THREADS);
+    cfg.blockDim = dim3(Roles::THREADS);
     cfg.dynamicSmemBytes = std::max((size_t)a.nst * stage, sums) + 1024;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -965,7 +992,7 @@ inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_ti
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = PAIR || S > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_gemm_tc<RAW, PAIR, NC, SUB>, (const TcArgs)a);
+    return cudaLaunchKernelEx(&cfg, k_gemm_tc<RAW, FORM>, (const TcArgs)a);
 }
 
 // out = epilogue(W x) for the M tokens of an operand image; jb: the second matrix of a gate/up pair or one that follows.
@@ -984,12 +1011,13 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
     auto fit = [&](int ctas) { return ctas <= 2 ? sms : ctas == 4 ? 132 : 112; };
     // the form and the number of k parts with the shortest longest chain: waves of CTAs x stages x what a stage takes, in
     // units of a 128-row, 128-token MMA stage
-    auto plan = [&](bool pair, int& S, int& NT) {
-        const int most = pair ? 256 : 128, tok_tiles = (a.Mp + most - 1) / most, unit = pair ? 32 : 16;
+    auto plan = [&](int form, int& S, int& NT) {
+        const bool pair = form == TC_PAIR;
+        const int most = pair ? 256 : form == TC_HALF ? 32 : 128, tok_tiles = (a.Mp + most - 1) / most, unit = pair ? 32 : 16;
         NT = ((a.Mp + tok_tiles - 1) / tok_tiles + unit - 1) / unit * unit;
         double best = 1e30;
         for (int s = 1; s <= (pair ? 4 : 8) && s <= ja.m.nb; s *= 2) {
-            const int ctas = (pair ? (tiles + 1) & ~1 : tiles) * tok_tiles * s, at_once = fit(pair ? 2 * s : s);
+            const int ctas = (pair ? (tiles + 1) & ~1 : tiles) * tok_tiles * s, at_once = fit(pair ? 2 * s : s) * (form == TC_HALF ? 2 : 1);
             const double stage = pair ? 0.4 + 1.2 * NT / 128 : 0.6 + 1.2 * NT / 128;
             const double t = (double)((ctas + at_once - 1) / at_once) * ((4.5 * ((ja.m.nb + s - 1) / s) * stage) + 6 + (s > 1 ? 3 : 0));
             if (t < best) best = t, S = s;
@@ -997,13 +1025,16 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
         return best;
     };
     int S = 1, S2 = 1, NT2 = 0;
-    const double single = plan(false, S, a.NT);
-    if (M > 128 && plan(true, S2, NT2) < single) {
-        a.NT = NT2;
-        return q4 ? launch_tc<RawQ4, true, 64, 1>(stream, sms, a, tiles, S2) : launch_tc<RawQ6, true, 128, 1>(stream, sms, a, tiles, S2);
+    if (M <= 32) {
+        plan(TC_HALF, S, a.NT);
+        return q4 ? launch_tc<RawQ4, TC_HALF>(stream, sms, a, tiles, S) : launch_tc<RawQ6, TC_HALF>(stream, sms, a, tiles, S);
     }
-    if (a.NT <= 32) return q4 ? launch_tc<RawQ4, false, 8, 4>(stream, sms, a, tiles, S) : launch_tc<RawQ6, false, 8, 2>(stream, sms, a, tiles, S);
-    return q4 ? launch_tc<RawQ4, false, 32, 1>(stream, sms, a, tiles, S) : launch_tc<RawQ6, false, 32, 1>(stream, sms, a, tiles, S);
+    const double single = plan(TC_SINGLE, S, a.NT);
+    if (M > 128 && plan(TC_PAIR, S2, NT2) < single) {
+        a.NT = NT2;
+        return q4 ? launch_tc<RawQ4, TC_PAIR>(stream, sms, a, tiles, S2) : launch_tc<RawQ6, TC_PAIR>(stream, sms, a, tiles, S2);
+    }
+    return q4 ? launch_tc<RawQ4, TC_SINGLE>(stream, sms, a, tiles, S) : launch_tc<RawQ6, TC_SINGLE>(stream, sms, a, tiles, S);
 }
 
 }  // namespace tfr
