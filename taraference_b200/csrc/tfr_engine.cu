@@ -281,17 +281,27 @@ static void configure_kernels_once() {
     const int dev = current_device_slot();
     if (done[dev]) return;
     done[dev] = true;
-    configure_kernel(k_gemv<BlockQ4, EpiQkv>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiStore>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiStore>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiSilu>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiStore>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiLogits>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiAllReduce>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiAllReduce>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiAllReduce>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiLogits>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiLogits>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiLogits, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiAllReduce, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiAllReduce, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiAllReduce, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiLogits, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiLogits, GEMV_THREADS>, true);
 #ifdef TFR_TEST_AIDS
     configure_kernel(k_int_dots<BlockQ8>, true);
     configure_kernel(k_int_dots<BlockQ4>, true);

@@ -13,6 +13,7 @@ namespace tfr {
 
 // y = W x (+y) (+bias): kernels/gemv.cu:367-373 residual rule (2 = accumulate in place).
 struct EpiStore {
+    static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_PAIRS;
     float* out;
     const float* bias;
@@ -43,6 +44,7 @@ struct EpiStore {
 
 // h = silu(gate.x) * (up.x), kernels/gemv.cu:2570-2574.  Pair p = (gate row p, up row p).
 struct EpiSilu {
+    static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_ZIP;
     float* out;
     __device__ __forceinline__ bool wants_residual() const { return false; }
@@ -59,6 +61,7 @@ struct EpiSilu {
 // (kernels/ops.cu:471-486).  Q and K rows were re-ordered at upload so that the RoPE
 // partners (i, i + hd/2) of a head are the two rows of a pair; biases likewise.
 struct EpiQkv {
+    static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_PAIRS;
     float* q_out;            // [n_head * hd] natural order
     unsigned short* kc;      // layer base [max_seq][kvdim]; with a TokenState: its cache + kv_off
@@ -135,6 +138,7 @@ __device__ __forceinline__ void advance_state(TokenState* st, int tok, int* out_
 }
 
 struct EpiLogits {
+    static constexpr bool SHARES_SM = false;
     static constexpr int MODE = EPI_PAIRS;
     float* logits;
     int* out_tokens;   // ring of emitted tokens, indexed by TokenState::step
@@ -252,9 +256,18 @@ struct F32Seg {
 // its weight tiles, then sleeps in griddepcontrol.wait until the previous kernel's results are
 // complete, so launch latency and the first tiles' fetch hide behind the predecessor's tail.
 constexpr size_t GEMV_SMEM_MAX = 225 * 1024;  // opt-in limit is 227 KB including the kernels' small static arrays
+// Threads of a CTA.  1 024 fill the register file: the next kernel's CTAs then start when this one's have left, and its
+// prologue (1.3 us) and the first trip of its weights to memory are in nobody's shadow.  Two smaller sizes share an SM:
+//   GEMV_SMALL   matrices of a few tiles per CTA (QKV, o-proj): a warp per tile is all they can use;
+//   GEMV_MID     larger ones whose tiles all fit beside a small CTA's: 24 warps take the same two rounds over a gate/up
+//                CTA's 38 tiles as 32 do.
+// With 56 registers a thread the two together have the SM's 65 536.
+constexpr int GEMV_SMALL = 384, GEMV_MID = 768;
+__host__ __device__ constexpr int gemv_regs(int threads) { return threads == GEMV_THREADS ? 64 : 56; }
+constexpr size_t GEMV_SMALL_SMEM = 60 * 1024, GEMV_MID_SMEM = 198 * 1024;
 constexpr int GEMV_L2_AHEAD = 4;  // tiles per warp requested into L2 beyond the one in its ring slot
-inline size_t gemv_smem_fixed(int K, bool with_xf, bool has_norm, int pbuf_floats) {
-    size_t act_bytes = (act_smem_bytes(K, with_xf, has_norm) + 15) & ~(size_t)15;
+inline size_t gemv_smem_fixed(int K, bool with_xf, int pbuf_floats) {
+    size_t act_bytes = (act_smem_bytes(K, with_xf, false) + 15) & ~(size_t)15;
     return act_bytes + (size_t)pbuf_floats * sizeof(float) + 272 * sizeof(float);
 }
 inline int gemv_pbuf_floats(int rows_a, int rows_b, int nb) {
@@ -263,13 +276,13 @@ inline int gemv_pbuf_floats(int rows_a, int rows_b, int nb) {
 }
 
 // Row sums from the per-block partials and the epilogue.  LPR lanes add up one row.
-template <int MODE, class Epi>
+template <int MODE, int W, class Epi>
 __device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, int n_rows, int nb, int id0, Epi& epi) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (nb <= 16) {
         const int LPR = nb <= 8 ? 8 : 16, RPW = 32 / LPR;
         const int k = lane & (LPR - 1), rl = lane / LPR;
-        for (int base = warp * RPW; base < n_rows; base += GEMV_WARPS * RPW) {
+        for (int base = warp * RPW; base < n_rows; base += W * RPW) {
             const int r = base + rl;
             const bool on = r < n_rows && k < nb;
             float a = on ? pa[r * nb + k] : 0.f;
@@ -287,7 +300,7 @@ __device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, in
         }
     } else {
         const int items = MODE == EPI_ZIP ? n_rows : (n_rows + 1) >> 1;
-        for (int it = warp; it < items; it += GEMV_WARPS) {
+        for (int it = warp; it < items; it += W) {
             const float* ra = MODE == EPI_ZIP ? pa + it * nb : pa + (2 * it) * nb;
             const float* rb = MODE == EPI_ZIP ? pb + it * nb : ra + nb;
             const bool has_b = MODE == EPI_ZIP || 2 * it + 1 < n_rows;
@@ -312,10 +325,11 @@ __device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, in
 // after a single barrier, rows are summed in a fixed order and handed to the epilogue.  When
 // the CTA has more tiles than slots (the vocabulary head), a warp owns one slot and refills
 // it itself after each tile.
-template <class BLK, class Epi>
-__global__ void __launch_bounds__(GEMV_THREADS, 1)
+template <class BLK, class Epi, int T>
+__global__ void __maxnreg__(gemv_regs(T))
 k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pbuf_floats, int slots, TokenState* st) {
     extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int W = T / 32;
     prof_mark(0, pa.prof_id);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x;
     const bool has_norm = pa.normw != nullptr;
@@ -323,8 +337,8 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     // the fp32-route rows, the embedding source
     const bool with_xf = has_norm || fseg.m.data != nullptr || pa.vec == nullptr;
     Epi epi = epi_in;
-    Act act = act_carve(smem, K, with_xf, has_norm);
-    const size_t act_bytes = (act_smem_bytes(K, with_xf, has_norm) + 15) & ~(size_t)15;
+    Act act = act_carve(smem, K, with_xf, false);
+    const size_t act_bytes = (act_smem_bytes(K, with_xf, false) + 15) & ~(size_t)15;
     float* pbuf = reinterpret_cast<float*>(smem + act_bytes);
     float* red = pbuf + pbuf_floats;
     unsigned long long* full = reinterpret_cast<unsigned long long*>(red + 272);
@@ -350,7 +364,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     // Tile j of the CTA belongs to warp j % stride.  Without reuse every tile has its own slot; with
     // reuse (more tiles than slots) warp w owns slot w and walks its tiles through it in order.
     const bool reuse = n_jobs > slots;
-    const int stride = reuse ? slots : GEMV_WARPS;
+    const int stride = reuse ? slots : W;
     auto issue = [&](int j) {
         const int s = reuse ? warp : j;
         mbar_expect_tx(full + s, TB);
@@ -372,7 +386,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             if (reuse) break;
         }
     }
-    if (fseg.m.data && tid == GEMV_THREADS - 1) {
+    if (fseg.m.data && tid == T - 1) {
         // the fp32-route rows are read with plain loads later: have their tiles in L2 by then
         const int r0 = 2 * fseg.sh.begin(cta), r1 = r0 + 2 * fseg.sh.count(cta);
         if (r1 > r0) {
@@ -387,11 +401,11 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     if (has_norm) {
 #pragma unroll
         for (int k = 0; k < NORM_REGS; k++) {
-            const int i4 = k * GEMV_THREADS + tid;
+            const int i4 = k * T + tid;
             wreg[k] = i4 < (K >> 2) ? reinterpret_cast<const float4*>(pa.normw)[i4] : make_float4(1.f, 1.f, 1.f, 1.f);
         }
     }
-    if (pa.l2_row_bytes && st && tid == GEMV_THREADS - 32) {
+    if (pa.l2_row_bytes && st && tid == T - 32) {
         // Never in a layer 0: behind the kernel that begins a call the state may not have landed yet.
         const int rows = st->pos + 1, per = (rows + (int)gridDim.x - 1) / (int)gridDim.x;
         const int r0 = cta * per, r1 = min(rows, r0 + per);
@@ -424,17 +438,17 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     if (pa.vec && !with_xf) {
         // plain vector: quantise pass by pass straight from the registers that fetched it
         if (!done) {
-            for (int base = 0; base < n4; base += STAGE_REGS * GEMV_THREADS) {
+            for (int base = 0; base < n4; base += STAGE_REGS * T) {
                 float4 sx[STAGE_REGS];
 #pragma unroll
                 for (int k = 0; k < STAGE_REGS; k++) {
-                    const int i4 = base + k * GEMV_THREADS + tid;
+                    const int i4 = base + k * T + tid;
                     sx[k] = i4 < n4 ? reinterpret_cast<const float4*>(pa.vec)[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (int k = 0; k < STAGE_REGS; k++) {
-                    const int i4 = base + k * GEMV_THREADS + tid;
-                    if (base + k * GEMV_THREADS < n4) act_quantize4(act, sx[k], i4, i4 < n4, nb);
+                    const int i4 = base + k * T + tid;
+                    if (base + k * T < n4) act_quantize4(act, sx[k], i4, i4 < n4, nb);
                 }
             }
         }
@@ -442,7 +456,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         prof_mark(6, pa.prof_id);
     } else {
         if (pa.vec) {
-            for (int i4 = tid; i4 < n4; i4 += GEMV_THREADS)
+            for (int i4 = tid; i4 < n4; i4 += T)
                 *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = reinterpret_cast<const float4*>(pa.vec)[i4];
         } else {
             int tok = st ? st->token : pa.token;
@@ -451,7 +465,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                 tok = 0;
             }
             const SrcEmbed src{pa.embed, tok};
-            for (int i = tid; i < K; i += GEMV_THREADS) {
+            for (int i = tid; i < K; i += T) {
                 const float v = src.get(i);
                 xs[xs_idx(i)] = v;
                 if (cta == 0 && pa.raw_out && !done) pa.raw_out[i] = v;
@@ -462,7 +476,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         if (!done) {
             if (has_norm) scale = rms_scale_staged(xs, K, pa.eps, red);
             prof_mark(6, pa.prof_id);
-            for (int k0 = 0; k0 < n4; k0 += GEMV_THREADS) {
+            for (int k0 = 0; k0 < n4; k0 += T) {
                 const int i4 = k0 + tid;
                 const bool on = i4 < n4;
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -470,8 +484,8 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                     x = *reinterpret_cast<const float4*>(xs + xs_idx(4 * i4));
                     if (has_norm) {
                         float4 w = wreg[0];
-                        if (k0 == GEMV_THREADS) w = wreg[1];
-                        if (k0 >= NORM_REGS * GEMV_THREADS) w = reinterpret_cast<const float4*>(pa.normw)[i4];
+                        if (k0 == T) w = wreg[1];
+                        if (k0 >= NORM_REGS * T) w = reinterpret_cast<const float4*>(pa.normw)[i4];
                         x.x = x.x * scale * w.x;
                         x.y = x.y * scale * w.y;
                         x.z = x.z * scale * w.z;
@@ -518,7 +532,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         const int chunk = (pbuf_floats / (2 * per_row)) * (2 * per_row);  // whole row pairs per chunk
         for (int t0 = 0; t0 < tasks; t0 += chunk) {
             const int tn = min(chunk, tasks - t0);
-            for (int t = tid; t < tn; t += GEMV_THREADS) {
+            for (int t = tid; t < tn; t += T) {
                 const int task = t0 + t;
                 const int row_l = task / per_row, rem = task - row_l * per_row;
                 const int row_g = 2 * pbase + row_l;
@@ -528,7 +542,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             }
             __syncthreads();
             const int pairs_here = tn / (2 * per_row), pair_first = t0 / (2 * per_row);
-            for (int rr = warp; rr < pairs_here; rr += GEMV_WARPS) {
+            for (int rr = warp; rr < pairs_here; rr += W) {
                 const float* a = pbuf + (2 * rr) * per_row;
                 float s0 = 0.f, s1 = 0.f;
                 for (int i = lane; i < per_row; i += 32) {
@@ -584,7 +598,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     }
     if (f32_fused) {
         const int pbase = fseg.sh.begin(cta), per_row = 16 * nb;
-        for (int t = GEMV_THREADS - 1 - tid; t < f32_tasks; t += GEMV_THREADS) {
+        for (int t = T - 1 - tid; t < f32_tasks; t += T) {
             const int row_l = t / per_row, rem = t - row_l * per_row;
             const int row_g = 2 * pbase + row_l;
             float v = 0.f;
@@ -598,7 +612,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     if (f32_fused) {
         // the same sums as the stand-alone route: lanes stride over a row's runs, then the warp tree
         const int pbase = fseg.sh.begin(cta), per_row = 16 * nb, pairs = f32_tasks / (2 * per_row);
-        for (int rr = GEMV_WARPS - 1 - warp; rr < pairs; rr += GEMV_WARPS) {
+        for (int rr = W - 1 - warp; rr < pairs; rr += W) {
             const float* a = pbuf + f32_off + (2 * rr) * per_row;
             float s0 = 0.f, s1 = 0.f;
             for (int i = lane; i < per_row; i += 32) {
@@ -612,10 +626,10 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     }
     // phase B: row sums in a fixed order + epilogue
     if (Epi::MODE == EPI_ZIP) {
-        reduce_rows<EPI_ZIP>(part_a, part_b, rows_a, nb, ja.id_base + rows_a0, epi);
+        reduce_rows<EPI_ZIP, W>(part_a, part_b, rows_a, nb, ja.id_base + rows_a0, epi);
     } else {
-        reduce_rows<EPI_PAIRS>(part_a, part_a, rows_a, nb, ja.id_base + (rows_a0 >> 1), epi);
-        if (rows_b > 0) reduce_rows<EPI_PAIRS>(part_b, part_b, rows_b, nb, jb.id_base + (rows_b0 >> 1), epi);
+        reduce_rows<EPI_PAIRS, W>(part_a, part_a, rows_a, nb, ja.id_base + (rows_a0 >> 1), epi);
+        if (rows_b > 0) reduce_rows<EPI_PAIRS, W>(part_b, part_b, rows_b, nb, jb.id_base + (rows_b0 >> 1), epi);
     }
     epi.end(st);
     if (late_slot >= 0) mbar_wait(full + late_slot, late_parity);  // bounded: a second limit, then the CTA leaves regardless
@@ -653,16 +667,25 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     if (fseg.m.data && pf < 2 * 16 * nb) pf = 2 * 16 * nb;
     const bool has_norm = pa.normw != nullptr;
     const bool with_xf = has_norm || fseg.m.data != nullptr || pa.vec == nullptr;  // as in the kernel
-    const size_t fixed = gemv_smem_fixed(K, with_xf, has_norm, pf);
-    // tiles a CTA can need: each matrix's share may straddle one extra tile at either end
-    const int need = (ra * nb + 31) / 32 + 1 + (rb ? (rb * nb + 31) / 32 + 1 : 0);
+    const size_t fixed = gemv_smem_fixed(K, with_xf, pf);
+    // tiles a CTA can need: where row groups are no whole tiles, a matrix's share may straddle an extra one
+    const int straddle = (ROW_GROUP * nb) % 32 ? 1 : 0;
+    const int need = (ra * nb + 31) / 32 + straddle + (rb ? (rb * nb + 31) / 32 + straddle : 0);
     if (fixed + 256 + 1024 + TB > GEMV_SMEM_MAX) return cudaErrorInvalidValue;
     int slots = (int)((GEMV_SMEM_MAX - fixed - 256 - 1024) / (TB + 8));
-    if (slots >= need) slots = need;
+    const bool resident = slots >= need;
+    if (resident) slots = need;
     else if (slots > GEMV_WARPS) slots = GEMV_WARPS;  // reuse: one slot per warp
     if (slots < 1) slots = 1;
     const size_t smem = fixed + (size_t)slots * 8 + 256 + (size_t)slots * TB;
-    return launch_pdl(k_gemv<BLK, Epi>, dim3(grid), dim3(GEMV_THREADS), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+    if constexpr (Epi::SHARES_SM) {
+        const int f32_tasks = fseg.m.data ? 2 * (fseg.sh.quot + 1) * 16 * nb : 0;
+        if (resident && need <= GEMV_SMALL / 32 && f32_tasks <= 2 * GEMV_SMALL && K <= 4 * 4 * GEMV_SMALL && smem <= GEMV_SMALL_SMEM)
+            return launch_pdl(k_gemv<BLK, Epi, GEMV_SMALL>, dim3(grid), dim3(GEMV_SMALL), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+        if (resident && smem <= GEMV_MID_SMEM)
+            return launch_pdl(k_gemv<BLK, Epi, GEMV_MID>, dim3(grid), dim3(GEMV_MID), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+    }
+    return launch_pdl(k_gemv<BLK, Epi, GEMV_THREADS>, dim3(grid), dim3(GEMV_THREADS), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
 }
 
 inline RowJob make_job(const Mat& m, int C, int id_base = 0) {
