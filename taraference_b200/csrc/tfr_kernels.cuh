@@ -13,6 +13,7 @@ namespace tfr {
 
 // y = W x (+y) (+bias): kernels/gemv.cu:367-373 residual rule (2 = accumulate in place).
 struct EpiStore {
+    static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_PAIRS;
     float* out;
@@ -44,6 +45,7 @@ struct EpiStore {
 
 // h = silu(gate.x) * (up.x), kernels/gemv.cu:2570-2574.  Pair p = (gate row p, up row p).
 struct EpiSilu {
+    static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_ZIP;
     float* out;
@@ -61,6 +63,7 @@ struct EpiSilu {
 // (kernels/ops.cu:471-486).  Q and K rows were re-ordered at upload so that the RoPE
 // partners (i, i + hd/2) of a head are the two rows of a pair; biases likewise.
 struct EpiQkv {
+    static constexpr bool STAGES_BIAS = true;
     static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_PAIRS;
     float* q_out;            // [n_head * hd] natural order
@@ -71,6 +74,9 @@ struct EpiQkv {
     float theta;
     int pos;
     size_t kv_off;
+    // the biases of the CTA's rows in shared memory, when it staged them: row v of a segment at v - off
+    const float* sbias = nullptr;
+    int off_q, off_k, off_v;
     __device__ void begin(const TokenState* st) {
         if (st) {
             pos = st->pos;
@@ -83,7 +89,11 @@ struct EpiQkv {
     __device__ __forceinline__ void set_residual(const float*, int) {}
     __device__ __forceinline__ void apply(int p, float x0, float x1) {
         const int v = 2 * p;
-        if (bias) {
+        if (sbias) {
+            const float2 b = *reinterpret_cast<const float2*>(sbias + v - (v < nq ? off_q : v < nq + nk ? off_k : off_v));
+            x0 += b.x;
+            x1 += b.y;
+        } else if (bias) {
             x0 += bias[v];
             x1 += bias[v + 1];
         }
@@ -138,6 +148,7 @@ __device__ __forceinline__ void advance_state(TokenState* st, int tok, int* out_
 }
 
 struct EpiLogits {
+    static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = false;
     static constexpr int MODE = EPI_PAIRS;
     float* logits;
@@ -277,8 +288,9 @@ inline int gemv_pbuf_floats(int rows_a, int rows_b, int nb) {
 
 // Row sums from the per-block partials and the epilogue.  LPR lanes add up one row.
 template <int MODE, int W, class Epi>
-__device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, int n_rows, int nb, int id0, Epi& epi) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, int n_rows, int nb, int id0, Epi& epi, int first = 0) {
+    // first: the warp that takes the first rows
+    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - first, warp = w < 0 ? w + W : w;
     if (nb <= 16) {
         const int LPR = nb <= 8 ? 8 : 16, RPW = 32 / LPR;
         const int k = lane & (LPR - 1), rl = lane / LPR;
@@ -418,6 +430,17 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             }
         }
     }
+    // So are the biases of the CTA's rows: fetched by the row sums, they cost the epilogue a trip to L2 per matrix (1 us).
+    float biasv = 0.f;
+    bool bias_pre = false;
+    const int rows_f = Epi::STAGES_BIAS && fseg.m.data ? 2 * fseg.sh.count(cta) : 0;
+    if constexpr (Epi::STAGES_BIAS) {
+        bias_pre = epi.bias && rows_a + rows_b + rows_f <= 256;
+        if (bias_pre && tid < rows_a + rows_b + rows_f)
+            biasv = epi.bias[tid < rows_a            ? 2 * ja.id_base + rows_a0 + tid
+                             : tid < rows_a + rows_b ? 2 * jb.id_base + rows_b0 + tid - rows_a
+                                                     : 2 * (fseg.id_base + fseg.sh.begin(cta)) + tid - rows_a - rows_b];
+    }
     __syncwarp();
     prof_mark(1, pa.prof_id);
     // Everything below reads what earlier kernels wrote (the vector, the decode state).
@@ -516,6 +539,15 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     if (res_pre) {
         if (tid < rows_a) red[tid] = resv;  // red is free once the norm's reduction is over
         epi.set_residual(red, res_row0);
+    }
+    if constexpr (Epi::STAGES_BIAS) {
+        if (bias_pre) {
+            if (tid < rows_a + rows_b + rows_f) red[tid] = biasv;
+            epi.sbias = red;
+            epi.off_q = 2 * ja.id_base + rows_a0;
+            epi.off_k = 2 * jb.id_base + rows_b0 - rows_a;
+            epi.off_v = 2 * (fseg.id_base + fseg.sh.begin(cta)) - rows_a - rows_b;
+        }
     }
     __syncthreads();
 
@@ -629,7 +661,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         reduce_rows<EPI_ZIP, W>(part_a, part_b, rows_a, nb, ja.id_base + rows_a0, epi);
     } else {
         reduce_rows<EPI_PAIRS, W>(part_a, part_a, rows_a, nb, ja.id_base + (rows_a0 >> 1), epi);
-        if (rows_b > 0) reduce_rows<EPI_PAIRS, W>(part_b, part_b, rows_b, nb, jb.id_base + (rows_b0 >> 1), epi);
+        if (rows_b > 0) reduce_rows<EPI_PAIRS, W>(part_b, part_b, rows_b, nb, jb.id_base + (rows_b0 >> 1), epi, W / 2);
     }
     epi.end(st);
     if (late_slot >= 0) mbar_wait(full + late_slot, late_parity);  // bounded: a second limit, then the CTA leaves regardless
