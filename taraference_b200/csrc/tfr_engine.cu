@@ -29,6 +29,7 @@
 #include "tfr_kernels.cuh"
 #include "tfr_chunk.cuh"
 #include "tfr_gemm_tc.cuh"
+#include "tfr_gemm_mma.cuh"
 #include "tfr_loop.cuh"
 
 using namespace tfr;
@@ -323,8 +324,14 @@ static void configure_kernels_once() {
     configure_kernel(k_gemm_tc<RawQ6, TC_PAIR>, true);
     configure_kernel(k_gemm_tc<RawQ4, TC_SINGLE>, true);
     configure_kernel(k_gemm_tc<RawQ6, TC_SINGLE>, true);
-    configure_kernel(k_gemm_tc<RawQ4, TC_HALF>, true);
-    configure_kernel(k_gemm_tc<RawQ6, TC_HALF>, true);
+    configure_kernel(k_prep_mma, true);
+    configure_kernel(k_gemm_mma<MmaQ4, 1>, true);
+    configure_kernel(k_gemm_mma<MmaQ4, 2>, true);
+    configure_kernel(k_gemm_mma<MmaQ4, 3>, true);
+    configure_kernel(k_gemm_mma<MmaQ4, 4>, true);
+    configure_kernel(k_gemm_mma<MmaQ4, 5>, true);
+    configure_kernel(k_gemm_mma<MmaQ6, 1>, true);
+    configure_kernel(k_gemm_mma<MmaQ6, 2>, true);
     configure_kernel(k_attn_chunk_merge, false);
     // the attention kernel also has static shared memory: ask for exactly the dynamic part it uses
     configure_kernel(k_attn_decode<64>, false);
@@ -1712,7 +1719,7 @@ static int chunk_buffers(tfr_engine* e, int M) {
     CU(e, cudaMalloc(&e->cattn, (size_t)cap * mix_width * 4));
     CU(e, cudaMalloc(&e->ch, (size_t)cap * P.ff * 4));
     CU(e, cudaMalloc(&e->cact, (size_t)cap * e->cact_stride));
-    CU(e, cudaMalloc(&e->cimage, tc_image_bytes(kmax, cap)));
+    CU(e, cudaMalloc(&e->cimage, std::max(tc_image_bytes(kmax, cap), mma_image_bytes(kmax))));
     CU(e, cudaMalloc(&e->ctscale, (size_t)tc_pad_tokens(cap) * 4));
     if (c.hybrid) {
         CU(e, cudaMalloc(&e->cproj, (size_t)cap * std::max(channels + vd + 2 * c.ssm_time_step_rank, 2 * P.nq + 2 * P.nkv) * 4));
@@ -1732,9 +1739,15 @@ static int chunk_buffers(tfr_engine* e, int M) {
     return TFR_OK;
 }
 
-// Batches from five tokens on: projections of Q4_K and Q6_K matrices on the tensor cores.  Fewer tokens leave those idle
-// and keep the dp4a kernel, as Q8_0 matrices do; TFR_GEMM_DP4A=1 in the environment keeps everything there (a test aid).
-static bool gemm_on_tc(int type, int M) { return M >= GEMM_TC_MIN_TOKENS && tc_type(type) && !getenv("TFR_GEMM_DP4A"); }
+// The kernel of a batch's projections.  Fewer than five tokens leave the tensor cores idle and keep the dp4a kernel, as Q8_0
+// matrices do (TFR_GEMM_DP4A=1 in the environment keeps everything there, a test aid).  mma.sync where it is the faster one:
+// up to 80 tokens on Q4_K (11 008 gate and up rows of 2 048: 15 us for 16 tokens, 54 for 80; tcgen05 29 and 59) and up to 32
+// on Q6_K, whose MMAs are half as deep (2 048 rows of 11 008: 15 and 21 us; 26 and 29; at 48 tokens both take 35).
+enum { GEMM_DP4A, GEMM_MMA, GEMM_TC };
+static int gemm_route(int type, int nb, int M) {
+    if (M < GEMM_TC_MIN_TOKENS || !tc_type(type) || getenv("TFR_GEMM_DP4A")) return GEMM_DP4A;
+    return M <= (type == TFR_Q4_K ? 80 : 32) && mma_tiles(nb, M) > 0 ? GEMM_MMA : GEMM_TC;
+}
 
 static cudaError_t launch_gemm_typed(cudaStream_t s, int grid, int type, const unsigned char* act, size_t stride, const float* xn, int M,
                                      const RowJob& ja, const RowJob& jb, const F32Seg& fseg, const ChunkEpi& epi, int K, TokenState* st) {
@@ -1755,24 +1768,31 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     cudaStream_t s = e->stream;
     int n = 0;
     // x -> RMSNorm (optional) -> Q8, in the form the projections that follow read
-    auto prep = [&](bool tc, const float* x, int ldx, int width, const float* normw, float* xn) -> cudaError_t {
+    auto prep = [&](int route, int type, const float* x, int ldx, int width, const float* normw, float* xn) -> cudaError_t {
         n++;
-        if (tc) {
+        if (route == GEMM_TC) {
             PrepTcArgs a{x, ldx, width, M, normw, c.rms_eps, e->cimage, e->ctscale, xn};
             return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(TC_PREP_THREADS), tc_prep_smem(width), s, a);
+        }
+        if (route == GEMM_MMA) {
+            PrepMmaArgs a{x, ldx, width, M, normw, c.rms_eps, e->cimage, xn, type == TFR_Q6_K};
+            return launch_pdl(k_prep_mma, dim3((M + 15) & ~15), dim3(MMA_PREP_THREADS), normw ? tc_prep_smem(width) : 0, s, a);
         }
         PrepRowsArgs a{x, ldx, width, normw, c.rms_eps, e->cact, e->cact_stride, xn};
         const size_t smem = normw ? (xs_floats(width) + 272) * sizeof(float) : 0;
         return launch_pdl(k_prep_rows, dim3(M), dim3(GEMV_THREADS), smem, s, a);
     };
+    auto gemm = [&](int route, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep) -> cudaError_t {
+        n++;
+        if (route == GEMM_TC) return launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, ja, jb, ep, e->st);
+        if (route == GEMM_MMA) return launch_gemm_mma(s, cap, e->cimage, M, ja, jb, ep, e->st);
+        return launch_gemm_typed(s, cap, ja.m.type, e->cact, e->cact_stride, nullptr, M, ja, jb, F32Seg{}, ep, ja.m.K, e->st);
+    };
     // RMSNorm + Q8 + W x + epilogue
     auto project = [&](const float* x, int width, const float* normw, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep) -> cudaError_t {
-        const bool tc = gemm_on_tc(ja.m.type, M);
-        cudaError_t r = prep(tc, x, width, width, normw, nullptr);
-        if (r != cudaSuccess) return r;
-        n++;
-        if (tc) return launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, ja, jb, ep, e->st);
-        return launch_gemm_typed(s, cap, ja.m.type, e->cact, e->cact_stride, nullptr, M, ja, jb, F32Seg{}, ep, width, e->st);
+        const int route = gemm_route(ja.m.type, ja.m.nb, M);
+        const cudaError_t r = prep(route, ja.m.type, x, width, width, normw, nullptr);
+        return r != cudaSuccess ? r : gemm(route, ja, jb, ep);
     };
     auto store_epi = [&](float* out, int ldo, int rows, int use_res) {
         ChunkEpi ep{};
@@ -1812,9 +1832,10 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             wout = L.ssm_out;
         } else {
         // 1. RMSNorm + Q8, Q/K/V (+bias); dense layers: RoPE + f16 KV rows
-        const bool gated = L.kind == LAYER_FULL_GATED, tc_qk = gemm_on_tc(TFR_Q4_K, M);
+        const bool gated = L.kind == LAYER_FULL_GATED;
+        const int route = gemm_route(TFR_Q4_K, L.wq->m.nb, M);
         const int q_rows = gated ? 2 * nq : nq;
-        if (prep(tc_qk, e->cx, K, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
+        if (prep(route, TFR_Q4_K, e->cx, K, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
         {
             const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, q_rows / 2);
             F32Seg fseg{};
@@ -1831,15 +1852,15 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
                 ep.nq = nq, ep.nk = nkv, ep.hd = hd, ep.kvdim = nkv, ep.pos0 = pos0, ep.theta = c.rope_theta;
             }
             ep.bias = L.bias_qkv;
-            if (tc_qk) {
+            if (route != GEMM_DP4A) {
                 // the fp32-route V rows keep the decode kernels' arithmetic bit for bit
                 if (launch_rows_f32(s, cap, fseg.m, fseg.id_base, e->cxn, M, ep) != cudaSuccess) return -1;
                 n++;
-                if (launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, jq, jk, ep, e->st) != cudaSuccess) return -1;
-            } else if (launch_gemm<BlockQ4>(s, cap, e->cact, e->cact_stride, e->cxn, M, jq, jk, fseg, ep, K, e->st) != cudaSuccess) {
-                return -1;
+                if (gemm(route, jq, jk, ep) != cudaSuccess) return -1;
+            } else {
+                if (launch_gemm<BlockQ4>(s, cap, e->cact, e->cact_stride, e->cxn, M, jq, jk, fseg, ep, K, e->st) != cudaSuccess) return -1;
+                n++;
             }
-            n++;
         }
         if (gated) {
             QkNormArgs qa{};

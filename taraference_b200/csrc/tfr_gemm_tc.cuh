@@ -368,34 +368,31 @@ struct RawQ6 {
 // tokens' two planes of B.  Warps 4-11 turn weights into A tiles, lanes of warp 1 request the B planes as bulk copies, lane
 // 0 of warps 0 and 2 issues the MMAs, the warps behind drain the accumulators (two buffers in TMEM) into the row sums they
 // hold in registers (TMEM lanes 32 (w & 3) .., a share of the tokens); every role runs ahead of the next as far as the
-// rings allow.  (With all warps doing everything in turn a stage took 4 500 cycles.)  Three forms:
+// rings allow.  (With all warps doing everything in turn a stage took 4 500 cycles.)  Two forms:
 //
 //   pair    batches of more than 128 tokens.  Two CTAs on adjacent row tiles share up to 256 tokens with cta_group::2
 //           MMAs of 256 x 256 x 16: each holds its own rows of A and half of the tokens' B, which halves what B costs in
 //           L2 reads and in shared-memory reads per MMA.  One CTA alone on 2 x 128 rows x 128 tokens ran at a third of it.
 //   single  up to 128 tokens.  The high and the low terms of the tokens are columns of ONE MMA, so A is read once for both.
-//   half    up to 32 tokens: the same in half an SM.  What a stage costs there is the chain unpack -> MMA -> slot free ->
-//           unpack (about 3 000 cycles, most of it barriers) and a CTA another 9 000 before and after its stages; a second
-//           CTA on the SM, of this or of the next kernel, works through the first one's waits.
 //
 // Gate / up pairs (ZIP) alternate the two matrices' rows in the tile, so that a gate value meets its up value in the
 // neighbouring lane, as the two rows of a RoPE pair do.  The k range is cut over the CTAs of a cluster (grid.y) where a
 // matrix has too few rows to fill the chip: their sums meet through distributed shared memory, each CTA finishing its
 // share of the tokens.
 constexpr int TC_C_WARPS = 4, TC_A_WARPS = 8, TC_MAX_STAGES = 6;
-constexpr size_t TC_SMEM_MAX = 225 * 1024, TC_SMEM_HALF = 111 * 1024;
-enum { TC_PAIR, TC_SINGLE, TC_HALF };
+constexpr size_t TC_SMEM_MAX = 225 * 1024;
+enum { TC_PAIR, TC_SINGLE };
 // Draining warps and the registers of a thread of each role (what they add up to is what the launch has).  Draining is a
 // chain of TMEM loads (300 cycles for 16 columns, waited for one by one), so sixteen warps share the columns; the pairs on
 // Q6_K matrices, whose third MMA leaves more time, keep eight and leave the registers to the unpacking.
 template <int FORM, bool Q4>
 struct TcRoles {
-    static constexpr int D_WARPS = FORM == TC_HALF ? 4 : FORM == TC_PAIR && !Q4 ? 8 : 16, THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + D_WARPS);
-    static constexpr int CTAS = FORM == TC_HALF ? 2 : 1, LAUNCH_REGS = FORM == TC_HALF ? 64 : D_WARPS == 8 ? 96 : 72;
+    static constexpr int D_WARPS = FORM == TC_PAIR && !Q4 ? 8 : 16, THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + D_WARPS);
+    static constexpr int LAUNCH_REGS = D_WARPS == 8 ? 96 : 72;
     static constexpr int C_REGS = D_WARPS == 8 ? 32 : 24, A_REGS = D_WARPS == 8 ? 64 : FORM == TC_PAIR ? 48 : 72,
-                         D_REGS = FORM == TC_HALF ? 88 : D_WARPS == 8 ? 160 : FORM == TC_PAIR ? 96 : 80;
+                         D_REGS = D_WARPS == 8 ? 160 : FORM == TC_PAIR ? 96 : 80;
     static constexpr int NC = FORM == TC_PAIR ? 1024 / D_WARPS : 32;  // tokens of a draining warp
-    static_assert(32 * (TC_C_WARPS * C_REGS + TC_A_WARPS * A_REGS + D_WARPS * D_REGS) <= THREADS * LAUNCH_REGS && CTAS * THREADS * LAUNCH_REGS <= 65536,
+    static_assert(32 * (TC_C_WARPS * C_REGS + TC_A_WARPS * A_REGS + D_WARPS * D_REGS) <= THREADS * LAUNCH_REGS && THREADS * LAUNCH_REGS <= 65536,
                   "more registers than the launch has");
 };
 // Registers of a role: N of the LAUNCH a thread has.  Fewer must be given back, more asked for.
@@ -428,7 +425,7 @@ struct TcRing {
 };
 
 template <class RAW, int FORM>
-__global__ void __launch_bounds__(TcRoles<FORM, RAW::PLANES == 1>::THREADS, TcRoles<FORM, RAW::PLANES == 1>::CTAS) k_gemm_tc(const TcArgs a) {
+__global__ void __launch_bounds__(TcRoles<FORM, RAW::PLANES == 1>::THREADS, 1) k_gemm_tc(const TcArgs a) {
     constexpr bool Q4 = RAW::PLANES == 1, PAIR = FORM == TC_PAIR;
     using Roles = TcRoles<FORM, Q4>;
     constexpr int TC_D_WARPS = Roles::D_WARPS, CGS = TC_D_WARPS / 4, NC = Roles::NC;  // column groups of NC tokens
@@ -474,7 +471,7 @@ __global__ void __launch_bounds__(TcRoles<FORM, RAW::PLANES == 1>::THREADS, TcRo
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int A_SUB = RAW::PLANES * 16384;            // A of 64 weights: one 16 KB tile per plane
     const int b_plane = ntc * 128, stage_bytes = A_SUB + 2 * (a.NT / CG) * 128;
-    constexpr unsigned ACC_COLS = (PAIR ? 1 : 2) * CGS * NC, TMEM_COLS = 2 * ACC_COLS;  // the tokens; single, half: high then low terms
+    constexpr unsigned ACC_COLS = (PAIR ? 1 : 2) * CGS * NC, TMEM_COLS = 2 * ACC_COLS;  // the tokens; single: high then low terms
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
             // every CTA's own A warps and B (with the bytes); the leader's also the word that the peer's are complete
@@ -975,8 +972,8 @@ inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_ti
     using Roles = TcRoles<FORM, RAW::PLANES == 1>;
     constexpr bool PAIR = FORM == TC_PAIR;
     const int stage = RAW::PLANES * 16384 + 2 * (a.NT / (PAIR ? 2 : 1)) * 128;
-    a.nst = std::min(TC_MAX_STAGES, (int)(((FORM == TC_HALF ? TC_SMEM_HALF : TC_SMEM_MAX) - 1024) / stage));
-    a.ahead = S == 1 && row_tiles > sms * Roles::CTAS ? sms * Roles::CTAS : 0;
+    a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024) / stage));
+    a.ahead = S == 1 && row_tiles > sms ? sms : 0;
     const size_t sums = S > 1 ? (size_t)a.NT * 512 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(PAIR ? (row_tiles + 1) & ~1 : row_tiles, S, (a.Mp + a.NT - 1) / a.NT);
@@ -1013,11 +1010,11 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
     // units of a 128-row, 128-token MMA stage
     auto plan = [&](int form, int& S, int& NT) {
         const bool pair = form == TC_PAIR;
-        const int most = pair ? 256 : form == TC_HALF ? 32 : 128, tok_tiles = (a.Mp + most - 1) / most, unit = pair ? 32 : 16;
+        const int most = pair ? 256 : 128, tok_tiles = (a.Mp + most - 1) / most, unit = pair ? 32 : 16;
         NT = ((a.Mp + tok_tiles - 1) / tok_tiles + unit - 1) / unit * unit;
         double best = 1e30;
         for (int s = 1; s <= (pair ? 4 : 8) && s <= ja.m.nb; s *= 2) {
-            const int ctas = (pair ? (tiles + 1) & ~1 : tiles) * tok_tiles * s, at_once = fit(pair ? 2 * s : s) * (form == TC_HALF ? 2 : 1);
+            const int ctas = (pair ? (tiles + 1) & ~1 : tiles) * tok_tiles * s, at_once = fit(pair ? 2 * s : s);
             const double stage = pair ? 0.4 + 1.2 * NT / 128 : 0.6 + 1.2 * NT / 128;
             const double t = (double)((ctas + at_once - 1) / at_once) * ((4.5 * ((ja.m.nb + s - 1) / s) * stage) + 6 + (s > 1 ? 3 : 0));
             if (t < best) best = t, S = s;
@@ -1025,10 +1022,6 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
         return best;
     };
     int S = 1, S2 = 1, NT2 = 0;
-    if (M <= 32) {
-        plan(TC_HALF, S, a.NT);
-        return q4 ? launch_tc<RawQ4, TC_HALF>(stream, sms, a, tiles, S) : launch_tc<RawQ6, TC_HALF>(stream, sms, a, tiles, S);
-    }
     const double single = plan(TC_SINGLE, S, a.NT);
     if (M > 128 && plan(TC_PAIR, S2, NT2) < single) {
         a.NT = NT2;

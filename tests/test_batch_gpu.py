@@ -1,4 +1,4 @@
-"""Token batches at the edges of the batched kernels' tiles: the tcgen05 projections against the dp4a ones, the hybrid
+"""Token batches at the edges of the batched kernels' tiles: the tensor-core projections against the dp4a ones, the hybrid
 layers against the step-by-step route (needs a B200)."""
 import numpy as np
 import pytest
@@ -28,9 +28,9 @@ def _state(m, kv, cfg, n):
 
 
 @pytest.mark.parametrize("cfg", [ODD, WIDE], ids=["odd", "wide"])
-@pytest.mark.parametrize("n", [5, 16, 17, 32, 33, 64, 128, 129, 224, 256, 257, 640])
+@pytest.mark.parametrize("n", [5, 16, 17, 32, 33, 48, 80, 81, 128, 129, 224, 256, 257, 640])
 def test_projections_of_batches_at_tile_edges(E, cfg, n, monkeypatch):
-    """One layer, all tokens in one batch: 16- and 32-token paddings, the forms for up to 32, 128 and more tokens, several
+    """One layer, all tokens in one batch: 16- and 32-token paddings, mma.sync up to 80 tokens (Q6_K: 32), the tcgen05 forms, several
     token tiles, tiles that end inside a column group.  V rows are the same bits, the logits differ by a flip at most."""
     m = E.CudaModel.load_with(cfg, S.make_dense_model(cfg, seed=31))
     prompt = [int(t) for t in np.random.default_rng(n).integers(0, cfg["n_vocab"], n)]
