@@ -267,7 +267,7 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
     // CTA): a thread unpacks the sixteen weights of its task ONCE, keeps them in registers and walks the tokens of the
     // whole launch, every token's normalised vector straight from global memory; with fewer tasks than threads the
     // tokens of a group are shared out among the threads of a task.  Same operations in the same order as
-    // q6k_run_dot_f32_g, hence the same bits.
+    // Q6Run::dot, hence the same bits.
     bool f32_done = false;
     if (fseg.m.data) {
         const int np = fseg.sh.count(cta), pbase = fseg.sh.begin(cta);
@@ -332,8 +332,11 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
                     const int row_l = t / per_row, rem = t - row_l * per_row;
                     const int row_g = 2 * (pbase + p0) + row_l;
                     float v = 0.f;
-                    if (row_g < fseg.m.N)
-                        v = q6k_run_dot_f32_g(fseg.m, mat_flat(nb, row_g, rem >> 4), rem >> 4, rem & 15, xn + (size_t)(m0 + m) * K);
+                    if (row_g < fseg.m.N) {
+                        Q6Run run;
+                        run.load(fseg.m, mat_flat(nb, row_g, rem >> 4), rem & 15);
+                        v = run.dot(xn + (size_t)(m0 + m) * K + 16 * rem);
+                    }
                     pbuf[(size_t)m * g.pbuf_floats + t] = v;
                 }
                 __syncthreads();

@@ -412,83 +412,55 @@ __device__ __forceinline__ float block_dot(BlockQ8, const uint8_t* tile, int lan
     return acc;
 }
 
-// One run of 16 elements (scale group c = 8n + 2j + is) of Q6_K block f against the fp32
-// activation staged in shared memory — the reference's route for a Q6_K attn_v,
-// kernels/gemv.cu:233-264: acc += d * scale * q * x with x unquantised.  b = block index in the row.
-__device__ __forceinline__ float q6k_run_dot_f32(const Mat& m, long long f, int b, int c, const float* xf) {
-    const int n = c >> 3, j = (c >> 1) & 3, is = c & 1;
-    const int4 ql = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 64 * n + 32 * (j & 1) + 16 * is)));
-    const int4 qh = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 128 + 32 * n + 16 * is)));
-    const float sc = (float)(int)*reinterpret_cast<const signed char*>(block_byte(m, f, 192 + 8 * n + is + 2 * j));
-    const float d = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(block_byte(m, f, 208))));
-    const float dsc = d * sc;
-    const float4* x4 = reinterpret_cast<const float4*>(xf + xs_idx(256 * b + 16 * c));
-    const int qlw[4] = {ql.x, ql.y, ql.z, ql.w};
-    const int qhw[4] = {qh.x, qh.y, qh.z, qh.w};
-    const int nsh = 4 * (j >> 1), hsh = 2 * j;
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float4 x = x4[k];
-        const float xv[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int by = 0; by < 4; by++) {
-            const int nib = (qlw[k] >> (8 * by + nsh)) & 0xF;
-            const int hb = (qhw[k] >> (8 * by + hsh)) & 3;
-            acc += dsc * (float)((nib | (hb << 4)) - 32) * xv[by];
-        }
+// One run of 16 elements (scale group c = 8n + 2j + is) of Q6_K block f on the fp32 activation route, the reference's for a
+// Q6_K attn_v (kernels/gemv.cu:233-264): acc += d * scale * q * x with x unquantised.  Loading and multiplying are separate,
+// so that a thread has several runs' words in flight.  The weights are unpacked four bytes at a time and become floats under
+// an exponent (the byte, plus 2^23, minus 2^23 + 32: exact) instead of by a conversion each, which runs at a quarter rate.
+struct Q6Run {
+    int4 ql, qh;
+    float dsc;
+    int nsh, hsh;
+    __device__ __forceinline__ void load(const Mat& m, long long f, int c) {
+        const int n = c >> 3, j = (c >> 1) & 3, is = c & 1;
+        ql = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 64 * n + 32 * (j & 1) + 16 * is)));
+        qh = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 128 + 32 * n + 16 * is)));
+        const float sc = (float)(int)*reinterpret_cast<const signed char*>(block_byte(m, f, 192 + 8 * n + is + 2 * j));
+        dsc = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(block_byte(m, f, 208)))) * sc;
+        nsh = 4 * (j >> 1), hsh = 2 * j;
     }
-    return acc;
-}
-
-// The same run against a plain fp32 vector in global memory (x = the row's start): the chunk kernels keep no staged
-// copy per token.  Same operations in the same order as q6k_run_dot_f32.
-__device__ __forceinline__ float q6k_run_dot_f32_g(const Mat& m, long long f, int b, int c, const float* x) {
-    const int n = c >> 3, j = (c >> 1) & 3, is = c & 1;
-    const int4 ql = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 64 * n + 32 * (j & 1) + 16 * is)));
-    const int4 qh = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 128 + 32 * n + 16 * is)));
-    const float sc = (float)(int)*reinterpret_cast<const signed char*>(block_byte(m, f, 192 + 8 * n + is + 2 * j));
-    const float d = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(block_byte(m, f, 208))));
-    const float dsc = d * sc;
-    const float4* x4 = reinterpret_cast<const float4*>(x + 256 * b + 16 * c);
-    const int qlw[4] = {ql.x, ql.y, ql.z, ql.w};
-    const int qhw[4] = {qh.x, qh.y, qh.z, qh.w};
-    const int nsh = 4 * (j >> 1), hsh = 2 * j;
-    float acc = 0.f;
+    // factors 4 k .. 4 k + 3
+    __device__ __forceinline__ void weights(int k, float (&w)[4]) const {
+        const unsigned l = (unsigned)(k == 0 ? ql.x : k == 1 ? ql.y : k == 2 ? ql.z : ql.w), h = (unsigned)(k == 0 ? qh.x : k == 1 ? qh.y : k == 2 ? qh.z : qh.w);
+        const unsigned q = ((l >> nsh) & 0x0f0f0f0fu) | (((h >> hsh) & 0x03030303u) << 4);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float4 xq = x4[k];
-        const float xv[4] = {xq.x, xq.y, xq.z, xq.w};
-#pragma unroll
-        for (int by = 0; by < 4; by++) {
-            const int nib = (qlw[k] >> (8 * by + nsh)) & 0xF;
-            const int hb = (qhw[k] >> (8 * by + hsh)) & 3;
-            acc += dsc * (float)((nib | (hb << 4)) - 32) * xv[by];
-        }
+        for (int i = 0; i < 4; i++) w[i] = dsc * (__uint_as_float(__byte_perm(q, 0x4b000000u, 0x7440 + i)) - 8388640.f);
     }
-    return acc;
-}
-
-// The sixteen weights of that run as the factors q6k_run_dot_f32_g multiplies x by, d * scale * (q - 32) in its order of
-// operations, and the dot with a vector piece in its order of additions: weights kept in registers serve many tokens.
+    __device__ __forceinline__ float dot(const float* x16) const {
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float4 x = reinterpret_cast<const float4*>(x16)[k];
+            float w[4];
+            weights(k, w);
+            acc += w[0] * x.x;
+            acc += w[1] * x.y;
+            acc += w[2] * x.z;
+            acc += w[3] * x.w;
+        }
+        return acc;
+    }
+};
+// The sixteen factors of a run: weights kept in registers serve many tokens.
 __device__ __forceinline__ void q6k_run_weights_f32(const Mat& m, long long f, int c, float (&w)[16]) {
-    const int n = c >> 3, j = (c >> 1) & 3, is = c & 1;
-    const int4 ql = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 64 * n + 32 * (j & 1) + 16 * is)));
-    const int4 qh = __ldg(reinterpret_cast<const int4*>(block_byte(m, f, 128 + 32 * n + 16 * is)));
-    const float sc = (float)(int)*reinterpret_cast<const signed char*>(block_byte(m, f, 192 + 8 * n + is + 2 * j));
-    const float d = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(block_byte(m, f, 208))));
-    const float dsc = d * sc;
-    const int qlw[4] = {ql.x, ql.y, ql.z, ql.w};
-    const int qhw[4] = {qh.x, qh.y, qh.z, qh.w};
-    const int nsh = 4 * (j >> 1), hsh = 2 * j;
+    Q6Run r;
+    r.load(m, f, c);
 #pragma unroll
-    for (int k = 0; k < 4; k++)
+    for (int k = 0; k < 4; k++) {
+        float v[4];
+        r.weights(k, v);
 #pragma unroll
-        for (int by = 0; by < 4; by++) {
-            const int nib = (qlw[k] >> (8 * by + nsh)) & 0xF;
-            const int hb = (qhw[k] >> (8 * by + hsh)) & 3;
-            w[4 * k + by] = dsc * (float)((nib | (hb << 4)) - 32);
-        }
+        for (int i = 0; i < 4; i++) w[4 * k + i] = v[i];
+    }
 }
 __device__ __forceinline__ float q6k_run_dot_weights(const float (&w)[16], const float* x16) {
     const float4* x4 = reinterpret_cast<const float4*>(x16);

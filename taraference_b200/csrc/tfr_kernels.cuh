@@ -1,5 +1,8 @@
 // __global__ kernels of the batch-1 decode path and their launch helpers.
 #pragma once
+#include <algorithm>
+#include <type_traits>
+
 #include "tfr_attn.cuh"
 #include "tfr_gdn.cuh"
 #include "tfr_gemv.cuh"
@@ -13,6 +16,7 @@ namespace tfr {
 
 // y = W x (+y) (+bias): kernels/gemv.cu:367-373 residual rule (2 = accumulate in place).
 struct EpiStore {
+    static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_PAIRS;
@@ -45,6 +49,7 @@ struct EpiStore {
 
 // h = silu(gate.x) * (up.x), kernels/gemv.cu:2570-2574.  Pair p = (gate row p, up row p).
 struct EpiSilu {
+    static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_ZIP;
@@ -63,6 +68,7 @@ struct EpiSilu {
 // (kernels/ops.cu:471-486).  Q and K rows were re-ordered at upload so that the RoPE
 // partners (i, i + hd/2) of a head are the two rows of a pair; biases likewise.
 struct EpiQkv {
+    static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = true;
     static constexpr bool SHARES_SM = true;
     static constexpr int MODE = EPI_PAIRS;
@@ -148,6 +154,7 @@ __device__ __forceinline__ void advance_state(TokenState* st, int tok, int* out_
 }
 
 struct EpiLogits {
+    static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = false;
     static constexpr int MODE = EPI_PAIRS;
@@ -342,12 +349,14 @@ __global__ void __maxnreg__(gemv_regs(T))
 k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pbuf_floats, int slots, TokenState* st) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int W = T / 32;
+    // only the kernels that have fp32-route rows carry their code
+    const bool f32 = Epi::F32_ROWS && std::is_same<BLK, BlockQ4>::value && fseg.m.data != nullptr;
     prof_mark(0, pa.prof_id);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x;
     const bool has_norm = pa.normw != nullptr;
     // the fp32 copy of the vector is staged only where something reads it back: the norm's reduction,
     // the fp32-route rows, the embedding source
-    const bool with_xf = has_norm || fseg.m.data != nullptr || pa.vec == nullptr;
+    const bool with_xf = has_norm || f32 || pa.vec == nullptr;
     Epi epi = epi_in;
     Act act = act_carve(smem, K, with_xf, false);
     const size_t act_bytes = (act_smem_bytes(K, with_xf, false) + 15) & ~(size_t)15;
@@ -383,6 +392,20 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         bulk_load(ring + (size_t)s * TB, job_src(j), TB, full + s);
     };
 
+    // RMSNorm weights are constants: fetched before the wait (the first 8 x threads of them).  The CTAs of 1 024 threads,
+    // wide layers' with a ring full of tiles, ask for them ahead of those, which would hold them up until the quantiser needs
+    // them (2 us on 5 120 inputs); the smaller ones ask for their tiles first.
+    constexpr int NORM_REGS = 2;
+    float4 wreg[NORM_REGS];
+    auto norm_weights = [&]() {
+#pragma unroll
+        for (int k = 0; k < NORM_REGS; k++) {
+            const int i4 = k * T + tid;
+            wreg[k] = i4 < (K >> 2) ? reinterpret_cast<const float4*>(pa.normw)[i4] : make_float4(1.f, 1.f, 1.f, 1.f);
+        }
+    };
+    if (T == GEMV_THREADS && has_norm) norm_weights();
+
     // Weights do not depend on the previous kernel: every warp requests its first tiles at once.  (Requesting
     // the tiles of a large CTA only after its vector has arrived was measured: the vector then lands within
     // 0.5 us instead of 2-3, but a bulk request costs its issuing thread a third of a microsecond, and paying
@@ -398,7 +421,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             if (reuse) break;
         }
     }
-    if (fseg.m.data && tid == T - 1) {
+    if (f32 && tid == T - 1) {
         // the fp32-route rows are read with plain loads later: have their tiles in L2 by then
         const int r0 = 2 * fseg.sh.begin(cta), r1 = r0 + 2 * fseg.sh.count(cta);
         if (r1 > r0) {
@@ -407,16 +430,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
             bulk_prefetch_l2(fseg.m.data + t0 * Q6_TILE_BYTES, (unsigned)((t1 - t0) * Q6_TILE_BYTES));
         }
     }
-    // RMSNorm weights are constants: fetch them before the wait (K <= 4 * threads on this path)
-    constexpr int NORM_REGS = 2;
-    float4 wreg[NORM_REGS];
-    if (has_norm) {
-#pragma unroll
-        for (int k = 0; k < NORM_REGS; k++) {
-            const int i4 = k * T + tid;
-            wreg[k] = i4 < (K >> 2) ? reinterpret_cast<const float4*>(pa.normw)[i4] : make_float4(1.f, 1.f, 1.f, 1.f);
-        }
-    }
+    if (T != GEMV_THREADS && has_norm) norm_weights();
     if (pa.l2_row_bytes && st && tid == T - 32) {
         // Never in a layer 0: behind the kernel that begins a call the state may not have landed yet.
         const int rows = st->pos + 1, per = (rows + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -433,7 +447,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     // So are the biases of the CTA's rows: fetched by the row sums, they cost the epilogue a trip to L2 per matrix (1 us).
     float biasv = 0.f;
     bool bias_pre = false;
-    const int rows_f = Epi::STAGES_BIAS && fseg.m.data ? 2 * fseg.sh.count(cta) : 0;
+    const int rows_f = Epi::STAGES_BIAS && f32 ? 2 * fseg.sh.count(cta) : 0;
     if constexpr (Epi::STAGES_BIAS) {
         bias_pre = epi.bias && rows_a + rows_b + rows_f <= 256;
         if (bias_pre && tid < rows_a + rows_b + rows_f)
@@ -452,7 +466,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     const int done = st ? st->done : 0;
     // residual values of this CTA's rows (pair-ordered epilogues only), one per thread
     const int res_row0 = 2 * (ja.id_base + (rows_a0 >> 1));
-    const bool res_pre = Epi::MODE == EPI_PAIRS && epi.wants_residual() && rows_a <= 256 && rows_b == 0 && !fseg.m.data;
+    const bool res_pre = Epi::MODE == EPI_PAIRS && epi.wants_residual() && rows_a <= 256 && rows_b == 0 && !f32;
     float resv = 0.f;
     if (res_pre && tid < rows_a) resv = epi.residual(res_row0 + tid);
     constexpr int STAGE_REGS = 6;  // float4 per thread and pass: one pass up to K = 12288
@@ -513,7 +527,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                         x.y = x.y * scale * w.y;
                         x.z = x.z * scale * w.z;
                         x.w = x.w * scale * w.w;
-                        if (fseg.m.data) *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = x;
+                        if (f32) *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = x;
                     }
                 }
                 act_quantize4(act, x, i4, on, nb);
@@ -555,10 +569,10 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     // block partials of the tiles (the usual case: a CTA holds one or two V row pairs), the tasks run side by side
     // with the tile dots — taken from the last thread downwards, so the few warps that own tiles keep to their tiles —
     // and share the tile dots' barrier; otherwise they run first, chunk by chunk, with barriers of their own.
-    const int f32_tasks = fseg.m.data ? 2 * fseg.sh.count(cta) * 16 * nb : 0;
+    const int f32_tasks = f32 ? 2 * fseg.sh.count(cta) * 16 * nb : 0;
     const int f32_off = blocks_a + blocks_b;
     const bool f32_fused = f32_tasks > 0 && f32_off + f32_tasks <= pbuf_floats;
-    if (fseg.m.data && !f32_fused) {
+    if (f32 && !f32_fused) {
         const int np = fseg.sh.count(cta), pbase = fseg.sh.begin(cta);
         const int per_row = 16 * nb, tasks = 2 * np * per_row;
         const int chunk = (pbuf_floats / (2 * per_row)) * (2 * per_row);  // whole row pairs per chunk
@@ -569,7 +583,11 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                 const int row_l = task / per_row, rem = task - row_l * per_row;
                 const int row_g = 2 * pbase + row_l;
                 float v = 0.f;
-                if (row_g < fseg.m.N) v = q6k_run_dot_f32(fseg.m, mat_flat(nb, row_g, rem >> 4), rem >> 4, rem & 15, xs);
+                if (row_g < fseg.m.N) {
+                    Q6Run run;
+                    run.load(fseg.m, mat_flat(nb, row_g, rem >> 4), rem & 15);
+                    v = run.dot(xs + xs_idx(16 * rem));
+                }
                 pbuf[t] = v;
             }
             __syncthreads();
@@ -630,12 +648,19 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     }
     if (f32_fused) {
         const int pbase = fseg.sh.begin(cta), per_row = 16 * nb;
-        for (int t = T - 1 - tid; t < f32_tasks; t += T) {
-            const int row_l = t / per_row, rem = t - row_l * per_row;
-            const int row_g = 2 * pbase + row_l;
-            float v = 0.f;
-            if (row_g < fseg.m.N) v = q6k_run_dot_f32(fseg.m, mat_flat(nb, row_g, rem >> 4), rem >> 4, rem & 15, xs);
-            pbuf[f32_off + t] = v;
+        // two runs of a thread in flight: their words come from L2
+        for (int t = T - 1 - tid; t < f32_tasks; t += 2 * T) {
+            Q6Run run[2];
+            int rem[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int ti = min(t + i * T, f32_tasks - 1), row_l = ti / per_row;
+                rem[i] = ti - row_l * per_row;
+                run[i].load(fseg.m, mat_flat(nb, min(2 * pbase + row_l, fseg.m.N - 1), rem[i] >> 4), rem[i] & 15);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                if (t + i * T < f32_tasks) pbuf[f32_off + t + i * T] = run[i].dot(xs + xs_idx(16 * rem[i]));
         }
     }
     if (!ok && st) st->err = 2;  // a bulk copy never completed: results of this step are invalid
@@ -696,7 +721,12 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     constexpr int TB = BLK::TILE_BYTES;
     const int ra = ja.rows_max(), rb = jb.m.data ? jb.rows_max() : 0;
     int pf = gemv_pbuf_floats(ra, rb, nb);
-    if (fseg.m.data && pf < 2 * 16 * nb) pf = 2 * 16 * nb;
+    if (fseg.m.data) {
+        // room for the fp32-route rows' partials beside the tiles': without it they run by the piece, two barriers each
+        // (four of them, 8 us, for the 1 024 V rows of 5 120)
+        const int beside = (ra + rb) * nb + 2 * (fseg.sh.quot + 1) * 16 * nb;
+        pf = std::max(pf, beside <= 8192 ? (beside + 3) & ~3 : 2 * 16 * nb);
+    }
     const bool has_norm = pa.normw != nullptr;
     const bool with_xf = has_norm || fseg.m.data != nullptr || pa.vec == nullptr;  // as in the kernel
     const size_t fixed = gemv_smem_fixed(K, with_xf, pf);
