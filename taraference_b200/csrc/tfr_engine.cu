@@ -283,20 +283,32 @@ static void configure_kernels_once() {
     if (done[dev]) return;
     done[dev] = true;
     configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_SMALL>, true);
     configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_MID>, true);
     configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_SMALL>, true);
     configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_MID>, true);
     configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_SMALL>, true);
     configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_MID>, true);
     configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_SMALL>, true);
     configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_MID>, true);
     configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_SMALL>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_SMALL>, true);
     configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_MID>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_MID>, true);
     configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ8, EpiLogits, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ8, EpiAllReduce, GEMV_THREADS>, true);
     configure_kernel(k_gemv<BlockQ4, EpiAllReduce, GEMV_THREADS>, true);
@@ -1419,7 +1431,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
         pa.prof_id = n;
         const RowJob job = make_job(w->m, cap);
         if (P.tp == 1) {
-            EpiStore epi{e->x, nullptr, 2, K};
+            EpiResidual epi{{e->x, nullptr, 2, K}};
             return launch_typed(s, cap, w->m.type, pa, job, RowJob{}, F32Seg{}, epi, width, e->st);
         }
         if (e->use_nccl) {
@@ -1560,7 +1572,9 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             epi.hd = hd;
             epi.kvdim = nkv;
             epi.theta = c.rope_theta;
-            if (launch_gemv<BlockQ4, EpiQkv>(s, cap, pn, jq, jk, fseg, epi, K, e->st) != cudaSuccess) return -1;
+            const cudaError_t qkv = li == 0 ? launch_gemv<BlockQ4, EpiQkvFirst>(s, cap, pn, jq, jk, fseg, EpiQkvFirst{epi}, K, e->st)
+                                            : launch_gemv<BlockQ4, EpiQkv>(s, cap, pn, jq, jk, fseg, epi, K, e->st);
+            if (qkv != cudaSuccess) return -1;
             n++;
             // 2. attention
             a.prof_id = n;

@@ -16,6 +16,7 @@ namespace tfr {
 
 // y = W x (+y) (+bias): kernels/gemv.cu:367-373 residual rule (2 = accumulate in place).
 struct EpiStore {
+    static constexpr bool EMBED = true, NORM = true;
     static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
@@ -49,6 +50,7 @@ struct EpiStore {
 
 // h = silu(gate.x) * (up.x), kernels/gemv.cu:2570-2574.  Pair p = (gate row p, up row p).
 struct EpiSilu {
+    static constexpr bool EMBED = false, NORM = true;
     static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
@@ -68,6 +70,7 @@ struct EpiSilu {
 // (kernels/ops.cu:471-486).  Q and K rows were re-ordered at upload so that the RoPE
 // partners (i, i + hd/2) of a head are the two rows of a pair; biases likewise.
 struct EpiQkv {
+    static constexpr bool EMBED = false, NORM = true;
     static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = true;
     static constexpr bool SHARES_SM = true;
@@ -154,6 +157,7 @@ __device__ __forceinline__ void advance_state(TokenState* st, int tok, int* out_
 }
 
 struct EpiLogits {
+    static constexpr bool EMBED = false, NORM = true;
     static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = false;
@@ -229,6 +233,16 @@ struct EpiLogits {
 };
 
 // ------------------------------------------------------------------ the GEMV kernel
+
+// What a kernel instance can meet is part of its epilogue's type, so that it carries no other code (the fp32-route rows' in
+// every kernel cost 2 to 6 % of a token): EMBED: the source may be an embedding row; NORM: a norm may be fused; F32_ROWS:
+// rows on the fp32 route.
+struct EpiQkvFirst : EpiQkv {  // layer 0
+    static constexpr bool EMBED = true;
+};
+struct EpiResidual : EpiStore {  // o-proj, down: plain vector in, sum into the residual stream
+    static constexpr bool EMBED = false, NORM = false, F32_ROWS = false;
+};
 
 struct PrepArgs {
     const float* vec;     // source vector; nullptr -> embedding row of TokenState::token
@@ -353,10 +367,10 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     const bool f32 = Epi::F32_ROWS && std::is_same<BLK, BlockQ4>::value && fseg.m.data != nullptr;
     prof_mark(0, pa.prof_id);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x;
-    const bool has_norm = pa.normw != nullptr;
+    const bool has_norm = Epi::NORM && pa.normw != nullptr, embed = Epi::EMBED && pa.vec == nullptr;
     // the fp32 copy of the vector is staged only where something reads it back: the norm's reduction,
     // the fp32-route rows, the embedding source
-    const bool with_xf = has_norm || f32 || pa.vec == nullptr;
+    const bool with_xf = has_norm || f32 || embed;
     Epi epi = epi_in;
     Act act = act_carve(smem, K, with_xf, false);
     const size_t act_bytes = (act_smem_bytes(K, with_xf, false) + 15) & ~(size_t)15;
@@ -384,7 +398,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     };
     // Tile j of the CTA belongs to warp j % stride.  Without reuse every tile has its own slot; with
     // reuse (more tiles than slots) warp w owns slot w and walks its tiles through it in order.
-    const bool reuse = n_jobs > slots;
+    const bool reuse = T == GEMV_THREADS && n_jobs > slots;  // smaller CTAs are launched with a slot for every tile
     const int stride = reuse ? slots : W;
     auto issue = [&](int j) {
         const int s = reuse ? warp : j;
@@ -472,7 +486,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     constexpr int STAGE_REGS = 6;  // float4 per thread and pass: one pass up to K = 12288
     const int n4 = K >> 2;
     float scale = 1.f;
-    if (pa.vec && !with_xf) {
+    if (!embed && !with_xf) {
         // plain vector: quantise pass by pass straight from the registers that fetched it
         if (!done) {
             for (int base = 0; base < n4; base += STAGE_REGS * T) {
@@ -492,7 +506,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         prof_mark(2, pa.prof_id);
         prof_mark(6, pa.prof_id);
     } else {
-        if (pa.vec) {
+        if (!embed) {
             for (int i4 = tid; i4 < n4; i4 += T)
                 *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = reinterpret_cast<const float4*>(pa.vec)[i4];
         } else {
