@@ -16,7 +16,7 @@ namespace tfr {
 
 // y = W x (+y) (+bias): kernels/gemv.cu:367-373 residual rule (2 = accumulate in place).
 struct EpiStore {
-    static constexpr bool EMBED = true, NORM = true;
+    static constexpr bool EMBED = true, NORM = true, TWO = true;
     static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
@@ -50,7 +50,7 @@ struct EpiStore {
 
 // h = silu(gate.x) * (up.x), kernels/gemv.cu:2570-2574.  Pair p = (gate row p, up row p).
 struct EpiSilu {
-    static constexpr bool EMBED = false, NORM = true;
+    static constexpr bool EMBED = false, NORM = true, TWO = true;
     static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
@@ -70,7 +70,7 @@ struct EpiSilu {
 // (kernels/ops.cu:471-486).  Q and K rows were re-ordered at upload so that the RoPE
 // partners (i, i + hd/2) of a head are the two rows of a pair; biases likewise.
 struct EpiQkv {
-    static constexpr bool EMBED = false, NORM = true;
+    static constexpr bool EMBED = false, NORM = true, TWO = true;
     static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = true;
     static constexpr bool SHARES_SM = true;
@@ -157,7 +157,7 @@ __device__ __forceinline__ void advance_state(TokenState* st, int tok, int* out_
 }
 
 struct EpiLogits {
-    static constexpr bool EMBED = false, NORM = true;
+    static constexpr bool EMBED = false, NORM = true, TWO = true;
     static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = false;
@@ -236,12 +236,12 @@ struct EpiLogits {
 
 // What a kernel instance can meet is part of its epilogue's type, so that it carries no other code (the fp32-route rows' in
 // every kernel cost 2 to 6 % of a token): EMBED: the source may be an embedding row; NORM: a norm may be fused; F32_ROWS:
-// rows on the fp32 route.
+// rows on the fp32 route; TWO: a second matrix.
 struct EpiQkvFirst : EpiQkv {  // layer 0
     static constexpr bool EMBED = true;
 };
 struct EpiResidual : EpiStore {  // o-proj, down: plain vector in, sum into the residual stream
-    static constexpr bool EMBED = false, NORM = false, F32_ROWS = false;
+    static constexpr bool EMBED = false, NORM = false, F32_ROWS = false, TWO = false;
 };
 
 struct PrepArgs {
@@ -385,7 +385,8 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
 
     // flat block ranges of this CTA in A and B, and the tiles that cover them
     const int rows_a0 = ja.row0(cta), rows_a = max(0, ja.rows(cta)), blocks_a = group_rows(rows_a) * nb;
-    const int rows_b0 = jb.m.data ? jb.row0(cta) : 0, rows_b = jb.m.data ? max(0, jb.rows(cta)) : 0, blocks_b = group_rows(rows_b) * nb;
+    const bool two = Epi::TWO && jb.m.data != nullptr;
+    const int rows_b0 = two ? jb.row0(cta) : 0, rows_b = two ? max(0, jb.rows(cta)) : 0, blocks_b = group_rows(rows_b) * nb;
     const long long fa0 = (long long)rows_a0 * nb, fa1 = fa0 + blocks_a;
     const long long fb0 = (long long)rows_b0 * nb, fb1 = fb0 + blocks_b;
     const int ta0 = (int)(fa0 >> 5), tiles_a = rows_a > 0 ? (int)((fa1 + 31) >> 5) - ta0 : 0;
@@ -483,7 +484,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     const bool res_pre = Epi::MODE == EPI_PAIRS && epi.wants_residual() && rows_a <= 256 && rows_b == 0 && !f32;
     float resv = 0.f;
     if (res_pre && tid < rows_a) resv = epi.residual(res_row0 + tid);
-    constexpr int STAGE_REGS = 6;  // float4 per thread and pass: one pass up to K = 12288
+    constexpr int STAGE_REGS = T == GEMV_THREADS ? 6 : 4;  // float4 per thread and pass: one pass up to K = 24 576, 12 288 and 6 144
     const int n4 = K >> 2;
     float scale = 1.f;
     if (!embed && !with_xf) {
@@ -586,7 +587,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     const int f32_tasks = f32 ? 2 * fseg.sh.count(cta) * 16 * nb : 0;
     const int f32_off = blocks_a + blocks_b;
     const bool f32_fused = f32_tasks > 0 && f32_off + f32_tasks <= pbuf_floats;
-    if (f32 && !f32_fused) {
+    if (T == GEMV_THREADS && f32 && !f32_fused) {
         const int np = fseg.sh.count(cta), pbase = fseg.sh.begin(cta);
         const int per_row = 16 * nb, tasks = 2 * np * per_row;
         const int chunk = (pbuf_floats / (2 * per_row)) * (2 * per_row);  // whole row pairs per chunk
@@ -699,8 +700,10 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     if (Epi::MODE == EPI_ZIP) {
         reduce_rows<EPI_ZIP, W>(part_a, part_b, rows_a, nb, ja.id_base + rows_a0, epi);
     } else {
-        reduce_rows<EPI_PAIRS, W>(part_a, part_a, rows_a, nb, ja.id_base + (rows_a0 >> 1), epi);
-        if (rows_b > 0) reduce_rows<EPI_PAIRS, W>(part_b, part_b, rows_b, nb, jb.id_base + (rows_b0 >> 1), epi, W / 2);
+#pragma unroll 1
+        for (int m = 0; m < (Epi::TWO && rows_b > 0 ? 2 : 1); m++)  // one copy of the code
+            reduce_rows<EPI_PAIRS, W>(m ? part_b : part_a, nullptr, m ? rows_b : rows_a, nb, m ? jb.id_base + (rows_b0 >> 1) : ja.id_base + (rows_a0 >> 1),
+                                      epi, m ? W / 2 : 0);
     }
     epi.end(st);
     if (late_slot >= 0) mbar_wait(full + late_slot, late_parity);  // bounded: a second limit, then the CTA leaves regardless
@@ -756,9 +759,10 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     const size_t smem = fixed + (size_t)slots * 8 + 256 + (size_t)slots * TB;
     if constexpr (Epi::SHARES_SM) {
         const int f32_tasks = fseg.m.data ? 2 * (fseg.sh.quot + 1) * 16 * nb : 0;
-        if (resident && need <= GEMV_SMALL / 32 && f32_tasks <= 2 * GEMV_SMALL && K <= 4 * 4 * GEMV_SMALL && smem <= GEMV_SMALL_SMEM)
+        const bool f32_beside = (ra + rb) * nb + f32_tasks <= pf;
+        if (resident && f32_beside && need <= GEMV_SMALL / 32 && f32_tasks <= 2 * GEMV_SMALL && K <= 4 * 4 * GEMV_SMALL && smem <= GEMV_SMALL_SMEM)
             return launch_pdl(k_gemv<BLK, Epi, GEMV_SMALL>, dim3(grid), dim3(GEMV_SMALL), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
-        if (resident && smem <= GEMV_MID_SMEM)
+        if (resident && f32_beside && smem <= GEMV_MID_SMEM)
             return launch_pdl(k_gemv<BLK, Epi, GEMV_MID>, dim3(grid), dim3(GEMV_MID), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
     }
     return launch_pdl(k_gemv<BLK, Epi, GEMV_THREADS>, dim3(grid), dim3(GEMV_THREADS), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
