@@ -282,39 +282,57 @@ static void configure_kernels_once() {
     const int dev = current_device_slot();
     if (done[dev]) return;
     done[dev] = true;
-    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_SMALL>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_MID>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiLogits, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ8, EpiAllReduce, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiAllReduce, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiAllReduce, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ4, EpiLogits, GEMV_THREADS>, true);
-    configure_kernel(k_gemv<BlockQ6, EpiLogits, GEMV_THREADS>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_SMALL, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_SMALL, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_MID, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_MID, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkv, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiQkvFirst, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_SMALL, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_MID, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiStore, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiResidual, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_SMALL, true>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_MID, true>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiStore, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiResidual, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiSilu, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_SMALL, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_SMALL, true>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_MID, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_MID, true>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiStore, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiResidual, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiLogits, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiLogits, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ8, EpiAllReduce, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiAllReduce, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiAllReduce, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiLogits, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ4, EpiLogits, GEMV_THREADS, true>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiLogits, GEMV_THREADS, false>, true);
+    configure_kernel(k_gemv<BlockQ6, EpiLogits, GEMV_THREADS, true>, true);
 #ifdef TFR_TEST_AIDS
     configure_kernel(k_int_dots<BlockQ8>, true);
     configure_kernel(k_int_dots<BlockQ4>, true);

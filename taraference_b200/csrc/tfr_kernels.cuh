@@ -16,7 +16,7 @@ namespace tfr {
 
 // y = W x (+y) (+bias): kernels/gemv.cu:367-373 residual rule (2 = accumulate in place).
 struct EpiStore {
-    static constexpr bool EMBED = true, NORM = true, TWO = true;
+    static constexpr bool EMBED = true, NORM = true, TWO = true, ROW_TILES = false;
     static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
@@ -50,7 +50,7 @@ struct EpiStore {
 
 // h = silu(gate.x) * (up.x), kernels/gemv.cu:2570-2574.  Pair p = (gate row p, up row p).
 struct EpiSilu {
-    static constexpr bool EMBED = false, NORM = true, TWO = true;
+    static constexpr bool EMBED = false, NORM = true, TWO = true, ROW_TILES = false;
     static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = true;
@@ -70,7 +70,7 @@ struct EpiSilu {
 // (kernels/ops.cu:471-486).  Q and K rows were re-ordered at upload so that the RoPE
 // partners (i, i + hd/2) of a head are the two rows of a pair; biases likewise.
 struct EpiQkv {
-    static constexpr bool EMBED = false, NORM = true, TWO = true;
+    static constexpr bool EMBED = false, NORM = true, TWO = true, ROW_TILES = true;
     static constexpr bool F32_ROWS = true;
     static constexpr bool STAGES_BIAS = true;
     static constexpr bool SHARES_SM = true;
@@ -157,7 +157,7 @@ __device__ __forceinline__ void advance_state(TokenState* st, int tok, int* out_
 }
 
 struct EpiLogits {
-    static constexpr bool EMBED = false, NORM = true, TWO = true;
+    static constexpr bool EMBED = false, NORM = true, TWO = true, ROW_TILES = true;
     static constexpr bool F32_ROWS = false;
     static constexpr bool STAGES_BIAS = false;
     static constexpr bool SHARES_SM = false;
@@ -236,12 +236,12 @@ struct EpiLogits {
 
 // What a kernel instance can meet is part of its epilogue's type, so that it carries no other code (the fp32-route rows' in
 // every kernel cost 2 to 6 % of a token): EMBED: the source may be an embedding row; NORM: a norm may be fused; F32_ROWS:
-// rows on the fp32 route; TWO: a second matrix.
+// rows on the fp32 route; TWO: a second matrix; ROW_TILES: an instance exists for rows of eight blocks (below).
 struct EpiQkvFirst : EpiQkv {  // layer 0
     static constexpr bool EMBED = true;
 };
 struct EpiResidual : EpiStore {  // o-proj, down: plain vector in, sum into the residual stream
-    static constexpr bool EMBED = false, NORM = false, F32_ROWS = false, TWO = false;
+    static constexpr bool EMBED = false, NORM = false, F32_ROWS = false, TWO = false, ROW_TILES = true;
 };
 
 struct PrepArgs {
@@ -358,7 +358,10 @@ __device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, in
 // after a single barrier, rows are summed in a fixed order and handed to the epilogue.  When
 // the CTA has more tiles than slots (the vocabulary head), a warp owns one slot and refills
 // it itself after each tile.
-template <class BLK, class Epi, int T>
+// WHOLE: rows of eight blocks (2 048 inputs), where a tile is a whole row group.  A warp then sums its tile's four rows by
+// shuffles, in reduce_rows' order of additions, and hands them to the epilogue: no partials, no barrier, and the vocabulary
+// head's row sums run under its stream instead of behind it (7 us).
+template <class BLK, class Epi, int T, bool WHOLE>
 __global__ void __maxnreg__(gemv_regs(T))
 k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pbuf_floats, int slots, TokenState* st) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -642,7 +645,16 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
                 late_slot = s;
                 late_parity = reuse ? (it & 1) : 0;
             }
-            if (mine) {
+            if constexpr (WHOLE) {
+                float v = mine && landed ? block_dot<true>(BLK{}, ring + (size_t)s * TB, lane, act, lane / ROW_GROUP, nb, nullptr) : 0.f;
+                v += __shfl_xor_sync(TFR_FULL_MASK, v, 16);
+                v += __shfl_xor_sync(TFR_FULL_MASK, v, 8);
+                v += __shfl_xor_sync(TFR_FULL_MASK, v, 4);
+                const float other = __shfl_down_sync(TFR_FULL_MASK, v, 1);
+                const int row = ROW_GROUP * (is_b ? j - tiles_a : j) + lane;
+                if ((lane == 0 || lane == 2) && row < (is_b ? rows_b : rows_a))
+                    epi.apply((is_b ? jb.id_base + (rows_b0 >> 1) : ja.id_base + (rows_a0 >> 1)) + (row >> 1), v, other);
+            } else if (mine) {
                 int row, b;
                 flat_row_block((int)(f - (is_b ? fb0 : fa0)), nb, row, b);
                 (is_b ? part_b : part_a)[row * nb + b] = landed ? block_dot<true>(BLK{}, ring + (size_t)s * TB, lane, act, b, nb, nullptr) : 0.f;
@@ -679,7 +691,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         }
     }
     if (!ok && st) st->err = 2;  // a bulk copy never completed: results of this step are invalid
-    __syncthreads();
+    if (!WHOLE || f32_fused) __syncthreads();
     prof_mark(4, pa.prof_id);
     if (f32_fused) {
         // the same sums as the stand-alone route: lanes stride over a row's runs, then the warp tree
@@ -697,7 +709,8 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
         }
     }
     // phase B: row sums in a fixed order + epilogue
-    if (Epi::MODE == EPI_ZIP) {
+    if constexpr (WHOLE) {
+    } else if (Epi::MODE == EPI_ZIP) {
         reduce_rows<EPI_ZIP, W>(part_a, part_b, rows_a, nb, ja.id_base + rows_a0, epi);
     } else {
 #pragma unroll 1
@@ -757,15 +770,23 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     else if (slots > GEMV_WARPS) slots = GEMV_WARPS;  // reuse: one slot per warp
     if (slots < 1) slots = 1;
     const size_t smem = fixed + (size_t)slots * 8 + 256 + (size_t)slots * TB;
+    auto launch = [&](auto threads, auto whole) {
+        constexpr int T = decltype(threads)::value;
+        return launch_pdl(k_gemv<BLK, Epi, T, decltype(whole)::value>, dim3(grid), dim3(T), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+    };
+    auto by_rows = [&](auto threads) {
+        if constexpr (Epi::ROW_TILES)
+            if (ROW_GROUP * nb == 32) return launch(threads, std::true_type{});
+        return launch(threads, std::false_type{});
+    };
     if constexpr (Epi::SHARES_SM) {
         const int f32_tasks = fseg.m.data ? 2 * (fseg.sh.quot + 1) * 16 * nb : 0;
         const bool f32_beside = (ra + rb) * nb + f32_tasks <= pf;
         if (resident && f32_beside && need <= GEMV_SMALL / 32 && f32_tasks <= 2 * GEMV_SMALL && K <= 4 * 4 * GEMV_SMALL && smem <= GEMV_SMALL_SMEM)
-            return launch_pdl(k_gemv<BLK, Epi, GEMV_SMALL>, dim3(grid), dim3(GEMV_SMALL), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
-        if (resident && f32_beside && smem <= GEMV_MID_SMEM)
-            return launch_pdl(k_gemv<BLK, Epi, GEMV_MID>, dim3(grid), dim3(GEMV_MID), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+            return by_rows(std::integral_constant<int, GEMV_SMALL>{});
+        if (resident && f32_beside && smem <= GEMV_MID_SMEM) return by_rows(std::integral_constant<int, GEMV_MID>{});
     }
-    return launch_pdl(k_gemv<BLK, Epi, GEMV_THREADS>, dim3(grid), dim3(GEMV_THREADS), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+    return by_rows(std::integral_constant<int, GEMV_THREADS>{});
 }
 
 inline RowJob make_job(const Mat& m, int C, int id_base = 0) {

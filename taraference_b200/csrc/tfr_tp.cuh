@@ -82,7 +82,7 @@ __device__ __forceinline__ bool tp_wait_cell(const uint4* cell, unsigned epoch, 
 // Row-parallel epilogue: x += sum over ranks of (W_rank . act_rank), kernels/gemv.cu:367-373 residual
 // rule (2 = accumulate in place) applied once to the reduced sum.
 struct EpiAllReduce {
-    static constexpr bool SHARES_SM = false, STAGES_BIAS = false, F32_ROWS = false, EMBED = false, NORM = false, TWO = false;
+    static constexpr bool SHARES_SM = false, STAGES_BIAS = false, F32_ROWS = false, EMBED = false, NORM = false, TWO = false, ROW_TILES = false;
     static constexpr int MODE = EPI_PAIRS;
     float* x;          // [n_rows] replicated residual stream, updated in place
     int n_rows;
