@@ -281,10 +281,9 @@ struct F32Seg {
 
 // Shared-memory map of k_gemv:
 //   [ Act | partial sums (pbuf_floats) | 272 floats | full[slots] mbarriers | tile slots ].
-// One CTA owns an SM (1024 threads, nearly all shared memory): 32 warps and up to ~46 tile slots
-// keep the dot phase at HBM speed.  (Half-SM CTAs, which would let the next kernel's CTA sit
-// beside this one and prefetch, were measured slower: fewer warps and slots cost more than the
-// overlap gained.)  Kernels are chained with programmatic stream serialisation: a CTA requests
+// A large CTA owns an SM (1024 threads, nearly all shared memory): 32 warps and up to ~46 tile slots
+// keep the dot phase at HBM speed.  (Half an SM for every CTA was measured
+// slower: fewer warps and slots cost more than the overlap gained.)  Kernels are chained with programmatic stream serialisation: a CTA requests
 // its weight tiles, then sleeps in griddepcontrol.wait until the previous kernel's results are
 // complete, so launch latency and the first tiles' fetch hide behind the predecessor's tail.
 constexpr size_t GEMV_SMEM_MAX = 225 * 1024;  // opt-in limit is 227 KB including the kernels' small static arrays
@@ -349,7 +348,7 @@ __device__ __forceinline__ void reduce_rows(const float* pa, const float* pb, in
     }
 }
 
-// One CTA of 1024 threads per SM.  The weight tiles of the CTA's rows are pulled into
+// One CTA per SM (threads: GEMV_SMALL above).  The weight tiles of the CTA's rows are pulled into
 // shared memory by bulk copies (TMA, one 4.5 / 6.6 KB request per tile).  Every warp requests
 // its own tiles at kernel entry (one issuing thread cannot keep HBM busy: a thread issues
 // only a few copies per microsecond), so they stream from HBM while all warps stage,
