@@ -10,8 +10,9 @@
 //   k_gemm_q8        every weight tile is brought on chip once per launch and dotted with the activations of up
 //                    to Mt tokens at a time; same block dots, row sums and epilogues as the batch-1 kernels
 //                    (Q8_0 matrices, batches of fewer than five tokens)
-//   k_gemm_tc        the other projections, on the tensor cores (tfr_gemm_tc.cuh, with a k_prep_tc of its own; the
-//                    fp32-route V rows beside it are k_rows_f32)
+//   k_gemm_mma, k_gemm_tc   the other projections, on the tensor cores (tfr_gemm_mma.cuh for small batches, tfr_gemm_tc.cuh
+//                    for larger ones, each with a preparation kernel of its own; the fp32-route V rows beside them are
+//                    k_rows_f32)
 //   k_attn_chunk / k_attn_chunk_mma   causal attention of a tile of query tokens x the query heads of one KV head
 //                    over the f16 cache, on CUDA cores / on the tensor cores (head sizes up to 128)
 //   k_argmax_rows    greedy token of every row                                        (kernels/ops.cu:601-629)
