@@ -234,7 +234,8 @@ float tfr_last_device_ms(const tfr_engine* e);
  * "k"/"v" = cache of `layer`, "layer_x" = residual stream after every layer; the first "layer_x"
  * request switches that tap on for later steps and returns zeros).  "layer_attn", "layer_mid", "layer_h" (dense
  * single-GPU models, chained kernels): per layer the attention output, the residual stream after the output
- * projection and SiLU*mul, i.e. the vectors a layer rounds to int8 besides its input; switched on the same way. */
+ * projection and SiLU*mul, i.e. the vectors a layer rounds to int8 besides its input; switched on the same way.  A prompt
+ * fed in chunks leaves the per-layer vectors of its last token. */
 int tfr_debug_read(tfr_engine* e, tfr_kv* kv, const char* what, int layer, void* out, size_t nbytes);
 
 /* Test aid: when device_buffer != NULL, thread 0 of every CTA of the matrix-vector and attention kernels stores the
@@ -292,6 +293,13 @@ int tfr_op_int_dots(const tfr_mat* w, const int8_t* q8, const float* d8, int32_t
  * b (Q4_K) the 32-group sums exactly as the dots' activation record holds them. */
 #ifdef TFR_TEST_AIDS
 int tfr_op_int_dots_x(const tfr_mat* w, const float* x, int32_t* a, int32_t* b, int8_t* q8_out, void* stream);
+#endif
+/* A batch's projection by itself (test aid): x[M][K] through RMSNorm (norm_w != NULL) and the Q8 quantiser, then out[M][N] =
+ * a x (use_res 2: out += a x), or with b the gate/up pair silu(a x) * (b x).  route: 0 dp4a, 1 mma.sync, 2 tcgen05, -1 the kernel
+ * prompts of M tokens take; TFR_E_UNSUPPORTED where that kernel does not cover the matrix or M.  Allocates and waits. */
+#ifdef TFR_TEST_AIDS
+int tfr_op_project_rows(const tfr_mat* a, const tfr_mat* b, const float* x, int M, const float* norm_w, float eps, int route,
+                        int use_res, float* out, void* stream);
 #endif
 /* attn_flash_partial + attn_flash_reduce, kernels/attn/flash.cu:16-255, for one query token
  * at position pos over cache rows [0, pos].  kc / vc: [max_seq][n_kv*head_dim] f16 bits.  The split-KV scratch

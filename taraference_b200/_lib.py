@@ -40,7 +40,7 @@ def declared_aid_symbols() -> list[str]:
 
 _lib = None
 AID_NAMES = ("tfr_debug_set_timeline", "tfr_debug_set_loop_timeline", "tfr_debug_f32_to_f16", "tfr_op_int_dots",
-             "tfr_op_int_dots_x", "tfr_synth_quantize")
+             "tfr_op_int_dots_x", "tfr_op_project_rows", "tfr_synth_quantize")
 _aids = None
 _use_aids = False
 
@@ -149,6 +149,7 @@ def _load(path: Path, with_aids: bool) -> C.CDLL:
         "tfr_ffn_block_host": (i32, [vp, vp, vp, vp, vp]),
         "tfr_op_int_dots": (i32, [vp, vp, vp, vp, vp, vp]),
         "tfr_op_int_dots_x": (i32, [vp, vp, vp, vp, vp, vp]),
+        "tfr_op_project_rows": (i32, [vp, vp, vp, i32, vp, f32, i32, i32, vp, vp]),
         "tfr_op_attention": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, vp]),
         "tfr_op_attention_noalloc": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, vp]),
         "tfr_op_qkv_rope_store": (i32, [vp] * 8 + [f32, f32, i32, i32, vp, vp, vp, vp]),

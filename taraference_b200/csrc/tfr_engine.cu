@@ -1788,6 +1788,36 @@ static cudaError_t launch_gemm_typed(cudaStream_t s, int grid, int type, const u
     return launch_gemm<BlockQ6>(s, grid, act, stride, xn, M, ja, jb, fseg, epi, K, st);
 }
 
+// What a batch's projections read and report through: the activations in the form of the kernel that follows, the error word.
+struct BatchBufs {
+    unsigned char* image;  // GEMM_TC, GEMM_MMA
+    unsigned char* act;    // GEMM_DP4A: Act arrays, act_stride bytes apart
+    size_t act_stride;
+    float* tscale;
+    TokenState* st;
+};
+// M rows of x -> RMSNorm (optional) -> Q8, in the form the projections of `route` read
+static cudaError_t batch_prep(cudaStream_t s, int route, int type, const float* x, int width, int M, const float* normw, float eps,
+                              const BatchBufs& b, float* xn) {
+    if (route == GEMM_TC) {
+        PrepTcArgs a{x, width, width, M, normw, eps, b.image, b.tscale, xn};
+        return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(TC_PREP_THREADS), tc_prep_smem(width), s, a);
+    }
+    if (route == GEMM_MMA) {
+        PrepMmaArgs a{x, width, width, M, normw, eps, b.image, xn, type == TFR_Q6_K};
+        return launch_pdl(k_prep_mma, dim3((M + 15) & ~15), dim3(MMA_PREP_THREADS), normw ? tc_prep_smem(width) : 0, s, a);
+    }
+    PrepRowsArgs a{x, width, width, normw, eps, b.act, b.act_stride, xn};
+    const size_t smem = normw ? (xs_floats(width) + 272) * sizeof(float) : 0;
+    return launch_pdl(k_prep_rows, dim3(M), dim3(GEMV_THREADS), smem, s, a);
+}
+// out = epilogue(W x) over them; jb: the second matrix of a gate/up pair or one that follows
+static cudaError_t batch_gemm(cudaStream_t s, int sms, int route, int M, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep, const BatchBufs& b) {
+    if (route == GEMM_TC) return launch_gemm_tc(s, sms, b.image, b.tscale, M, ja, jb, ep, b.st);
+    if (route == GEMM_MMA) return launch_gemm_mma(s, sms, b.image, M, ja, jb, ep, b.st);
+    return launch_gemm_typed(s, sms, ja.m.type, b.act, b.act_stride, nullptr, M, ja, jb, F32Seg{}, ep, ja.m.K, b.st);
+}
+
 // M tokens (device ids at tok) at positions pos0 .. pos0 + M - 1 through all layers: their K / V rows land in the
 // cache and e->cx holds their residual streams.  rec0: tokens the recurrent state (hybrid models) has absorbed before
 // them.  all_rows: also the greedy token after every position, to
@@ -1799,31 +1829,19 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     const int cap = e->prop.multiProcessorCount;
     cudaStream_t s = e->stream;
     int n = 0;
-    // x -> RMSNorm (optional) -> Q8, in the form the projections that follow read
-    auto prep = [&](int route, int type, const float* x, int ldx, int width, const float* normw, float* xn) -> cudaError_t {
+    const BatchBufs bufs{e->cimage, e->cact, e->cact_stride, e->ctscale, e->st};
+    auto prep = [&](int route, int type, const float* x, int width, const float* normw, float* xn) -> cudaError_t {
         n++;
-        if (route == GEMM_TC) {
-            PrepTcArgs a{x, ldx, width, M, normw, c.rms_eps, e->cimage, e->ctscale, xn};
-            return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(TC_PREP_THREADS), tc_prep_smem(width), s, a);
-        }
-        if (route == GEMM_MMA) {
-            PrepMmaArgs a{x, ldx, width, M, normw, c.rms_eps, e->cimage, xn, type == TFR_Q6_K};
-            return launch_pdl(k_prep_mma, dim3((M + 15) & ~15), dim3(MMA_PREP_THREADS), normw ? tc_prep_smem(width) : 0, s, a);
-        }
-        PrepRowsArgs a{x, ldx, width, normw, c.rms_eps, e->cact, e->cact_stride, xn};
-        const size_t smem = normw ? (xs_floats(width) + 272) * sizeof(float) : 0;
-        return launch_pdl(k_prep_rows, dim3(M), dim3(GEMV_THREADS), smem, s, a);
+        return batch_prep(s, route, type, x, width, M, normw, c.rms_eps, bufs, xn);
     };
     auto gemm = [&](int route, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep) -> cudaError_t {
         n++;
-        if (route == GEMM_TC) return launch_gemm_tc(s, cap, e->cimage, e->ctscale, M, ja, jb, ep, e->st);
-        if (route == GEMM_MMA) return launch_gemm_mma(s, cap, e->cimage, M, ja, jb, ep, e->st);
-        return launch_gemm_typed(s, cap, ja.m.type, e->cact, e->cact_stride, nullptr, M, ja, jb, F32Seg{}, ep, ja.m.K, e->st);
+        return batch_gemm(s, cap, route, M, ja, jb, ep, bufs);
     };
     // RMSNorm + Q8 + W x + epilogue
     auto project = [&](const float* x, int width, const float* normw, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep) -> cudaError_t {
         const int route = gemm_route(ja.m.type, ja.m.nb, M);
-        const cudaError_t r = prep(route, ja.m.type, x, width, width, normw, nullptr);
+        const cudaError_t r = prep(route, ja.m.type, x, width, normw, nullptr);
         return r != cudaSuccess ? r : gemm(route, ja, jb, ep);
     };
     auto store_epi = [&](float* out, int ldo, int rows, int use_res) {
@@ -1867,7 +1885,7 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
         const bool gated = L.kind == LAYER_FULL_GATED;
         const int route = gemm_route(TFR_Q4_K, L.wq->m.nb, M);
         const int q_rows = gated ? 2 * nq : nq;
-        if (prep(route, TFR_Q4_K, e->cx, K, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
+        if (prep(route, TFR_Q4_K, e->cx, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
         {
             const RowJob jq = make_job(L.wq->m, cap, 0), jk = make_job(L.wk->m, cap, q_rows / 2);
             F32Seg fseg{};
@@ -1948,15 +1966,23 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
             n++;
         }
         }
+        // the last token's vectors, as a decode step's taps hold them
+        auto tap = [&](float* dst, const float* src, int width) {
+            return !dst || cudaMemcpyAsync(dst + (size_t)li * width, src + (size_t)(M - 1) * width, (size_t)width * 4, cudaMemcpyDeviceToDevice, s) == cudaSuccess;
+        };
+        if (!tap(e->tap_attn, e->cattn, P.attn_width)) return -1;
         // 3. Q8 + output projection + residual
         if (project(e->cattn, mix_width, nullptr, make_job(wout->m, cap), RowJob{}, store_epi(e->cx, K, K, 2)) != cudaSuccess) return -1;
+        if (!tap(e->tap_mid, e->cx, K)) return -1;
         // 4. RMSNorm + Q8 + gate/up + SiLU*mul
         ChunkEpi ep{};
         ep.kind = CEPI_SILU;
         ep.out = e->ch, ep.ldo = FF;
         if (project(e->cx, K, L.ffn_norm, make_job(L.gate->m, cap), make_job(L.up->m, cap), ep) != cudaSuccess) return -1;
+        if (!tap(e->tap_h, e->ch, FF)) return -1;
         // 5. Q8 + down + residual
         if (project(e->ch, FF, nullptr, make_job(L.down->m, cap), RowJob{}, store_epi(e->cx, K, K, 2)) != cudaSuccess) return -1;
+        if (!tap(e->layer_taps, e->cx, K)) return -1;
     }
     if (all_rows) {
         if (project(e->cx, K, e->output_norm, make_job(e->head->m, cap), RowJob{}, store_epi(e->clogits, V, V, 0)) != cudaSuccess) return -1;
@@ -2518,6 +2544,38 @@ extern "C" int tfr_op_int_dots(const tfr_mat* w, const int8_t* q8, const float* 
 extern "C" int tfr_op_int_dots_x(const tfr_mat* w, const float* x, int32_t* a, int32_t* b, int8_t* q8_out, void* stream) {
     if (!x) return TFR_E_INVALID;
     return int_dots_impl(w, x, nullptr, nullptr, a, b, q8_out, stream);
+}
+
+// Test aid: a batch's projection by itself, by the kernel of `route` (GEMM_DP4A, GEMM_MMA, GEMM_TC; -1: the one the engine takes).
+extern "C" int tfr_op_project_rows(const tfr_mat* a, const tfr_mat* b, const float* x, int M, const float* norm_w, float eps, int route,
+                                   int use_res, float* out, void* stream) {
+    if (!a || !x || !out || M <= 0 || M > CHUNK_MAX_TOKENS || (use_res != 0 && use_res != 2)) return TFR_E_INVALID;
+    if (b && (b->m.K != a->m.K || b->m.N != a->m.N || b->m.type != a->m.type || use_res)) return TFR_E_INVALID;
+    if (route < 0) route = gemm_route(a->m.type, a->m.nb, M);
+    if (route > GEMM_TC || (route != GEMM_DP4A && !tc_type(a->m.type))) return TFR_E_UNSUPPORTED;
+    if (route == GEMM_MMA && (M > (a->m.type == TFR_Q4_K ? MMA_MAX_TOKENS : 32) || mma_tiles(a->m.nb, M) == 0)) return TFR_E_UNSUPPORTED;
+    configure_kernels_once();
+    cudaStream_t s = (cudaStream_t)stream;
+    const int K = a->m.K, sms = sm_count_cached();
+    BatchBufs bufs{};
+    bufs.act_stride = (act_smem_bytes(K, false, false) + 255) & ~(size_t)255;
+    const size_t image = std::max(tc_image_bytes(K, M), mma_image_bytes(K)), parts[4] = {image, bufs.act_stride * M, (size_t)tc_pad_tokens(M) * 4, sizeof(TokenState)};
+    size_t total = 0, at[4];
+    for (int i = 0; i < 4; i++) at[i] = total, total += (parts[i] + 255) & ~(size_t)255;
+    unsigned char* mem = nullptr;
+    if (cudaMalloc(&mem, total) != cudaSuccess) return TFR_E_CUDA;
+    bufs.image = mem + at[0], bufs.act = mem + at[1], bufs.tscale = (float*)(mem + at[2]), bufs.st = (TokenState*)(mem + at[3]);
+    ChunkEpi ep{};
+    ep.kind = b ? CEPI_SILU : CEPI_STORE;
+    ep.out = out, ep.ldo = ep.n_rows = a->m.N, ep.use_res = use_res;
+    TokenState st{};
+    cudaError_t r = cudaMemsetAsync(bufs.st, 0, sizeof(TokenState), s);
+    if (r == cudaSuccess) r = batch_prep(s, route, a->m.type, x, K, M, norm_w, eps, bufs, nullptr);
+    if (r == cudaSuccess) r = batch_gemm(s, sms, route, M, make_job(a->m, sms), b ? make_job(b->m, sms) : RowJob{}, ep, bufs);
+    if (r == cudaSuccess) r = cudaMemcpyAsync(&st, bufs.st, sizeof st, cudaMemcpyDeviceToHost, s);
+    if (r == cudaSuccess) r = cudaStreamSynchronize(s);
+    cudaFree(mem);
+    return r != cudaSuccess || st.err ? TFR_E_CUDA : TFR_OK;
 }
 
 #endif  // TFR_TEST_AIDS

@@ -431,6 +431,12 @@ def op_int_dots_x(w: GpuMat, x, a, b=None, q8_out=None, stream: int = 0) -> None
     _ok(_lib.aids().tfr_op_int_dots_x(w._h, _ptr(x), _ptr(a), _ptr(b), _ptr(q8_out), stream), "int_dots_x")
 
 
+def op_project_rows(a: GpuMat, x, out, m: int, b: GpuMat | None = None, norm_w=None, eps: float = 1e-6, route: int = -1,
+                    use_res: int = 0, stream: int = 0) -> None:
+    _ok(_lib.aids().tfr_op_project_rows(a._h, b._h if b else None, _ptr(x), m, _ptr(norm_w), eps, route, use_res, _ptr(out), stream),
+        "project_rows")
+
+
 def debug_f32_to_f16(src, dst, n: int, stream: int = 0) -> None:
     """Test aid: the KV store's f32 -> f16 rounding over n device floats."""
     _ok(_lib.aids().tfr_debug_f32_to_f16(_ptr(src), _ptr(dst), int(n), stream), "debug_f32_to_f16")

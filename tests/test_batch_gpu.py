@@ -27,26 +27,133 @@ def _state(m, kv, cfg, n):
     return [m.debug_read(w, n * kvdim, np.uint16, kv=kv, layer=0) for w in "kv"]
 
 
+# Sums of the same int8 products by two kernels, of the largest value.  Measured against float64: the tcgen05 forms, whose
+# accumulators truncate, are off by up to 5.5e-6 of a result's rms, the others by 1.6e-6; a largest value is three to four rms.
+# Twice that sum.
+SAME_INT8 = 4e-6
+
+
 @pytest.mark.parametrize("cfg", [ODD, WIDE], ids=["odd", "wide"])
 @pytest.mark.parametrize("n", [5, 16, 17, 32, 33, 48, 80, 81, 128, 129, 224, 256, 257, 640])
-def test_projections_of_batches_at_tile_edges(E, cfg, n, monkeypatch):
+def test_projections_of_batches_at_tile_edges(E, oracle, cfg, n, monkeypatch):
     """One layer, all tokens in one batch: 16- and 32-token paddings, mma.sync up to 80 tokens (Q6_K: 32), the tcgen05 forms, several
-    token tiles, tiles that end inside a column group.  V rows are the same bits, the logits differ by a flip at most."""
-    m = E.CudaModel.load_with(cfg, S.make_dense_model(cfg, seed=31))
+    token tiles, tiles that end inside a column group.  V rows are the dp4a route's bits, K rows the same up to f16 steps.  The last
+    token's vectors are held against the decode kernels stage by stage, each fed the batch's own vector, so that both round the
+    same values to int8 and only the order of the fp32 sums differs."""
+    tens = S.make_dense_model(cfg, seed=31)
+    m = E.CudaModel.load_with(cfg, tens)
+    K, FF, nq = cfg["n_embd"], cfg["n_ff"], cfg["n_head"] * cfg["head_dim"]
+    taps = [("layer_attn", nq), ("layer_mid", K), ("layer_h", FF), ("layer_x", K)]
+    for name, width in taps:
+        m.debug_read(name, width)  # switch the taps on
     prompt = [int(t) for t in np.random.default_rng(n).integers(0, cfg["n_vocab"], n)]
     out = []
     for dp4a in (True, False):
         (monkeypatch.setenv if dp4a else monkeypatch.delenv)(*(("TFR_GEMM_DP4A", "1") if dp4a else ("TFR_GEMM_DP4A",)))
         kv = m.alloc_kv(n + 8)
         m.forward_greedy(prompt, kv)
-        out.append((m.current_logits(), *_state(m, kv, cfg, n)))
+        out.append((*_state(m, kv, cfg, n), [m.debug_read(*t) for t in taps]))
         kv.free()
-    (la, ka, va), (lb, kb, vb) = out
+    (ka, va, ta), (kb, vb, tb) = out
+    logits = m.current_logits()
     assert np.array_equal(va, vb)
     f = lambda a: a.view(np.float16).astype(np.float32)
     assert _rel(f(kb), f(ka)) < 5e-4
-    assert _rel(lb, la) < TF_WORST
+    assert _rel(tb[0], ta[0]) < 1e-4  # K values that fell to the other f16: 5e-4 of the largest, fewer than one in a hundred
+    attn, mid, h, x = (torch.from_numpy(v).cuda() for v in tb)
+    mats = {k: E.GpuMat(*tens[k][:3], tens[k][3]) for k in tens if k == "token_embd.weight" or ("blk" in k and isinstance(tens[k], tuple))}
+    vec = lambda k: torch.from_numpy(tens[k]).cuda()
+    wtype, k, _, raw = tens["token_embd.weight"]
+    row = np.ascontiguousarray(raw.reshape(cfg["n_vocab"], -1)[prompt[-1]])
+    want = [torch.from_numpy(oracle.dequant_rows(wtype, row, k, 1).reshape(-1)).cuda(), torch.empty(FF, device="cuda"), mid.clone(),
+            torch.empty(cfg["n_vocab"], device="cuda")]
+    E.op_gemv(mats["blk.0.attn_output.weight"], attn, want[0], use_res=2)
+    E.op_ffn_gate_up(mats["blk.0.ffn_gate.weight"], mats["blk.0.ffn_up.weight"], mid, want[1], norm_w=vec("blk.0.ffn_norm.weight"), eps=cfg["eps"])
+    E.op_gemv(mats["blk.0.ffn_down.weight"], h, want[2], use_res=2)
+    E.op_gemv(mats["token_embd.weight"], x, want[3], norm_w=vec("output_norm.weight"), eps=cfg["eps"])
+    for name, got, w in zip(("mid", "h", "x", "logits"), (mid, h, x, torch.from_numpy(logits)), want):
+        assert _rel(got.cpu().numpy(), w.cpu().numpy()) < SAME_INT8, name
+    for w in mats.values():
+        w.free()
     m.destroy()
+
+
+def _q4_k_exact(raw, K, N):
+    """GGUF bytes -> float64 weights, exactly (kernels/common.cu:40-84)."""
+    b = raw.reshape(N, K // 256, 144)
+    d, dmin = (b[..., i:i + 2].copy().view(np.float16)[..., 0].astype(np.float64) for i in (0, 2))
+    s = b[..., 4:16].astype(np.int64)
+    sc = np.concatenate([s[..., :4] & 63, (s[..., 8:] & 15) | (s[..., :4] >> 6 << 4)], -1)
+    mn = np.concatenate([s[..., 4:8] & 63, (s[..., 8:] >> 4) | (s[..., 4:8] >> 6 << 4)], -1)
+    q = b[..., 16:].astype(np.int64).reshape(N, K // 256, 4, 32)
+    q = np.stack([q & 15, q >> 4], axis=3).reshape(N, K // 256, 8, 32)
+    return (d[..., None, None] * sc[..., None] * q - (dmin[..., None] * mn)[..., None]).reshape(N, K)
+
+
+def _q6_k_exact(raw, K, N):
+    """GGUF bytes -> float64 weights, exactly (kernels/gemv.cu:302-337)."""
+    b = raw.reshape(N, K // 256, 210)
+    ql, qh = b[..., :128].astype(np.int64).reshape(N, -1, 2, 64), b[..., 128:192].astype(np.int64).reshape(N, -1, 2, 32)
+    sc = b[..., 192:208].copy().view(np.int8).astype(np.float64).reshape(N, -1, 2, 8)
+    w = np.empty((N, K // 256, 2, 128))
+    for j in range(4):
+        q = (ql[..., 32 * (j & 1):32 * (j & 1) + 32] >> (4 * (j >> 1)) & 15) | (qh >> (2 * j) & 3) << 4
+        w[..., 32 * j:32 * j + 32] = sc[..., 2 * j:2 * j + 2].repeat(16, axis=-1) * (q - 32)
+    return (w * b[..., 208:].copy().view(np.float16).astype(np.float64)[..., None]).reshape(N, K)
+
+
+DP4A, MMA, TC = 0, 1, 2
+
+
+def _matrix(E, wtype, K, N, rng, scale=0.02):
+    raw = S.quantize(wtype, (rng.standard_normal((N, K)) * scale).astype(np.float32)).reshape(-1)
+    exact = (_q4_k_exact if wtype == S.Q4_K else _q6_k_exact)(raw, K, N)
+    return E.GpuMat(wtype, K, N, raw), torch.from_numpy(exact).cuda()
+
+
+def _exact_q8(E, x):
+    """The int8 activations and their scales as float64."""
+    M, K = x.shape
+    q8, d8 = torch.empty(M * K, dtype=torch.int8, device="cuda"), torch.empty(M * K // 32, device="cuda")
+    E.op_quantize_q8(x.view(-1), q8, d8)
+    return (q8.view(-1, 32).double() * d8.view(-1, 1).double()).view(M, K)
+
+
+def _errors(E, w, exact, x, routes, **kw):
+    """Relative error (2-norm) of a batch's projection against float64 sums of the same int8 activations, by route."""
+    ref = _exact_q8(E, x) @ exact.T
+    errs = []
+    for route in routes:
+        out = torch.full((x.shape[0], w.N), float("nan"), device="cuda")
+        E.op_project_rows(w, x, out, x.shape[0], route=route, **kw)
+        errs.append(float((out.double() - ref).norm() / ref.norm()))
+    return errs
+
+
+@pytest.mark.parametrize("wtype", [S.Q4_K, S.Q6_K], ids=["q4", "q6"])
+@pytest.mark.parametrize("K,N", [(256, 3), (768, 130), (2816, 257), (11008, 64)])
+def test_projection_routes_agree_on_equal_int8(E, wtype, K, N):
+    """The three projection kernels on the same int8 activations, against float64, where tiles, token paddings, clusters over
+    the k range and pairs of CTAs end; then residuals added, and gate/up pairs with a fused norm."""
+    rng = np.random.default_rng(K + N)
+    w, exact = _matrix(E, wtype, K, N, rng)
+    for M in (5, 16, 17, 32, 33, 80, 81, 128, 129, 257):
+        x = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).cuda()
+        routes = [DP4A, TC] + ([MMA] if M <= (80 if wtype == S.Q4_K else 32) else [])
+        assert max(_errors(E, w, exact, x, routes)) < SAME_INT8, M
+    M, norm = 37, torch.from_numpy(rng.uniform(0.5, 2, K).astype(np.float32)).cuda()
+    x = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).cuda()
+    w2, _ = _matrix(E, wtype, K, N, rng)
+    res = torch.randn((M, N), device="cuda")
+    for kw in (dict(use_res=2), dict(b=w2, norm_w=norm) if K < 4096 else dict(b=w2)):
+        outs = []
+        for route in (DP4A, TC, -1):
+            out = res.clone() if "use_res" in kw else torch.full_like(res, float("nan"))
+            E.op_project_rows(w, x, out, M, route=route, **kw)
+            outs.append(out.cpu().numpy())
+        assert _rel(outs[1], outs[0]) < SAME_INT8 and _rel(outs[2], outs[0]) < SAME_INT8, kw.keys()
+    w.free()
+    w2.free()
 
 
 @pytest.mark.parametrize("chunk,n", [(2, 7), (16, 16), (16, 45), (64, 19), (2048, 41)])
