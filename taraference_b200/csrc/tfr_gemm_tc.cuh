@@ -38,6 +38,15 @@ __host__ __device__ inline size_t tc_image_bytes(int K, int M) {
     return (size_t)(K / TC_STAGE_K + tc_min_stages(K)) * tc_pad_tokens(M) * 256;
 }
 __host__ __device__ inline size_t tc_plane(int stage, int plane, int Mp) { return ((size_t)stage * 2 + plane) * Mp * 128; }
+// x as two tf32 terms, each rounded to nearest: 2^-24 of x is lost.  (The tensor core cuts off what does not fit: a high term cut
+// off instead of rounded leaves a low term of 13 bits, of which it would drop two, always towards zero.)
+__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
+    unsigned h, l;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
+    hi = __uint_as_float(h);
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - hi));
+    lo = __uint_as_float(l);
+}
 __device__ __forceinline__ unsigned tc_swz(int row, int chunk) { return (unsigned)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
 
 struct PrepTcArgs {

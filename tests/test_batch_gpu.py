@@ -156,6 +156,25 @@ def test_projection_routes_agree_on_equal_int8(E, wtype, K, N):
     w2.free()
 
 
+# Rounding errors of fp32 sums of exact products grow with the kernel's order of additions alone: dp4a adds a row's blocks as a
+# tree, the tensor-core kernels one by one, which measures up to 1.17 times dp4a's error (Q4_K, 11 008 inputs 1.02; the int8
+# kernel for chunks before them: 1.05 to 1.17).  The rest is the spread of a sample of a few thousand results.
+PRECISION = 1.25
+
+
+@pytest.mark.parametrize("wtype", [S.Q4_K, S.Q6_K], ids=["q4", "q6"])
+@pytest.mark.parametrize("K", [768, 2048, 11008])
+def test_small_batches_are_as_precise_as_dp4a(E, wtype, K):
+    """Error of k_gemm_mma against float64 sums of the same int8 activations, against dp4a's."""
+    rng = np.random.default_rng(K)
+    w, exact = _matrix(E, wtype, K, 200, rng)
+    for M in (16, 32, 77) if wtype == S.Q4_K else (16, 32):
+        x = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).cuda()
+        dp4a, mma = _errors(E, w, exact, x, (DP4A, MMA))
+        assert mma < PRECISION * dp4a, (M, dp4a, mma)
+    w.free()
+
+
 @pytest.mark.parametrize("chunk,n", [(2, 7), (16, 16), (16, 45), (64, 19), (2048, 41)])
 def test_hybrid_prompt_in_batches_equals_step_by_step(E, chunk, n):
     """Batches of a hybrid model: conv history across batches (shorter ones than the kernel, too), scan tiles of 16 tokens,
