@@ -196,7 +196,6 @@ struct tfr_engine {
     int chunk_cap = 0;  // tokens the chunk buffers have room for
     unsigned char* cact = nullptr;
     unsigned char* cimage = nullptr;  // operand image of the tensor-core projections (tfr_gemm_tc.cuh), its token scales
-    float* ctscale = nullptr;
     size_t cact_stride = 0;
     // hybrid layers of a batch: raw projections, the mixer's q / k / v (or the output gates of a full layer), decay and write strength
     float *cproj = nullptr, *cmix = nullptr, *cgates = nullptr;
@@ -350,10 +349,8 @@ static void configure_kernels_once() {
     configure_kernel(k_prep_tc, true);
     configure_kernel(k_rows_f32<4, 4, false>, true);
     configure_kernel(k_rows_f32<8, 8, true>, true);
-    configure_kernel(k_gemm_tc<RawQ4, TC_PAIR>, true);
-    configure_kernel(k_gemm_tc<RawQ6, TC_PAIR>, true);
-    configure_kernel(k_gemm_tc<RawQ4, TC_SINGLE>, true);
-    configure_kernel(k_gemm_tc<RawQ6, TC_SINGLE>, true);
+    configure_kernel(k_gemm_tc<RawQ4>, true);
+    configure_kernel(k_gemm_tc<RawQ6>, true);
     configure_kernel(k_prep_mma, true);
     configure_kernel(k_gemm_mma<MmaQ4, 1>, true);
     configure_kernel(k_gemm_mma<MmaQ4, 2>, true);
@@ -681,7 +678,7 @@ extern "C" void tfr_destroy(tfr_engine* e) {
     for (auto& kv : e->vecs) cudaFree(kv.second.dev);
     for (auto& L : e->layers) cudaFree(L.bias_qkv);
     void* ws[] = {e->x, e->q, e->attn, e->h, e->logits, e->partial, e->counters, e->st, e->prompt,
-                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->ctscale, e->cproj, e->cmix, e->cgates, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
+                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->cproj, e->cmix, e->cgates, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
     for (void* p : ws) cudaFree(p);
     if (e->st_host) cudaFreeHost(e->st_host);
     if (e->logits_host) cudaFreeHost(e->logits_host);
@@ -1738,7 +1735,7 @@ static int chunk_buffers(tfr_engine* e, int M) {
     const int mix_width = std::max(P.attn_width, vd), kmax = std::max(std::max(K, P.ff), mix_width);
     CU(e, cudaStreamSynchronize(e->stream));
     void** grown[] = {(void**)&e->cx, (void**)&e->cxn, (void**)&e->cq, (void**)&e->cattn, (void**)&e->ch, (void**)&e->cact, (void**)&e->cpart,
-                      (void**)&e->cimage, (void**)&e->ctscale, (void**)&e->cproj, (void**)&e->cmix, (void**)&e->cgates};
+                      (void**)&e->cimage, (void**)&e->cproj, (void**)&e->cmix, (void**)&e->cgates};
     e->chunk_cap = 0;
     for (void** p : grown) {
         cudaFree(*p);
@@ -1752,7 +1749,6 @@ static int chunk_buffers(tfr_engine* e, int M) {
     CU(e, cudaMalloc(&e->ch, (size_t)cap * P.ff * 4));
     CU(e, cudaMalloc(&e->cact, (size_t)cap * e->cact_stride));
     CU(e, cudaMalloc(&e->cimage, std::max(tc_image_bytes(kmax, cap), mma_image_bytes(kmax))));
-    CU(e, cudaMalloc(&e->ctscale, (size_t)tc_pad_tokens(cap) * 4));
     if (c.hybrid) {
         CU(e, cudaMalloc(&e->cproj, (size_t)cap * std::max(channels + vd + 2 * c.ssm_time_step_rank, 2 * P.nq + 2 * P.nkv) * 4));
         CU(e, cudaMalloc(&e->cmix, (size_t)cap * std::max(channels, P.nq) * 4));
@@ -1793,14 +1789,13 @@ struct BatchBufs {
     unsigned char* image;  // GEMM_TC, GEMM_MMA
     unsigned char* act;    // GEMM_DP4A: Act arrays, act_stride bytes apart
     size_t act_stride;
-    float* tscale;
     TokenState* st;
 };
 // M rows of x -> RMSNorm (optional) -> Q8, in the form the projections of `route` read
 static cudaError_t batch_prep(cudaStream_t s, int route, int type, const float* x, int width, int M, const float* normw, float eps,
                               const BatchBufs& b, float* xn) {
     if (route == GEMM_TC) {
-        PrepTcArgs a{x, width, width, M, normw, eps, b.image, b.tscale, xn};
+        PrepTcArgs a{x, width, width, M, normw, eps, b.image, xn};
         return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(TC_PREP_THREADS), tc_prep_smem(width), s, a);
     }
     if (route == GEMM_MMA) {
@@ -1813,7 +1808,7 @@ static cudaError_t batch_prep(cudaStream_t s, int route, int type, const float* 
 }
 // out = epilogue(W x) over them; jb: the second matrix of a gate/up pair or one that follows
 static cudaError_t batch_gemm(cudaStream_t s, int sms, int route, int M, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep, const BatchBufs& b) {
-    if (route == GEMM_TC) return launch_gemm_tc(s, sms, b.image, b.tscale, M, ja, jb, ep, b.st);
+    if (route == GEMM_TC) return launch_gemm_tc(s, sms, b.image, M, ja, jb, ep, b.st);
     if (route == GEMM_MMA) return launch_gemm_mma(s, sms, b.image, M, ja, jb, ep, b.st);
     return launch_gemm_typed(s, sms, ja.m.type, b.act, b.act_stride, nullptr, M, ja, jb, F32Seg{}, ep, ja.m.K, b.st);
 }
@@ -1829,7 +1824,7 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     const int cap = e->prop.multiProcessorCount;
     cudaStream_t s = e->stream;
     int n = 0;
-    const BatchBufs bufs{e->cimage, e->cact, e->cact_stride, e->ctscale, e->st};
+    const BatchBufs bufs{e->cimage, e->cact, e->cact_stride, e->st};
     auto prep = [&](int route, int type, const float* x, int width, const float* normw, float* xn) -> cudaError_t {
         n++;
         return batch_prep(s, route, type, x, width, M, normw, c.rms_eps, bufs, xn);
@@ -2559,12 +2554,12 @@ extern "C" int tfr_op_project_rows(const tfr_mat* a, const tfr_mat* b, const flo
     const int K = a->m.K, sms = sm_count_cached();
     BatchBufs bufs{};
     bufs.act_stride = (act_smem_bytes(K, false, false) + 255) & ~(size_t)255;
-    const size_t image = std::max(tc_image_bytes(K, M), mma_image_bytes(K)), parts[4] = {image, bufs.act_stride * M, (size_t)tc_pad_tokens(M) * 4, sizeof(TokenState)};
-    size_t total = 0, at[4];
-    for (int i = 0; i < 4; i++) at[i] = total, total += (parts[i] + 255) & ~(size_t)255;
+    const size_t image = std::max(tc_image_bytes(K, M), mma_image_bytes(K)), parts[3] = {image, bufs.act_stride * M, sizeof(TokenState)};
+    size_t total = 0, at[3];
+    for (int i = 0; i < 3; i++) at[i] = total, total += (parts[i] + 255) & ~(size_t)255;
     unsigned char* mem = nullptr;
     if (cudaMalloc(&mem, total) != cudaSuccess) return TFR_E_CUDA;
-    bufs.image = mem + at[0], bufs.act = mem + at[1], bufs.tscale = (float*)(mem + at[2]), bufs.st = (TokenState*)(mem + at[3]);
+    bufs.image = mem + at[0], bufs.act = mem + at[1], bufs.st = (TokenState*)(mem + at[2]);
     ChunkEpi ep{};
     ep.kind = b ? CEPI_SILU : CEPI_STORE;
     ep.out = out, ep.ldo = ep.n_rows = a->m.N, ep.use_res = use_res;

@@ -5,19 +5,20 @@
 // activation group's fp32 scale, scaled per 256-weight block by the block's fp16 d, minus (Q4_K) dmin times the scaled
 // group sums.  An integer MMA would have to leave its accumulator after every 32 (Q4_K) or 16 (Q6_K) weights to meet the
 // activation's scale, which binds the kernel to that scale arithmetic on CUDA cores (9 % of the tensor pipe, 90 us for
-// the 22 016 x 2 048 gate/up pair and 64 tokens).  Here the scales travel inside the f16 operands instead:
+// the 22 016 x 2 048 gate/up pair and 64 tokens).  Here the weights' scales travel inside the f16 operand instead:
 //
 //   A = scale * quant      an integer.  Q4_K: at most 63 * 15, exact in f16.  Q6_K: at most 128 * 32, so an f16 term and
 //                          a residual of at most one unit (a second operand tile);
-//   B = d8 * q8 * 2^s      as two f16 terms (22 bits; s per token puts the token's largest value at 2^9 .. 2^10, far from
-//                          both ends of f16);
+//   B = q8                 an integer.
 //
-// the accumulator (fp32, in TMEM) runs over 64 weights and is then joined to the row's sum by fma(d, accumulator, sum) in
-// registers, round to nearest.  The tensor core truncates as it adds: accumulators over whole 256-weight blocks left sums
-// four times less accurate than fp32 sums of the integer dots (1e-6 of the largest logit against 2.5e-7), over 64 weights
-// with the small products first they are as accurate.  The min
-// term of Q4_K, sum over groups of dmin * m * (d8 * sum q8), is a product of its own with 1 / 32 of the depth, run as
-// tf32 (two terms each; no range to fit) ahead of the blocks.
+// The accumulator (fp32, in TMEM) runs over one group of 32 weights.  All products and their sum are integers below 2^24
+// (4 096 * 127 * 32), so the tensor core's truncating additions lose nothing: it holds the exact dot that dp4a computes, and
+// meets the group's d8 and the block's d in fp32 multiply-adds in registers, round to nearest.  (With d8 inside the operand, as
+// two f16 terms, an accumulator could run over 128 weights, but truncated: 5-10e-7 against float64 where this has 1.9-2.2e-7,
+// and groups far smaller than their token's largest lost their low terms among the f16 subnormals.)
+//
+// The min term of Q4_K, sum over a block's groups of m * (d8 * sum q8), is a tf32 product of 8 terms: m is exact, the group sums
+// are two rounded terms whose products stay in accumulators of their own.
 #pragma once
 #include "tfr_chunk.cuh"
 
@@ -27,17 +28,18 @@ namespace tfr {
 
 // Both operands lie in shared memory as K-major rows of 128 bytes with the 128-byte swizzle: 16-byte chunk c of row r at
 // r * 128 + ((c ^ (r & 7)) << 4), 8-row atoms of 1 KB.  The activations are written to global memory in exactly that
-// image, so a stage of a CTA's token tile is one run of bytes per plane and travels as one untiled bulk copy:
-//   [stage][plane: high term, low term][token / 8][1 KB atom]
-// stages 0 .. K/64 - 1 hold 64 values of f16 each, the next ceil(K / 1024) hold 32 group sums of tf32 each.
+// image, so a stage of a CTA's token tile is one run of bytes and travels as one untiled bulk copy:
+//   [stage of 64 values][token / 8][1 KB atom]       f16
+//   [pair of blocks][token / 8][1 KB atom]           group sums of a block as tf32: 8 high terms, 8 low terms; the second block
+//   [stage][token][its two groups]                   d8
 constexpr int TC_STAGE_K = 64;
-__host__ __device__ inline int tc_min_stages(int K) { return (K + 1023) / 1024; }
-// Padding tokens make MMA widths: multiples of 16 columns, of 32 for the two-CTA MMAs of larger batches.
-__host__ __device__ inline int tc_pad_tokens(int M) { return M > 128 ? (M + 31) & ~31 : (M + 15) & ~15; }
+__host__ __device__ inline int tc_pad_tokens(int M) { return (M + 7) & ~7; }  // whole atoms
+__host__ __device__ inline size_t tc_sums_at(int K, int Mp) { return (size_t)(K / TC_STAGE_K) * Mp * 128; }
+__host__ __device__ inline size_t tc_d8_at(int K, int Mp) { return tc_sums_at(K, Mp) + (size_t)((K / 256 + 1) / 2) * Mp * 128; }
 __host__ __device__ inline size_t tc_image_bytes(int K, int M) {
-    return (size_t)(K / TC_STAGE_K + tc_min_stages(K)) * tc_pad_tokens(M) * 256;
+    const int Mp = tc_pad_tokens(M);
+    return tc_d8_at(K, Mp) + (size_t)(K / TC_STAGE_K) * Mp * 8;
 }
-__host__ __device__ inline size_t tc_plane(int stage, int plane, int Mp) { return ((size_t)stage * 2 + plane) * Mp * 128; }
 // x as two tf32 terms, each rounded to nearest: 2^-24 of x is lost.  (The tensor core cuts off what does not fit: a high term cut
 // off instead of rounded leaves a low term of 13 bits, of which it would drop two, always towards zero.)
 __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
@@ -55,7 +57,6 @@ struct PrepTcArgs {
     const float* normw;  // RMSNorm weight or nullptr
     float eps;
     unsigned char* image;
-    float* tscale;       // [Mp]: 2^-s of every token
     float* xn;           // optional [M][K]: the normalised vector (fp32-route rows read it)
 };
 
@@ -74,59 +75,40 @@ __global__ void __launch_bounds__(TC_PREP_THREADS) k_prep_tc(PrepTcArgs a) {
     griddep_wait();
     griddep_launch_dependents();
     const float* x = a.x + (size_t)(live ? m : 0) * a.ldx;
-    float amax = 0.f;
-    for (int i4 = tid; i4 < (K >> 2); i4 += TC_PREP_THREADS) {
-        float4 v = live ? reinterpret_cast<const float4*>(x)[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = v;
-        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    }
+    float scale = 1.f;
     if (a.normw) {
+        for (int i4 = tid; i4 < (K >> 2); i4 += TC_PREP_THREADS)
+            *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = reinterpret_cast<const float4*>(x)[i4];
         __syncthreads();
-        const float scale = rms_scale_staged(xs, K, a.eps, red);
-        amax = 0.f;
-        for (int i4 = tid; i4 < (K >> 2); i4 += TC_PREP_THREADS) {
-            float4 v = *reinterpret_cast<const float4*>(xs + xs_idx(4 * i4));
-            const float4 w = reinterpret_cast<const float4*>(a.normw)[i4];
-            v.x = v.x * scale * w.x;
-            v.y = v.y * scale * w.y;
-            v.z = v.z * scale * w.z;
-            v.w = v.w * scale * w.w;
-            *reinterpret_cast<float4*>(xs + xs_idx(4 * i4)) = v;
-            if (a.xn && live) reinterpret_cast<float4*>(a.xn + (size_t)m * K)[i4] = v;
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-        }
+        scale = rms_scale_staged(xs, K, a.eps, red);
     }
-    __syncthreads();  // red is free, the staged vector is final
-    amax = warp_max(amax);
-    if (lane == 0) red[tid >> 5] = amax;
-    __syncthreads();
-    if (tid < 32) {
-        const float v = warp_max(tid < TC_PREP_THREADS / 32 ? red[tid] : 0.f);
-        if (tid == 0) red[32] = v;
-    }
-    __syncthreads();
-    amax = red[32];
-    // 2^s with amax * 2^s in [2^9, 2^10): exponents outside +-100 are left alone (all zero, or no finite vector)
-    int e = 0;
-    if (amax > 1e-30f && amax < 1e30f) e = 9 - ((int)((__float_as_uint(amax) >> 23) & 0xff) - 127);
-    const float up = __uint_as_float((unsigned)(127 + e) << 23);
-    if (tid == 0) a.tscale[m] = __uint_as_float((unsigned)(127 - e) << 23);
     unsigned char* tok = a.image + (size_t)(m >> 3) * 1024;
+    unsigned char* d8 = a.image + tc_d8_at(K, Mp) + (size_t)m * 8;
     for (int i0 = 0; i0 < n8; i0 += TC_PREP_THREADS) {
         const int i = i0 + tid;  // values 8 i .. 8 i + 7; four lanes share a 32-value group
         const bool on = i < n8;
         float v[8];
-        const float4 v0 = on ? *reinterpret_cast<const float4*>(xs + xs_idx(8 * i)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 v1 = on ? *reinterpret_cast<const float4*>(xs + xs_idx(8 * i + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[0] = v0.x, v[1] = v0.y, v[2] = v0.z, v[3] = v0.w, v[4] = v1.x, v[5] = v1.y, v[6] = v1.z, v[7] = v1.w;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (on && live) {
+                u = a.normw ? *reinterpret_cast<const float4*>(xs + xs_idx(8 * i + 4 * h)) : reinterpret_cast<const float4*>(x)[2 * i + h];
+                if (a.normw) {
+                    const float4 w = reinterpret_cast<const float4*>(a.normw)[2 * i + h];
+                    u.x = u.x * scale * w.x, u.y = u.y * scale * w.y, u.z = u.z * scale * w.z, u.w = u.w * scale * w.w;
+                    if (a.xn) reinterpret_cast<float4*>(a.xn + (size_t)m * K)[2 * i + h] = u;
+                }
+            }
+            v[4 * h] = u.x, v[4 * h + 1] = u.y, v[4 * h + 2] = u.z, v[4 * h + 3] = u.w;
+        }
         float g = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; k++) g = fmaxf(g, fabsf(v[k]));
         g = fmaxf(g, __shfl_xor_sync(TFR_FULL_MASK, g, 1));
         g = fmaxf(g, __shfl_xor_sync(TFR_FULL_MASK, g, 2));
-        const float d = g * (1.0f / 127.0f), du = d * up;
+        const float d = g * (1.0f / 127.0f);
         int sum = 0;
-        unsigned hi[4], lo[4];
+        unsigned q[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             int q0 = 0, q1 = 0;
@@ -135,68 +117,41 @@ __global__ void __launch_bounds__(TC_PREP_THREADS) k_prep_tc(PrepTcArgs a) {
                 q1 = (int)(signed char)__float2int_rn(v[2 * k + 1] / d);
             }
             sum += q0 + q1;
-            const float f0 = (float)q0, f1 = (float)q1;
-            const __half h0 = __float2half_rn(du * f0), h1 = __float2half_rn(du * f1);
-            hi[k] = pack_f16x2(h0, h1);
-            lo[k] = pack_f16x2(__float2half_rn(fmaf(du, f0, -__half2float(h0))), __float2half_rn(fmaf(du, f1, -__half2float(h1))));
+            q[k] = pack_f16x2(__int2half_rn(q0), __int2half_rn(q1));
         }
         sum += __shfl_xor_sync(TFR_FULL_MASK, sum, 1);
         sum += __shfl_xor_sync(TFR_FULL_MASK, sum, 2);
         if (!on) continue;  // whole groups: n8 is a multiple of 32
-        const unsigned at = tc_swz(row, i & 7);
-        *reinterpret_cast<uint4*>(tok + tc_plane(i >> 3, 0, Mp) + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(tok + tc_plane(i >> 3, 1, Mp) + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4*>(tok + (size_t)(i >> 3) * Mp * 128 + tc_swz(row, i & 7)) = make_uint4(q[0], q[1], q[2], q[3]);
         if ((i & 3) == 0) {
-            const int grp = i >> 2;
-            const float s = d * (float)sum * up, sh = __uint_as_float(__float_as_uint(s) & 0xffffe000u);
-            const size_t o = tc_plane(K / TC_STAGE_K + (grp >> 5), 0, Mp) + tc_swz(row, (grp & 31) >> 2) + (grp & 3) * 4;
-            *reinterpret_cast<float*>(tok + o) = sh;
-            *reinterpret_cast<float*>(tok + o + (size_t)Mp * 128) = s - sh;
+            const int grp = i >> 2, b = grp >> 3;
+            float hi, lo;
+            split_tf32(d * (float)sum, hi, lo);
+            unsigned char* p = tok + tc_sums_at(K, Mp) + (size_t)(b >> 1) * Mp * 128;
+            const int chunk = 4 * (b & 1) + ((grp >> 2) & 1), at = (grp & 3) * 4;
+            *reinterpret_cast<float*>(p + tc_swz(row, chunk) + at) = hi;
+            *reinterpret_cast<float*>(p + tc_swz(row, chunk + 2) + at) = lo;
+            *reinterpret_cast<float*>(d8 + (size_t)(grp >> 1) * Mp * 8 + (grp & 1) * 4) = d;
         }
     }
-    // groups past the end of the last stage of sums
-    for (int grp = K / 32 + tid; grp < 32 * tc_min_stages(K); grp += TC_PREP_THREADS) {
-        const size_t o = tc_plane(K / TC_STAGE_K + (grp >> 5), 0, Mp) + tc_swz(row, (grp & 31) >> 2) + (grp & 3) * 4;
-        *reinterpret_cast<float*>(tok + o) = 0.f;
-        *reinterpret_cast<float*>(tok + o + (size_t)Mp * 128) = 0.f;
-    }
 }
 
-// ------------------------------------------------------------------ tcgen05 primitives (CG: CTAs an MMA runs on)
+// ------------------------------------------------------------------ tcgen05 primitives
 
-template <int CG>
 __device__ __forceinline__ void tc_alloc(unsigned* slot, unsigned cols) {
-    if (CG == 2) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-    } else {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
 }
-template <int CG>
 __device__ __forceinline__ void tc_dealloc(unsigned addr, unsigned cols) {
-    if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols));
-    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols));
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Arrives at the barrier when the MMAs issued so far are done; in both CTAs of a pair whose leader has cluster rank `lead`.
-template <int CG>
-__device__ __forceinline__ void tc_commit(unsigned long long* bar, int lead) {
-    if (CG == 2)
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-                     "h"((unsigned short)(3 << lead))
-                     : "memory");
-    else
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// Barriers by their shared-memory address.  Arrives when the MMAs issued so far are done:
+__device__ __forceinline__ void tc_commit(unsigned bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Arrives at the barrier at the same place in CTA `rank` of the cluster.
-__device__ __forceinline__ void tc_arrive_at(unsigned long long* bar, int rank) {
-    unsigned remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(rank));
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
+__device__ __forceinline__ void tc_arrive(unsigned bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // Shared-memory descriptor of a K-major operand with the 128-byte swizzle: start address, (unused) leading offset, 1 KB
 // between 8-row atoms, version 1, swizzle mode 2.
 __device__ __forceinline__ unsigned long long tc_desc(unsigned addr) {
@@ -204,24 +159,19 @@ __device__ __forceinline__ unsigned long long tc_desc(unsigned addr) {
 }
 // Instruction descriptor: fp32 accumulator, K-major operands of type `ty` (0: f16, 2: tf32), m x n.
 __device__ __forceinline__ unsigned tc_idesc(unsigned ty, unsigned m, unsigned n) { return (1u << 4) | (ty << 7) | (ty << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
-template <bool TF32, int CG>
+template <bool TF32>
 __device__ __forceinline__ void tc_mma(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
 #define TFR_TC_MMA(form)                                                                                                    \
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\ttcgen05.mma." form " [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), \
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\ttcgen05.mma.cta_group::1." form " [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), \
                  "l"(b), "r"(idesc), "r"(accumulate)                                                                         \
                  : "memory")
-    if (CG == 2) {
-        if (TF32) TFR_TC_MMA("cta_group::2.kind::tf32");
-        else TFR_TC_MMA("cta_group::2.kind::f16");
-    } else {
-        if (TF32) TFR_TC_MMA("cta_group::1.kind::tf32");
-        else TFR_TC_MMA("cta_group::1.kind::f16");
-    }
+    if (TF32) TFR_TC_MMA("kind::tf32");
+    else TFR_TC_MMA("kind::f16");
 #undef TFR_TC_MMA
 }
 // Columns addr .. addr + W - 1 of this warp's 32 lanes; the values are there after tc_ld_wait.
 template <int W>
-__device__ __forceinline__ void tc_ld(float (&v)[W], unsigned addr) {
+__device__ __forceinline__ void tc_ld(float* v, unsigned addr) {
     static_assert(W == 8 || W == 16, "");
     if constexpr (W == 8)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -232,6 +182,11 @@ __device__ __forceinline__ void tc_ld(float (&v)[W], unsigned addr) {
                      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
                        "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
                      : "r"(addr));
+}
+// 24 columns of this warp's 32 lanes.
+__device__ __forceinline__ void tc_ld24(float* v, unsigned addr) {
+    tc_ld<16>(v, addr);
+    tc_ld<8>(v + 16, addr + 16);
 }
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
@@ -249,18 +204,14 @@ __device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
     return d;
 }
 // Bounded mbarrier wait of a pipeline: once one wait has run out, `dead` lets all others pass at once (the call is then
-// reported as failed; what is computed meanwhile is not used).  CLUSTER: arrivals may come from another CTA.
-template <bool CLUSTER>
-__device__ __forceinline__ void tc_wait(unsigned long long* bar, unsigned parity, volatile int* dead) {
+// reported as failed; what is computed meanwhile is not used).
+__device__ __forceinline__ void tc_wait(unsigned bar, unsigned parity, volatile int* dead) {
     for (int i = 0; i < MBAR_POLL_LIMIT; i++) {
         unsigned ok;
-        if (CLUSTER)
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok)
-                         : "r"(smem_u32(bar)), "r"(parity)
-                         : "memory");
-        else
-            ok = mbar_try_wait(bar, parity);
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
         if (ok) return;
         if ((i & 63) == 63 && *dead) return;
     }
@@ -281,17 +232,25 @@ __device__ __forceinline__ unsigned tc_bits(__half2 h) { return *reinterpret_cas
 // takes the 16 bytes of every 64 weights that start at byte 16 h.
 struct RawQ4 {
     static constexpr int WPS = 4, PLANES = 1;
-    unsigned s0, s2;  // of the header's three scale words, the two that hold the sub-block scales
+    unsigned s0, s1, s2;  // scale words of the header
+    unsigned n0, n1, n2;  // of the next block's
     unsigned w[4][WPS];
-    // What stage s alone uses; the header with the last one.
+    // What stage s alone uses; the header with the first one, because its words are needed to the block's end.
     __device__ __forceinline__ void load_stage(int s, const uint8_t* data, int f, int h) {
         const uint8_t* p = data + (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16;
         const int4 v = ldg_stream(p + (1 + 2 * s + h) * 512);
         w[s][0] = v.x, w[s][1] = v.y, w[s][2] = v.z, w[s][3] = v.w;
-        if (s == 3) {
+        if (s == 0) {
             const int4 hdr = ldg_stream(p);
-            s0 = (unsigned)hdr.y, s2 = (unsigned)hdr.w;
+            n0 = (unsigned)hdr.y, n1 = (unsigned)hdr.z, n2 = (unsigned)hdr.w;
         }
+    }
+    __device__ __forceinline__ void begin_block() { s0 = n0, s1 = n1, s2 = n2; }
+    // The eight mins of a block as tf32, four per thread (the first 32 bytes of a row).
+    __device__ __forceinline__ void store_mins(unsigned char* tile, int row, int h) const {
+        const unsigned m = h ? ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4) : s1 & 0x3f3f3f3fu;
+        *reinterpret_cast<float4*>(tile + tc_swz(row, h)) =
+            make_float4(i2f_small((int)(m & 0xff)), i2f_small((int)((m >> 8) & 0xff)), i2f_small((int)((m >> 16) & 0xff)), i2f_small((int)(m >> 24)));
     }
     __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
 #pragma unroll
@@ -336,6 +295,7 @@ struct RawQ6 {
         hq[n][0] = c.x, hq[n][1] = c.y, hq[n][2] = c.z, hq[n][3] = c.w;
         if (s == 3) sc = ldg_stream(p + 12 * 512);
     }
+    __device__ __forceinline__ void begin_block() {}
     __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
         load_stage(1, data, f, h);
         load_stage(3, data, f, h);
@@ -373,49 +333,47 @@ struct RawQ6 {
 
 // ------------------------------------------------------------------ the kernel
 
-// CTA = 128 weight rows x a tile of tokens x a part of the k range, in stages of 64 weights: 16 KB of A per plane, and the
-// tokens' two planes of B.  Warps 4-11 turn weights into A tiles, lanes of warp 1 request the B planes as bulk copies, lane
-// 0 of warps 0 and 2 issues the MMAs, the warps behind drain the accumulators (two buffers in TMEM) into the row sums they
-// hold in registers (TMEM lanes 32 (w & 3) .., a share of the tokens); every role runs ahead of the next as far as the
-// rings allow.  (With all warps doing everything in turn a stage took 4 500 cycles.)  Two forms:
+// The tokens are the rows of the product (128 lanes of TMEM per CTA), the weight rows its columns: a thread that drains an
+// accumulator has one token, whose d8 it holds in a register, and the columns' d come once a block.  (The other way round every
+// d8 was a broadcast read of shared memory: 770 of 2 000 cycles a stage.)
 //
-//   pair    batches of more than 128 tokens.  Two CTAs on adjacent row tiles share up to 256 tokens with cta_group::2
-//           MMAs of 256 x 256 x 16: each holds its own rows of A and half of the tokens' B, which halves what B costs in
-//           L2 reads and in shared-memory reads per MMA.  One CTA alone on 2 x 128 rows x 128 tokens ran at a third of it.
-//   single  up to 128 tokens.  The high and the low terms of the tokens are columns of ONE MMA, so A is read once for both.
+// CTA = 128 tokens x a tile of 96 weight rows x a part of the k range, in stages of 64 weights (and one for the mins of a block).
+// Lane 0 of warps 1 and 3 requests the tokens' operand as bulk copies, the unpacking warps turn weights into the other
+// operand, lane 0 of warps 0 and 2 issues the MMAs, the sixteen warps behind drain the accumulators (two buffers in TMEM, each
+// with the two groups of a stage side by side) into the block's and the row's sums they hold in registers (TMEM lanes
+// 32 (w & 3) .., a quarter of the columns); every role runs ahead of the next as far as the rings allow.
 //
-// Gate / up pairs (ZIP) alternate the two matrices' rows in the tile, so that a gate value meets its up value in the
-// neighbouring lane, as the two rows of a RoPE pair do.  The k range is cut over the CTAs of a cluster (grid.y) where a
-// matrix has too few rows to fill the chip: their sums meet through distributed shared memory, each CTA finishing its
-// share of the tokens.
-constexpr int TC_C_WARPS = 4, TC_A_WARPS = 8, TC_MAX_STAGES = 6;
+// Gate / up pairs (ZIP) alternate the two matrices' rows in the tile, so that a thread holds a gate value beside its up value,
+// as the two rows of a RoPE pair.  The k range is cut over the CTAs of a cluster (grid.y) where a matrix has too few rows to
+// fill the chip, or so many blocks that a chain of additions over them would cost precision: the parts' sums meet through
+// distributed shared memory, each CTA finishing its share of the columns.
+constexpr int TC_C_WARPS = 4, TC_D_WARPS = 16, TC_MAX_STAGES = 8, TC_LANES = 128, TC_ROWS = 96, TC_COLSCALE_BYTES = TC_D_WARPS * 2 * (TC_ROWS / 4) * 4;
 constexpr size_t TC_SMEM_MAX = 225 * 1024;
-enum { TC_PAIR, TC_SINGLE };
-// Draining warps and the registers of a thread of each role (what they add up to is what the launch has).  Draining is a
-// chain of TMEM loads (300 cycles for 16 columns, waited for one by one), so sixteen warps share the columns; the pairs on
-// Q6_K matrices, whose third MMA leaves more time, keep eight and leave the registers to the unpacking.
-template <int FORM, bool Q4>
-struct TcRoles {
-    static constexpr int D_WARPS = FORM == TC_PAIR && !Q4 ? 8 : 16, THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + D_WARPS);
-    static constexpr int LAUNCH_REGS = D_WARPS == 8 ? 96 : 72;
-    static constexpr int C_REGS = D_WARPS == 8 ? 32 : 24, A_REGS = D_WARPS == 8 ? 64 : FORM == TC_PAIR ? 48 : 72,
-                         D_REGS = D_WARPS == 8 ? 160 : FORM == TC_PAIR ? 96 : 80;
-    static constexpr int NC = FORM == TC_PAIR ? 1024 / D_WARPS : 32;  // tokens of a draining warp
-    static_assert(32 * (TC_C_WARPS * C_REGS + TC_A_WARPS * A_REGS + D_WARPS * D_REGS) <= THREADS * LAUNCH_REGS && THREADS * LAUNCH_REGS <= 65536,
+// Unpacking warps, two threads per row (a warpgroup's registers change together: the last two idle), and the registers of a
+// thread of each role; what they add up to is what the launch has.
+constexpr int TC_A_WARPS = 8, TC_A_BUSY = TC_ROWS / 16, TC_THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + TC_D_WARPS), TC_LAUNCH_REGS = 72;
+template <bool Q4>
+struct TcRegs {
+    static constexpr int C = 24, A = Q4 ? 48 : 64, D = Q4 ? 96 : 88;
+    static_assert(32 * (TC_C_WARPS * C + TC_A_WARPS * A + TC_D_WARPS * D) <= TC_THREADS * TC_LAUNCH_REGS && TC_THREADS * TC_LAUNCH_REGS <= 65536,
                   "more registers than the launch has");
 };
 // Registers of a role: N of the LAUNCH a thread has.  Fewer must be given back, more asked for.
-template <int N, int LAUNCH>
+template <int N>
 __device__ __forceinline__ void tc_regs() {
     static_assert(N % 8 == 0, "");
-    if constexpr (N < LAUNCH) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-    else if constexpr (N > LAUNCH) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+    if constexpr (N < TC_LAUNCH_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+    else if constexpr (N > TC_LAUNCH_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
 }
+
+// Most blocks a CTA adds up one after the other.  The rounding of such a chain grows with the root of its length: Q6_K rows of 43
+// and 108 blocks in one piece 1.30e-7 and 1.94e-7 against float64, in pieces of 22 and 27 1.07e-7 and 1.2e-7 (dp4a, which adds
+// them as a tree, 0.93e-7 and 0.98e-7).
+constexpr int TC_CHAIN = 27;
 
 struct TcArgs {
     const unsigned char* image;
-    const float* tscale;
-    int M, Mp, NT;   // tokens, with padding; tokens per tile
+    int M, Mp;       // tokens, with padding
     Mat A1, A2;      // ZIP: the pair; otherwise A2 (optional) follows A1 in the grid
     int tiles1;      // row tiles of A1
     int id1, id2, zip, nst;
@@ -433,406 +391,334 @@ struct TcRing {
     }
 };
 
-template <class RAW, int FORM>
-__global__ void __launch_bounds__(TcRoles<FORM, RAW::PLANES == 1>::THREADS, 1) k_gemm_tc(const TcArgs a) {
-    constexpr bool Q4 = RAW::PLANES == 1, PAIR = FORM == TC_PAIR;
-    using Roles = TcRoles<FORM, Q4>;
-    constexpr int TC_D_WARPS = Roles::D_WARPS, CGS = TC_D_WARPS / 4, NC = Roles::NC;  // column groups of NC tokens
-    constexpr int CG = PAIR ? 2 : 1;  // CTAs of an MMA
-    constexpr int DR = PAIR ? 2 : 1;  // stages an accumulator runs over
+template <class RAW>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
+    constexpr bool Q4 = RAW::PLANES == 1;
+    using Regs = TcRegs<Q4>;
+    constexpr int NC = TC_ROWS / (TC_D_WARPS / 4);  // columns of a draining warp
+    constexpr int SPB = Q4 ? 5 : 4;                 // stages of a block: four of weights, one of mins
+    constexpr int T_BYTES = TC_LANES * 128, W_PLANE = TC_ROWS * 128, STAGE = T_BYTES + RAW::PLANES * W_PLANE;
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
-    __shared__ unsigned long long full[TC_MAX_STAGES], empty[TC_MAX_STAGES], accfull[2], accempty[2];
+    __shared__ unsigned long long bars[2 * TC_MAX_STAGES + 4];
     __shared__ unsigned tmem_slot;
     __shared__ int dead_s;
-    __shared__ float tscale_s[PAIR ? 256 : 128];
     volatile int* dead = &dead_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int S = gridDim.y, part = blockIdx.y;           // k parts
-    const int pr = PAIR ? blockIdx.x & 1 : 0;             // this CTA of the pair; 0 leads
-    const int lead = PAIR ? 2 * part : part;              // cluster rank of the pair's leader (single: of this CTA)
-    const bool cluster = PAIR || S > 1;
-    const int n0 = blockIdx.z * a.NT, nt = min(a.NT, a.Mp - n0), nst = a.nst;
-    const int ntc = nt / CG, nc0 = n0 + pr * ntc;         // the tokens whose B this CTA holds
-    const bool second = !a.zip && a.A2.data != nullptr && (int)blockIdx.x >= a.tiles1;
+    const unsigned full = smem_u32(bars), empty = full + 8 * TC_MAX_STAGES, accfull = empty + 8 * TC_MAX_STAGES, accempty = accfull + 16;
+    const int S = gridDim.y, part = blockIdx.y;  // k parts
+    const int n0 = blockIdx.z * TC_LANES, nt = min(TC_LANES, a.Mp - n0), nst = a.nst;  // this CTA's tokens
+    const int tile = blockIdx.x;
+    const bool second = !a.zip && a.A2.data != nullptr && tile >= a.tiles1;
     const Mat& A = second ? a.A2 : a.A1;
     const int nb = A.nb, K = A.K, N = A.N;
-    const int row0 = ((int)blockIdx.x - (second ? a.tiles1 : 0)) * (a.zip ? 64 : 128);
+    const int row0 = (tile - (second ? a.tiles1 : 0)) * (a.zip ? TC_ROWS / 2 : TC_ROWS);
     const int b0 = nb * part / S, b1 = nb * (part + 1) / S;
-    // stages of group sums come in two: the high terms of dmin * m with both of the sums' terms, its low terms with the high ones
-    const int n_min = Q4 ? tc_min_stages(K) : 0, m0 = n_min * part / S, m1 = n_min * (part + 1) / S;
     if (warp == 3) {
-        // The tile's weights start towards L2 at once, and so do those of the CTA that will follow on this SM: the registers
+        // The rows this CTA unpacks start towards L2 at once, and so do those of the CTA that will follow on this SM: the registers
         // of the unpacking warps hold one block ahead, which covers an L2 hit but not a trip to memory.
-        auto ahead = [&](const Mat& m, int group) {
-            if (group * ROW_GROUP >= m.N) return;
-            const size_t f = (size_t)group * ROW_GROUP * nb, t0 = (f + ROW_GROUP * b0) >> 5, t1 = (f + ROW_GROUP * b1 + 31) >> 5;
+        auto ahead = [&](const Mat& m, int row) {
+            if (row >= m.N) return;
+            const size_t f = mat_flat(nb, row, 0), t0 = (f + ROW_GROUP * b0) >> 5, t1 = (f + ROW_GROUP * b1 + 31) >> 5;
             constexpr size_t TB = Q4 ? Q4_TILE_BYTES : Q6_TILE_BYTES;
             bulk_prefetch_l2(m.data + t0 * TB, (unsigned)((t1 - t0) * TB));
         };
         for (int w = 0; w <= 1; w++) {
-            const int row = row0 + w * a.ahead * (a.zip ? 64 : 128);
             if (w == 1 && a.ahead == 0) break;
-            if (a.zip) ahead(lane & 1 ? a.A2 : A, row / ROW_GROUP + (lane >> 1));
-            else ahead(A, row / ROW_GROUP + lane);
+            const int t = row0 + w * a.ahead * (a.zip ? TC_ROWS / 2 : TC_ROWS);
+            if (lane < TC_ROWS / ROW_GROUP) {
+                if (a.zip) ahead(lane & 1 ? a.A2 : A, t + (lane >> 1) * ROW_GROUP);
+                else ahead(A, t + lane * ROW_GROUP);
+            }
         }
     }
-    const int min_stages = 2 * (m1 - m0), stages = min_stages + 4 * (b1 - b0);
+    const int stages = SPB * (b1 - b0);
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr int A_SUB = RAW::PLANES * 16384;            // A of 64 weights: one 16 KB tile per plane
-    const int b_plane = ntc * 128, stage_bytes = A_SUB + 2 * (a.NT / CG) * 128;
-    constexpr unsigned ACC_COLS = (PAIR ? 1 : 2) * CGS * NC, TMEM_COLS = 2 * ACC_COLS;  // the tokens; single: high then low terms
+    constexpr unsigned ACC_COLS = 2 * TC_ROWS, TMEM_COLS = 512;  // the rows for a stage's first and second group, twice
+    float* colscales = reinterpret_cast<float*>(smem + (size_t)nst * STAGE);  // d and -dmin of every draining warp's columns
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
-            // every CTA's own A warps and B (with the bytes); the leader's also the word that the peer's are complete
-            mbar_init(full + i, TC_A_WARPS + 1 + (PAIR && pr == 0));
-            mbar_init(empty + i, 1);
+            mbar_init(bars + i, TC_A_BUSY + 1);  // the unpacking warps and the tokens (with the bytes)
+            mbar_init(bars + TC_MAX_STAGES + i, 1);
         }
         for (int i = 0; i < 2; i++) {
-            mbar_init(accfull + i, 1);
-            mbar_init(accempty + i, TC_D_WARPS + (PAIR && pr == 0));
+            mbar_init(bars + 2 * TC_MAX_STAGES + i, 1);
+            mbar_init(bars + 2 * TC_MAX_STAGES + 2 + i, TC_D_WARPS);
         }
         dead_s = 0;
         mbar_fence_init();
     }
-    if (warp == 0) tc_alloc<CG>(&tmem_slot, TMEM_COLS);
+    if (warp == 0) tc_alloc(&tmem_slot, TMEM_COLS);
     tc_fence_before();
     __syncthreads();
-    if (cluster) cluster_sync_all();  // the barriers of the cluster exist
     tc_fence_after();
     const unsigned tmem = tmem_slot;
-    float* sums = reinterpret_cast<float*>(smem);  // S > 1: [token][128 rows], over the stages once every MMA has read them
+    float* sums = reinterpret_cast<float*>(smem);  // S > 1: [column][128 tokens], over the stages once every MMA has read them
 
     if (warp < TC_C_WARPS) {
-        tc_regs<Roles::C_REGS, Roles::LAUNCH_REGS>();
-        if ((warp & 1) == 0 && pr == 0) {
-            // Two issuing threads take turns by accumulator: a wait costs one about 300 cycles even when there is nothing to
-            // wait for, and the MMAs of a stage 650.
+        tc_regs<Regs::C>();
+        if ((warp & 1) == 0) {
+            // Two issuing threads take turns by accumulator: with 28 warps at work a wait costs one 300 cycles even when there is
+            // nothing to wait for, and four MMAs 400.
             if (lane == 0) {
                 TcRing ring;
                 const unsigned long long d0 = tc_desc(smem_u32(smem));
-                for (int j = 0; j < stages; j++) {
-                    const int r = j / DR, buf = r & 1;
-                    if (buf != warp >> 1) {
-                        ring.next(nst);
-                        continue;
-                    }
-                    const bool fresh = j % DR == 0;
-                    if (fresh && r >= 2) tc_wait<PAIR>(accempty + buf, ((r >> 1) - 1) & 1, dead);
-                    tc_wait<PAIR>(full + ring.slot, ring.lap, dead);
+                const unsigned id = tc_idesc(0, TC_LANES, TC_ROWS), idm = tc_idesc(2, TC_LANES, TC_ROWS);
+                const int buf = warp >> 1;
+                const unsigned acc = tmem + buf * ACC_COLS;
+                if (buf) ring.next(nst);
+                for (int j = buf; j < stages; j += 2) {
+                    tc_wait(full + 8 * ring.slot, ring.lap, dead);
                     // what the unpacking warps stored becomes visible to the tensor core here, not where they store it: a
                     // fence there waits for the warp's loads in flight, the next block's words (900 to 2 200 cycles a block)
                     fence_proxy_async();
+                    const unsigned long long dt = d0 + ((ring.slot * STAGE) >> 4), dw = dt + (T_BYTES >> 4);
+                    if (j >= 2) tc_wait(accempty + 8 * buf, ((j >> 1) - 1) & 1, dead);  // last: nothing else stands behind the draining
                     tc_fence_after();
-                    const unsigned acc = tmem + buf * ACC_COLS;
-                    const unsigned long long da = d0 + ((ring.slot * stage_bytes) >> 4), db = da + (A_SUB >> 4);
-                    if (Q4 && j < min_stages) {
-                        const unsigned id = tc_idesc(2, 128 * CG, nt), id2 = tc_idesc(2, 128, 2 * nt);
-                        const bool high = !(j & 1);
-                        if (!PAIR && high) {
-#pragma unroll
-                            for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, da + 2 * kk, db + 2 * kk, id2, !fresh || kk > 0);
-                        } else {
-                            // the small products go first: the tensor core truncates as it adds, so what counts is how
-                            // often it adds to the full sum
-                            if (PAIR && high)
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, da + 2 * kk, db + (b_plane >> 4) + 2 * kk, id, !fresh || kk > 0);
-#pragma unroll
-                            for (int kk = 0; kk < 4; kk++) tc_mma<true, CG>(acc, da + 2 * kk, db + 2 * kk, id, !fresh || (PAIR && high) || kk > 0);
-                        }
+                    if (Q4 && j % SPB == 4) {
+                        // high terms of the group sums to the first columns, low terms to the second
+                        const int odd = 4 * ((b0 + j / SPB) & 1);
+                        tc_mma<true>(acc, dt + odd, dw, idm, 0);
+                        tc_mma<true>(acc + TC_ROWS, dt + odd + 2, dw, idm, 0);
                     } else {
-                        const unsigned id = tc_idesc(0, 128 * CG, nt), id2 = tc_idesc(0, 128, 2 * nt);
-                        if (PAIR) {
 #pragma unroll
-                            for (int kk = 0; kk < 4; kk++) {
-                                tc_mma<false, CG>(acc, da + 2 * kk, db + (b_plane >> 4) + 2 * kk, id, !fresh || kk > 0);
-                                if (!Q4) tc_mma<false, CG>(acc, da + 1024 + 2 * kk, db + 2 * kk, id, 1);
-                            }
-#pragma unroll
-                            for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(acc, da + 2 * kk, db + 2 * kk, id, 1);
-                        } else {
-                            // Q6_K: the residuals of A touch the high columns alone and go first as well
-                            if (!Q4) {
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(acc, da + 1024 + 2 * kk, db + 2 * kk, id2, !fresh || kk > 0);
-                            }
-#pragma unroll
-                            for (int kk = 0; kk < 4; kk++) tc_mma<false, CG>(acc, da + 2 * kk, db + 2 * kk, id2, !Q4 || !fresh || kk > 0);
+                        for (int kk = 0; kk < 4; kk++) {
+                            tc_mma<false>(acc + (kk >> 1) * TC_ROWS, dt + 2 * kk, dw + 2 * kk, id, kk & 1);
+                            if (!Q4) tc_mma<false>(acc + (kk >> 1) * TC_ROWS, dt + 2 * kk, dw + (W_PLANE >> 4) + 2 * kk, id, 1);
                         }
                     }
-                    tc_commit<CG>(empty + ring.slot, lead);
-                    if (j % DR == DR - 1) tc_commit<CG>(accfull + buf, lead);
+                    tc_commit(accfull + 8 * buf);
+                    tc_commit(empty + 8 * ring.slot);
+                    ring.next(nst);
                     ring.next(nst);
                 }
             }
             __syncwarp();
-        } else if (PAIR && (warp & 1) == 0) {
-            // The second CTA of a pair passes its barriers' phases on to the leader's: one thread each, because an arrival at
-            // another CTA that releases at cluster scope holds up the warp that makes it.
+        } else {
+            // two threads take turns: a bulk request costs the one that makes it 300 to 560 cycles
+            griddep_wait();  // the image comes from the previous kernel
             if (lane == 0) {
                 TcRing ring;
-                if (warp == 0)
-                    for (int j = 0; j < stages; j++) {
-                        tc_wait<false>(full + ring.slot, ring.lap, dead);
-                        fence_proxy_async();
-                        tc_arrive_at(full + ring.slot, lead);
-                        ring.next(nst);
-                    }
-                else
-                    for (int r = 0; r < stages / DR - 2; r++) {
-                        tc_wait<false>(accempty + (r & 1), (r >> 1) & 1, dead);
-                        tc_arrive_at(accempty + (r & 1), lead);
-                    }
+                const size_t plane = (size_t)a.Mp * 128;
+                const unsigned char* src = a.image + (size_t)n0 * 128;
+                if (warp >> 1) ring.next(nst);
+                for (int j = warp >> 1; j < stages; j += 2) {
+                    const int b = b0 + j / SPB, s = j % SPB;
+                    if (j >= nst) tc_wait(empty + 8 * ring.slot, ring.lap ^ 1, dead);
+                    unsigned long long* bar = bars + ring.slot;
+                    mbar_expect_tx(bar, nt * 128);
+                    bulk_load(smem + ring.slot * STAGE, src + (s == 4 ? tc_sums_at(K, a.Mp) + (b >> 1) * plane : (4 * b + s) * plane), nt * 128, bar);
+                    ring.next(nst);
+                    ring.next(nst);
+                }
             }
             __syncwarp();
-        } else if (warp == 1) {
-            griddep_wait();  // the image comes from the previous kernel
-            TcRing ring;
-            const size_t plane = (size_t)a.Mp * 128;
-            const unsigned char* src = a.image + (size_t)nc0 * 128 + (lane & 1) * plane;
-            for (int j = 0; j < stages; j++) {
-                const bool mins = j < min_stages;
-                // a lane per plane; the low terms of dmin * m meet the high plane alone
-                const int image_stage = mins ? K / TC_STAGE_K + m0 + (j >> 1) : 4 * b0 + (j - min_stages);
-                const int copies = mins && (j & 1) ? 1 : 2;
-                if (j >= nst) tc_wait<false>(empty + ring.slot, ring.lap ^ 1, dead);
-                if (lane == 0) mbar_expect_tx(full + ring.slot, copies * b_plane);
-                __syncwarp();
-                if (lane < copies)
-                    bulk_load(smem + ring.slot * stage_bytes + A_SUB + lane * b_plane, src + (size_t)2 * image_stage * plane, b_plane, full + ring.slot);
-                __syncwarp();
-                ring.next(nst);
-            }
         }
         griddep_launch_dependents();
-        if (S > 1) cluster_sync_all();
-        if (cluster) cluster_sync_all();
-        else asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");  // the last accumulator has been read
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");  // the last accumulator has been read
         tc_fence_after();
-        if (warp == 0) tc_dealloc<CG>(tmem, TMEM_COLS);
+        if (warp == 0) tc_dealloc(tmem, TMEM_COLS);
+        if (S > 1) cluster_sync_all();
+        if (S > 1) cluster_sync_all();
         return;
     }
 
     if (warp < TC_C_WARPS + TC_A_WARPS) {
-        tc_regs<Roles::A_REGS, Roles::LAUNCH_REGS>();
-        // this thread's row of the tile and its half of the row's blocks; rows past the matrix repeat its last row
-        const int wa = warp - TC_C_WARPS, row_l = (wa & 3) * 32 + lane, h = wa >> 2;
-        const uint8_t* wdata = (a.zip && (row_l & 1)) ? a.A2.data : A.data;
-        const int f0 = (int)mat_flat(nb, min(row0 + (a.zip ? row_l >> 1 : row_l), N - 1), 0);
-        RAW raw;
-        raw.load(wdata, f0 + ROW_GROUP * b0, h);  // weights do not depend on earlier kernels
+        tc_regs<Regs::A>();
+        const int ta = tid - 32 * TC_C_WARPS;
         griddep_launch_dependents();
-        TcRing ring;
-        int j = 0;
-        auto acquire = [&]() {
-            if (j >= nst) tc_wait<false>(empty + ring.slot, ring.lap ^ 1, dead);
-            return smem + ring.slot * stage_bytes;
-        };
-        auto publish = [&]() {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(full + ring.slot);
-            ring.next(nst);
-            j++;
-        };
-        if constexpr (Q4) {
-            for (int c = m0; c < m1; c++) {
-                // groups of 32 weights 32 c .. 32 c + 31 = blocks 4 c .. 4 c + 3, two of them this thread's
+        if (ta < 2 * TC_ROWS) {
+            // this thread's row and its half of the row's blocks; rows past the matrix repeat its last row
+            const int h = ta >= TC_ROWS, row_l = ta - h * TC_ROWS;
+            const uint8_t* wdata = (a.zip && (row_l & 1)) ? a.A2.data : A.data;
+            const int f0 = (int)mat_flat(nb, min(row0 + (a.zip ? row_l >> 1 : row_l), N - 1), 0);
+            RAW raw;
+            raw.load(wdata, f0 + ROW_GROUP * b0, h);  // weights do not depend on earlier kernels
+            TcRing ring;
+            int j = 0;
+            auto acquire = [&]() {
+                if (j >= nst) tc_wait(empty + 8 * ring.slot, ring.lap ^ 1, dead);
+                return smem + ring.slot * STAGE + T_BYTES;
+            };
+            auto publish = [&]() {
+                __syncwarp();
+                if (lane == 0) tc_arrive(full + 8 * ring.slot);
+                ring.next(nst);
+                j++;
+            };
+            for (int b = b0; b < b1; b++) {
                 unsigned char* t = nullptr;
-#pragma unroll 1
-                for (int p = 0; p < 2; p++) {
+                raw.begin_block();
+#pragma unroll
+                for (int s = 0; s < 4; s++) {
                     t = acquire();
-#pragma unroll 1
-                    for (int i = 0; i < 2; i++) {
-                        const int b = 4 * c + 2 * h + i, f = f0 + ROW_GROUP * min(b, nb - 1);
-                        const int4 hdr = __ldg(reinterpret_cast<const int4*>(wdata + (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16));
-                        const unsigned s1 = (unsigned)hdr.z, s2 = (unsigned)hdr.w;
-                        const unsigned ml = s1 & 0x3f3f3f3fu, mh = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
-                        const float dmin = b < nb ? f16_to_f32((unsigned short)((unsigned)hdr.x >> 16)) : 0.f;
-#pragma unroll
-                        for (int half = 0; half < 2; half++) {
-                            const unsigned mm = half ? mh : ml;
-                            unsigned o[4];
-#pragma unroll
-                            for (int k = 0; k < 4; k++) {
-                                const float v = dmin * i2f_small((int)((mm >> (8 * k)) & 0xff));
-                                const unsigned top = __float_as_uint(v) & 0xffffe000u;
-                                o[k] = p ? __float_as_uint(v - __uint_as_float(top)) : top;
-                            }
-                            *reinterpret_cast<uint4*>(t + tc_swz(row_l, 2 * (2 * h + i) + half)) = make_uint4(o[0], o[1], o[2], o[3]);
-                        }
-                    }
+                    raw.store(s, t, row_l, h, W_PLANE);
+                    publish();
+                    if (b + 1 < b1) raw.load_stage(s, wdata, f0 + ROW_GROUP * (b + 1), h);  // the words just used, of the next block
+                }
+                if constexpr (Q4) {
+                    t = acquire();
+                    raw.store_mins(t, row_l, h);
                     publish();
                 }
             }
         }
-        for (int b = b0; b < b1; b++) {
-            unsigned char* t = nullptr;
-#pragma unroll
-            for (int s = 0; s < 4; s++) {
-                t = acquire();
-                raw.store(s, t, row_l, h, 16384);
-                publish();
-                if (b + 1 < b1) raw.load_stage(s, wdata, f0 + ROW_GROUP * (b + 1), h);  // the words just used, of the next block
-            }
-        }
         if (S > 1) cluster_sync_all();
-        if (cluster) cluster_sync_all();
+        if (S > 1) cluster_sync_all();
         return;
     }
 
-    tc_regs<Roles::D_REGS, Roles::LAUNCH_REGS>();
-    const int quad = warp & 3, cg = (warp - TC_C_WARPS - TC_A_WARPS) >> 2, row_d = quad * 32 + lane;
-    float2 tot[NC / 2];  // token pairs: one packed multiply-add joins two accumulators to their sums
+    tc_regs<Regs::D>();
+    const int dwarp = warp - TC_C_WARPS - TC_A_WARPS, quad = warp & 3, cg = dwarp >> 2, tok = quad * 32 + lane, m = n0 + tok;
+    static_assert(NC == 24 && TC_COLSCALE_BYTES == TC_D_WARPS * 2 * NC * 4, "");
+    float* colscale = colscales + dwarp * 2 * NC;
+    float2 tot[NC / 2];  // of the token and its columns: over the row
 #pragma unroll
     for (int i = 0; i < NC / 2; i++) tot[i] = make_float2(0.f, 0.f);
     {
-        const uint8_t* ddata = (a.zip && (row_d & 1)) ? a.A2.data : A.data;
-        const int df = (int)mat_flat(nb, min(row0 + (a.zip ? row_d >> 1 : row_d), N - 1), 0);
+        // lanes below NC hold a column's d, and dmin above it, a block ahead
+        const int col = cg * NC + min(lane, NC - 1);
+        const uint8_t* ddata = (a.zip && (col & 1)) ? a.A2.data : A.data;
+        const int df = (int)mat_flat(nb, min(row0 + (a.zip ? col >> 1 : col), N - 1), 0);
         auto load_d = [&](int b) {
-            const int f = df + ROW_GROUP * min(b, nb - 1);
-            const uint8_t* p = ddata + (Q4 ? (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16
-                                           : (size_t)(f >> 5) * Q6_TILE_BYTES + Q6_PIECES * 512 + (f & 31) * 2);
-            return f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(p)));
+            const int f = df + ROW_GROUP * b;
+            return Q4 ? __ldg(reinterpret_cast<const unsigned*>(ddata + (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16))
+                      : (unsigned)__ldg(reinterpret_cast<const unsigned short*>(ddata + (size_t)(f >> 5) * Q6_TILE_BYTES + Q6_PIECES * 512 + (f & 31) * 2));
         };
-        float dnext = load_d(b0), dcur = -1.f;
+        unsigned dnext = load_d(b0);
         griddep_launch_dependents();
-        griddep_wait();  // nothing reaches an accumulator before the image is complete; token scales and residuals are then, too
-        const int td = tid - 32 * (TC_C_WARPS + TC_A_WARPS);
-        if (td < nt) tscale_s[td] = n0 + td < a.M ? a.tscale[n0 + td] : 0.f;
-        const int min_rounds = min_stages / DR;
-        int left = min_rounds;  // rounds until the factor changes
-        for (int r = 0; r < stages / DR; r++) {
-            const bool minus = Q4 && r < min_rounds;
-            if (left == 0) {
-                dcur = dnext;
-                dnext = load_d(b0 + (r - min_rounds) / (4 / DR) + 1);
-                left = 4 / DR;
-            }
-            left--;
-            const int buf = r & 1;
-            tc_wait<false>(accfull + buf, (r >> 1) & 1, dead);
+        griddep_wait();  // nothing reaches an accumulator before the image is complete; residuals are then, too
+        const unsigned lanes = tmem + ((unsigned)quad << 21) + cg * NC;
+        float2 sum[NC / 2];  // of the block without its d
+        // d8 of the token's groups, two stages ahead
+        const float2* d8 = reinterpret_cast<const float2*>(a.image + tc_d8_at(K, a.Mp)) + (size_t)(4 * b0) * a.Mp + min(m, a.Mp - 1);
+        const int d8_end = 4 * (b1 - b0);
+        auto load_d8 = [&](int i) { return __ldcg(d8 + (size_t)min(i, d8_end - 1) * a.Mp); };  // L1 may hold the last image
+        float2 knext[2] = {load_d8(0), load_d8(1)};
+        int j = 0;
+        float v[NC];
+        // the two accumulators of stage j, one after the other: use(which)
+        auto drain = [&](auto&& use) {
+            const int buf = j & 1;
+            tc_wait(accfull + 8 * buf, (j >> 1) & 1, dead);
             tc_fence_after();
-            const unsigned at = tmem + ((unsigned)quad << 21) + buf * ACC_COLS + cg * NC;
-            // The truncations cost an accumulator, on average, about half (Q4_K) or three quarters (Q6_K) of a unit in its
-            // last place (measured against float64); raising the factor by one unit in as many stages gives it back.
-            const float f = (r & 3) < (Q4 ? 2 : 3) ? dcur * 1.00000012f : dcur;
-            const float2 ff = make_float2(f, f);
-            const bool low = !PAIR && !(minus && (r & 1));  // there are low columns
 #pragma unroll
-            for (int c = 0; c < NC; c += 16) {  // columns of a load
-                if (cg * NC + c >= nt) break;
-                float v[16], w[16];
-                tc_ld<16>(v, at + c);
-                if (low) tc_ld<16>(w, at + nt + c);
+            for (int g = 0; g < 2; g++) {
+                tc_ld24(v, lanes + buf * ACC_COLS + g * TC_ROWS);
                 tc_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 8; i++) tot[c / 2 + i] = fma_f32x2(ff, make_float2(v[2 * i], v[2 * i + 1]), tot[c / 2 + i]);
-                if (low) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) tot[c / 2 + i] = fma_f32x2(ff, make_float2(w[2 * i], w[2 * i + 1]), tot[c / 2 + i]);
+                if (g == 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) tc_arrive(accempty + 8 * buf);
                 }
+                use(g);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(accempty + buf);
+            j++;
+        };
+        for (int b = b0; b < b1; b++) {
+            if (lane < NC) {
+                colscale[lane] = f16_to_f32((unsigned short)dnext);
+                if (Q4) colscale[NC + lane] = -f16_to_f32((unsigned short)(dnext >> 16));
+            }
+            if (b + 1 < b1) dnext = load_d(b + 1);
+#pragma unroll
+            for (int s = 0; s < 4; s++) {
+                const float2 k = knext[s & 1];
+                knext[s & 1] = load_d8(4 * (b - b0) + s + 2);
+                drain([&](int g) {
+                    const float kg = g ? k.y : k.x;
+#pragma unroll
+                    for (int i = 0; i < NC / 2; i++) {
+                        const float2 t = make_float2(v[2 * i], v[2 * i + 1]);
+                        sum[i] = s == 0 && g == 0 ? mul_f32x2(t, make_float2(kg, kg)) : fma_f32x2(t, make_float2(kg, kg), sum[i]);
+                    }
+                });
+            }
+            // the block's d * sums - dmin * mins, and once more rounded into the row's sum
+            const float4* dc = reinterpret_cast<const float4*>(colscale);
+#pragma unroll
+            for (int i = 0; i < NC / 4; i++) {
+                const float4 d = dc[i];
+                sum[2 * i] = mul_f32x2(make_float2(d.x, d.y), sum[2 * i]), sum[2 * i + 1] = mul_f32x2(make_float2(d.z, d.w), sum[2 * i + 1]);
+            }
+            if constexpr (Q4)
+                drain([&](int) {
+#pragma unroll
+                    for (int i = 0; i < NC / 4; i++) {
+                        const float4 m = dc[NC / 4 + i];
+                        sum[2 * i] = fma_f32x2(make_float2(m.x, m.y), make_float2(v[4 * i], v[4 * i + 1]), sum[2 * i]);
+                        sum[2 * i + 1] = fma_f32x2(make_float2(m.z, m.w), make_float2(v[4 * i + 2], v[4 * i + 3]), sum[2 * i + 1]);
+                    }
+                });
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) tot[i] = fma_f32x2(make_float2(1.f, 1.f), sum[i], tot[i]);
+            __syncwarp();  // the columns' scales have been read
         }
     }
-    if (!cluster) asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");
-    else asm volatile("bar.sync 1, %0;" ::"n"(32 * TC_D_WARPS) : "memory");  // the token scales
+    tc_fence_before();
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");
 
-    // ---- epilogue
-    auto total = [&](int i) { return (i & 1) ? tot[i >> 1].y : tot[i >> 1].x; };
+    // ---- epilogue: column pairs (RoPE pairs, gate and up) of the thread's token
     const int id_base = second ? a.id2 : a.id1;
-    const int row = row0 + (a.zip ? row_d >> 1 : row_d);
-    const bool odd = lane & 1, store = a.epi.kind == CEPI_STORE;
-    ChunkEpi epi = a.epi;
-    epi.bias = nullptr;  // added here, once per row
-    const float bias = a.epi.bias && row < N ? a.epi.bias[2 * id_base + row] : 0.f;
-    // items of two adjacent lanes (RoPE pairs, gate and up): id of the item and whether it exists
-    const int item = id_base + (a.zip ? row : row >> 1);
-    const bool item_on = a.zip ? row < N : (row & ~1) < N;
+    const bool live = m < a.M;
     if (S == 1) {
-        const int t0 = n0 + cg * NC, tn = min(NC, min(nt, a.M - n0) - cg * NC);
+        const ChunkEpi& e = a.epi;
+        const int rows = a.zip ? NC / 2 : NC, row = row0 + cg * rows, first = (a.zip ? id_base : 2 * id_base) + row;
+        float* o = e.out + (size_t)m * e.ldo + first;
+        const bool wide = row + rows <= N && (e.ldo & 3) == 0 && (first & 3) == 0 && (reinterpret_cast<uintptr_t>(e.out) & 15) == 0;
+        if (!live) {
+        } else if (e.kind == CEPI_SILU && wide) {
 #pragma unroll
-        for (int i0 = 0; i0 < NC; i0 += 8) {
-            if (i0 >= tn) break;
-            // eight tokens' scales and residuals in flight together: a load behind each store would cost a trip to L2
-            float v[8];
-            {
-                float ts[8], res[8];
+            for (int i = 0; i < NC / 2; i += 4) {
+                float h[4];
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const bool on = i0 + i < tn;
-                    ts[i] = on ? tscale_s[cg * NC + i0 + i] : 0.f;
-                    res[i] = on && store && epi.use_res == 2 && row < N ? epi.out[(size_t)(t0 + i0 + i) * epi.ldo + 2 * id_base + row] : 0.f;
-                }
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = total(i0 + i) * ts[i] + res[i] + bias;
+                for (int q = 0; q < 4; q++) h[q] = (tot[i + q].x / (1.f + __expf(-tot[i + q].x))) * tot[i + q].y;  // as ChunkEpiTok::apply
+                *reinterpret_cast<float4*>(o + i) = make_float4(h[0], h[1], h[2], h[3]);
             }
-            if (store) {
+        } else if (e.kind == CEPI_STORE && wide && !e.bias) {
+            // all residuals in flight together: a load behind each store would cost a trip to L2
+            float4 r[NC / 4];
 #pragma unroll
-                for (int i = 0; i < 8; i++)
-                    if (i0 + i < tn && row < N) epi.out[(size_t)(t0 + i0 + i) * epi.ldo + 2 * id_base + row] = v[i];
-            } else {
+            for (int i = 0; i < NC / 4; i++) r[i] = e.use_res == 2 ? reinterpret_cast<const float4*>(o)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    // the even lane takes token i, the odd one token i + 1
-                    const float got = __shfl_xor_sync(TFR_FULL_MASK, odd ? v[i] : v[i + 1], 1);
-                    const int t = i0 + i + (odd ? 1 : 0);
-                    if (t < tn && item_on) ChunkEpiTok{&epi, t0 + t}.apply(item, odd ? got : v[i], odd ? v[i + 1] : got);
-                }
+            for (int i = 0; i < NC / 4; i++)
+                reinterpret_cast<float4*>(o)[i] =
+                    make_float4(tot[2 * i].x + r[i].x, tot[2 * i].y + r[i].y, tot[2 * i + 1].x + r[i].z, tot[2 * i + 1].y + r[i].w);
+        } else {
+            const ChunkEpiTok t{&a.epi, m};
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) {
+                const int r = a.zip ? row + i : row + 2 * i;
+                if (r < N) t.apply(id_base + (a.zip ? r : r >> 1), tot[i].x, tot[i].y);
             }
         }
     } else {
-        if (cg * NC < nt) {
+        // [pair of columns][token]
+        float2* mine = reinterpret_cast<float2*>(sums) + (size_t)cg * (NC / 2) * TC_LANES + tok;
 #pragma unroll
-            for (int i = 0; i < NC; i++)
-                if (cg * NC + i < nt) sums[(cg * NC + i) * 128 + row_d] = total(i);
-        }
+        for (int i = 0; i < NC / 2; i++) mine[i * TC_LANES] = tot[i];
         cluster_sync_all();
-        const int per = (nt + S - 1) / S, c0 = part * per, cn = min(per, min(nt, a.M - n0) - c0);
-        for (int c4 = c0 + cg; c4 < c0 + cn; c4 += 4 * CGS) {
-            // four tokens' residuals and the parts' sums in flight together
-            float res[4], v[4];
+        const int i0 = NC / 2 * part / S, i1 = NC / 2 * (part + 1) / S;
+        for (int i = i0; i < i1; i++) {
+            const unsigned at0 = smem_u32(mine + i * TC_LANES);
+            float2 x[8];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int c = c4 + q * CGS;
-                res[q] = c < c0 + cn && store && epi.use_res == 2 && row < N ? epi.out[(size_t)(n0 + c) * epi.ldo + 2 * id_base + row] : 0.f;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int c = min(c4 + q * CGS, c0 + cn - 1);
-                const unsigned at0 = smem_u32(sums + c * 128 + row_d);
-                float x[8];
-#pragma unroll
-                for (int p = 0; p < 8; p++) {
-                    x[p] = 0.f;
-                    if (p < S) {
-                        unsigned remote;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at0), "r"(PAIR ? 2 * p + pr : p));
-                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x[p]) : "r"(remote) : "memory");
-                    }
-                }
-                v[q] = 0.f;
-#pragma unroll
-                for (int p = 0; p < 8; p++) v[q] += x[p];
-                v[q] = v[q] * tscale_s[c] + res[q] + bias;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int c = c4 + q * CGS;
-                if (c >= c0 + cn) break;
-                if (store) {
-                    if (row < N) epi.out[(size_t)(n0 + c) * epi.ldo + 2 * id_base + row] = v[q];
-                } else {
-                    const float got = __shfl_xor_sync(TFR_FULL_MASK, v[q], 1);
-                    if (!odd && item_on) ChunkEpiTok{&epi, n0 + c}.apply(item, v[q], got);
+            for (int p = 0; p < 8; p++) {
+                x[p] = make_float2(0.f, 0.f);
+                if (p < S) {
+                    unsigned remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at0), "r"(p));
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x[p].x), "=f"(x[p].y) : "r"(remote) : "memory");
                 }
             }
+            float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int p = 0; p < 8; p++) v.x += x[p].x, v.y += x[p].y;
+            const int r = row0 + (a.zip ? cg * (NC / 2) + i : cg * NC + 2 * i);
+            if (live && r < N) ChunkEpiTok{&a.epi, m}.apply(id_base + (a.zip ? r : r >> 1), v.x, v.y);
         }
     }
     if (tid == 32 * (TC_C_WARPS + TC_A_WARPS) && dead_s && a.st) a.st->err = 2;
-    if (cluster) cluster_sync_all();  // nobody leaves while others use its barriers, operands or sums
+    if (S > 1) cluster_sync_all();  // nobody leaves while others read its sums
 }
 
 // ------------------------------------------------------------------ rows on the fp32 activation route
@@ -976,67 +862,53 @@ inline cudaError_t launch_rows_f32(cudaStream_t stream, int sms, const Mat& w, i
 
 inline bool tc_type(int type) { return type == TFR_Q4_K || type == TFR_Q6_K; }
 
-template <class RAW, int FORM>
+template <class RAW>
 inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_tiles, int S) {
-    using Roles = TcRoles<FORM, RAW::PLANES == 1>;
-    constexpr bool PAIR = FORM == TC_PAIR;
-    const int stage = RAW::PLANES * 16384 + 2 * (a.NT / (PAIR ? 2 : 1)) * 128;
-    a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024) / stage));
+    constexpr int stage = TC_LANES * 128 + RAW::PLANES * TC_ROWS * 128;
+    a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024 - TC_COLSCALE_BYTES) / stage));
     a.ahead = S == 1 && row_tiles > sms ? sms : 0;
-    const size_t sums = S > 1 ? (size_t)a.NT * 512 : 0;
+    const size_t sums = S > 1 ? (size_t)TC_ROWS * TC_LANES * 4 : 0;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(PAIR ? (row_tiles + 1) & ~1 : row_tiles, S, (a.Mp + a.NT - 1) / a.NT);
-    cfg.blockDim = dim3(Roles::THREADS);
-    cfg.dynamicSmemBytes = std::max((size_t)a.nst * stage, sums) + 1024;
+    cfg.gridDim = dim3(row_tiles, S, (a.M + TC_LANES - 1) / TC_LANES);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = std::max((size_t)a.nst * stage + TC_COLSCALE_BYTES, sums) + 1024;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = PAIR ? 2 : 1;
+    attr[1].val.clusterDim.x = 1;
     attr[1].val.clusterDim.y = S;
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = PAIR || S > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_gemm_tc<RAW, FORM>, (const TcArgs)a);
+    cfg.numAttrs = S > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k_gemm_tc<RAW>, (const TcArgs)a);
 }
 
 // out = epilogue(W x) for the M tokens of an operand image; jb: the second matrix of a gate/up pair or one that follows.
-inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned char* image, const float* tscale, int M, const RowJob& ja,
+inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned char* image, int M, const RowJob& ja,
                                   const RowJob& jb, const ChunkEpi& epi, TokenState* st) {
     TcArgs a{};
-    a.image = image, a.tscale = tscale, a.M = M, a.Mp = tc_pad_tokens(M);
+    a.image = image, a.M = M, a.Mp = tc_pad_tokens(M);
     a.A1 = ja.m, a.A2 = jb.m, a.id1 = ja.id_base, a.id2 = jb.id_base;
     a.zip = epi.kind == CEPI_SILU;
     a.epi = epi, a.st = st;
-    const bool q4 = ja.m.type == TFR_Q4_K;
-    const int rows = a.zip ? 64 : 128;
+    const int rows = a.zip ? TC_ROWS / 2 : TC_ROWS;
     a.tiles1 = (ja.m.N + rows - 1) / rows;
-    const int tiles = a.tiles1 + (!a.zip && jb.m.data ? (jb.m.N + rows - 1) / rows : 0);
+    const int tiles = a.tiles1 + (!a.zip && jb.m.data ? (jb.m.N + rows - 1) / rows : 0), groups = (M + TC_LANES - 1) / TC_LANES;
     // CTAs the device runs at once by cluster size (GPCs hold whole clusters)
     auto fit = [&](int ctas) { return ctas <= 2 ? sms : ctas == 4 ? 132 : 112; };
-    // the form and the number of k parts with the shortest longest chain: waves of CTAs x stages x what a stage takes, in
-    // units of a 128-row, 128-token MMA stage
-    auto plan = [&](int form, int& S, int& NT) {
-        const bool pair = form == TC_PAIR;
-        const int most = pair ? 256 : 128, tok_tiles = (a.Mp + most - 1) / most, unit = pair ? 32 : 16;
-        NT = ((a.Mp + tok_tiles - 1) / tok_tiles + unit - 1) / unit * unit;
-        double best = 1e30;
-        for (int s = 1; s <= (pair ? 4 : 8) && s <= ja.m.nb; s *= 2) {
-            const int ctas = (pair ? (tiles + 1) & ~1 : tiles) * tok_tiles * s, at_once = fit(pair ? 2 * s : s);
-            const double stage = pair ? 0.4 + 1.2 * NT / 128 : 0.6 + 1.2 * NT / 128;
-            const double t = (double)((ctas + at_once - 1) / at_once) * ((4.5 * ((ja.m.nb + s - 1) / s) * stage) + 6 + (s > 1 ? 3 : 0));
-            if (t < best) best = t, S = s;
-        }
-        return best;
-    };
-    int S = 1, S2 = 1, NT2 = 0;
-    const double single = plan(TC_SINGLE, S, a.NT);
-    if (M > 128 && plan(TC_PAIR, S2, NT2) < single) {
-        a.NT = NT2;
-        return q4 ? launch_tc<RawQ4, TC_PAIR>(stream, sms, a, tiles, S2) : launch_tc<RawQ6, TC_PAIR>(stream, sms, a, tiles, S2);
+    // the number of k parts with the shortest longest chain: waves of CTAs x (blocks x what a block takes + the ends), in units of
+    // a quarter of a block (0.8 us)
+    int S = 1;
+    double best = 1e30;
+    for (int s = 1; s <= 8 && s <= ja.m.nb; s *= 2) {
+        if (s < 8 && (ja.m.nb + s - 1) / s > TC_CHAIN) continue;
+        const int ctas = tiles * groups * s;
+        const double t = (double)((ctas + fit(s) - 1) / fit(s)) * (4.5 * ((ja.m.nb + s - 1) / s) + 6 + (s > 1 ? 3 : 0));
+        if (t < best) best = t, S = s;
     }
-    return q4 ? launch_tc<RawQ4, TC_SINGLE>(stream, sms, a, tiles, S) : launch_tc<RawQ6, TC_SINGLE>(stream, sms, a, tiles, S);
+    return ja.m.type == TFR_Q4_K ? launch_tc<RawQ4>(stream, sms, a, tiles, S) : launch_tc<RawQ6>(stream, sms, a, tiles, S);
 }
 
 }  // namespace tfr

@@ -27,10 +27,9 @@ def _state(m, kv, cfg, n):
     return [m.debug_read(w, n * kvdim, np.uint16, kv=kv, layer=0) for w in "kv"]
 
 
-# Sums of the same int8 products by two kernels, of the largest value.  Measured against float64: the tcgen05 forms, whose
-# accumulators truncate, are off by up to 5.5e-6 of a result's rms, the others by 1.6e-6; a largest value is three to four rms.
-# Twice that sum.
-SAME_INT8 = 4e-6
+# Sums of the same int8 products by two kernels, of the largest value.  Measured against float64: no kernel is off by more than
+# 2e-6 of a result's rms, and a largest value is three to four rms: 1.3e-6.  One and a half times that.
+SAME_INT8 = 2e-6
 
 
 @pytest.mark.parametrize("cfg", [ODD, WIDE], ids=["odd", "wide"])
@@ -173,6 +172,28 @@ def test_small_batches_are_as_precise_as_dp4a(E, wtype, K):
         dp4a, mma = _errors(E, w, exact, x, (DP4A, MMA))
         assert mma < PRECISION * dp4a, (M, dp4a, mma)
     w.free()
+
+
+@pytest.mark.parametrize("wtype", [S.Q4_K, S.Q6_K], ids=["q4", "q6"])
+@pytest.mark.parametrize("K,N,M", [(768, 200, 81), (2048, 500, 128), (2048, 500, 300), (11008, 500, 100), (11008, 1536, 1300)])
+def test_larger_batches_are_as_precise_as_dp4a(E, wtype, K, N, M):
+    """Error of k_gemm_tc against float64 sums of the same int8 activations, against dp4a's.  Also with blocks of the input spread
+    over five decades and weights that make up for it, so that small groups count as much as the token's largest; the last shape
+    has so many tiles that nothing but the length of a row's chain of additions asks for parts of the k range."""
+    from taraference_b200 import synth_gpu as G
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K + M)
+    for spread in (0, 5):
+        f = 10.0 ** (-spread * torch.rand(K // 256, generator=gen, device="cuda")).repeat_interleave(256)
+        w32 = torch.randn((N, K), generator=gen, device="cuda") * (0.005 / f)
+        raw = torch.empty(N * K // 256 * S.BLOCK_BYTES[wtype], dtype=torch.uint8, device="cuda")
+        E.synth_quantize(wtype, w32, raw)
+        raw = raw.cpu().numpy()
+        exact = torch.from_numpy((_q4_k_exact if wtype == S.Q4_K else _q6_k_exact)(raw, K, N)).cuda()
+        w = E.GpuMat(wtype, K, N, raw)
+        dp4a, tc = _errors(E, w, exact, torch.randn((M, K), generator=gen, device="cuda") * f, (DP4A, TC))
+        assert tc < PRECISION * dp4a, (spread, dp4a, tc)
+        w.free()
 
 
 @pytest.mark.parametrize("chunk,n", [(2, 7), (16, 16), (16, 45), (64, 19), (2048, 41)])
