@@ -348,6 +348,7 @@ struct RawQ6 {
 // fill the chip, or so many blocks that a chain of additions over them would cost precision: the parts' sums meet through
 // distributed shared memory, each CTA finishing its share of the columns.
 constexpr int TC_C_WARPS = 4, TC_D_WARPS = 16, TC_MAX_STAGES = 8, TC_LANES = 128, TC_ROWS = 96, TC_COLSCALE_BYTES = TC_D_WARPS * 2 * (TC_ROWS / 4) * 4;
+constexpr int TC_SUM_STRIDE = TC_ROWS / 2 + 1;  // float2 of a token's sums in the epilogue; odd, so that 16 tokens' pairs lie in 32 banks
 constexpr size_t TC_SMEM_MAX = 225 * 1024;
 // Unpacking warps, two threads per row (a warpgroup's registers change together: the last two idle), and the registers of a
 // thread of each role; what they add up to is what the launch has.
@@ -452,7 +453,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = tmem_slot;
-    float* sums = reinterpret_cast<float*>(smem);  // S > 1: [column][128 tokens], over the stages once every MMA has read them
 
     if (warp < TC_C_WARPS) {
         tc_regs<Regs::C>();
@@ -657,65 +657,51 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
     tc_fence_before();
     asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");
 
-    // ---- epilogue: column pairs (RoPE pairs, gate and up) of the thread's token
-    const int id_base = second ? a.id2 : a.id1;
-    const bool live = m < a.M;
-    if (S == 1) {
-        const ChunkEpi& e = a.epi;
-        const int rows = a.zip ? NC / 2 : NC, row = row0 + cg * rows, first = (a.zip ? id_base : 2 * id_base) + row;
-        float* o = e.out + (size_t)m * e.ldo + first;
-        const bool wide = row + rows <= N && (e.ldo & 3) == 0 && (first & 3) == 0 && (reinterpret_cast<uintptr_t>(e.out) & 15) == 0;
-        if (!live) {
-        } else if (e.kind == CEPI_SILU && wide) {
+    // ---- epilogue: [token][pair of columns] through shared memory (of the cluster's CTAs), then lanes along the columns: RoPE
+    // pairs, gate and up values.  A thread's own token and columns would touch 32 rows of the output with every access (a down
+    // projection of 2 048 tokens: 620 us).
+    constexpr int PAIRS = TC_ROWS / 2, BATCH = 4;
+    float2* mine = reinterpret_cast<float2*>(smem) + tok * TC_SUM_STRIDE + cg * (NC / 2);
 #pragma unroll
-            for (int i = 0; i < NC / 2; i += 4) {
-                float h[4];
+    for (int i = 0; i < NC / 2; i++) mine[i] = tot[i];
+    if (S > 1) cluster_sync_all();
+    else asm volatile("bar.sync 2, %0;" ::"n"(32 * TC_D_WARPS) : "memory");
+    const int id_base = second ? a.id2 : a.id1, td = tid - 32 * (TC_C_WARPS + TC_A_WARPS);
+    const int t0 = TC_LANES * part / S, items = min(TC_LANES / S, a.M - n0 - t0) * PAIRS;  // S is a power of two
+    const bool res = a.epi.kind == CEPI_STORE && a.epi.use_res == 2;
+    ChunkEpi epi = a.epi;
+    epi.use_res = 0;
+    for (int k0 = td; k0 < items; k0 += BATCH * 32 * TC_D_WARPS) {
+        // the parts' sums and the residuals of four items in flight together
+        float2 v[BATCH], r[BATCH];
+        int m[BATCH], id[BATCH];
 #pragma unroll
-                for (int q = 0; q < 4; q++) h[q] = (tot[i + q].x / (1.f + __expf(-tot[i + q].x))) * tot[i + q].y;  // as ChunkEpiTok::apply
-                *reinterpret_cast<float4*>(o + i) = make_float4(h[0], h[1], h[2], h[3]);
+        for (int q = 0; q < BATCH; q++) {
+            const int k = k0 + q * 32 * TC_D_WARPS, t = t0 + k / PAIRS, pair = k % PAIRS;
+            const int row = row0 + (a.zip ? pair : 2 * pair);
+            const bool on = k < items && row < N;
+            m[q] = n0 + t, id[q] = on ? id_base + (a.zip ? row : row >> 1) : -1;
+            v[q] = r[q] = make_float2(0.f, 0.f);
+            if (!on) continue;
+            if (res) {
+                const float* o = epi.out + (size_t)m[q] * epi.ldo + 2 * id[q];
+                r[q].x = o[0];
+                if (2 * id[q] + 1 < epi.n_rows) r[q].y = o[1];
             }
-        } else if (e.kind == CEPI_STORE && wide && !e.bias) {
-            // all residuals in flight together: a load behind each store would cost a trip to L2
-            float4 r[NC / 4];
-#pragma unroll
-            for (int i = 0; i < NC / 4; i++) r[i] = e.use_res == 2 ? reinterpret_cast<const float4*>(o)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < NC / 4; i++)
-                reinterpret_cast<float4*>(o)[i] =
-                    make_float4(tot[2 * i].x + r[i].x, tot[2 * i].y + r[i].y, tot[2 * i + 1].x + r[i].z, tot[2 * i + 1].y + r[i].w);
-        } else {
-            const ChunkEpiTok t{&a.epi, m};
-#pragma unroll
-            for (int i = 0; i < NC / 2; i++) {
-                const int r = a.zip ? row + i : row + 2 * i;
-                if (r < N) t.apply(id_base + (a.zip ? r : r >> 1), tot[i].x, tot[i].y);
-            }
-        }
-    } else {
-        // [pair of columns][token]
-        float2* mine = reinterpret_cast<float2*>(sums) + (size_t)cg * (NC / 2) * TC_LANES + tok;
-#pragma unroll
-        for (int i = 0; i < NC / 2; i++) mine[i * TC_LANES] = tot[i];
-        cluster_sync_all();
-        const int i0 = NC / 2 * part / S, i1 = NC / 2 * (part + 1) / S;
-        for (int i = i0; i < i1; i++) {
-            const unsigned at0 = smem_u32(mine + i * TC_LANES);
-            float2 x[8];
+            const unsigned at = smem_u32(smem) + (t * TC_SUM_STRIDE + pair) * 8;
 #pragma unroll
             for (int p = 0; p < 8; p++) {
-                x[p] = make_float2(0.f, 0.f);
-                if (p < S) {
-                    unsigned remote;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at0), "r"(p));
-                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x[p].x), "=f"(x[p].y) : "r"(remote) : "memory");
-                }
+                if (p >= S) break;
+                float2 x;
+                unsigned remote;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(p));
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"(remote) : "memory");
+                v[q].x += x.x, v[q].y += x.y;
             }
-            float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int p = 0; p < 8; p++) v.x += x[p].x, v.y += x[p].y;
-            const int r = row0 + (a.zip ? cg * (NC / 2) + i : cg * NC + 2 * i);
-            if (live && r < N) ChunkEpiTok{&a.epi, m}.apply(id_base + (a.zip ? r : r >> 1), v.x, v.y);
         }
+#pragma unroll
+        for (int q = 0; q < BATCH; q++)
+            if (id[q] >= 0) ChunkEpiTok{&epi, m[q]}.apply(id[q], v[q].x + r[q].x, v[q].y + r[q].y);
     }
     if (tid == 32 * (TC_C_WARPS + TC_A_WARPS) && dead_s && a.st) a.st->err = 2;
     if (S > 1) cluster_sync_all();  // nobody leaves while others read its sums
@@ -867,11 +853,11 @@ inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_ti
     constexpr int stage = TC_LANES * 128 + RAW::PLANES * TC_ROWS * 128;
     a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024 - TC_COLSCALE_BYTES) / stage));
     a.ahead = S == 1 && row_tiles > sms ? sms : 0;
-    const size_t sums = S > 1 ? (size_t)TC_ROWS * TC_LANES * 4 : 0;
+    static_assert(TC_LANES * TC_SUM_STRIDE * 8 <= 2 * stage, "the epilogue's sums lie over the first stages");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(row_tiles, S, (a.M + TC_LANES - 1) / TC_LANES);
     cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = std::max((size_t)a.nst * stage + TC_COLSCALE_BYTES, sums) + 1024;
+    cfg.dynamicSmemBytes = (size_t)a.nst * stage + TC_COLSCALE_BYTES + 1024;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
