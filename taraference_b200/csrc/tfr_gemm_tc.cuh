@@ -228,104 +228,100 @@ __device__ __forceinline__ __half2 tc_bytes_1024(unsigned w) {
 }
 __device__ __forceinline__ unsigned tc_bits(__half2 h) { return *reinterpret_cast<const unsigned*>(&h); }
 
-// Raw words of one 256-weight block that a thread turns into operand values: two threads share a row's block, thread h
-// takes the 16 bytes of every 64 weights that start at byte 16 h.
+// Raw words of half g of a 256-weight block (two stages of 64 weights) that a thread turns into operand values.
 struct RawQ4 {
-    static constexpr int WPS = 4, PLANES = 1;
+    static constexpr int PLANES = 1;
     unsigned s0, s1, s2;  // scale words of the header
     unsigned n0, n1, n2;  // of the next block's
-    unsigned w[4][WPS];
-    // What stage s alone uses; the header with the first one, because its words are needed to the block's end.
-    __device__ __forceinline__ void load_stage(int s, const uint8_t* data, int f, int h) {
+    unsigned w[2][8];     // 64 weights: [stage of the half]
+    // Stage i of the half; the header with the first one, because its words are needed to the block's end.
+    __device__ __forceinline__ void load_stage(int i, const uint8_t* data, int f, int g) {
         const uint8_t* p = data + (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16;
-        const int4 v = ldg_stream(p + (1 + 2 * s + h) * 512);
-        w[s][0] = v.x, w[s][1] = v.y, w[s][2] = v.z, w[s][3] = v.w;
-        if (s == 0) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int4 v = ldg_stream(p + (1 + 2 * (2 * g + i) + h) * 512);
+            w[i][4 * h] = v.x, w[i][4 * h + 1] = v.y, w[i][4 * h + 2] = v.z, w[i][4 * h + 3] = v.w;
+        }
+        if (i == 0) {
             const int4 hdr = ldg_stream(p);
             n0 = (unsigned)hdr.y, n1 = (unsigned)hdr.z, n2 = (unsigned)hdr.w;
         }
     }
     __device__ __forceinline__ void begin_block() { s0 = n0, s1 = n1, s2 = n2; }
-    // The eight mins of a block as tf32, four per thread (the first 32 bytes of a row).
-    __device__ __forceinline__ void store_mins(unsigned char* tile, int row, int h) const {
-        const unsigned m = h ? ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4) : s1 & 0x3f3f3f3fu;
-        *reinterpret_cast<float4*>(tile + tc_swz(row, h)) =
-            make_float4(i2f_small((int)(m & 0xff)), i2f_small((int)((m >> 8) & 0xff)), i2f_small((int)((m >> 16) & 0xff)), i2f_small((int)(m >> 24)));
-    }
-    __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
+    // The eight mins of a block as tf32 (the first 32 bytes of a row).
+    __device__ __forceinline__ void store_mins(unsigned char* tile, int row) const {
 #pragma unroll
-        for (int s = 0; s < 4; s++) load_stage(s, data, f, h);
+        for (int h = 0; h < 2; h++) {
+            const unsigned m = h ? ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4) : s1 & 0x3f3f3f3fu;
+            *reinterpret_cast<float4*>(tile + tc_swz(row, h)) =
+                make_float4(i2f_small((int)(m & 0xff)), i2f_small((int)((m >> 8) & 0xff)), i2f_small((int)((m >> 16) & 0xff)), i2f_small((int)(m >> 24)));
+        }
     }
-    // 64 weights of stage s: low nibbles = sub-block 2 s, high nibbles = sub-block 2 s + 1 (kernels/common.cu:40-84)
-    __device__ __forceinline__ void store(int s, unsigned char* tile, int row, int h, int) const {
-        const unsigned sc4 = s < 2 ? s0 & 0x3f3f3f3fu : (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
+    // 64 weights of stage 2 g + i: low nibbles = sub-block 2 (2 g + i), high nibbles the next (kernels/common.cu:40-84)
+    __device__ __forceinline__ void store(int i, unsigned char* tile, int row, int g, int) const {
+        const unsigned sc4 = g == 0 ? s0 & 0x3f3f3f3fu : (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
         const __half2 bias = __half2half2(__ushort_as_half(0x6400)), m1024 = __half2half2(__ushort_as_half(0xe400));
-        const unsigned sa = __byte_perm(sc4, 0x64646464u, (s & 1) ? 0x4242 : 0x4040), sb = __byte_perm(sc4, 0x64646464u, (s & 1) ? 0x4343 : 0x4141);
+        const unsigned sa = __byte_perm(sc4, 0x64646464u, i ? 0x4242 : 0x4040), sb = __byte_perm(sc4, 0x64646464u, i ? 0x4343 : 0x4141);
         const __half2 scl = __hsub2(*reinterpret_cast<const __half2*>(&sa), bias), sch = __hsub2(*reinterpret_cast<const __half2*>(&sb), bias);
         const __half2 ofl = __hmul2(scl, m1024), ofh = __hmul2(sch, m1024);
 #pragma unroll
-        for (int c = 0; c < WPS / 2; c++) {
+        for (int c = 0; c < 4; c++) {
             unsigned lo[4], hi[4];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const unsigned x = w[s][2 * c + k], l = x & 0x0f0f0f0fu, u = (x >> 4) & 0x0f0f0f0fu;
+                const unsigned x = w[i][2 * c + k], l = x & 0x0f0f0f0fu, u = (x >> 4) & 0x0f0f0f0fu;
                 // (1024 + q) * sc - 1024 * sc: both products below 2^16, the difference q * sc exact
                 lo[2 * k] = tc_bits(__hfma2(tc_bytes_1024<0>(l), scl, ofl)), lo[2 * k + 1] = tc_bits(__hfma2(tc_bytes_1024<1>(l), scl, ofl));
                 hi[2 * k] = tc_bits(__hfma2(tc_bytes_1024<0>(u), sch, ofh)), hi[2 * k + 1] = tc_bits(__hfma2(tc_bytes_1024<1>(u), sch, ofh));
             }
-            const int chunk = (WPS / 2) * h + c;
-            *reinterpret_cast<uint4*>(tile + tc_swz(row, chunk)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            *reinterpret_cast<uint4*>(tile + tc_swz(row, 4 + chunk)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(tile + tc_swz(row, c)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            *reinterpret_cast<uint4*>(tile + tc_swz(row, 4 + c)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         }
     }
 };
 
 struct RawQ6 {
-    static constexpr int WPS = 4, PLANES = 2;
-    int4 sc;
-    unsigned la[2][WPS], lb[2][WPS], hq[2][WPS];
-    // What the stages up to s are the last to use: half n = s >> 1 after its second stage.
-    __device__ __forceinline__ void load_stage(int s, const uint8_t* data, int f, int h) {
-        if (!(s & 1)) return;
+    static constexpr int PLANES = 2;
+    unsigned sc[2];  // the half's eight scales
+    unsigned la[8], lb[8], hq[8];
+    // Both stages of the half use the same words, in different bits: they come with the second.
+    __device__ __forceinline__ void load_stage(int i, const uint8_t* data, int f, int g) {
+        if (i == 0) return;
         const uint8_t* p = data + (size_t)(f >> 5) * Q6_TILE_BYTES + (f & 31) * 16;
-        const int n = s >> 1;
-        const int4 a = ldg_stream(p + (4 * n + h) * 512), b = ldg_stream(p + (4 * n + 2 + h) * 512), c = ldg_stream(p + (8 + 2 * n + h) * 512);
-        la[n][0] = a.x, la[n][1] = a.y, la[n][2] = a.z, la[n][3] = a.w;
-        lb[n][0] = b.x, lb[n][1] = b.y, lb[n][2] = b.z, lb[n][3] = b.w;
-        hq[n][0] = c.x, hq[n][1] = c.y, hq[n][2] = c.z, hq[n][3] = c.w;
-        if (s == 3) sc = ldg_stream(p + 12 * 512);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int4 a = ldg_stream(p + (4 * g + h) * 512), b = ldg_stream(p + (4 * g + 2 + h) * 512), c = ldg_stream(p + (8 + 2 * g + h) * 512);
+            la[4 * h] = a.x, la[4 * h + 1] = a.y, la[4 * h + 2] = a.z, la[4 * h + 3] = a.w;
+            lb[4 * h] = b.x, lb[4 * h + 1] = b.y, lb[4 * h + 2] = b.z, lb[4 * h + 3] = b.w;
+            hq[4 * h] = c.x, hq[4 * h + 1] = c.y, hq[4 * h + 2] = c.z, hq[4 * h + 3] = c.w;
+        }
+        const uint2 s = __ldg(reinterpret_cast<const uint2*>(p + 12 * 512 + 8 * g));
+        sc[0] = s.x, sc[1] = s.y;
     }
     __device__ __forceinline__ void begin_block() {}
-    __device__ __forceinline__ void load(const uint8_t* data, int f, int h) {
-        load_stage(1, data, f, h);
-        load_stage(3, data, f, h);
-    }
-    // 64 weights of stage s = runs j = 2 (s & 1), + 1 of half n = s >> 1 (kernels/gemv.cu:302-337, as in block_dot):
+    // 64 weights of stage 2 g + i = runs j = 2 i, 2 i + 1 of half g (kernels/gemv.cu:302-337, as in block_dot):
     // scale * (q - 32) as its f16 rounding and the residual (0 or +-1: |scale * q| <= 4096)
-    __device__ __forceinline__ void store(int s, unsigned char* tile, int row, int h, int plane_bytes) const {
-        const int n = s >> 1;
+    __device__ __forceinline__ void store(int i, unsigned char* tile, int row, int, int plane_bytes) const {
         const __half2 off = __half2half2(__ushort_as_half(0x6420));  // 1024 + 32
 #pragma unroll
         for (int jl = 0; jl < 2; jl++) {
-            const int j = 2 * (s & 1) + jl;
-            // scale byte 8 n + h + 2 j: word 2 n + (j >> 1), byte h + 2 (j & 1)
-            const int word = n == 0 ? ((s & 1) ? sc.y : sc.x) : ((s & 1) ? sc.w : sc.z);
-            const __half2 sch = __half2half2(__int2half_rn((int)(signed char)((word >> (8 * (h + 2 * jl))) & 0xff)));
+            const int j = 2 * i + jl;
 #pragma unroll
-            for (int c = 0; c < WPS / 2; c++) {
+            for (int c = 0; c < 4; c++) {
+                const int h = c >> 1;  // scale byte 2 j + h of the half
+                const __half2 sch = __half2half2(__int2half_rn((int)(signed char)((sc[i] >> (8 * (2 * jl + h))) & 0xff)));
                 unsigned hi[4], lo[4];
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
-                    const unsigned nib = jl ? lb[n][2 * c + k] : la[n][2 * c + k];
-                    const unsigned q = ((nib >> (4 * (s & 1))) & 0x0f0f0f0fu) | (((hq[n][2 * c + k] >> (2 * j)) & 0x03030303u) << 4);
+                    const unsigned nib = jl ? lb[2 * c + k] : la[2 * c + k];
+                    const unsigned q = ((nib >> (4 * i)) & 0x0f0f0f0fu) | (((hq[2 * c + k] >> (2 * j)) & 0x03030303u) << 4);
                     const __half2 q0 = __hsub2(tc_bytes_1024<0>(q), off), q1 = __hsub2(tc_bytes_1024<1>(q), off);
                     const __half2 p0 = __hmul2(sch, q0), p1 = __hmul2(sch, q1);
                     hi[2 * k] = tc_bits(p0), hi[2 * k + 1] = tc_bits(p1);
                     lo[2 * k] = tc_bits(__hfma2(sch, q0, __hneg2(p0))), lo[2 * k + 1] = tc_bits(__hfma2(sch, q1, __hneg2(p1)));
                 }
-                const int chunk = 4 * jl + (WPS / 2) * h + c;
-                *reinterpret_cast<uint4*>(tile + tc_swz(row, chunk)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(tile + plane_bytes + tc_swz(row, chunk)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                *reinterpret_cast<uint4*>(tile + tc_swz(row, 4 * jl + c)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(tile + plane_bytes + tc_swz(row, 4 * jl + c)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
         }
     }
@@ -350,7 +346,8 @@ struct RawQ6 {
 constexpr int TC_C_WARPS = 4, TC_D_WARPS = 16, TC_MAX_STAGES = 8, TC_LANES = 128, TC_ROWS = 96, TC_COLSCALE_BYTES = TC_D_WARPS * 2 * (TC_ROWS / 4) * 4;
 constexpr int TC_SUM_STRIDE = TC_ROWS / 2 + 1;  // float2 of a token's sums in the epilogue; odd, so that 16 tokens' pairs lie in 32 banks
 constexpr size_t TC_SMEM_MAX = 225 * 1024;
-// Unpacking warps, two threads per row (a warpgroup's registers change together: the last two idle), and the registers of a
+// Unpacking warps, two threads per row, one for each half of its blocks (a warpgroup's registers change together: the last two
+// idle; two threads on every stage paid the ring's price, 900 of 1 500 cycles, twice as often), and the registers of a
 // thread of each role; what they add up to is what the launch has.
 constexpr int TC_A_WARPS = 8, TC_A_BUSY = TC_ROWS / 16, TC_THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + TC_D_WARPS), TC_LAUNCH_REGS = 72;
 template <bool Q4>
@@ -438,7 +435,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
     float* colscales = reinterpret_cast<float*>(smem + (size_t)nst * STAGE);  // d and -dmin of every draining warp's columns
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
-            mbar_init(bars + i, TC_A_BUSY + 1);  // the unpacking warps and the tokens (with the bytes)
+            mbar_init(bars + i, TC_A_BUSY / 2 + 1);  // the warps that unpack a half and the tokens (with the bytes)
             mbar_init(bars + TC_MAX_STAGES + i, 1);
         }
         for (int i = 0; i < 2; i++) {
@@ -527,39 +524,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
         const int ta = tid - 32 * TC_C_WARPS;
         griddep_launch_dependents();
         if (ta < 2 * TC_ROWS) {
-            // this thread's row and its half of the row's blocks; rows past the matrix repeat its last row
-            const int h = ta >= TC_ROWS, row_l = ta - h * TC_ROWS;
+            // three warps per half of the blocks, a thread per row; rows past the matrix repeat its last row
+            const int g = ta >= TC_ROWS, row_l = ta - g * TC_ROWS;
             const uint8_t* wdata = (a.zip && (row_l & 1)) ? a.A2.data : A.data;
             const int f0 = (int)mat_flat(nb, min(row0 + (a.zip ? row_l >> 1 : row_l), N - 1), 0);
             RAW raw;
-            raw.load(wdata, f0 + ROW_GROUP * b0, h);  // weights do not depend on earlier kernels
-            TcRing ring;
-            int j = 0;
-            auto acquire = [&]() {
-                if (j >= nst) tc_wait(empty + 8 * ring.slot, ring.lap ^ 1, dead);
-                return smem + ring.slot * STAGE + T_BYTES;
-            };
-            auto publish = [&]() {
+            raw.load_stage(0, wdata, f0 + ROW_GROUP * b0, g);  // weights do not depend on earlier kernels
+            raw.load_stage(1, wdata, f0 + ROW_GROUP * b0, g);
+            int slot = 0, j0 = 0;  // of the block's first stage
+            unsigned lap = 0;
+            // stage s of the block: its slot free, filled by `fill`, handed on
+            auto stage = [&](int s, auto&& fill) {
+                const bool wrap = slot + s >= nst;
+                const int at = slot + s - (wrap ? nst : 0);
+                if (j0 + s >= nst) tc_wait(empty + 8 * at, (lap ^ (wrap ? 1u : 0u)) ^ 1u, dead);
+                fill(smem + at * STAGE + T_BYTES);
                 __syncwarp();
-                if (lane == 0) tc_arrive(full + 8 * ring.slot);
-                ring.next(nst);
-                j++;
+                if (lane == 0) tc_arrive(full + 8 * at);
             };
             for (int b = b0; b < b1; b++) {
-                unsigned char* t = nullptr;
                 raw.begin_block();
 #pragma unroll
-                for (int s = 0; s < 4; s++) {
-                    t = acquire();
-                    raw.store(s, t, row_l, h, W_PLANE);
-                    publish();
-                    if (b + 1 < b1) raw.load_stage(s, wdata, f0 + ROW_GROUP * (b + 1), h);  // the words just used, of the next block
+                for (int i = 0; i < 2; i++) {
+                    stage(2 * g + i, [&](unsigned char* t) { raw.store(i, t, row_l, g, W_PLANE); });
+                    if (b + 1 < b1) raw.load_stage(i, wdata, f0 + ROW_GROUP * (b + 1), g);  // the words just used, of the next block
                 }
-                if constexpr (Q4) {
-                    t = acquire();
-                    raw.store_mins(t, row_l, h);
-                    publish();
-                }
+                if constexpr (Q4)
+                    if (g == (b & 1)) stage(4, [&](unsigned char* t) { raw.store_mins(t, row_l); });
+                j0 += SPB, slot += SPB;
+                if (slot >= nst) slot -= nst, lap ^= 1;
             }
         }
         if (S > 1) cluster_sync_all();
@@ -852,6 +845,7 @@ template <class RAW>
 inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_tiles, int S) {
     constexpr int stage = TC_LANES * 128 + RAW::PLANES * TC_ROWS * 128;
     a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024 - TC_COLSCALE_BYTES) / stage));
+    static_assert((TC_SMEM_MAX - 1024 - TC_COLSCALE_BYTES) / stage >= 5, "the ring holds a block's stages");
     a.ahead = S == 1 && row_tiles > sms ? sms : 0;
     static_assert(TC_LANES * TC_SUM_STRIDE * 8 <= 2 * stage, "the epilogue's sums lie over the first stages");
     cudaLaunchConfig_t cfg{};
