@@ -461,7 +461,7 @@ inline int mma_parts(int nb, int mt) {
 }
 template <class RAW, int MT>
 inline cudaError_t launch_mma(cudaStream_t stream, int sms, MmaArgs& a, int strips, int S) {
-    const int nb = a.A1.nb, z = (a.M + 16 * MT - 1) / (16 * MT), ctas = std::max(1, std::min(strips, (S == 1 ? sms : S <= 2 ? sms & ~1 : S == 4 ? 132 : 112) / (S * z))), nbk = (nb + S - 1) / S;
+    const int nb = a.A1.nb, z = (a.M + 16 * MT - 1) / (16 * MT), ctas = std::max(1, std::min(strips, cluster_ctas(k_gemm_mma<RAW, MT>, MMA_THREADS, S, sms) / (S * z))), nbk = (nb + S - 1) / S;
     a.sh = make_share(strips, ctas);
     const int most = a.sh.quot + (a.sh.rem ? 1 : 0);
     // warps per strip: rounds x (blocks of a warp x what a block costs + what a round costs)

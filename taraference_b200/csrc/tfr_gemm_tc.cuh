@@ -839,6 +839,38 @@ inline cudaError_t launch_rows_f32(cudaStream_t stream, int sms, const Mat& w, i
                       tt, epi);
 }
 
+// CTAs of a kernel, one to an SM, that the device runs at once in clusters of S along grid.y (GPCs hold whole clusters): the
+// driver's answer, asked once per device, kernel type and S.  threads: of a CTA; it is taken to fill the shared memory.
+template <class F>
+inline int cluster_ctas(F* kernel, int threads, int S, int sms) {
+    static std::atomic<int> known[16][4];
+    if (S <= 1) return sms;
+    int dev = 0, slot = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return S;
+    while ((1 << slot) < S) slot++;
+    std::atomic<int>& k = known[dev & 15][slot];
+    if (dev < 16 && k.load() > 0) return k.load();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(64, S);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = 200 * 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = S;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = sms / (2 * S);  // no answer: count on half of the chip
+    }
+    const int ctas = std::max(1, n) * S;
+    if (dev < 16) k.store(ctas);
+    return ctas;
+}
+
 inline bool tc_type(int type) { return type == TFR_Q4_K || type == TFR_Q6_K; }
 
 template <class RAW>
@@ -876,16 +908,14 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
     const int rows = a.zip ? TC_ROWS / 2 : TC_ROWS;
     a.tiles1 = (ja.m.N + rows - 1) / rows;
     const int tiles = a.tiles1 + (!a.zip && jb.m.data ? (jb.m.N + rows - 1) / rows : 0), groups = (M + TC_LANES - 1) / TC_LANES;
-    // CTAs the device runs at once by cluster size (GPCs hold whole clusters)
-    auto fit = [&](int ctas) { return ctas <= 2 ? sms : ctas == 4 ? 132 : 112; };
     // the number of k parts with the shortest longest chain: waves of CTAs x (blocks x what a block takes + the ends), in units of
     // a quarter of a block (0.8 us)
     int S = 1;
     double best = 1e30;
     for (int s = 1; s <= 8 && s <= ja.m.nb; s *= 2) {
         if (s < 8 && (ja.m.nb + s - 1) / s > TC_CHAIN) continue;
-        const int ctas = tiles * groups * s;
-        const double t = (double)((ctas + fit(s) - 1) / fit(s)) * (4.5 * ((ja.m.nb + s - 1) / s) + 6 + (s > 1 ? 3 : 0));
+        const int ctas = tiles * groups * s, at_once = cluster_ctas(k_gemm_tc<RawQ4>, TC_THREADS, s, sms);
+        const double t = (double)((ctas + at_once - 1) / at_once) * (4.5 * ((ja.m.nb + s - 1) / s) + 6 + (s > 1 ? 3 : 0));
         if (t < best) best = t, S = s;
     }
     return ja.m.type == TFR_Q4_K ? launch_tc<RawQ4>(stream, sms, a, tiles, S) : launch_tc<RawQ6>(stream, sms, a, tiles, S);
