@@ -7,7 +7,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 from taraference_b200 import synth as S  # noqa: E402
-from tests.test_engine_gpu import TF_WORST, _rel  # noqa: E402
+from tests.test_engine_gpu import TF_WORST, _rel, margin_gated_equal  # noqa: E402
 
 # rows that fill neither row tiles nor row groups' tiles (FF = 1 280, K = 768: three and five blocks), a vocabulary of odd size
 ODD = dict(arch="qwen2", n_layer=1, n_embd=768, n_head=6, n_kv=2, head_dim=128, n_ff=1280, n_vocab=3001,
@@ -216,5 +216,79 @@ def test_hybrid_prompt_in_batches_equals_step_by_step(E, chunk, n):
         logits.append(row)
         kv.free()
     rels = [_rel(b, a) for a, b in zip(*logits)]
+    assert max(rels) < cfg["n_layer"] * TF_WORST, rels
+    m.destroy()
+
+
+def _mixed_types(cfg, seed):
+    """The tensor mix of real hybrid files: of a linear layer's four projections one is Q8_0 (from Q5_K) and three are Q4_K, so
+    that they stay four matrices; attn_output is Q8_0."""
+    tens, rng = S.make_model(cfg, seed=seed), np.random.default_rng(seed)
+    for name, t in list(tens.items()):
+        if name.endswith(("attn_qkv.weight", "ssm_out.weight")):
+            tens[name] = (S.Q5_K, *t[1:3], S.random_q5_k(rng, t[2] * (t[1] // 256), d_sigma=0.0015).reshape(-1))
+        elif name.endswith("attn_output.weight"):
+            tens[name] = (S.Q8_0, *t[1:3], S.quantize_q8_0(rng.normal(0, 0.02, (t[2], t[1])).astype(np.float32)).reshape(-1))
+    return tens
+
+
+def _recurrent_state(m, kv, cfg):
+    return [m.debug_read("ssm_state", cfg["ssm_n_v"] * 128 * 128, kv=kv, layer=i) for i in range(cfg["n_layer"]) if S.is_linear_layer(cfg, i)]
+
+
+@pytest.mark.parametrize("mixed", [False, True], ids=["q4", "mixed"])
+@pytest.mark.parametrize("n", [2, 9, 16, 23])
+def test_hybrid_verification_in_one_pass(E, n, mixed):
+    """forward_greedy_all of a hybrid model as batches (its default) against one decode step per token: the greedy token after every
+    position wherever the step's margin is above what a flip moves, the logits, the recurrent state, and a step that continues
+    from it.  23 tokens take two passes."""
+    cfg = S.TINY_HYBRID
+    m = E.CudaModel.load_with(cfg, _mixed_types(cfg, 6) if mixed else S.make_model(cfg, seed=6))
+    toks = [int(t) for t in np.random.default_rng(n).integers(0, cfg["n_vocab"], n)]
+    m.set_prefill_chunk(0)
+    kv = m.alloc_kv(64)
+    m.forward_greedy([1, 2, 3], kv)
+    want, margins = [], []
+    for t in toks:
+        want.append(m.forward_greedy([t], kv))
+        top = np.sort(m.current_logits())[-2:]
+        margins.append(float(top[1] - top[0]))
+    a = [m.current_logits(), *_recurrent_state(m, kv, cfg)]
+    m.forward_greedy([4], kv)
+    a.append(m.current_logits())
+    kv.free()
+    m.set_prefill_chunk(64)
+    kv = m.alloc_kv(64)
+    m.forward_greedy([1, 2, 3], kv)
+    launches = m.launch_count()
+    got = m.forward_greedy_all(toks, kv)
+    launches = m.launch_count() - launches
+    assert kv.len == 3 + n
+    b = [m.current_logits(), *_recurrent_state(m, kv, cfg)]
+    m.forward_greedy([4], kv)
+    b.append(m.current_logits())
+    assert launches < n * 10 * cfg["n_layer"] or n == 2, launches  # a pass over the layers, not one for every token
+    scale = float(np.abs(a[0]).max())
+    assert margin_gated_equal(list(got), want, margins, gate=cfg["n_layer"] * TF_WORST * scale)
+    rels = [_rel(y, x) for x, y in zip(a, b)]
+    assert max(rels) < cfg["n_layer"] * TF_WORST, rels
+    kv.free()
+    m.destroy()
+
+
+@pytest.mark.parametrize("n", [3, 7, 40, 100])
+def test_hybrid_prompt_of_mixed_types_equals_step_by_step(E, n):
+    """Four projections of different types in a batch: Q8_0 ones on dp4a beside Q4_K ones on mma.sync and tcgen05."""
+    cfg = S.TINY_HYBRID
+    m = E.CudaModel.load_with(cfg, _mixed_types(cfg, 7))
+    prompt = [int(t) for t in np.random.default_rng(n).integers(0, cfg["n_vocab"], n)]
+    out = []
+    for tokens in (0, 2048):
+        m.set_prefill_chunk(tokens)
+        kv = m.alloc_kv(128)
+        m.forward_greedy(prompt, kv)
+        out.append([m.current_logits(), *_recurrent_state(m, kv, cfg)])
+        kv.free()
+    rels = [_rel(y, x) for x, y in zip(*out)]
     assert max(rels) < cfg["n_layer"] * TF_WORST, rels
     m.destroy()
