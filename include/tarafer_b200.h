@@ -148,7 +148,7 @@ int tfr_zero_recurrent(tfr_engine* e, tfr_kv* kv); /* CudaModel::zero_recurrent,
 /* ---- token loop ---- */
 /* CudaModel::forward_greedy, forward.rs:42-71: feeds n tokens at positions kv.len.., returns the
  * greedy next token, advances kv.len by n.  n == 0 -> TFR_E_EMPTY, overflow -> TFR_E_FULL.
- * Prompts (n > 1) are fed through the decode kernels one position at a time. */
+ * Prompts (n > 1) go through the layers in chunks (tfr_set_prefill_chunk). */
 int tfr_forward_greedy(tfr_engine* e, tfr_kv* kv, const uint32_t* tokens, int n, uint32_t* next_token);
 /* CudaModel::forward_greedy_all, forward.rs:268-290 (the verification primitive of speculative decoding,
  * session.rs:321-367): feeds tokens[0..n) at positions kv.len .. and returns in out[i] the greedy prediction
@@ -220,9 +220,10 @@ int tfr_decode_path(const tfr_engine* e);
 /* Prompts and verification batches go through the engine in chunks of up to `tokens` tokens, each chunk reading
  * the weights once (CudaModel::forward_chunk, crates/core/src/cuda/forward.rs:54-65, 360-407; MAX_BATCH,
  * MAX_VERIFY_TOKENS, crates/core/src/cuda/types.rs:7-9).  tokens = 0 feeds every token of a prompt as a decode step;
- * values above the engine's chunk capacity are clamped.  tfr_prefill_chunk returns the size in effect, 0 for models
- * the chunk kernels do not cover (tensor parallelism), which keep the step-by-step route, and for hybrid models, whose
- * recurrent layers step through the tokens inside a chunk. */
+ * values above the engine's chunk capacity are clamped.  tfr_prefill_chunk returns the size in effect; 0 when the
+ * step-by-step route is in effect (tokens = 0, tensor parallelism).  It also returns 0 for hybrid models, which is not that:
+ * their prompts and verification passes go through in chunks of the size set, too; their recurrent layers step through the
+ * tokens inside a chunk. */
 int tfr_set_prefill_chunk(tfr_engine* e, int tokens);
 int tfr_prefill_chunk(const tfr_engine* e);
 /* Kernel launches issued by this engine so far (graph replays count their kernel nodes). */

@@ -2323,8 +2323,9 @@ extern "C" int tfr_set_prefill_chunk(tfr_engine* e, int tokens) {
     e->chunk_tokens = tokens > CHUNK_MAX_TOKENS ? CHUNK_MAX_TOKENS : tokens;
     return TFR_OK;
 }
-// Tokens per chunk in effect: 0 when prompts are fed by decode steps (switched off, or a model the chunk kernels do
-// not cover) and, as ever, for hybrid models, whose recurrent layers step through the tokens inside a chunk.
+// Tokens per batch of models whose layers take all of a batch's tokens at once: 0 when prompts are fed by decode steps (switched
+// off, or a model the chunk kernels do not cover).  Hybrid models report 0 as well, although their prompts and verification
+// passes go through in batches of the same size: callers take 0 for "tokens depend on one another inside a batch".
 extern "C" int tfr_prefill_chunk(const tfr_engine* e) { return e && e->finalized && e->chunk_ok && !is_hybrid(e) ? e->chunk_tokens : 0; }
 
 extern "C" int tfr_decode_path(const tfr_engine* e) {

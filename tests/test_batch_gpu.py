@@ -292,3 +292,21 @@ def test_hybrid_prompt_of_mixed_types_equals_step_by_step(E, n):
     rels = [_rel(y, x) for x, y in zip(*out)]
     assert max(rels) < cfg["n_layer"] * TF_WORST, rels
     m.destroy()
+
+
+def test_prefill_chunk_of_a_hybrid_model(E):
+    """tfr_prefill_chunk reports the batches of models whose layers take all tokens at once and 0 for hybrid models (callers rely on
+    it), whose prompts go through in batches all the same: far fewer launches than with batches switched off."""
+    cfg = S.TINY_HYBRID
+    m = E.CudaModel.load_with(cfg, S.make_model(cfg, seed=2))
+    launches = []
+    for tokens in (0, 64):
+        m.set_prefill_chunk(tokens)
+        assert m.prefill_chunk() == 0
+        kv = m.alloc_kv(64)
+        before = m.launch_count()
+        m.forward_greedy([int(t) for t in np.random.default_rng(1).integers(0, cfg["n_vocab"], 48)], kv)
+        launches.append(m.launch_count() - before)
+        kv.free()
+    assert launches[1] < launches[0] / 5, launches
+    m.destroy()
