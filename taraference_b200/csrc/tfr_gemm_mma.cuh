@@ -3,18 +3,18 @@
 // The arithmetic is that of the decode kernels: exact integer sub-block dots, each scaled by the weights' scale and the
 // activation group's, summed in fp32.  A sub-block of 32 (Q4_K) or 16 (Q6_K) weights is one MMA: 16 tokens (A: the int8
 // activations) x 8 weight rows (B: the 4- or 6-bit values as they are).  Its accumulator starts at 1.5 * 2^23, so that its
-// bits are that float plus the dot, and costs six packed operations for its 128 sums.  tcgen05 would need the scales
-// inside its f16 operands (tfr_gemm_tc.cuh): unpacking weights to them costs 1 900 warp instructions per 128 rows x 64
-// weights and a pipeline of barriers, whatever the batch; here a batch of 16 costs 450, of 80 tokens 1 500, and there is
-// no barrier between a CTA's first weight and its last.
+// bits are that float plus the dot, and costs six packed operations for its 128 sums.  tcgen05 needs the weights' scales
+// inside its f16 operand (tfr_gemm_tc.cuh): unpacking to it and a pipeline of barriers cost the same whatever the batch (2 900
+// warp instructions per 96 rows x 64 weights x up to 128 tokens; here 860 for 16 tokens, 2 600 for 80), and there is no barrier
+// here between a CTA's first weight and its last.
 //
 // A block's sums are joined to the row's once per block.  Relative error against float64, Gaussian values: Q4_K 1.9-2.2e-7
 // for 512 to 27 648 inputs, Q6_K 0.8-1.15e-7 (dp4a 1.8-1.95e-7 and 0.7-1.0e-7); with one chain over a row's sub-blocks and
 // terms cut off instead of rounded it was 3.3-4.5e-7 and 0.8-1.3e-7.
 //
-//   What bounds it: the chains of shared-memory read, MMA and sums, about 60 cycles of a scheduler per MMA whatever the
-//   batch (11 008 gate and up rows of 2 048: 15 us for 16 tokens, 26 for 48, 54 for 80).  As f16 MMAs on 1024 + q, whose sums
-//   need no conversion but twice the MMAs and reads, the same took 18.5, 43 and 67 us.
+//   What bounds it: the chains of shared-memory read, MMA and sums, 80 cycles of a scheduler per MMA with five token tiles (11 008
+//   gate and up rows of 2 048, a launch by itself: 20 us for 16 tokens, 31 for 48, 62 for 80; the tensor pipe is 10 to 16 %
+//   busy, the schedulers issue in 34 to 36 % of the cycles).
 #pragma once
 #include "tfr_gemm_tc.cuh"
 

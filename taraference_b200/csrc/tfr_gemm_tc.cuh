@@ -4,12 +4,11 @@
 // 4- or 6-bit weights with the int8 activations, scaled per sub-block by the weight's 6- or 8-bit scale and the
 // activation group's fp32 scale, scaled per 256-weight block by the block's fp16 d, minus (Q4_K) dmin times the scaled
 // group sums.  An integer MMA would have to leave its accumulator after every 32 (Q4_K) or 16 (Q6_K) weights to meet the
-// activation's scale, which binds the kernel to that scale arithmetic on CUDA cores (9 % of the tensor pipe, 90 us for
-// the 22 016 x 2 048 gate/up pair and 64 tokens).  Here the weights' scales travel inside the f16 operand instead:
+// activation's scale, and on the way meet the weight's.  Here the weights' scales travel inside the f16 operand instead:
 //
-//   A = scale * quant      an integer.  Q4_K: at most 63 * 15, exact in f16.  Q6_K: at most 128 * 32, so an f16 term and
-//                          a residual of at most one unit (a second operand tile);
-//   B = q8                 an integer.
+//   weights   scale * quant   an integer.  Q4_K: at most 63 * 15, exact in f16.  Q6_K: at most 128 * 32, so an f16 term and
+//                             a residual of at most one unit (a second operand tile);
+//   tokens    q8              an integer.
 //
 // The accumulator (fp32, in TMEM) runs over one group of 32 weights.  All products and their sum are integers below 2^24
 // (4 096 * 127 * 32), so the tensor core's truncating additions lose nothing: it holds the exact dot that dp4a computes, and
@@ -19,6 +18,12 @@
 //
 // The min term of Q4_K, sum over a block's groups of m * (d8 * sum q8), is a tf32 product of 8 terms: m is exact, the group sums
 // are two rounded terms whose products stay in accumulators of their own.
+//
+//   What bounds it: the schedulers and the chain through the two accumulators, about 1 450 cycles a stage of 96 rows x 128 tokens x
+//   64 weights (the schedulers issue in half of the cycles, the tensor pipe is 12 % busy on Q4_K, 25 % on Q6_K; with no work left
+//   in any role the waits alone take 860).  Gate and up rows of 2 048 inputs, 2 048 tokens: 787 us; 11 008 inputs to 2 048 rows: 373.
+//   Tried: pairs of CTAs on one tile of rows (cta_group::2; an arrival at the other CTA takes 1 000 cycles: 1 011 us), eight draining
+//   warps with 48 columns each (865 to 920).
 #pragma once
 #include "tfr_chunk.cuh"
 

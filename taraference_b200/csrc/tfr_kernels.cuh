@@ -291,7 +291,7 @@ constexpr size_t GEMV_SMEM_MAX = 225 * 1024;  // opt-in limit is 227 KB includin
 // prologue (1.3 us) and the first trip of its weights to memory are in nobody's shadow.  Two smaller sizes share an SM:
 //   GEMV_SMALL   matrices of a few tiles per CTA (QKV, o-proj): a warp per tile is all they can use;
 //   GEMV_MID     larger ones whose tiles all fit beside a small CTA's: 24 warps take the same two rounds over a gate/up
-//                CTA's 38 tiles as 32 do.
+//                CTA's 38 tiles as 32 do.  Q8_0 rows 2 560 x 8 192 and 4 096 x 2 560 in turn 11.0 us a launch, 13.6 without it.
 // With 56 registers a thread the two together have the SM's 65 536.
 constexpr int GEMV_SMALL = 384, GEMV_MID = 768;
 __host__ __device__ constexpr int gemv_regs(int threads) { return threads == GEMV_THREADS ? 64 : 56; }
@@ -774,7 +774,8 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
         return launch_pdl(k_gemv<BLK, Epi, T, decltype(whole)::value>, dim3(grid), dim3(T), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
     };
     auto by_rows = [&](auto threads) {
-        if constexpr (Epi::ROW_TILES)
+        // (Q8_0: no gain, 2 048 x 8 192 and 2 048 x 2 048 residual rows in turn 9.15 us without and 9.14 with such an instance)
+        if constexpr (Epi::ROW_TILES && !std::is_same<BLK, BlockQ8>::value)
             if (ROW_GROUP * nb == 32) return launch(threads, std::true_type{});
         return launch(threads, std::false_type{});
     };
