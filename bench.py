@@ -485,7 +485,7 @@ def main():
     prefill = {"tokens": int(PROMPT_LEN), "device_ms": model.last_device_ms(),
                "tokens_per_s": PROMPT_LEN / max(model.last_device_ms(), 1e-9) * 1e3, "chunk_tokens": model.prefill_chunk(),
                "what": "tfr_forward_greedy over the whole prompt: chunks of chunk_tokens through the batched kernels "
-                       "(0: one decode step per token), the last token as a decode step with the head"}
+                       "(0: one decode step per token), the head on the last token's row"}
 
     def barrier():
         if world > 1:
