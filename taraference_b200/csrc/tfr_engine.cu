@@ -1766,8 +1766,8 @@ static int chunk_buffers(tfr_engine* e, int M) {
 
 // The kernel of a batch's projections.  Fewer than five tokens leave the tensor cores idle and keep the dp4a kernel, as Q8_0
 // matrices do (TFR_GEMM_DP4A=1 in the environment keeps everything there, a test aid).  mma.sync where it is the faster one:
-// up to 80 tokens on Q4_K (11 008 gate and up rows of 2 048, a launch by itself: 20 us for 16 tokens, 62 for 80; tcgen05 65 and
-// 66) and up to 32 on Q6_K, whose MMAs are half as deep (2 048 rows of 11 008: 18 us for 16 tokens and 25 for 32; tcgen05 42).
+// up to 80 tokens on Q4_K (11 008 gate and up rows of 2 048, a launch by itself: 20 us for 16 tokens, 62 for 80; tcgen05 62 and
+// 63) and up to 32 on Q6_K, whose MMAs are half as deep (2 048 rows of 11 008: 18 us for 16 tokens and 25 for 32; tcgen05 40).
 enum { GEMM_DP4A, GEMM_MMA, GEMM_TC };
 static int gemm_route(int type, int nb, int M) {
     if (M < GEMM_TC_MIN_TOKENS || !tc_type(type) || getenv("TFR_GEMM_DP4A")) return GEMM_DP4A;

@@ -19,11 +19,11 @@
 // The min term of Q4_K, sum over a block's groups of m * (d8 * sum q8), is a tf32 product of 8 terms: m is exact, the group sums
 // are two rounded terms whose products stay in accumulators of their own.
 //
-//   What bounds it: the schedulers and the chain through the two accumulators, about 1 450 cycles a stage of 96 rows x 128 tokens x
+//   What bounds it: the schedulers and the chain through the two accumulators, about 1 400 cycles a stage of 96 rows x 128 tokens x
 //   64 weights (the schedulers issue in half of the cycles, the tensor pipe is 12 % busy on Q4_K, 25 % on Q6_K; with no work left
-//   in any role the waits alone take 860).  Gate and up rows of 2 048 inputs, 2 048 tokens: 787 us; 11 008 inputs to 2 048 rows: 373.
-//   Tried: pairs of CTAs on one tile of rows (cta_group::2; an arrival at the other CTA takes 1 000 cycles: 1 011 us), eight draining
-//   warps with 48 columns each (865 to 920).
+//   in any role the waits alone take 860).  Gate and up rows of 2 048 inputs, 2 048 tokens: 768 us; 11 008 inputs to 2 048 rows: 341.
+//   Tried: pairs of CTAs on one tile of rows (cta_group::2; an arrival at the other CTA takes 1 000 cycles: 1 011 us where one CTA took 814), eight draining
+//   warps with 48 columns each (865 to 920 where sixteen took 817).
 #pragma once
 #include "tfr_chunk.cuh"
 
@@ -152,6 +152,12 @@ __device__ __forceinline__ void tc_dealloc(unsigned addr, unsigned cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// One thread of a converged warp, always the same.
+__device__ __forceinline__ bool tc_elect() {
+    unsigned p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // Barriers by their shared-memory address.  Arrives when the MMAs issued so far are done:
 __device__ __forceinline__ void tc_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -459,23 +465,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
     if (warp < TC_C_WARPS) {
         tc_regs<Regs::C>();
         if ((warp & 1) == 0) {
-            // Two issuing threads take turns by accumulator: with 28 warps at work a wait costs one 300 cycles even when there is
-            // nothing to wait for, and four MMAs 400.
-            if (lane == 0) {
-                TcRing ring;
-                const unsigned long long d0 = tc_desc(smem_u32(smem));
-                const unsigned id = tc_idesc(0, TC_LANES, TC_ROWS), idm = tc_idesc(2, TC_LANES, TC_ROWS);
-                const int buf = warp >> 1;
-                const unsigned acc = tmem + buf * ACC_COLS;
-                if (buf) ring.next(nst);
-                for (int j = buf; j < stages; j += 2) {
-                    tc_wait(full + 8 * ring.slot, ring.lap, dead);
-                    // what the unpacking warps stored becomes visible to the tensor core here, not where they store it: a
-                    // fence there waits for the warp's loads in flight, the next block's words (900 to 2 200 cycles a block)
-                    fence_proxy_async();
-                    const unsigned long long dt = d0 + ((ring.slot * STAGE) >> 4), dw = dt + (T_BYTES >> 4);
-                    if (j >= 2) tc_wait(accempty + 8 * buf, ((j >> 1) - 1) & 1, dead);  // last: nothing else stands behind the draining
-                    tc_fence_after();
+            // Two issuing warps take turns by accumulator: with 28 warps at work a wait costs one 300 cycles even when there is
+            // nothing to wait for.  The whole warp walks the loop and one thread of it issues: that way operands stand in uniform
+            // registers.
+            TcRing ring;
+            const unsigned long long d0 = tc_desc(smem_u32(smem));
+            const unsigned id = tc_idesc(0, TC_LANES, TC_ROWS), idm = tc_idesc(2, TC_LANES, TC_ROWS);
+            const int buf = __shfl_sync(TFR_FULL_MASK, warp >> 1, 0);
+            const unsigned acc = __shfl_sync(TFR_FULL_MASK, tmem, 0) + buf * ACC_COLS;
+            if (buf) ring.next(nst);
+            for (int j = buf; j < stages; j += 2) {
+                tc_wait(full + 8 * ring.slot, ring.lap, dead);
+                // what the unpacking warps stored becomes visible to the tensor core here, not where they store it: a
+                // fence there waits for the warp's loads in flight, the next block's words (900 to 2 200 cycles a block)
+                fence_proxy_async();
+                const unsigned long long dt = d0 + ((ring.slot * STAGE) >> 4), dw = dt + (T_BYTES >> 4);
+                if (j >= 2) tc_wait(accempty + 8 * buf, ((j >> 1) - 1) & 1, dead);  // last: nothing else stands behind the draining
+                tc_fence_after();
+                if (tc_elect()) {
                     if (Q4 && j % SPB == 4) {
                         // high terms of the group sums to the first columns, low terms to the second
                         const int odd = 4 * ((b0 + j / SPB) & 1);
@@ -490,11 +497,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
                     }
                     tc_commit(accfull + 8 * buf);
                     tc_commit(empty + 8 * ring.slot);
-                    ring.next(nst);
-                    ring.next(nst);
                 }
+                __syncwarp();
+                ring.next(nst);
+                ring.next(nst);
             }
-            __syncwarp();
         } else {
             // two threads take turns: a bulk request costs the one that makes it 300 to 560 cycles
             griddep_wait();  // the image comes from the previous kernel
