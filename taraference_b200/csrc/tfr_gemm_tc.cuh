@@ -13,17 +13,17 @@
 // The accumulator (fp32, in TMEM) runs over one group of 32 weights.  All products and their sum are integers below 2^24
 // (4 096 * 127 * 32), so the tensor core's truncating additions lose nothing: it holds the exact dot that dp4a computes, and
 // meets the group's d8 and the block's d in fp32 multiply-adds in registers, round to nearest.  (With d8 inside the operand, as
-// two f16 terms, an accumulator could run over 128 weights, but truncated: 5-10e-7 against float64 where this has 1.9-2.2e-7,
+// two f16 terms, an accumulator could run over 128 weights, but truncated: 5-10e-7 against float64 where this has 1.75-2.1e-7,
 // and groups far smaller than their token's largest lost their low terms among the f16 subnormals.)
 //
 // The min term of Q4_K, sum over a block's groups of m * (d8 * sum q8), is a tf32 product of 8 terms: m is exact, the group sums
 // are two rounded terms whose products stay in accumulators of their own.
 //
 //   What bounds it: the schedulers and the chain through the two accumulators, about 1 400 cycles a stage of 96 rows x 128 tokens x
-//   64 weights (the schedulers issue in half of the cycles, the tensor pipe is 12 % busy on Q4_K, 25 % on Q6_K; with no work left
+//   64 weights (the schedulers issue in half of the cycles, the tensor pipe is 13 % busy on Q4_K, 28 % on Q6_K; with no work left
 //   in any role the waits alone take 860).  Gate and up rows of 2 048 inputs, 2 048 tokens: 768 us; 11 008 inputs to 2 048 rows: 341.
-//   Tried: pairs of CTAs on one tile of rows (cta_group::2; an arrival at the other CTA takes 1 000 cycles: 1 011 us where one CTA took 814), eight draining
-//   warps with 48 columns each (865 to 920 where sixteen took 817).
+//   Tried: pairs of CTAs on one tile of rows (cta_group::2; an arrival at the other CTA takes 1 000 cycles: 1 011 us where one CTA
+//   took 814), eight draining warps with 48 columns each (865 to 920 where sixteen took 817).
 #pragma once
 #include "tfr_chunk.cuh"
 
@@ -376,7 +376,7 @@ __device__ __forceinline__ void tc_regs() {
 }
 
 // Most blocks a CTA adds up one after the other.  The rounding of such a chain grows with the root of its length: Q6_K rows of 43
-// and 108 blocks in one piece 1.30e-7 and 1.94e-7 against float64, in pieces of 22 and 27 1.07e-7 and 1.2e-7 (dp4a, which adds
+// and 108 blocks in one piece 1.30e-7 and 1.94e-7 against float64, in pieces of 22 and 27 1.04e-7 and 1.16e-7 (dp4a, which adds
 // them as a tree, 0.93e-7 and 0.98e-7).
 constexpr int TC_CHAIN = 27;
 
