@@ -196,6 +196,7 @@ struct tfr_engine {
     size_t cpart_floats = 0;
     int chunk_cap = 0;  // tokens the chunk buffers have room for
     unsigned char* cact = nullptr;
+    float2* cpark = nullptr;          // parked sums of k_gemm_tc (tc_park_bytes)
     unsigned char* cimage = nullptr;  // operand image of the tensor-core projections (tfr_gemm_tc.cuh), its token scales
     size_t cact_stride = 0;
     // hybrid layers of a batch: raw projections, the mixer's q / k / v (or the output gates of a full layer), decay and write strength
@@ -266,6 +267,12 @@ static void configure_kernel(F f, bool dynamic) {
     // one L1/shared split for every kernel of the token loop: a change of carve-out between two
     // launches drains the SMs
     cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+
+template <class RAW, int ROWS>
+static void configure_gemm_tc() {
+    cudaFuncSetAttribute(k_gemm_tc<RAW, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcGeom<RAW::PLANES == 1, ROWS>::SMEM);
+    configure_kernel(k_gemm_tc<RAW, ROWS>, false);
 }
 
 // CUDA function attributes, occupancy answers and the stand-alone operators' scratch are per-device state: one
@@ -346,8 +353,10 @@ static void configure_kernels_once() {
     configure_kernel(k_prep_tc, true);
     configure_kernel(k_rows_f32<4, 4, false>, true);
     configure_kernel(k_rows_f32<8, 8, true>, true);
-    configure_kernel(k_gemm_tc<RawQ4>, true);
-    configure_kernel(k_gemm_tc<RawQ6>, true);
+    configure_gemm_tc<RawQ4, 96>();
+    configure_gemm_tc<RawQ4, 64>();
+    configure_gemm_tc<RawQ6, 96>();
+    configure_gemm_tc<RawQ6, 64>();
     configure_kernel(k_prep_mma, true);
     configure_kernel(k_gemm_mma<MmaQ4, 1>, true);
     configure_kernel(k_gemm_mma<MmaQ4, 2>, true);
@@ -675,7 +684,7 @@ extern "C" void tfr_destroy(tfr_engine* e) {
     for (auto& kv : e->vecs) cudaFree(kv.second.dev);
     for (auto& L : e->layers) cudaFree(L.bias_qkv);
     void* ws[] = {e->x, e->q, e->attn, e->h, e->logits, e->partial, e->counters, e->st, e->prompt,
-                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cimage, e->cproj, e->cmix, e->cgates, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
+                  e->layer_taps, e->tap_attn, e->tap_mid, e->tap_h, e->proj, e->qgate, e->loop_layers, e->loop_bar, e->loop_best, e->loop_vec, e->cx, e->cq, e->cattn, e->ch, e->cxn, e->clogits, e->cpart, e->cact, e->cpark, e->cimage, e->cproj, e->cmix, e->cgates, e->ckeys, e->ccount, e->loop_blob, e->loop_head_tasks};
     for (void* p : ws) cudaFree(p);
     if (e->st_host) cudaFreeHost(e->st_host);
     if (e->logits_host) cudaFreeHost(e->logits_host);
@@ -1746,6 +1755,8 @@ static int chunk_buffers(tfr_engine* e, int M) {
     CU(e, cudaMalloc(&e->ch, (size_t)cap * P.ff * 4));
     CU(e, cudaMalloc(&e->cact, (size_t)cap * e->cact_stride));
     CU(e, cudaMalloc(&e->cimage, std::max(tc_image_bytes(kmax, cap), mma_image_bytes(kmax))));
+    if (!e->cpark && tc_park_bytes(kmax / 256, e->prop.multiProcessorCount))
+        CU(e, cudaMalloc(&e->cpark, tc_park_bytes(kmax / 256, e->prop.multiProcessorCount)));
     if (c.hybrid) {
         CU(e, cudaMalloc(&e->cproj, (size_t)cap * std::max(channels + vd + 2 * c.ssm_time_step_rank, 2 * P.nq + 2 * P.nkv) * 4));
         CU(e, cudaMalloc(&e->cmix, (size_t)cap * std::max(channels, P.nq) * 4));
@@ -1784,6 +1795,7 @@ static cudaError_t launch_gemm_typed(cudaStream_t s, int grid, int type, const u
 // What a batch's projections read and report through: the activations in the form of the kernel that follows, the error word.
 struct BatchBufs {
     unsigned char* image;  // GEMM_TC, GEMM_MMA
+    float2* park;          // GEMM_TC
     unsigned char* act;    // GEMM_DP4A: Act arrays, act_stride bytes apart
     size_t act_stride;
     TokenState* st;
@@ -1805,7 +1817,7 @@ static cudaError_t batch_prep(cudaStream_t s, int route, int type, const float* 
 }
 // out = epilogue(W x) over them; jb: the second matrix of a gate/up pair or one that follows
 static cudaError_t batch_gemm(cudaStream_t s, int sms, int route, int M, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep, const BatchBufs& b) {
-    if (route == GEMM_TC) return launch_gemm_tc(s, sms, b.image, M, ja, jb, ep, b.st);
+    if (route == GEMM_TC) return launch_gemm_tc(s, sms, b.image, b.park, M, ja, jb, ep, b.st);
     if (route == GEMM_MMA) return launch_gemm_mma(s, sms, b.image, M, ja, jb, ep, b.st);
     return launch_gemm_typed(s, sms, ja.m.type, b.act, b.act_stride, nullptr, M, ja, jb, F32Seg{}, ep, ja.m.K, b.st);
 }
@@ -1821,7 +1833,7 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     const int cap = e->prop.multiProcessorCount;
     cudaStream_t s = e->stream;
     int n = 0;
-    const BatchBufs bufs{e->cimage, e->cact, e->cact_stride, e->st};
+    const BatchBufs bufs{e->cimage, e->cpark, e->cact, e->cact_stride, e->st};
     auto prep = [&](int route, int type, const float* x, int width, const float* normw, float* xn) -> cudaError_t {
         n++;
         return batch_prep(s, route, type, x, width, M, normw, c.rms_eps, bufs, xn);
@@ -2552,12 +2564,13 @@ extern "C" int tfr_op_project_rows(const tfr_mat* a, const tfr_mat* b, const flo
     const int K = a->m.K, sms = sm_count_cached();
     BatchBufs bufs{};
     bufs.act_stride = (act_smem_bytes(K, false, false) + 255) & ~(size_t)255;
-    const size_t image = std::max(tc_image_bytes(K, M), mma_image_bytes(K)), parts[3] = {image, bufs.act_stride * M, sizeof(TokenState)};
-    size_t total = 0, at[3];
-    for (int i = 0; i < 3; i++) at[i] = total, total += (parts[i] + 255) & ~(size_t)255;
+    const size_t image = std::max(tc_image_bytes(K, M), mma_image_bytes(K)),
+                 parts[4] = {image, bufs.act_stride * M, sizeof(TokenState), tc_park_bytes(K / 256, sms)};
+    size_t total = 0, at[4];
+    for (int i = 0; i < 4; i++) at[i] = total, total += (parts[i] + 255) & ~(size_t)255;
     unsigned char* mem = nullptr;
     if (cudaMalloc(&mem, total) != cudaSuccess) return TFR_E_CUDA;
-    bufs.image = mem + at[0], bufs.act = mem + at[1], bufs.st = (TokenState*)(mem + at[2]);
+    bufs.image = mem + at[0], bufs.act = mem + at[1], bufs.st = (TokenState*)(mem + at[2]), bufs.park = (float2*)(mem + at[3]);
     ChunkEpi ep{};
     ep.kind = b ? CEPI_SILU : CEPI_STORE;
     ep.out = out, ep.ldo = ep.n_rows = a->m.N, ep.use_res = use_res;

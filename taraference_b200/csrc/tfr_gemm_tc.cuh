@@ -19,11 +19,14 @@
 // The min term of Q4_K, sum over a block's groups of m * (d8 * sum q8), is a tf32 product of 8 terms: m is exact, the group sums
 // are two rounded terms whose products stay in accumulators of their own.
 //
-//   What bounds it: the schedulers and the chain through the two accumulators, about 1 400 cycles a stage of 96 rows x 128 tokens x
-//   64 weights (the schedulers issue in half of the cycles, the tensor pipe is 13 % busy on Q4_K, 28 % on Q6_K; with no work left
-//   in any role the waits alone take 860).  Gate and up rows of 2 048 inputs, 2 048 tokens: 768 us; 11 008 inputs to 2 048 rows: 341.
-//   Tried: pairs of CTAs on one tile of rows (cta_group::2; an arrival at the other CTA takes 1 000 cycles: 1 011 us where one CTA
-//   took 814), eight draining warps with 48 columns each (865 to 920 where sixteen took 817).
+//   What bounds it: instructions, and the waits between the roles.  The schedulers issue in two thirds of the cycles; a block of 256
+//   weights x 96 rows x 128 tokens takes 4 300 cycles, of which the tensor pipe works a fifth.  Gate and up rows of 2 048 inputs,
+//   2 048 tokens: 477 us (before: 744), without the unpacking 433, without the MMAs 385, without the multiply-adds 433, with none of
+//   them and without the blocks' ends 212.  11 008 inputs to 2 048 rows: 281 us (before: 326).
+//   What made the difference: waits looked at before their loop (tc_wait), one hand-over for both groups of a stage (532 us with one
+//   for each), d and dmin from TMEM (tc_mma of ones), a CTA that goes on with the next tile, no register spills (local memory is an
+//   L2 round trip where shared memory takes all of L1).  Tried on the way: eight draining warps with 48 or 64 columns each (532 us),
+//   one issuing warp (534), pairs of CTAs on one tile of rows (an arrival at the other CTA takes 1 000 cycles).
 #pragma once
 #include "tfr_chunk.cuh"
 
@@ -116,10 +119,11 @@ __global__ void __launch_bounds__(TC_PREP_THREADS) k_prep_tc(PrepTcArgs a) {
         unsigned q[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
+            const int at = (k & 1) + 4 * (k >> 1);  // values 0, 2, 1, 3 of every four: the order in which weights unpack
             int q0 = 0, q1 = 0;
             if (g != 0.f) {
-                q0 = (int)(signed char)__float2int_rn(v[2 * k] / d);
-                q1 = (int)(signed char)__float2int_rn(v[2 * k + 1] / d);
+                q0 = (int)(signed char)__float2int_rn(v[at] / d);
+                q1 = (int)(signed char)__float2int_rn(v[at + 2] / d);
             }
             sum += q0 + q1;
             q[k] = pack_f16x2(__int2half_rn(q0), __int2half_rn(q1));
@@ -168,6 +172,10 @@ __device__ __forceinline__ void tc_arrive(unsigned bar) { asm volatile("mbarrier
 __device__ __forceinline__ unsigned long long tc_desc(unsigned addr) {
     return (unsigned long long)((addr & 0x3ffffu) >> 4) | (1ull << 16) | ((unsigned long long)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
+// The same for a K-major operand without swizzle, 32 bytes a row: cores of 8 rows x 16 bytes, 128 bytes apart along k, 256 along the rows.
+__device__ __forceinline__ unsigned long long tc_desc_plain(unsigned addr) {
+    return (unsigned long long)((addr & 0x3ffffu) >> 4) | ((unsigned long long)(128 >> 4) << 16) | ((unsigned long long)(256 >> 4) << 32) | (1ull << 46);
+}
 // Instruction descriptor: fp32 accumulator, K-major operands of type `ty` (0: f16, 2: tf32), m x n.
 __device__ __forceinline__ unsigned tc_idesc(unsigned ty, unsigned m, unsigned n) { return (1u << 4) | (ty << 7) | (ty << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
 template <bool TF32>
@@ -190,16 +198,43 @@ __device__ __forceinline__ void tc_ld(float* v, unsigned addr) {
                      : "r"(addr));
     else
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
-                       "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
                      : "r"(addr));
 }
-// 24 columns of this warp's 32 lanes.
-__device__ __forceinline__ void tc_ld24(float* v, unsigned addr) {
-    tc_ld<16>(v, addr);
-    tc_ld<8>(v + 16, addr + 16);
+// The same columns are stored; loads see them after tc_st_wait.
+template <int W>
+__device__ __forceinline__ void tc_st(unsigned addr, const float* v) {
+    if constexpr (W == 8)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                     : "memory");
+    else
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+                     : "memory");
 }
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// 16, 24 or 32 columns.
+template <int N>
+__device__ __forceinline__ void tc_ldn(float* v, unsigned addr) {
+#pragma unroll
+    for (int c = 0; c + 16 <= N; c += 16) tc_ld<16>(v + c, addr + c);
+    if constexpr (N % 16 == 8) tc_ld<8>(v + N - 8, addr + N - 8);
+}
+template <int N>
+__device__ __forceinline__ void tc_stn(unsigned addr, const float* v) {
+#pragma unroll
+    for (int c = 0; c + 16 <= N; c += 16) tc_st<16>(addr + c, v + c);
+    if constexpr (N % 16 == 8) tc_st<8>(addr + N - 8, v + N - 8);
+}
+// Waits for this warp's loads.  Uses of the values stay behind it if they are volatile assembly (fma_pair and the like); other uses
+// take the second form, which costs moves.
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+template <int W>
+__device__ __forceinline__ void tc_ld_wait(float* v) {
+    if constexpr (W == 8)
+        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])::"memory");
+    else
+        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])::"memory");
+}
 __device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
     float2 d;
     asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.ftz.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
@@ -214,27 +249,79 @@ __device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return d;
 }
+// The same on pairs that stay in one 64-bit register: x * k + acc, x the two values of an accumulator.  Volatile: put off past the
+// next load they would keep a third buffer of values alive.
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, const float* x, unsigned long long k) {
+    asm volatile("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tfma.rn.ftz.f32x2 %0, x, %3, %0;\n\t}" : "+l"(acc) : "f"(x[0]), "f"(x[1]), "l"(k));
+}
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, const float* x, const float* y) {
+    asm volatile("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%1, %2};\n\tmov.b64 y, {%3, %4};\n\tfma.rn.ftz.f32x2 %0, x, y, %0;\n\t}"
+                 : "+l"(acc)
+                 : "f"(x[0]), "f"(x[1]), "f"(y[0]), "f"(y[1]));
+}
+__device__ __forceinline__ void mul_pair(unsigned long long& acc, const float* x) {
+    asm volatile("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tmul.rn.ftz.f32x2 %0, x, %0;\n\t}" : "+l"(acc) : "f"(x[0]), "f"(x[1]));
+}
+__device__ __forceinline__ void add_pair(float* x, unsigned long long y) {
+    asm volatile("{\n\t.reg .b64 x;\n\tmov.b64 x, {%0, %1};\n\tadd.rn.ftz.f32x2 x, x, %2;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+f"(x[0]), "+f"(x[1]) : "l"(y));
+}
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
 // Bounded mbarrier wait of a pipeline: once one wait has run out, `dead` lets all others pass at once (the call is then
 // reported as failed; what is computed meanwhile is not used).
-__device__ __forceinline__ void tc_wait(unsigned bar, unsigned parity, volatile int* dead) {
+__device__ __forceinline__ bool tc_try(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void tc_wait_slow(unsigned bar, unsigned parity, volatile int* dead) {
     for (int i = 0; i < MBAR_POLL_LIMIT; i++) {
-        unsigned ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (ok) return;
+        if (tc_try(bar, parity)) return;
         if ((i & 63) == 63 && *dead) return;
     }
     *dead = 1;
 }
+// The first look stands before the loop: a wait that passes at once takes 67 cycles so, 142 as a pass through the loop.  Where
+// it can, a role looks earlier (tc_try) and comes here with what it saw.
+__device__ __forceinline__ void tc_wait(unsigned bar, unsigned parity, volatile int* dead, bool seen) {
+    if (__builtin_expect(!seen, 0)) tc_wait_slow(bar, parity, dead);
+}
+// Roles that run ahead of the others leave the schedulers alone between looks.
+__device__ __forceinline__ void tc_wait_idle(unsigned bar, unsigned parity, volatile int* dead) {
+    if (__builtin_expect(tc_try(bar, parity), 1)) return;
+    for (int i = 0; i < MBAR_POLL_LIMIT; i++) {
+        __nanosleep(32);
+        if (tc_try(bar, parity)) return;
+        if ((i & 63) == 63 && *dead) return;
+    }
+    *dead = 1;
+}
+__device__ __forceinline__ void tc_wait(unsigned bar, unsigned parity, volatile int* dead) { tc_wait(bar, parity, dead, tc_try(bar, parity)); }
 
 // ------------------------------------------------------------------ weights: registers -> operand tile
 
-// Two f16 integers 0 .. 255 out of bytes of w: the byte under an exponent that makes the f16 1024 + byte.
+// 16 bytes to shared memory, by its own address: an aligned-up pointer would be a generic one.
+__device__ __forceinline__ void sts16(unsigned addr, unsigned x, unsigned y, unsigned z, unsigned w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+// A row of an operand tile: where its chunk 0 lies; chunk c is at this ^ (c << 4).
+__device__ __forceinline__ unsigned tc_row_at(int row) { return (unsigned)(row * 128 + ((row & 7) << 4)); }
+
+// Two f16 integers out of the bits `mask` of w: under the exponent that makes the f16 1024 + them.
+__device__ __forceinline__ __half2 tc_bits_1024(unsigned w, unsigned mask) {
+    const unsigned r = (w & mask) | 0x64006400u;
+    return *reinterpret_cast<const __half2*>(&r);
+}
+// Out of bytes PAIR and PAIR + 2 of w.
 template <int PAIR>
 __device__ __forceinline__ __half2 tc_bytes_1024(unsigned w) {
-    const unsigned r = __byte_perm(w, 0x64646464u, PAIR ? 0x4342 : 0x4140);
+    const unsigned r = __byte_perm(w, 0x64646464u, PAIR ? 0x4341 : 0x4240);
     return *reinterpret_cast<const __half2*>(&r);
 }
 __device__ __forceinline__ unsigned tc_bits(__half2 h) { return *reinterpret_cast<const unsigned*>(&h); }
@@ -242,8 +329,8 @@ __device__ __forceinline__ unsigned tc_bits(__half2 h) { return *reinterpret_cas
 // Raw words of half g of a 256-weight block (two stages of 64 weights) that a thread turns into operand values.
 struct RawQ4 {
     static constexpr int PLANES = 1;
-    unsigned s0, s1, s2;  // scale words of the header
-    unsigned n0, n1, n2;  // of the next block's
+    unsigned dm, s0, s1, s2;  // header: d and dmin, scales
+    unsigned nd, n0, n1, n2;  // of the next block's
     unsigned w[2][8];     // 64 weights: [stage of the half]
     // Stage i of the half; the header with the first one, because its words are needed to the block's end.
     __device__ __forceinline__ void load_stage(int i, const uint8_t* data, int f, int g) {
@@ -255,38 +342,41 @@ struct RawQ4 {
         }
         if (i == 0) {
             const int4 hdr = ldg_stream(p);
-            n0 = (unsigned)hdr.y, n1 = (unsigned)hdr.z, n2 = (unsigned)hdr.w;
+            nd = (unsigned)hdr.x, n0 = (unsigned)hdr.y, n1 = (unsigned)hdr.z, n2 = (unsigned)hdr.w;
         }
     }
-    __device__ __forceinline__ void begin_block() { s0 = n0, s1 = n1, s2 = n2; }
-    // The eight mins of a block as tf32 (the first 32 bytes of a row).
-    __device__ __forceinline__ void store_mins(unsigned char* tile, int row) const {
+    __device__ __forceinline__ void begin_block() { dm = nd, s0 = n0, s1 = n1, s2 = n2; }
+    // The eight mins of a block as tf32, 32 bytes; behind them d and -dmin, each the first of eight with zeros after it.
+    __device__ __forceinline__ void store_mins(unsigned at) const {
+        auto f = [](unsigned m, int i) { return __float_as_uint(i2f_small((int)((m >> (8 * i)) & 0xff))); };
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const unsigned m = h ? ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4) : s1 & 0x3f3f3f3fu;
-            *reinterpret_cast<float4*>(tile + tc_swz(row, h)) =
-                make_float4(i2f_small((int)(m & 0xff)), i2f_small((int)((m >> 8) & 0xff)), i2f_small((int)((m >> 16) & 0xff)), i2f_small((int)(m >> 24)));
+            sts16(at ^ (h << 4), f(m, 0), f(m, 1), f(m, 2), f(m, 3));
+            sts16(at ^ ((2 + 2 * h) << 4), __float_as_uint(h ? -f16_to_f32((unsigned short)(dm >> 16)) : f16_to_f32((unsigned short)dm)), 0, 0, 0);
+            sts16(at ^ ((3 + 2 * h) << 4), 0, 0, 0, 0);
         }
     }
     // 64 weights of stage 2 g + i: low nibbles = sub-block 2 (2 g + i), high nibbles the next (kernels/common.cu:40-84)
-    __device__ __forceinline__ void store(int i, unsigned char* tile, int row, int g, int) const {
+    __device__ __forceinline__ void store(int i, unsigned at, int g, int) const {
         const unsigned sc4 = g == 0 ? s0 & 0x3f3f3f3fu : (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
         const __half2 bias = __half2half2(__ushort_as_half(0x6400)), m1024 = __half2half2(__ushort_as_half(0xe400));
         const unsigned sa = __byte_perm(sc4, 0x64646464u, i ? 0x4242 : 0x4040), sb = __byte_perm(sc4, 0x64646464u, i ? 0x4343 : 0x4141);
         const __half2 scl = __hsub2(*reinterpret_cast<const __half2*>(&sa), bias), sch = __hsub2(*reinterpret_cast<const __half2*>(&sb), bias);
-        const __half2 ofl = __hmul2(scl, m1024), ofh = __hmul2(sch, m1024);
+        // (1024 + q) * sc - 1024 * sc, the high nibbles where they stand: (1024 + 16 q) * sc / 16 - 64 * sc.  Products below 2^16, sc / 16
+        // and the difference q * sc exact
+        const __half2 ofl = __hmul2(scl, m1024), sch16 = __hmul2(sch, __half2half2(__ushort_as_half(0x2c00))), ofh = __hmul2(sch16, m1024);
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             unsigned lo[4], hi[4];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const unsigned x = w[i][2 * c + k], l = x & 0x0f0f0f0fu, u = (x >> 4) & 0x0f0f0f0fu;
-                // (1024 + q) * sc - 1024 * sc: both products below 2^16, the difference q * sc exact
-                lo[2 * k] = tc_bits(__hfma2(tc_bytes_1024<0>(l), scl, ofl)), lo[2 * k + 1] = tc_bits(__hfma2(tc_bytes_1024<1>(l), scl, ofl));
-                hi[2 * k] = tc_bits(__hfma2(tc_bytes_1024<0>(u), sch, ofh)), hi[2 * k + 1] = tc_bits(__hfma2(tc_bytes_1024<1>(u), sch, ofh));
+                const unsigned x = w[i][2 * c + k], y = x >> 8;
+                lo[2 * k] = tc_bits(__hfma2(tc_bits_1024(x, 0x000f000fu), scl, ofl)), lo[2 * k + 1] = tc_bits(__hfma2(tc_bits_1024(y, 0x000f000fu), scl, ofl));
+                hi[2 * k] = tc_bits(__hfma2(tc_bits_1024(x, 0x00f000f0u), sch16, ofh)), hi[2 * k + 1] = tc_bits(__hfma2(tc_bits_1024(y, 0x00f000f0u), sch16, ofh));
             }
-            *reinterpret_cast<uint4*>(tile + tc_swz(row, c)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            *reinterpret_cast<uint4*>(tile + tc_swz(row, 4 + c)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            sts16(at ^ (c << 4), lo[0], lo[1], lo[2], lo[3]);
+            sts16(at ^ ((4 + c) << 4), hi[0], hi[1], hi[2], hi[3]);
         }
     }
 };
@@ -312,7 +402,7 @@ struct RawQ6 {
     __device__ __forceinline__ void begin_block() {}
     // 64 weights of stage 2 g + i = runs j = 2 i, 2 i + 1 of half g (kernels/gemv.cu:302-337, as in block_dot):
     // scale * (q - 32) as its f16 rounding and the residual (0 or +-1: |scale * q| <= 4096)
-    __device__ __forceinline__ void store(int i, unsigned char* tile, int row, int, int plane_bytes) const {
+    __device__ __forceinline__ void store(int i, unsigned at, int, int plane_bytes) const {
         const __half2 off = __half2half2(__ushort_as_half(0x6420));  // 1024 + 32
 #pragma unroll
         for (int jl = 0; jl < 2; jl++) {
@@ -331,8 +421,8 @@ struct RawQ6 {
                     hi[2 * k] = tc_bits(p0), hi[2 * k + 1] = tc_bits(p1);
                     lo[2 * k] = tc_bits(__hfma2(sch, q0, __hneg2(p0))), lo[2 * k + 1] = tc_bits(__hfma2(sch, q1, __hneg2(p1)));
                 }
-                *reinterpret_cast<uint4*>(tile + tc_swz(row, 4 * jl + c)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(tile + plane_bytes + tc_swz(row, 4 * jl + c)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                sts16(at ^ ((4 * jl + c) << 4), hi[0], hi[1], hi[2], hi[3]);
+                sts16((at ^ ((4 * jl + c) << 4)) + plane_bytes, lo[0], lo[1], lo[2], lo[3]);
             }
         }
     }
@@ -344,29 +434,27 @@ struct RawQ6 {
 // accumulator has one token, whose d8 it holds in a register, and the columns' d come once a block.  (The other way round every
 // d8 was a broadcast read of shared memory: 770 of 2 000 cycles a stage.)
 //
-// CTA = 128 tokens x a tile of 96 weight rows x a part of the k range, in stages of 64 weights (and one for the mins of a block).
-// Lane 0 of warps 1 and 3 requests the tokens' operand as bulk copies, the unpacking warps turn weights into the other
-// operand, lane 0 of warps 0 and 2 issues the MMAs, the sixteen warps behind drain the accumulators (two buffers in TMEM, each
-// with the two groups of a stage side by side) into the block's and the row's sums they hold in registers (TMEM lanes
-// 32 (w & 3) .., a quarter of the columns); every role runs ahead of the next as far as the rings allow.
+// A CTA stays on its SM and walks over items: 128 tokens x ROWS weight rows, in stages of 64 weights (and one for the mins of a
+// block).  Lane 0 of warps 1 and 3 requests the tokens' operand as bulk copies, eight unpacking warps, a thread for each half of a
+// row's blocks, turn weights into the other operand (two threads on every stage paid the ring's price twice as often), one thread of
+// warps 0 and 2 issues the MMAs, sixteen warps drain the accumulators (two buffers in TMEM, each with the two groups of a stage side
+// by side) into the block's sums in registers and those into the row's sums in TMEM (lanes 32 (w & 3) .., a quarter of the columns).
+// Every role runs ahead of the next as far as the rings allow, over the end of an item too.
+//
+// A block's end needs d and dmin of every column in every lane.  They come as a product of their own: a column of ones times d is d,
+// exactly, in every lane of an accumulator, and TMEM is read four times as fast as shared memory broadcasts.
 //
 // Gate / up pairs (ZIP) alternate the two matrices' rows in the tile, so that a thread holds a gate value beside its up value,
-// as the two rows of a RoPE pair.  The k range is cut over the CTAs of a cluster (grid.y) where a matrix has too few rows to
-// fill the chip, or so many blocks that a chain of additions over them would cost precision: the parts' sums meet through
-// distributed shared memory, each CTA finishing its share of the columns.
-constexpr int TC_C_WARPS = 4, TC_D_WARPS = 16, TC_MAX_STAGES = 8, TC_LANES = 128, TC_ROWS = 96, TC_COLSCALE_BYTES = TC_D_WARPS * 2 * (TC_ROWS / 4) * 4;
-constexpr int TC_SUM_STRIDE = TC_ROWS / 2 + 1;  // float2 of a token's sums in the epilogue; odd, so that 16 tokens' pairs lie in 32 banks
-constexpr size_t TC_SMEM_MAX = 225 * 1024;
-// Unpacking warps, two threads per row, one for each half of its blocks (a warpgroup's registers change together: the last two
-// idle; two threads on every stage paid the ring's price, 900 of 1 500 cycles, twice as often), and the registers of a
-// thread of each role; what they add up to is what the launch has.
-constexpr int TC_A_WARPS = 8, TC_A_BUSY = TC_ROWS / 16, TC_THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + TC_D_WARPS), TC_LAUNCH_REGS = 72;
-template <bool Q4>
-struct TcRegs {
-    static constexpr int C = 24, A = Q4 ? 48 : 64, D = Q4 ? 96 : 88;
-    static_assert(32 * (TC_C_WARPS * C + TC_A_WARPS * A + TC_D_WARPS * D) <= TC_THREADS * TC_LAUNCH_REGS && TC_THREADS * TC_LAUNCH_REGS <= 65536,
-                  "more registers than the launch has");
-};
+// as the two rows of a RoPE pair.  Where the items are too few to fill the chip, the k range is cut over the CTAs of a cluster
+// (grid.y): the parts' sums meet through distributed shared memory, each CTA finishing its share of the tokens.
+constexpr int TC_C_WARPS = 4, TC_A_WARPS = 8, TC_D_WARPS = 16, TC_MAX_STAGES = 12, TC_LANES = 128;
+constexpr int TC_THREADS = 32 * (TC_C_WARPS + TC_A_WARPS + TC_D_WARPS), TC_LAUNCH_REGS = 72;
+constexpr size_t TC_SMEM_MAX = 227 * 1024 - 512;  // less what the kernel declares itself
+// Registers of a thread of each role; what they add up to is what the launch has.
+constexpr int TC_REGS_C = 24, TC_REGS_A = 64, TC_REGS_D = 88;
+static_assert(32 * (TC_C_WARPS * TC_REGS_C + TC_A_WARPS * TC_REGS_A + TC_D_WARPS * TC_REGS_D) <= TC_THREADS * TC_LAUNCH_REGS &&
+                  TC_THREADS * TC_LAUNCH_REGS <= 65536,
+              "more registers than the launch has");
 // Registers of a role: N of the LAUNCH a thread has.  Fewer must be given back, more asked for.
 template <int N>
 __device__ __forceinline__ void tc_regs() {
@@ -375,7 +463,7 @@ __device__ __forceinline__ void tc_regs() {
     else if constexpr (N > TC_LAUNCH_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// Most blocks a CTA adds up one after the other.  The rounding of such a chain grows with the root of its length: Q6_K rows of 43
+// Most blocks a thread adds up one after the other.  The rounding of such a chain grows with the root of its length: Q6_K rows of 43
 // and 108 blocks in one piece 1.30e-7 and 1.94e-7 against float64, in pieces of 22 and 27 1.04e-7 and 1.16e-7 (dp4a, which adds
 // them as a tree, 0.93e-7 and 0.98e-7).
 constexpr int TC_CHAIN = 27;
@@ -385,11 +473,15 @@ struct TcArgs {
     int M, Mp;       // tokens, with padding
     Mat A1, A2;      // ZIP: the pair; otherwise A2 (optional) follows A1 in the grid
     int tiles1;      // row tiles of A1
-    int id1, id2, zip, nst;
-    int ahead;       // row tiles between a CTA and the one that takes its place (0: none does)
+    int items;       // row tiles x token tiles
+    int groups;      // token tiles; an item's token tile is its index modulo this
+    int id1, id2, zip;
+    float2* park;    // sums of finished pieces of a chain (tc_park_bytes)
     ChunkEpi epi;
     TokenState* st;
 };
+
+constexpr int TC_ACCS = 4;  // accumulators in TMEM, two for a stage's groups, twice; behind them the sums of the rows
 
 // Position in a ring of n slots: slot, and the parity of the lap.
 struct TcRing {
@@ -400,171 +492,234 @@ struct TcRing {
     }
 };
 
-template <class RAW>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
+// What a CTA works on.
+template <int ROWS>
+struct TcItem {
+    int n0, nt, row0, N, id_base;
+    bool second;
+    const Mat* A;
+    __device__ __forceinline__ TcItem(const TcArgs& a, int item) {
+        const int tile = item / a.groups;
+        n0 = (item - tile * a.groups) * TC_LANES, nt = min(TC_LANES, a.Mp - n0);
+        second = !a.zip && a.A2.data != nullptr && tile >= a.tiles1;
+        A = second ? &a.A2 : &a.A1;
+        row0 = (tile - (second ? a.tiles1 : 0)) * (a.zip ? ROWS / 2 : ROWS);
+        N = A->N, id_base = second ? a.id2 : a.id1;
+    }
+    // matrix and row of the tile's row r; rows past the matrix repeat its last row
+    __device__ __forceinline__ const uint8_t* row(const TcArgs& a, int r, int& f) const {
+        f = (int)mat_flat(A->nb, min(row0 + (a.zip ? r >> 1 : r), N - 1), 0);
+        return (a.zip && (r & 1)) ? a.A2.data : A->data;
+    }
+};
+
+template <bool Q4, int ROWS>
+struct TcGeom {
+    static constexpr int NC = ROWS / (TC_D_WARPS / 4);  // columns of a draining warp
+    static constexpr int CH = 8;  // columns of a step at a block's end
+    static constexpr int T_BYTES = TC_LANES * 128, W_PLANE = ROWS * 128, STAGE = T_BYTES + (Q4 ? 1 : 2) * W_PLANE;
+    static constexpr int SUM_STRIDE = ROWS / 2 + 1;         // float2 of a token's sums when k parts meet; odd, so that 16 tokens' pairs lie in 32 banks
+    static constexpr int OUT_PAIRS = 4;               // pairs of columns a warp turns from tokens to columns at a time
+    static constexpr int WARP_BYTES = 32 * (OUT_PAIRS + 1) * 8 + NC * 4;  // a draining warp's own: that, and its columns' d and dmin
+    static constexpr int ONES_BYTES = Q4 ? TC_LANES * 32 : 0;  // a tf32 operand whose first column is ones, the others zero
+    static constexpr int NST_MAX = (int)((TC_SMEM_MAX - 1024 - TC_D_WARPS * WARP_BYTES - ONES_BYTES) / STAGE);
+    static constexpr int NST = NST_MAX < TC_MAX_STAGES ? NST_MAX : TC_MAX_STAGES;
+    static constexpr size_t SMEM = (size_t)NST * STAGE + TC_D_WARPS * WARP_BYTES + ONES_BYTES + 1024;
+    static_assert(NC % CH == 0 && WARP_BYTES % 16 == 0 && (TC_ACCS + 1) * ROWS <= 512 && NC % 8 == 0 && TC_LANES * SUM_STRIDE * 8 <= NST * STAGE, "");
+};
+constexpr size_t TC_PARK_BYTES = TC_LANES * 96 * 4;
+// Scratch for matrices of nb blocks a row: three CTAs' sums for every SM, where a chain can be cut at all.
+__host__ __device__ inline size_t tc_park_bytes(int nb, int sms) { return nb > TC_CHAIN ? (size_t)3 * sms * TC_PARK_BYTES : 0; }
+
+template <class RAW, int ROWS>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant__ TcArgs a) {
     constexpr bool Q4 = RAW::PLANES == 1;
-    using Regs = TcRegs<Q4>;
-    constexpr int NC = TC_ROWS / (TC_D_WARPS / 4);  // columns of a draining warp
-    constexpr int SPB = Q4 ? 5 : 4;                 // stages of a block: four of weights, one of mins
-    constexpr int T_BYTES = TC_LANES * 128, W_PLANE = TC_ROWS * 128, STAGE = T_BYTES + RAW::PLANES * W_PLANE;
+    using G = TcGeom<Q4, ROWS>;
+    constexpr int NC = G::NC, CH = G::CH;
+    constexpr int SPB = Q4 ? 5 : 4;  // stages of a block: four of weights, one of mins
+    constexpr int T_BYTES = G::T_BYTES, W_PLANE = G::W_PLANE, STAGE = G::STAGE, nst = G::NST;
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
-    __shared__ unsigned long long bars[2 * TC_MAX_STAGES + 4];
+    __shared__ unsigned long long bars[2 * TC_MAX_STAGES + 8];
     __shared__ unsigned tmem_slot;
     __shared__ int dead_s;
     volatile int* dead = &dead_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned full = smem_u32(bars), empty = full + 8 * TC_MAX_STAGES, accfull = empty + 8 * TC_MAX_STAGES, accempty = accfull + 16;
+    const unsigned full = smem_u32(bars), empty = full + 8 * TC_MAX_STAGES, accfull = empty + 8 * TC_MAX_STAGES, accempty = accfull + 32;
     const int S = gridDim.y, part = blockIdx.y;  // k parts
-    const int n0 = blockIdx.z * TC_LANES, nt = min(TC_LANES, a.Mp - n0), nst = a.nst;  // this CTA's tokens
-    const int tile = blockIdx.x;
-    const bool second = !a.zip && a.A2.data != nullptr && tile >= a.tiles1;
-    const Mat& A = second ? a.A2 : a.A1;
-    const int nb = A.nb, K = A.K, N = A.N;
-    const int row0 = (tile - (second ? a.tiles1 : 0)) * (a.zip ? TC_ROWS / 2 : TC_ROWS);
+    const int nb = a.A1.nb, K = a.A1.K;
     const int b0 = nb * part / S, b1 = nb * (part + 1) / S;
-    if (warp == 3) {
-        // The rows this CTA unpacks start towards L2 at once, and so do those of the CTA that will follow on this SM: the registers
-        // of the unpacking warps hold one block ahead, which covers an L2 hit but not a trip to memory.
-        auto ahead = [&](const Mat& m, int row) {
-            if (row >= m.N) return;
-            const size_t f = mat_flat(nb, row, 0), t0 = (f + ROW_GROUP * b0) >> 5, t1 = (f + ROW_GROUP * b1 + 31) >> 5;
-            constexpr size_t TB = Q4 ? Q4_TILE_BYTES : Q6_TILE_BYTES;
-            bulk_prefetch_l2(m.data + t0 * TB, (unsigned)((t1 - t0) * TB));
-        };
-        for (int w = 0; w <= 1; w++) {
-            if (w == 1 && a.ahead == 0) break;
-            const int t = row0 + w * a.ahead * (a.zip ? TC_ROWS / 2 : TC_ROWS);
-            if (lane < TC_ROWS / ROW_GROUP) {
-                if (a.zip) ahead(lane & 1 ? a.A2 : A, t + (lane >> 1) * ROW_GROUP);
-                else ahead(A, t + lane * ROW_GROUP);
-            }
-        }
-    }
-    const int stages = SPB * (b1 - b0);
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr unsigned ACC_COLS = 2 * TC_ROWS, TMEM_COLS = 512;  // the rows for a stage's first and second group, twice
-    float* colscales = reinterpret_cast<float*>(smem + (size_t)nst * STAGE);  // d and -dmin of every draining warp's columns
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
-            mbar_init(bars + i, TC_A_BUSY / 2 + 1);  // the warps that unpack a half and the tokens (with the bytes)
-            mbar_init(bars + TC_MAX_STAGES + i, 1);
+            mbar_init(bars + i, (ROWS + 31) / 32 + 1);  // the warps that unpack a half and the tokens (with the bytes)
+            mbar_init(bars + TC_MAX_STAGES + i, 2);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(bars + 2 * TC_MAX_STAGES + i, 1);
-            mbar_init(bars + 2 * TC_MAX_STAGES + 2 + i, TC_D_WARPS);
+            mbar_init(bars + 2 * TC_MAX_STAGES + 4 + i, TC_D_WARPS);
         }
         dead_s = 0;
         mbar_fence_init();
     }
-    if (warp == 0) tc_alloc(&tmem_slot, TMEM_COLS);
+    if (Q4 && tid < 2 * TC_LANES) {
+        // cores of even index hold the first half of eight rows
+        const float4 z = make_float4(tid & 8 ? 0.f : 1.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(smem + (size_t)nst * STAGE + TC_D_WARPS * G::WARP_BYTES + tid * 16) = z;
+    }
+    fence_proxy_async();
+    if (warp == 0) tc_alloc(&tmem_slot, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = tmem_slot;
 
     if (warp < TC_C_WARPS) {
-        tc_regs<Regs::C>();
+        tc_regs<TC_REGS_C>();
+        const int stages = SPB * (b1 - b0);
         if ((warp & 1) == 0) {
-            // Two issuing warps take turns by accumulator: with 28 warps at work a wait costs one 300 cycles even when there is
-            // nothing to wait for.  The whole warp walks the loop and one thread of it issues: that way operands stand in uniform
-            // registers.
-            TcRing ring;
-            const unsigned long long d0 = tc_desc(smem_u32(smem));
-            const unsigned id = tc_idesc(0, TC_LANES, TC_ROWS), idm = tc_idesc(2, TC_LANES, TC_ROWS);
-            const int buf = __shfl_sync(TFR_FULL_MASK, warp >> 1, 0);
-            const unsigned acc = __shfl_sync(TFR_FULL_MASK, tmem, 0) + buf * ACC_COLS;
-            if (buf) ring.next(nst);
-            for (int j = buf; j < stages; j += 2) {
-                tc_wait(full + 8 * ring.slot, ring.lap, dead);
-                // what the unpacking warps stored becomes visible to the tensor core here, not where they store it: a
-                // fence there waits for the warp's loads in flight, the next block's words (900 to 2 200 cycles a block)
-                fence_proxy_async();
-                const unsigned long long dt = d0 + ((ring.slot * STAGE) >> 4), dw = dt + (T_BYTES >> 4);
-                if (j >= 2) tc_wait(accempty + 8 * buf, ((j >> 1) - 1) & 1, dead);  // last: nothing else stands behind the draining
-                tc_fence_after();
-                if (tc_elect()) {
-                    if (Q4 && j % SPB == 4) {
-                        // high terms of the group sums to the first columns, low terms to the second
-                        const int odd = 4 * ((b0 + j / SPB) & 1);
-                        tc_mma<true>(acc, dt + odd, dw, idm, 0);
-                        tc_mma<true>(acc + TC_ROWS, dt + odd + 2, dw, idm, 0);
-                    } else {
+            // Two issuing warps take turns by stage, each with two accumulators of its own: a hand-over costs a warp some 200 cycles of
+            // waiting and branching.  A block's mins are one stage to both: d and -dmin, and the mins' product.
+            if (tc_elect()) {
+                const int w = warp >> 1;
+                TcRing ring;
+                if (w) ring.next(nst);
+                const unsigned base = smem_u32(smem) >> 4, dhi = (unsigned)(tc_desc(0) >> 32);
+                const unsigned id = tc_idesc(0, TC_LANES, ROWS), idm = tc_idesc(2, TC_LANES, ROWS);
+                auto desc = [&](unsigned at) { return ((unsigned long long)dhi << 32) | (at | (1u << 16)); };
+                const unsigned acc0 = tmem + 2 * w * ROWS, af = accfull + 8 * w, ae = accempty + 8 * w;
+                unsigned par = 1;     // of the accumulators' last reading; the first lap waits for none
+                const int items = (a.items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+                // a stage's two accumulators: free, filled by mmas, handed on
+                auto stage = [&](int step, int commits, auto&& mmas) {
+                    const bool there = tc_try(full + 8 * ring.slot, ring.lap), free_ = tc_try(ae, par);
+                    tc_wait(full + 8 * ring.slot, ring.lap, dead, there);
+                    // what the unpacking warps stored becomes visible to the tensor core here, not where they store it: a
+                    // fence there waits for the warp's loads in flight, the next block's words (900 to 2 200 cycles a block)
+                    fence_proxy_async();
+                    tc_wait(ae, par, dead, free_);
+                    tc_fence_after();
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            tc_mma<false>(acc + (kk >> 1) * TC_ROWS, dt + 2 * kk, dw + 2 * kk, id, kk & 1);
-                            if (!Q4) tc_mma<false>(acc + (kk >> 1) * TC_ROWS, dt + 2 * kk, dw + (W_PLANE >> 4) + 2 * kk, id, 1);
-                        }
+                    for (int g = 0; g < 2; g++) mmas(g);
+                    tc_commit(af);
+                    par ^= 1;
+                    for (int i = 0; i < commits; i++) tc_commit(empty + 8 * ring.slot);  // two a stage
+                    for (int i = 0; i < step; i++) ring.next(nst);
+                };
+                for (int j = items * (b1 - b0), b = b0; j > 0; j--) {
+#pragma unroll
+                    for (int s = 0; s < 2; s++) {
+                        const unsigned dt = base + ((ring.slot * STAGE) >> 4), dw = dt + (T_BYTES >> 4);
+                        stage(Q4 && s == 1 && w ? 1 : 2, 2, [&](int g) {
+#pragma unroll
+                            for (int q = 0; q < 2; q++) {
+                                const int kk = 2 * g + q;
+                                tc_mma<false>(acc0 + g * ROWS, desc(dt + 2 * kk), desc(dw + 2 * kk), id, q);
+                                if (!Q4) tc_mma<false>(acc0 + g * ROWS, desc(dt + 2 * kk), desc(dw + (W_PLANE >> 4) + 2 * kk), id, 1);
+                            }
+                        });
                     }
-                    tc_commit(accfull + 8 * buf);
-                    tc_commit(empty + 8 * ring.slot);
+                    if constexpr (Q4) {
+                        const unsigned dt = base + ((ring.slot * STAGE) >> 4) + 4 * (b & 1), dw = base + ((ring.slot * STAGE) >> 4) + (T_BYTES >> 4);
+                        // d and -dmin of the columns in every lane; the mins' product with the high and with the low terms of the group sums
+                        stage(w ? 2 : 1, 1, [&](int g) {
+                            if (w) tc_mma<true>(acc0 + g * ROWS, desc(dt + 2 * g), desc(dw), idm, 0);
+                            else tc_mma<true>(acc0 + g * ROWS, tc_desc_plain(smem_u32(smem) + nst * STAGE + TC_D_WARPS * G::WARP_BYTES), desc(dw + 2 + 2 * g), idm, 0);
+                        });
+                        if (++b == b1) b = b0;
+                    }
                 }
-                __syncwarp();
-                ring.next(nst);
-                ring.next(nst);
             }
+            __syncwarp();
         } else {
             // two threads take turns: a bulk request costs the one that makes it 300 to 560 cycles
             griddep_wait();  // the image comes from the previous kernel
             if (lane == 0) {
                 TcRing ring;
                 const size_t plane = (size_t)a.Mp * 128;
-                const unsigned char* src = a.image + (size_t)n0 * 128;
                 if (warp >> 1) ring.next(nst);
-                for (int j = warp >> 1; j < stages; j += 2) {
-                    const int b = b0 + j / SPB, s = j % SPB;
-                    if (j >= nst) tc_wait(empty + 8 * ring.slot, ring.lap ^ 1, dead);
-                    unsigned long long* bar = bars + ring.slot;
-                    mbar_expect_tx(bar, nt * 128);
-                    bulk_load(smem + ring.slot * STAGE, src + (s == 4 ? tc_sums_at(K, a.Mp) + (b >> 1) * plane : (4 * b + s) * plane), nt * 128, bar);
-                    ring.next(nst);
-                    ring.next(nst);
+                int j = warp >> 1, lap = 0;
+                for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+                    const int n0 = (item % a.groups) * TC_LANES, nt = min(TC_LANES, a.Mp - n0);
+                    const unsigned char* src = a.image + (size_t)n0 * 128;
+                    for (; j < stages; j += 2) {
+                        const int b = b0 + j / SPB, s = j % SPB;
+                        if (lap) tc_wait_idle(empty + 8 * ring.slot, ring.lap ^ 1, dead);
+                        if (*dead) break;
+                        unsigned long long* bar = bars + ring.slot;
+                        mbar_expect_tx(bar, nt * 128);
+                        bulk_load(smem + ring.slot * STAGE, src + (s == 4 ? tc_sums_at(K, a.Mp) + (b >> 1) * plane : (4 * b + s) * plane), nt * 128, bar);
+                        ring.next(nst);
+                        ring.next(nst);
+                        if (ring.lap) lap = 1;
+                    }
+                    j -= stages;
                 }
             }
             __syncwarp();
         }
+        if (*dead)  // after a wait that ran out: copies and MMAs in flight have this long to land before shared memory goes
+            for (int i = 0; i < 100; i++) __nanosleep(1000);
         griddep_launch_dependents();
         asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");  // the last accumulator has been read
         tc_fence_after();
-        if (warp == 0) tc_dealloc(tmem, TMEM_COLS);
+        if (warp == 0) tc_dealloc(tmem, 512);
         if (S > 1) cluster_sync_all();
         if (S > 1) cluster_sync_all();
         return;
     }
 
     if (warp < TC_C_WARPS + TC_A_WARPS) {
-        tc_regs<Regs::A>();
-        const int ta = tid - 32 * TC_C_WARPS;
+        tc_regs<TC_REGS_A>();
+        const int ta = tid - 32 * TC_C_WARPS, g = ta >> 7, row_l = ta & 127;  // half of the blocks; row of the tile
         griddep_launch_dependents();
-        if (ta < 2 * TC_ROWS) {
-            // three warps per half of the blocks, a thread per row; rows past the matrix repeat its last row
-            const int g = ta >= TC_ROWS, row_l = ta - g * TC_ROWS;
-            const uint8_t* wdata = (a.zip && (row_l & 1)) ? a.A2.data : A.data;
-            const int f0 = (int)mat_flat(nb, min(row0 + (a.zip ? row_l >> 1 : row_l), N - 1), 0);
-            RAW raw;
-            raw.load_stage(0, wdata, f0 + ROW_GROUP * b0, g);  // weights do not depend on earlier kernels
-            raw.load_stage(1, wdata, f0 + ROW_GROUP * b0, g);
-            int slot = 0, j0 = 0;  // of the block's first stage
+        if (row_l < ((ROWS + 31) & ~31)) {
+            const int r = min(row_l, ROWS - 1);
+            const bool on = row_l < ROWS;
+            const unsigned tile = smem_u32(smem) + T_BYTES + tc_row_at(r);  // the row in slot 0
+            int slot = 0;  // of the block's first stage
             unsigned lap = 0;
-            // stage s of the block: its slot free, filled by `fill`, handed on
-            auto stage = [&](int s, auto&& fill) {
-                const bool wrap = slot + s >= nst;
-                const int at = slot + s - (wrap ? nst : 0);
-                if (j0 + s >= nst) tc_wait(empty + 8 * at, (lap ^ (wrap ? 1u : 0u)) ^ 1u, dead);
-                fill(smem + at * STAGE + T_BYTES);
-                __syncwarp();
-                if (lane == 0) tc_arrive(full + 8 * at);
-            };
-            for (int b = b0; b < b1; b++) {
-                raw.begin_block();
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    stage(2 * g + i, [&](unsigned char* t) { raw.store(i, t, row_l, g, W_PLANE); });
-                    if (b + 1 < b1) raw.load_stage(i, wdata, f0 + ROW_GROUP * (b + 1), g);  // the words just used, of the next block
+            bool again = false;  // the ring has been round
+            for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+                const TcItem<ROWS> it(a, item);
+                int f0;
+                const uint8_t* wdata = it.row(a, r, f0);
+                RAW raw;
+                raw.load_stage(0, wdata, f0 + ROW_GROUP * b0, g);  // weights do not depend on earlier kernels
+                raw.load_stage(1, wdata, f0 + ROW_GROUP * b0, g);
+                // the rows of the CTA's next item start towards L2: the registers hold one block ahead, which covers an L2 hit but
+                // not a trip to memory
+                const int next = item + gridDim.x;
+                if (next < a.items && next % a.groups == 0 && g == 0 && (row_l & 3) == 0) {
+                    const TcItem<ROWS> in(a, next);
+                    // one request a row group of each matrix
+                    const int q = row_l >> 2, rows = a.zip ? ROWS / 2 : ROWS, rg = (a.zip ? q >> 1 : q) * ROW_GROUP;
+                    if (rg < rows && in.row0 + rg < in.N) {
+                        constexpr size_t TB = Q4 ? Q4_TILE_BYTES : Q6_TILE_BYTES;
+                        const size_t f = mat_flat(nb, in.row0 + rg, 0), t0 = (f + ROW_GROUP * b0) >> 5, t1 = (f + ROW_GROUP * b1 + 31) >> 5;
+                        bulk_prefetch_l2((a.zip && (q & 1) ? a.A2.data : in.A->data) + t0 * TB, (unsigned)((t1 - t0) * TB));
+                    }
                 }
-                if constexpr (Q4)
-                    if (g == (b & 1)) stage(4, [&](unsigned char* t) { raw.store_mins(t, row_l); });
-                j0 += SPB, slot += SPB;
-                if (slot >= nst) slot -= nst, lap ^= 1;
+                // stage s of the block: its slot free, filled by `fill`, handed on
+                auto stage = [&](int s, auto&& fill) {
+                    const bool wrap = slot + s >= nst;
+                    const int at = slot + s - (wrap ? nst : 0);
+                    if (again || wrap) tc_wait_idle(empty + 8 * at, (lap ^ (wrap ? 1u : 0u)) ^ 1u, dead);
+                    if (on) fill(tile + at * STAGE);
+                    __syncwarp();
+                    if (lane == 0) tc_arrive(full + 8 * at);
+                };
+                for (int b = b0; b < b1; b++) {
+                    raw.begin_block();
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        stage(2 * g + i, [&](unsigned t) { raw.store(i, t, g, W_PLANE); });
+                        if (b + 1 < b1) raw.load_stage(i, wdata, f0 + ROW_GROUP * (b + 1), g);  // the words just used, of the next block
+                    }
+                    if constexpr (Q4)
+                        if (g == (b & 1)) stage(4, [&](unsigned t) { raw.store_mins(t); });
+                    slot += SPB;
+                    if (slot >= nst) slot -= nst, lap ^= 1, again = true;
+                }
             }
         }
         if (S > 1) cluster_sync_all();
@@ -572,161 +727,296 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcArgs a) {
         return;
     }
 
-    tc_regs<Regs::D>();
-    const int dwarp = warp - TC_C_WARPS - TC_A_WARPS, quad = warp & 3, cg = dwarp >> 2, tok = quad * 32 + lane, m = n0 + tok;
-    static_assert(NC == 24 && TC_COLSCALE_BYTES == TC_D_WARPS * 2 * NC * 4, "");
-    float* colscale = colscales + dwarp * 2 * NC;
-    float2 tot[NC / 2];  // of the token and its columns: over the row
-#pragma unroll
-    for (int i = 0; i < NC / 2; i++) tot[i] = make_float2(0.f, 0.f);
-    {
-        // lanes below NC hold a column's d, and dmin above it, a block ahead
-        const int col = cg * NC + min(lane, NC - 1);
-        const uint8_t* ddata = (a.zip && (col & 1)) ? a.A2.data : A.data;
-        const int df = (int)mat_flat(nb, min(row0 + (a.zip ? col >> 1 : col), N - 1), 0);
+    tc_regs<TC_REGS_D>();
+    const int dwarp = warp - TC_C_WARPS - TC_A_WARPS, td = tid - 32 * (TC_C_WARPS + TC_A_WARPS), quad = warp & 3, cg = dwarp >> 2, tok = quad * 32 + lane;
+    unsigned char* own = smem + (size_t)nst * STAGE + dwarp * G::WARP_BYTES;
+    float2* turn = reinterpret_cast<float2*>(own);
+    float* colscale = reinterpret_cast<float*>(own + 32 * (G::OUT_PAIRS + 1) * 8);  // Q6_K: d of the warp's columns
+    const unsigned lanes = tmem + ((unsigned)quad << 21) + cg * NC;
+    const unsigned lanes_tot = lanes + TC_ACCS * ROWS;  // the row's sums of the token and its columns
+    griddep_launch_dependents();
+    griddep_wait();  // nothing reaches an accumulator before the image is complete; residuals are then, too
+    const int pieces = (b1 - b0 + TC_CHAIN - 1) / TC_CHAIN;
+    unsigned par = 0;  // of the buffers' first uses in a block; Q4_K uses them three times
+    for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+        // Q6_K: lanes hold two columns' d, a block ahead: column lane and, where there is one, 32 further
+        int df, dmore;  // flat index of the one; from there to the other
+        const uint8_t* dp;
+        unsigned d8_at;
+        {
+            const TcItem<ROWS> it(a, item);
+            int f;
+            dp = (a.zip && (lane & 1)) || it.second ? a.A2.data : a.A1.data;
+            d8_at = (unsigned)(4 * b0) * a.Mp + min(it.n0 + tok, a.Mp - 1);
+            it.row(a, cg * NC + min(lane, NC - 1), df);
+            it.row(a, cg * NC + (NC > 32 ? min(lane + 32, NC - 1) : 0), f);  // 32 is even: the same matrix, unless it repeats the last column
+            dmore = lane + 32 < NC ? f - df : 0;
+        }
+        float dnext[2];
         auto load_d = [&](int b) {
-            const int f = df + ROW_GROUP * b;
-            return Q4 ? __ldg(reinterpret_cast<const unsigned*>(ddata + (size_t)(f >> 5) * Q4_TILE_BYTES + (f & 31) * 16))
-                      : (unsigned)__ldg(reinterpret_cast<const unsigned short*>(ddata + (size_t)(f >> 5) * Q6_TILE_BYTES + Q6_PIECES * 512 + (f & 31) * 2));
-        };
-        unsigned dnext = load_d(b0);
-        griddep_launch_dependents();
-        griddep_wait();  // nothing reaches an accumulator before the image is complete; residuals are then, too
-        const unsigned lanes = tmem + ((unsigned)quad << 21) + cg * NC;
-        float2 sum[NC / 2];  // of the block without its d
-        // d8 of the token's groups, two stages ahead
-        const float2* d8 = reinterpret_cast<const float2*>(a.image + tc_d8_at(K, a.Mp)) + (size_t)(4 * b0) * a.Mp + min(m, a.Mp - 1);
-        const int d8_end = 4 * (b1 - b0);
-        auto load_d8 = [&](int i) { return __ldcg(d8 + (size_t)min(i, d8_end - 1) * a.Mp); };  // L1 may hold the last image
-        float2 knext[2] = {load_d8(0), load_d8(1)};
-        int j = 0;
-        float v[NC];
-        // the two accumulators of stage j, one after the other: use(which)
-        auto drain = [&](auto&& use) {
-            const int buf = j & 1;
-            tc_wait(accfull + 8 * buf, (j >> 1) & 1, dead);
-            tc_fence_after();
 #pragma unroll
-            for (int g = 0; g < 2; g++) {
-                tc_ld24(v, lanes + buf * ACC_COLS + g * TC_ROWS);
-                tc_ld_wait();
-                if (g == 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) tc_arrive(accempty + 8 * buf);
-                }
-                use(g);
+            for (int h = 0; h < (NC > 32 ? 2 : 1); h++) {
+                const int f = df + ROW_GROUP * b + (h ? dmore : 0);
+                dnext[h] = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(dp + (size_t)(f >> 5) * Q6_TILE_BYTES + Q6_PIECES * 512 + (f & 31) * 2)));
             }
-            j++;
         };
+        if (!Q4) load_d(b0);
+        // d8 of the token's groups, two stages ahead
+        int d8_left = 4 * (b1 - b0);
+        auto load_d8 = [&] {  // L1 may hold the last image
+            const float2 k = __ldcg(reinterpret_cast<const float2*>(a.image + tc_d8_at(K, a.Mp)) + d8_at);
+            if (--d8_left > 0) d8_at += a.Mp;
+            return k;
+        };
+        float2 knext[2];
+        knext[0] = load_d8(), knext[1] = load_d8();
+        int piece = 1, cut = b0 + (b1 - b0) / pieces;
+        auto clear = [&] {
+            float z[NC];
+#pragma unroll
+            for (int i = 0; i < NC; i++) z[i] = 0.f;
+            tc_stn<NC>(lanes_tot, z);
+            tc_st_wait();
+        };
+        clear();
         for (int b = b0; b < b1; b++) {
-            if (lane < NC) {
-                colscale[lane] = f16_to_f32((unsigned short)dnext);
-                if (Q4) colscale[NC + lane] = -f16_to_f32((unsigned short)(dnext >> 16));
+            if (!Q4) {
+                if (lane < NC) colscale[lane] = dnext[0];
+                if (NC > 32 && lane + 32 < NC) colscale[lane + 32] = dnext[1];
+                if (b + 1 < b1) load_d(b + 1);
             }
-            if (b + 1 < b1) dnext = load_d(b + 1);
+            // use k of the block of buffer `buf`
+            auto wait_full = [&](int buf, int k) {
+                tc_wait(accfull + 8 * buf, par ^ (k & 1), dead);
+                tc_fence_after();
+            };
+            auto release = [&](int buf) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc_arrive(accempty + 8 * buf);
+            };
+            unsigned long long sum[NC / 2];  // of the block without its d
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) sum[i] = 0;
 #pragma unroll
             for (int s = 0; s < 4; s++) {
-                const float2 k = knext[s & 1];
-                knext[s & 1] = load_d8(4 * (b - b0) + s + 2);
-                drain([&](int g) {
-                    const float kg = g ? k.y : k.x;
+                const int buf = s & 1;
+                const float2 k = knext[buf];
+                knext[buf] = load_d8();
+                float v[2][NC];
+                wait_full(buf, s >> 1);
+                tc_ldn<NC>(v[0], lanes + 2 * buf * ROWS);
+                tc_ld_wait();
+                tc_ldn<NC>(v[1], lanes + (2 * buf + 1) * ROWS);
+                {
+                    const unsigned long long kk = pair(k.x, k.x);
 #pragma unroll
-                    for (int i = 0; i < NC / 2; i++) {
-                        const float2 t = make_float2(v[2 * i], v[2 * i + 1]);
-                        sum[i] = s == 0 && g == 0 ? mul_f32x2(t, make_float2(kg, kg)) : fma_f32x2(t, make_float2(kg, kg), sum[i]);
-                    }
-                });
+                    for (int i = 0; i < NC / 2; i++) fma_pair(sum[i], v[0] + 2 * i, kk);
+                }
+                tc_ld_wait();
+                release(buf);
+                {
+                    const unsigned long long kk = pair(k.y, k.y);
+#pragma unroll
+                    for (int i = 0; i < NC / 2; i++) fma_pair(sum[i], v[1] + 2 * i, kk);
+                }
             }
             // the block's d * sums - dmin * mins, and once more rounded into the row's sum
-            const float4* dc = reinterpret_cast<const float4*>(colscale);
+            tc_st_wait();  // of the block before
+            if constexpr (Q4) {
+                float w[4][CH];
+                wait_full(0, 2);
 #pragma unroll
-            for (int i = 0; i < NC / 4; i++) {
-                const float4 d = dc[i];
-                sum[2 * i] = mul_f32x2(make_float2(d.x, d.y), sum[2 * i]), sum[2 * i + 1] = mul_f32x2(make_float2(d.z, d.w), sum[2 * i + 1]);
-            }
-            if constexpr (Q4)
-                drain([&](int) {
+                for (int c = 0; c < NC / CH; c++) {
+                    tc_ld<CH>(w[0], lanes + c * CH);
+                    tc_ld<CH>(w[1], lanes + ROWS + c * CH);
+                    tc_ld<CH>(w[3], lanes_tot + c * CH);
+                    if (c == 0) wait_full(1, 2);
+                    tc_ld<CH>(w[2], lanes + 2 * ROWS + c * CH);
+                    tc_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < NC / 4; i++) {
-                        const float4 m = dc[NC / 4 + i];
-                        sum[2 * i] = fma_f32x2(make_float2(m.x, m.y), make_float2(v[4 * i], v[4 * i + 1]), sum[2 * i]);
-                        sum[2 * i + 1] = fma_f32x2(make_float2(m.z, m.w), make_float2(v[4 * i + 2], v[4 * i + 3]), sum[2 * i + 1]);
+                    for (int i = 0; i < CH / 2; i++) {
+                        mul_pair(sum[c * (CH / 2) + i], w[0] + 2 * i);
+                        fma_pair(sum[c * (CH / 2) + i], w[1] + 2 * i, w[2] + 2 * i);
                     }
-                });
+                    tc_ld<CH>(w[2], lanes + 3 * ROWS + c * CH);
+                    tc_ld_wait();
+                    if (c == NC / CH - 1) {
+                        release(0);
+                        release(1);
+                    }
 #pragma unroll
-            for (int i = 0; i < NC / 2; i++) tot[i] = fma_f32x2(make_float2(1.f, 1.f), sum[i], tot[i]);
-            __syncwarp();  // the columns' scales have been read
+                    for (int i = 0; i < CH / 2; i++) {
+                        fma_pair(sum[c * (CH / 2) + i], w[1] + 2 * i, w[2] + 2 * i);
+                        add_pair(w[3] + 2 * i, sum[c * (CH / 2) + i]);
+                    }
+                    tc_st<CH>(lanes_tot + c * CH, w[3]);
+                }
+                par ^= 1;
+            } else {
+                __syncwarp();
+                float v[NC];
+                tc_ldn<NC>(v, lanes_tot);
+                tc_ld_wait();
+#pragma unroll
+                for (int q = 0; q < NC / 4; q++) {
+                    const float4 d = reinterpret_cast<const float4*>(colscale)[q];
+                    mul_pair(sum[2 * q], &d.x), mul_pair(sum[2 * q + 1], &d.z);
+                    add_pair(v + 4 * q, sum[2 * q]), add_pair(v + 4 * q + 2, sum[2 * q + 1]);
+                }
+                __syncwarp();  // the columns' scales have been read
+                tc_stn<NC>(lanes_tot, v);
+            }
+            if (pieces > 1 && b + 1 == cut) {
+                tc_st_wait();
+                // a piece of the chain is done: its sums wait in memory (a thread's own 8 bytes beside its neighbours')
+                const bool last = piece == pieces;
+                float2* park = a.park + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * (TC_PARK_BYTES / 8) + td;
+                float v[NC];
+                tc_ldn<NC>(v, lanes_tot);
+                tc_ld_wait();
+#pragma unroll
+                for (int i = 0; i < NC / 2; i++) {
+                    float2* p = park + i * (32 * TC_D_WARPS);
+                    if (piece > 1) {
+                        const float2 t = *p;
+                        add_pair(v + 2 * i, pair(t.x, t.y));
+                    }
+                    if (!last) {
+                        asm volatile("" : "+f"(v[2 * i]), "+f"(v[2 * i + 1]));
+                        *p = make_float2(v[2 * i], v[2 * i + 1]);
+                    }
+                }
+                if (last) {
+                    tc_stn<NC>(lanes_tot, v);
+                    tc_st_wait();
+                } else {
+                    clear();
+                }
+                piece++;
+                cut = b0 + (b1 - b0) * piece / pieces;
+            }
+        }
+
+        int again = item;  // looked up once more: it would cost registers in the loop
+        asm volatile("" : "+r"(again));
+        const TcItem<ROWS> it(a, again);
+        const int m = it.n0 + tok;
+        float2 tot[NC / 2];
+        tc_st_wait();
+#pragma unroll
+        for (int c = 0; c < NC / 8; c++) {
+            float v[8];
+            tc_ld<8>(v, lanes_tot + 8 * c);
+            tc_ld_wait<8>(v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) tot[4 * c + i] = make_float2(v[2 * i], v[2 * i + 1]);
+        }
+
+        // ---- epilogue.  A gate/up tile whose rows all exist leaves straight from the registers (gate and up of 2 048 tokens 4 % faster
+        // than the other way).  All else is turned first, so that lanes run along the columns: RoPE pairs, rows with residuals.  A thread's
+        // own token and columns would touch 32 rows of the output with every access (a down projection of 2 048 tokens: 620 us).
+        if (S > 1) {
+            float2* mine = reinterpret_cast<float2*>(smem) + tok * G::SUM_STRIDE + cg * (NC / 2);
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) mine[i] = tot[i];
+            break;  // one item a cluster
+        }
+        if (a.epi.kind == CEPI_SILU && it.row0 + ROWS / 2 <= it.N && ((a.epi.ldo | (it.id_base + it.row0)) & 3) == 0 &&
+            (reinterpret_cast<uintptr_t>(a.epi.out) & 15) == 0) {
+            if (m < a.M) {
+                float4* o = reinterpret_cast<float4*>(a.epi.out + (size_t)m * a.epi.ldo + it.id_base + it.row0 + cg * (NC / 2));
+#pragma unroll
+                for (int i = 0; i < NC / 2; i += 4) {
+                    float h[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) h[q] = (tot[i + q].x / (1.f + __expf(-tot[i + q].x))) * tot[i + q].y;  // as ChunkEpiTok::apply
+                    o[i / 4] = make_float4(h[0], h[1], h[2], h[3]);
+                }
+            }
+            continue;
+        }
+        constexpr int OP = G::OUT_PAIRS;
+        static_assert((NC / 2) % 4 == 0, "");
+        const bool res = a.epi.kind == CEPI_STORE && a.epi.use_res == 2;
+        ChunkEpi epi = a.epi;
+        epi.use_res = 0;
+#pragma unroll
+        for (int c = 0; c < NC / 2; c += OP) {
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < OP; i++)
+                if (c + i < NC / 2) turn[lane * (OP + 1) + i] = tot[c + i];
+            __syncwarp();
+            const int pl = lane & (OP - 1), pair = cg * (NC / 2) + c + pl;
+            const int row = it.row0 + (a.zip ? pair : 2 * pair);
+            const bool on = c + pl < NC / 2 && row < it.N;
+            const int id = it.id_base + (a.zip ? row : row >> 1);
+            float2 r[OP];
+#pragma unroll
+            for (int q = 0; q < OP; q++) {
+                const int mt = it.n0 + quad * 32 + q * (32 / OP) + lane / OP;
+                r[q] = make_float2(0.f, 0.f);
+                if (res && on && mt < a.M) {
+                    const float* o = epi.out + (size_t)mt * epi.ldo + 2 * id;
+                    r[q].x = o[0];
+                    if (2 * id + 1 < epi.n_rows) r[q].y = o[1];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < OP; q++) {
+                const int t = q * (32 / OP) + lane / OP, mt = it.n0 + quad * 32 + t;
+                const float2 x = turn[t * (OP + 1) + pl];
+                if (on && mt < a.M) ChunkEpiTok{&epi, mt}.apply(id, x.x + r[q].x, x.y + r[q].y);
+            }
         }
     }
     tc_fence_before();
     asm volatile("bar.sync 1, %0;" ::"n"(32 * (TC_D_WARPS + TC_C_WARPS)) : "memory");
-
-    // ---- epilogue.  A gate/up tile whose rows all exist leaves straight from the registers, twelve values of a token in three
-    // stores (gate and up of 2 048 tokens 4 % faster than the other way).  All else goes as [token][pair of columns] through
-    // shared memory (of the cluster's CTAs), then lanes along the columns: RoPE pairs, rows with residuals.  A thread's own token
-    // and columns would touch 32 rows of the output with every access (a down projection of 2 048 tokens: 620 us).
-    const int id_base = second ? a.id2 : a.id1;
-    if (S == 1 && a.epi.kind == CEPI_SILU && row0 + TC_ROWS / 2 <= N && ((a.epi.ldo | (id_base + row0)) & 3) == 0 &&
-        (reinterpret_cast<uintptr_t>(a.epi.out) & 15) == 0) {
-        if (m < a.M) {
-            float4* o = reinterpret_cast<float4*>(a.epi.out + (size_t)m * a.epi.ldo + id_base + row0 + cg * (NC / 2));
+    if (td == 0 && dead_s && a.st) a.st->err = 2;
+    if (S == 1) return;
+    cluster_sync_all();
+    {
+        const TcItem<ROWS> it(a, blockIdx.x);
+        constexpr int PAIRS = ROWS / 2, BATCH = 4;
+        const int t0 = TC_LANES * part / S, items = min(TC_LANES / S, a.M - it.n0 - t0) * PAIRS;  // S is a power of two
+        const bool res = a.epi.kind == CEPI_STORE && a.epi.use_res == 2;
+        ChunkEpi epi = a.epi;
+        epi.use_res = 0;
+        for (int k0 = td; k0 < items; k0 += BATCH * 32 * TC_D_WARPS) {
+            // the parts' sums and the residuals of four items in flight together
+            float2 v[BATCH], r[BATCH];
+            int m[BATCH], id[BATCH];
 #pragma unroll
-            for (int i = 0; i < NC / 2; i += 4) {
-                float h[4];
+            for (int q = 0; q < BATCH; q++) {
+                const int k = k0 + q * 32 * TC_D_WARPS, t = t0 + k / PAIRS, pair = k % PAIRS;
+                const int row = it.row0 + (a.zip ? pair : 2 * pair);
+                const bool on = k < items && row < it.N;
+                m[q] = it.n0 + t, id[q] = on ? it.id_base + (a.zip ? row : row >> 1) : -1;
+                v[q] = r[q] = make_float2(0.f, 0.f);
+                if (!on) continue;
+                if (res) {
+                    const float* o = epi.out + (size_t)m[q] * epi.ldo + 2 * id[q];
+                    r[q].x = o[0];
+                    if (2 * id[q] + 1 < epi.n_rows) r[q].y = o[1];
+                }
+                const unsigned at = smem_u32(smem) + (t * G::SUM_STRIDE + pair) * 8;
 #pragma unroll
-                for (int q = 0; q < 4; q++) h[q] = (tot[i + q].x / (1.f + __expf(-tot[i + q].x))) * tot[i + q].y;  // as ChunkEpiTok::apply
-                o[i / 4] = make_float4(h[0], h[1], h[2], h[3]);
+                for (int p = 0; p < 8; p++) {
+                    if (p >= S) break;
+                    float2 x;
+                    unsigned remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(p));
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"(remote) : "memory");
+                    v[q].x += x.x, v[q].y += x.y;
+                }
             }
+#pragma unroll
+            for (int q = 0; q < BATCH; q++)
+                if (id[q] >= 0) ChunkEpiTok{&epi, m[q]}.apply(id[q], v[q].x + r[q].x, v[q].y + r[q].y);
         }
-        if (tid == 32 * (TC_C_WARPS + TC_A_WARPS) && dead_s && a.st) a.st->err = 2;
-        return;
     }
-    constexpr int PAIRS = TC_ROWS / 2, BATCH = 4;
-    float2* mine = reinterpret_cast<float2*>(smem) + tok * TC_SUM_STRIDE + cg * (NC / 2);
-#pragma unroll
-    for (int i = 0; i < NC / 2; i++) mine[i] = tot[i];
-    if (S > 1) cluster_sync_all();
-    else asm volatile("bar.sync 2, %0;" ::"n"(32 * TC_D_WARPS) : "memory");
-    const int td = tid - 32 * (TC_C_WARPS + TC_A_WARPS);
-    const int t0 = TC_LANES * part / S, items = min(TC_LANES / S, a.M - n0 - t0) * PAIRS;  // S is a power of two
-    const bool res = a.epi.kind == CEPI_STORE && a.epi.use_res == 2;
-    ChunkEpi epi = a.epi;
-    epi.use_res = 0;
-    for (int k0 = td; k0 < items; k0 += BATCH * 32 * TC_D_WARPS) {
-        // the parts' sums and the residuals of four items in flight together
-        float2 v[BATCH], r[BATCH];
-        int m[BATCH], id[BATCH];
-#pragma unroll
-        for (int q = 0; q < BATCH; q++) {
-            const int k = k0 + q * 32 * TC_D_WARPS, t = t0 + k / PAIRS, pair = k % PAIRS;
-            const int row = row0 + (a.zip ? pair : 2 * pair);
-            const bool on = k < items && row < N;
-            m[q] = n0 + t, id[q] = on ? id_base + (a.zip ? row : row >> 1) : -1;
-            v[q] = r[q] = make_float2(0.f, 0.f);
-            if (!on) continue;
-            if (res) {
-                const float* o = epi.out + (size_t)m[q] * epi.ldo + 2 * id[q];
-                r[q].x = o[0];
-                if (2 * id[q] + 1 < epi.n_rows) r[q].y = o[1];
-            }
-            const unsigned at = smem_u32(smem) + (t * TC_SUM_STRIDE + pair) * 8;
-#pragma unroll
-            for (int p = 0; p < 8; p++) {
-                if (p >= S) break;
-                float2 x;
-                unsigned remote;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(p));
-                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"(remote) : "memory");
-                v[q].x += x.x, v[q].y += x.y;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < BATCH; q++)
-            if (id[q] >= 0) ChunkEpiTok{&epi, m[q]}.apply(id[q], v[q].x + r[q].x, v[q].y + r[q].y);
-    }
-    if (tid == 32 * (TC_C_WARPS + TC_A_WARPS) && dead_s && a.st) a.st->err = 2;
-    if (S > 1) cluster_sync_all();  // nobody leaves while others read its sums
+    cluster_sync_all();  // nobody leaves while others read its sums
 }
 
 // ------------------------------------------------------------------ rows on the fp32 activation route
@@ -902,17 +1192,14 @@ inline int cluster_ctas(F* kernel, int threads, int S, int sms) {
 
 inline bool tc_type(int type) { return type == TFR_Q4_K || type == TFR_Q6_K; }
 
-template <class RAW>
-inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_tiles, int S) {
-    constexpr int stage = TC_LANES * 128 + RAW::PLANES * TC_ROWS * 128;
-    a.nst = std::min(TC_MAX_STAGES, (int)((TC_SMEM_MAX - 1024 - TC_COLSCALE_BYTES) / stage));
-    static_assert((TC_SMEM_MAX - 1024 - TC_COLSCALE_BYTES) / stage >= 5, "the ring holds a block's stages");
-    a.ahead = S == 1 && row_tiles > sms ? sms : 0;
-    static_assert(TC_LANES * TC_SUM_STRIDE * 8 <= 2 * stage, "the epilogue's sums lie over the first stages");
+template <class RAW, int ROWS>
+inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int S) {
+    constexpr bool Q4 = RAW::PLANES == 1;
+    using G = TcGeom<Q4, ROWS>;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(row_tiles, S, (a.M + TC_LANES - 1) / TC_LANES);
+    cfg.gridDim = dim3(S > 1 ? a.items : std::min(a.items, sms), S);
     cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = (size_t)a.nst * stage + TC_COLSCALE_BYTES + 1024;
+    cfg.dynamicSmemBytes = G::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -923,31 +1210,42 @@ inline cudaError_t launch_tc(cudaStream_t stream, int sms, TcArgs& a, int row_ti
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = S > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_gemm_tc<RAW>, (const TcArgs)a);
+    return cudaLaunchKernelEx(&cfg, k_gemm_tc<RAW, ROWS>, (const TcArgs)a);
 }
 
 // out = epilogue(W x) for the M tokens of an operand image; jb: the second matrix of a gate/up pair or one that follows.
-inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned char* image, int M, const RowJob& ja,
+// park: tc_park_bytes.
+inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned char* image, float2* park, int M, const RowJob& ja,
                                   const RowJob& jb, const ChunkEpi& epi, TokenState* st) {
     TcArgs a{};
     a.image = image, a.M = M, a.Mp = tc_pad_tokens(M);
     a.A1 = ja.m, a.A2 = jb.m, a.id1 = ja.id_base, a.id2 = jb.id_base;
     a.zip = epi.kind == CEPI_SILU;
-    a.epi = epi, a.st = st;
-    const int rows = a.zip ? TC_ROWS / 2 : TC_ROWS;
-    a.tiles1 = (ja.m.N + rows - 1) / rows;
-    const int tiles = a.tiles1 + (!a.zip && jb.m.data ? (jb.m.N + rows - 1) / rows : 0), groups = (M + TC_LANES - 1) / TC_LANES;
-    // the number of k parts with the shortest longest chain: waves of CTAs x (blocks x what a block takes + the ends), in units of
-    // a quarter of a block (0.8 us)
-    int S = 1;
+    a.epi = epi, a.st = st, a.park = park;
+    a.groups = (M + TC_LANES - 1) / TC_LANES;
+    // Tile and number of k parts with the shortest longest chain: waves of CTAs x (blocks x what a block takes + the ends), in units of
+    // 3.2 us.  Measured: 96 rows 2.4 us a block, 64 rows 1.95; ends 3 us, cut k ranges 3 more.  Down rows of 11 008 inputs: 77 tokens
+    // 29.7 us (64 rows, four parts; 96 rows 32.8, one part 99.8), 300 tokens 58.6 (96 rows, two parts; one 103, four 66.6), 2 048
+    // tokens 284 (two parts; one 319).
+    int S = 1, rows = 96;
     double best = 1e30;
-    for (int s = 1; s <= 8 && s <= ja.m.nb; s *= 2) {
-        if (s < 8 && (ja.m.nb + s - 1) / s > TC_CHAIN) continue;
-        const int ctas = tiles * groups * s, at_once = cluster_ctas(k_gemm_tc<RawQ4>, TC_THREADS, s, sms);
-        const double t = (double)((ctas + at_once - 1) / at_once) * (4.5 * ((ja.m.nb + s - 1) / s) + 6 + (s > 1 ? 3 : 0));
-        if (t < best) best = t, S = s;
-    }
-    return ja.m.type == TFR_Q4_K ? launch_tc<RawQ4>(stream, sms, a, tiles, S) : launch_tc<RawQ6>(stream, sms, a, tiles, S);
+    auto tiles = [&](int r, int& first) {
+        const int per = a.zip ? r / 2 : r;
+        first = (ja.m.N + per - 1) / per;
+        return first + (!a.zip && jb.m.data ? (jb.m.N + per - 1) / per : 0);
+    };
+    for (int r : {96, 64})
+        for (int s = 1; s <= 8 && s <= ja.m.nb; s *= 2) {
+            int first;
+            const int ctas = tiles(r, first) * a.groups * s, at_once = cluster_ctas(k_gemm_tc<RawQ4, 96>, TC_THREADS, s, sms);
+            const int blocks = (ja.m.nb + s - 1) / s;
+            if (s > 1 && blocks > TC_CHAIN && ctas > 3 * sms) continue;  // parked sums have no room
+            const double t = (double)((ctas + at_once - 1) / at_once) * ((r == 96 ? 0.75 : 0.62) * blocks + 1 + (s > 1 ? 1 : 0));
+            if (t < best) best = t, S = s, rows = r;
+        }
+    a.items = tiles(rows, a.tiles1) * a.groups;
+    if (rows == 96) return ja.m.type == TFR_Q4_K ? launch_tc<RawQ4, 96>(stream, sms, a, S) : launch_tc<RawQ6, 96>(stream, sms, a, S);
+    return ja.m.type == TFR_Q4_K ? launch_tc<RawQ4, 64>(stream, sms, a, S) : launch_tc<RawQ6, 64>(stream, sms, a, S);
 }
 
 }  // namespace tfr
