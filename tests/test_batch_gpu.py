@@ -196,6 +196,23 @@ def test_larger_batches_are_as_precise_as_dp4a(E, wtype, K, N, M):
         w.free()
 
 
+@pytest.mark.parametrize("wtype,K,N,M", [(S.Q4_K, 512, 20000, 300), (S.Q4_K, 7680, 3000, 1000), (S.Q6_K, 7680, 3000, 1000), (S.Q6_K, 27648, 5120, 500),
+                                         (S.Q4_K, 27648, 97, 66), (S.Q6_K, 2048, 2048, 65)])
+def test_larger_batches_beyond_one_tile_a_cta(E, wtype, K, N, M):
+    """k_gemm_tc where a CTA works on several tiles, where a row's chain of additions is cut and its pieces wait in memory (in one
+    part, and in two), in tiles of 64 rows: against dp4a on the same int8 activations."""
+    from taraference_b200 import synth_gpu as G
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K + N)
+    w = E.GpuMat(wtype, K, N, G.quantized_matrix(wtype, K, N, gen, 0.02))
+    x, res = torch.randn((M, K), generator=gen, device="cuda"), torch.randn((M, N), generator=gen, device="cuda")
+    outs = [res.clone(), res.clone()]
+    for route, out in zip((DP4A, TC), outs):
+        E.op_project_rows(w, x, out, M, route=route, use_res=2)
+    assert _rel(outs[1].cpu().numpy(), outs[0].cpu().numpy()) < SAME_INT8
+    w.free()
+
+
 @pytest.mark.parametrize("chunk,n", [(2, 7), (16, 16), (16, 45), (64, 19), (2048, 41)])
 def test_hybrid_prompt_in_batches_equals_step_by_step(E, chunk, n):
     """Batches of a hybrid model: conv history across batches (shorter ones than the kernel, too), scan tiles of 16 tokens,
