@@ -230,7 +230,7 @@ k_gemm_q8(const unsigned char* act_g, const float* xn, RowJob ja, RowJob jb, F32
     unsigned char* act_s = smem;
     float* pbuf = reinterpret_cast<float*>(act_s + (size_t)Mt * g.act_b16);
     unsigned long long* full = reinterpret_cast<unsigned long long*>(pbuf + (size_t)Mt * g.pbuf_floats);
-    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(full + wa * nsw) + 127) & ~(uintptr_t)127);
+    unsigned char* ring = smem + (((unsigned)(Mt * (g.act_b16 + 4 * (size_t)g.pbuf_floats)) + 8u * (unsigned)(wa * nsw) + 127) & ~127u);  // an offset: stays a shared pointer
 
     const int rows_a0 = ja.row0(cta), rows_a = max(0, ja.rows(cta)), blocks_a = group_rows(rows_a) * nb;
     const int rows_b0 = jb.m.data ? jb.row0(cta) : 0, rows_b = jb.m.data ? max(0, jb.rows(cta)) : 0, blocks_b = group_rows(rows_b) * nb;

@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
     const int S = gridDim.y, part = blockIdx.y;  // k parts
     const int nb = a.A1.nb, K = a.A1.K;
     const int b0 = nb * part / S, b1 = nb * (part + 1) / S;
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* smem = tc_smem_raw + (-smem_u32(tc_smem_raw) & 1023u);
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
             mbar_init(bars + i, (ROWS + 31) / 32 + 1);  // the warps that unpack a half and the tokens (with the bytes)

@@ -382,8 +382,9 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     float* xs = act.xf;
     const int nb = K >> 8;
     constexpr int TB = BLK::TILE_BYTES;
-    unsigned char* ring = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(full + slots) + 127) & ~(uintptr_t)127);
+    // aligned as an offset, not as an address: the compiler then knows that tiles lie in shared memory and reads them as such
+    const unsigned ring_at = ((unsigned)act_bytes + ((unsigned)pbuf_floats + 272) * 4 + 8 * (unsigned)slots + 127) & ~127u;
+    unsigned char* ring = smem + ring_at;
 
     // flat block ranges of this CTA in A and B, and the tiles that cover them
     const int rows_a0 = ja.row0(cta), rows_a = max(0, ja.rows(cta)), blocks_a = group_rows(rows_a) * nb;
