@@ -35,7 +35,8 @@ struct GdnArgs {
 // The conv history is a ring indexed by position instead of the reference's shifted window
 // (deltanet.cu:552-558): nothing moves, and the two V heads that share a K head can both read
 // the Q/K history without racing against a shift.
-__device__ __forceinline__ float gdn_conv_channel(const GdnArgs& a, int c, int channels, int slot, bool write) {
+// The sum over the history, and with the current input the channel's value.
+__device__ __forceinline__ float gdn_conv_history(const GdnArgs& a, int c, int channels, int slot) {
     const int km1 = a.kernel - 1;
     float acc = 0.f;
 #pragma unroll
@@ -46,29 +47,39 @@ __device__ __forceinline__ float gdn_conv_channel(const GdnArgs& a, int c, int c
             acc += a.conv_w[(size_t)c * a.kernel + k] * a.conv_ring[(size_t)s * channels + c];
         }
     }
-    const float xt = a.proj[c];
-    acc += a.conv_w[(size_t)c * a.kernel + km1] * xt;
+    return acc;
+}
+__device__ __forceinline__ float gdn_conv_value(const GdnArgs& a, int c, int channels, int slot, bool write, float acc, float w, float xt) {
+    acc += w * xt;
     if (write) a.conv_ring[(size_t)slot * channels + c] = xt;
     return acc / (1.f + expf(-acc));
 }
 
+// Inside a token the kernel before this one is the layer's projection, which writes neither the state nor the conv history
+// and starts this kernel only when what ran before it is complete: the state (64 KB a head) and all that does not come from the
+// projection is asked for before the dependency wait and arrives under it.  A stand-alone call may follow another one on the same
+// state and waits first.
 __global__ void __launch_bounds__(GDN_THREADS, 1) k_gdn_step(GdnArgs a, const TokenState* st) {
-    griddep_wait();  // the projections come from the previous kernel
-    griddep_launch_dependents();
-    if (st && st->done) return;
+    int slot = a.slot, done = 0;
     if (st) {
+        done = st->done;
         a.conv_ring = st->kv_conv + a.conv_off;
         a.state = st->kv_ssm + a.state_off;
+        slot = (st->pos + st->ring_off) % a.kernel;
+    }
+    if (!st || done) {
+        griddep_wait();
+        griddep_launch_dependents();
+        if (done) return;
     }
     constexpr int D = GDN_D, R = D / GDN_PARTS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.x, hk = h % a.n_k;
     const int key_dim = a.n_k * D, val_dim = a.n_v * D, channels = 2 * key_dim + val_dim;
-    const int slot = st ? (st->pos + st->ring_off) % a.kernel : a.slot;
     const int j = tid & (D - 1), part = tid >> 7;
     float* S = a.state + (size_t)h * D * D;
 
-    __shared__ float sq[D], sk[D], sv[D];
+    __shared__ float sq[D], sk[D], sv[D], sz[D];
     __shared__ float red[GDN_PARTS][D];
     __shared__ float wred[16];
     __shared__ float sg, sb;
@@ -78,19 +89,28 @@ __global__ void __launch_bounds__(GDN_THREADS, 1) k_gdn_step(GdnArgs a, const To
 #pragma unroll
     for (int r = 0; r < R; r++) s[r] = __ldcs(S + (size_t)(part * R + r) * D + j);
 
-    float cv = 0.f;
+    // part 0: Q channel j of K head hk, part 1: K channel, part 2: V channel j of head h; part 3: the z gate of output j
+    const int c = part == 0 ? hk * D + j : part == 1 ? key_dim + hk * D + j : part == 2 ? 2 * key_dim + h * D + j : channels + h * D + j;
+    float cv = 0.f, cw = 0.f;
     if (part < 3) {
-        // part 0: Q channel j of K head hk, part 1: K channel, part 2: V channel j of head h
-        const int c = part == 0 ? hk * D + j : part == 1 ? key_dim + hk * D + j : 2 * key_dim + h * D + j;
-        cv = gdn_conv_channel(a, c, channels, slot, part == 2 || h < a.n_k);
+        cv = gdn_conv_history(a, c, channels, slot);
+        cw = a.conv_w[(size_t)c * a.kernel + a.kernel - 1];
     }
+    const float nw = a.norm_w[j], dt = tid == 0 ? a.ssm_dt[h] : 0.f, decay = tid == 0 ? a.ssm_a[h] : 0.f;
+    if (st) {
+        griddep_wait();  // the projections come from the previous kernel
+        griddep_launch_dependents();
+    }
+    const float xt = a.proj[c];
     if (tid == 0) {
         const float br = a.proj[channels + val_dim + h];
         sb = 1.f / (1.f + expf(-br));
-        const float z = a.proj[channels + val_dim + a.n_v + h] + a.ssm_dt[h];
+        const float z = a.proj[channels + val_dim + a.n_v + h] + dt;
         const float sp = (z > 20.f) ? z : log1pf(expf(z));
-        sg = expf(sp * a.ssm_a[h]);
+        sg = expf(sp * decay);
     }
+    if (part < 3) cv = gdn_conv_value(a, c, channels, slot, part == 2 || h < a.n_k, cv, cw, xt);
+    else sz[j] = xt;
     // L2 norms of Q and K (sum of squares, deltanet.cu:598-620)
     const float sqr = warp_sum(part < 2 ? cv * cv : 0.f);
     if (lane == 0) wred[warp] = sqr;
@@ -136,9 +156,9 @@ __global__ void __launch_bounds__(GDN_THREADS, 1) k_gdn_step(GdnArgs a, const To
     __syncthreads();
     if (part == 0) {
         const float scale = rsqrtf((wred[8] + wred[9] + wred[10] + wred[11]) * (1.f / (float)D) + a.eps);
-        const float gate = a.proj[channels + h * D + j];
+        const float gate = sz[j];
         const float silu = gate / (1.f + expf(-gate));
-        a.out[h * D + j] = oj * scale * a.norm_w[j] * silu;
+        a.out[h * D + j] = oj * scale * nw * silu;
     }
 }
 
@@ -347,18 +367,21 @@ struct QkNormArgs {
 };
 
 __global__ void __launch_bounds__(256) k_qk_norm_rope_store(QkNormArgs a, const TokenState* st) {
-    griddep_wait();
-    griddep_launch_dependents();
-    if (st && st->done) return;
+    // the state's words together and before the wait, as in k_gdn_step: the kernel before this one does not write them
+    int done = 0, pos0 = a.pos;
     if (st) {
+        done = st->done, pos0 = st->pos;
         a.kc = st->kv_k + a.kv_off;
         a.vc = st->kv_v + a.kv_off;
     }
+    griddep_wait();
+    griddep_launch_dependents();
+    if (done) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int head = blockIdx.x, hd = a.hd;
     const bool isq = head < a.n_head;
     const int hk = head - a.n_head;
-    const int m = blockIdx.y, pos = (st ? st->pos : a.pos) + m;
+    const int m = blockIdx.y, pos = pos0 + m;
     const int qn2 = 2 * a.n_head * hd, kvdim = a.n_kv * hd;
     const float* raw = a.raw + (size_t)m * (qn2 + 2 * kvdim);
     const float* src = isq ? raw + (size_t)head * 2 * hd : raw + qn2 + (size_t)hk * hd;
