@@ -1776,13 +1776,15 @@ static int chunk_buffers(tfr_engine* e, int M) {
 }
 
 // The kernel of a batch's projections.  Fewer than five tokens leave the tensor cores idle and keep the dp4a kernel, as Q8_0
-// matrices do (TFR_GEMM_DP4A=1 in the environment keeps everything there, a test aid).  mma.sync where it is the faster one:
-// up to 80 tokens on Q4_K (11 008 gate and up rows of 2 048, a launch by itself: 20 us for 16 tokens, 62 for 80; tcgen05 62 and
-// 63) and up to 32 on Q6_K, whose MMAs are half as deep (2 048 rows of 11 008: 18 us for 16 tokens and 25 for 32; tcgen05 40).
+// matrices do (TFR_GEMM_DP4A=1 in the environment keeps everything there, a test aid).  mma.sync where it is the faster one.
+// Launches by themselves, us, mma.sync against tcgen05: Q4_K, 11 008 gate and up rows of 2 048, 48 tokens 31 : 47, 64 tokens 50 : 48,
+// 65 tokens 60 : 47; 27 648 rows of 5 120, 48 tokens 170 : 203, 64 211 : 204, 65 367 : 204; few rows (2 048 of 2 048) 64 tokens
+// 10.5 : 14.8, 80 tokens 14.0 : 14.9.  Q6_K, whose MMAs are half as deep, 2 048 rows of 11 008: 32 tokens 26 : 35.
 enum { GEMM_DP4A, GEMM_MMA, GEMM_TC };
-static int gemm_route(int type, int nb, int M) {
+static int gemm_route(const Mat& m, int M) {
+    const int type = m.type, nb = m.nb;
     if (M < GEMM_TC_MIN_TOKENS || !tc_type(type) || getenv("TFR_GEMM_DP4A")) return GEMM_DP4A;
-    return M <= (type == TFR_Q4_K ? 80 : 32) && mma_tiles(nb, M) > 0 ? GEMM_MMA : GEMM_TC;
+    return M <= (type != TFR_Q4_K ? 32 : m.N <= 4096 ? 80 : 64) && mma_tiles(nb, M) > 0 ? GEMM_MMA : GEMM_TC;
 }
 
 static cudaError_t launch_gemm_typed(cudaStream_t s, int grid, int type, const unsigned char* act, size_t stride, const float* xn, int M,
@@ -1844,7 +1846,7 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
     };
     // RMSNorm + Q8 + W x + epilogue
     auto project = [&](const float* x, int width, const float* normw, const RowJob& ja, const RowJob& jb, const ChunkEpi& ep) -> cudaError_t {
-        const int route = gemm_route(ja.m.type, ja.m.nb, M);
+        const int route = gemm_route(ja.m, M);
         const cudaError_t r = prep(route, ja.m.type, x, width, normw, nullptr);
         return r != cudaSuccess ? r : gemm(route, ja, jb, ep);
     };
@@ -1887,7 +1889,7 @@ static int forward_chunk(tfr_engine* e, const tfr_kv* kv, const int* tok, int M,
         } else {
         // 1. RMSNorm + Q8, Q/K/V (+bias); dense layers: RoPE + f16 KV rows
         const bool gated = L.kind == LAYER_FULL_GATED;
-        const int route = gemm_route(TFR_Q4_K, L.wq->m.nb, M);
+        const int route = gemm_route(L.wq->m, M);
         const int q_rows = gated ? 2 * nq : nq;
         if (prep(route, TFR_Q4_K, e->cx, K, L.attn_norm, e->cxn) != cudaSuccess) return -1;
         {
@@ -2556,7 +2558,7 @@ extern "C" int tfr_op_project_rows(const tfr_mat* a, const tfr_mat* b, const flo
                                    int use_res, float* out, void* stream) {
     if (!a || !x || !out || M <= 0 || M > CHUNK_MAX_TOKENS || (use_res != 0 && use_res != 2)) return TFR_E_INVALID;
     if (b && (b->m.K != a->m.K || b->m.N != a->m.N || b->m.type != a->m.type || use_res)) return TFR_E_INVALID;
-    if (route < 0) route = gemm_route(a->m.type, a->m.nb, M);
+    if (route < 0) route = gemm_route(a->m, M);
     if (route > GEMM_TC || (route != GEMM_DP4A && !tc_type(a->m.type))) return TFR_E_UNSUPPORTED;
     if (route == GEMM_MMA && (M > (a->m.type == TFR_Q4_K ? MMA_MAX_TOKENS : 32) || mma_tiles(a->m.nb, M) == 0)) return TFR_E_UNSUPPORTED;
     configure_kernels_once();
