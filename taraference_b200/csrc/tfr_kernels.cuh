@@ -491,20 +491,20 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     const int n4 = K >> 2;
     float scale = 1.f;
     if (!embed && !with_xf) {
-        // plain vector: quantise pass by pass straight from the registers that fetched it
-        if (!done) {
-            for (int base = 0; base < n4; base += STAGE_REGS * T) {
-                float4 sx[STAGE_REGS];
+        // plain vector: quantise pass by pass straight from the registers that fetched it.  The vector is asked for beside `done`, not
+        // behind it: that were a second trip to L2 in a row
+        for (int base = 0; base < n4; base += STAGE_REGS * T) {
+            float4 sx[STAGE_REGS];
 #pragma unroll
-                for (int k = 0; k < STAGE_REGS; k++) {
-                    const int i4 = base + k * T + tid;
-                    sx[k] = i4 < n4 ? reinterpret_cast<const float4*>(pa.vec)[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+            for (int k = 0; k < STAGE_REGS; k++) {
+                const int i4 = base + k * T + tid;
+                sx[k] = i4 < n4 ? reinterpret_cast<const float4*>(pa.vec)[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (done) break;
 #pragma unroll
-                for (int k = 0; k < STAGE_REGS; k++) {
-                    const int i4 = base + k * T + tid;
-                    if (base + k * T < n4) act_quantize4(act, sx[k], i4, i4 < n4, nb);
-                }
+            for (int k = 0; k < STAGE_REGS; k++) {
+                const int i4 = base + k * T + tid;
+                if (base + k * T < n4) act_quantize4(act, sx[k], i4, i4 < n4, nb);
             }
         }
         prof_mark(2, pa.prof_id);
