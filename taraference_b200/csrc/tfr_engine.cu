@@ -1807,7 +1807,7 @@ static cudaError_t batch_prep(cudaStream_t s, int route, int type, const float* 
                               const BatchBufs& b, float* xn) {
     if (route == GEMM_TC) {
         PrepTcArgs a{x, width, width, M, normw, eps, b.image, xn};
-        return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(TC_PREP_THREADS), tc_prep_smem(width), s, a);
+        return launch_pdl(k_prep_tc, dim3(tc_pad_tokens(M)), dim3(tc_prep_threads(width)), tc_prep_smem(width), s, a);
     }
     if (route == GEMM_MMA) {
         PrepMmaArgs a{x, width, width, M, normw, eps, b.image, xn, type == TFR_Q6_K};
