@@ -57,8 +57,8 @@ __device__ __forceinline__ float gdn_conv_value(const GdnArgs& a, int c, int cha
 
 // Inside a token the kernel before this one is the layer's projection, which writes neither the state nor the conv history
 // and starts this kernel only when what ran before it is complete: the state (64 KB a head) and all that does not come from the
-// projection is asked for before the dependency wait and arrives under it.  A stand-alone call may follow another one on the same
-// state and waits first.
+// projection is asked for before the dependency wait and arrives under it (64 tokens in and 32 out on the hybrid 4B shape, with the
+// same in k_qk_norm_rope_store: 46.33 -> 44.57 ms).  A stand-alone call may follow another one on the same state and waits first.
 __global__ void __launch_bounds__(GDN_THREADS, 1) k_gdn_step(GdnArgs a, const TokenState* st) {
     int slot = a.slot, done = 0;
     if (st) {
