@@ -1367,6 +1367,8 @@ extern "C" int tfr_zero_recurrent(tfr_engine* e, tfr_kv* kv) {
 
 // ------------------------------------------------------------------ one token
 
+// A decode step's attention and recurrent kernels read the state, and what it points to, ahead of their dependency wait: they follow
+// a WaitsFirst.  Without a state (the operators) only attention reads ahead, rows that its caller has written before.
 static cudaError_t launch_attention(cudaStream_t s, const AttnArgs& a, int hd, const TokenState* st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(a.S, a.n_kv);
@@ -1391,9 +1393,19 @@ static cudaError_t launch_attention(cudaStream_t s, const AttnArgs& a, int hd, c
     if (hd == 128) return cudaLaunchKernelEx(&cfg, k_attn_decode<128, false>, a, st);
     return cudaLaunchKernelEx(&cfg, k_attn_decode<256, false>, a, st);
 }
+static cudaError_t launch_attention_behind(WaitsFirst before, cudaStream_t s, const AttnArgs& a, int hd, const TokenState* st) {
+    return before != cudaSuccess ? before.err : launch_attention(s, a, hd, st);
+}
+static cudaError_t launch_gdn_step_behind(WaitsFirst before, cudaStream_t s, const GdnArgs& g, const TokenState* st) {
+    return before != cudaSuccess ? before.err : launch_pdl(k_gdn_step, dim3(g.n_v), dim3(GDN_THREADS), 0, s, g, st);
+}
+// This one waits before it starts the next, too.
+static WaitsFirst launch_qk_norm_behind(WaitsFirst before, cudaStream_t s, const QkNormArgs& a, const TokenState* st) {
+    return before != cudaSuccess ? before : WaitsFirst{launch_pdl(k_qk_norm_rope_store, dim3(a.n_head + a.n_kv), dim3(256), 0, s, a, st)};
+}
 
 template <class Epi>
-static cudaError_t launch_typed(cudaStream_t s, int grid, int type, const PrepArgs& pa, const RowJob& ja, const RowJob& jb,
+static WaitsFirst launch_typed(cudaStream_t s, int grid, int type, const PrepArgs& pa, const RowJob& ja, const RowJob& jb,
                                 const F32Seg& fseg, const Epi& epi, int K, TokenState* st) {
     if (type == TFR_Q4_K) return launch_gemv<BlockQ4, Epi>(s, grid, pa, ja, jb, fseg, epi, K, st);
     if (type == TFR_Q8_0) return launch_gemv<BlockQ8, Epi>(s, grid, pa, ja, jb, fseg, epi, K, st);
@@ -1500,11 +1512,11 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
         const tfr_mat* wout = L.wo;
         if (L.kind == LAYER_LINEAR) {
             // 1. norm + quant + [qkv | z | beta | alpha] projections (layer.rs:736-798)
+            WaitsFirst proj{};
             if (L.gdn_proj) {
                 EpiStore ep{e->proj, nullptr, 0, L.gdn_proj->m.N};
-                if (launch_typed(s, cap, L.gdn_proj->m.type, pn, make_job(L.gdn_proj->m, cap), RowJob{}, F32Seg{}, ep, K, e->st) !=
-                    cudaSuccess)
-                    return -1;
+                proj = launch_typed(s, cap, L.gdn_proj->m.type, pn, make_job(L.gdn_proj->m, cap), RowJob{}, F32Seg{}, ep, K, e->st);
+                if (proj != cudaSuccess) return -1;
                 n++;
             } else {
                 // mixed weight types (e.g. a Q5_K attn_qkv beside a Q4_K attn_gate): one launch per matrix, as the
@@ -1519,8 +1531,8 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
                     }
                     pk.prof_id = n;
                     EpiStore ep{e->proj + off, nullptr, 0, w->m.N};
-                    if (launch_typed(s, cap, w->m.type, pk, make_job(w->m, cap), RowJob{}, F32Seg{}, ep, K, e->st) != cudaSuccess)
-                        return -1;
+                    proj = launch_typed(s, cap, w->m.type, pk, make_job(w->m, cap), RowJob{}, F32Seg{}, ep, K, e->st);
+                    if (proj != cudaSuccess) return -1;
                     off += w->m.N;
                     n++;
                 }
@@ -1539,7 +1551,7 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             g.n_v = c.ssm_time_step_rank;
             g.kernel = c.ssm_conv_kernel;
             g.eps = c.rms_eps;
-            if (launch_pdl(k_gdn_step, dim3(g.n_v), dim3(GDN_THREADS), 0, s, g, (const TokenState*)e->st) != cudaSuccess) return -1;
+            if (launch_gdn_step_behind(proj, s, g, e->st) != cudaSuccess) return -1;
             n++;
             mix_width = gdn_val_dim(c);
             wout = L.ssm_out;
@@ -1551,7 +1563,8 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             fseg.sh = make_share(nkv / 2, cap);
             fseg.id_base = (2 * nq + nkv) / 2;
             EpiStore ep{e->proj, L.bias_qkv, 0, 2 * nq + 2 * nkv};
-            if (launch_gemv<BlockQ4, EpiStore>(s, cap, pn, jq, jk, fseg, ep, K, e->st) != cudaSuccess) return -1;
+            const WaitsFirst proj = launch_gemv<BlockQ4, EpiStore>(s, cap, pn, jq, jk, fseg, ep, K, e->st);
+            if (proj != cudaSuccess) return -1;
             n++;
             // 2. per-head Q/K RMSNorm + partial RoPE, Q|gate split, f16 KV store (layer.rs:386-560)
             QkNormArgs qa{};
@@ -1567,13 +1580,13 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             qa.n_rot = (c.rope_dim > 0 && c.rope_dim < hd) ? c.rope_dim : hd;
             qa.theta = c.rope_theta;
             qa.eps = c.rms_eps;
-            if (launch_pdl(k_qk_norm_rope_store, dim3(P.n_head + P.n_kv), dim3(256), 0, s, qa, (const TokenState*)e->st) != cudaSuccess)
-                return -1;
+            const WaitsFirst normed = launch_qk_norm_behind(proj, s, qa, e->st);
+            if (normed != cudaSuccess) return -1;
             n++;
             // 3. attention with the sigmoid output gate (layer.rs:646-659)
             a.gate = e->qgate;
             a.prof_id = n;
-            if (launch_attention(s, a, hd, e->st) != cudaSuccess) return -1;
+            if (launch_attention_behind(normed, s, a, hd, e->st) != cudaSuccess) return -1;
             n++;
         } else {
             // 1. norm + quant + QKV + rope + KV store
@@ -1593,13 +1606,13 @@ static int record_token(tfr_engine* e, const tfr_kv* kv, bool with_head) {
             epi.hd = hd;
             epi.kvdim = nkv;
             epi.theta = c.rope_theta;
-            const cudaError_t qkv = li == 0 ? launch_gemv<BlockQ4, EpiQkvFirst>(s, cap, pn, jq, jk, fseg, EpiQkvFirst{epi}, K, e->st)
-                                            : launch_gemv<BlockQ4, EpiQkv>(s, cap, pn, jq, jk, fseg, epi, K, e->st);
+            const WaitsFirst qkv = li == 0 ? launch_gemv<BlockQ4, EpiQkvFirst>(s, cap, pn, jq, jk, fseg, EpiQkvFirst{epi}, K, e->st)
+                                           : launch_gemv<BlockQ4, EpiQkv>(s, cap, pn, jq, jk, fseg, epi, K, e->st);
             if (qkv != cudaSuccess) return -1;
             n++;
             // 2. attention
             a.prof_id = n;
-            if (launch_attention(s, a, hd, e->st) != cudaSuccess) return -1;
+            if (launch_attention_behind(qkv, s, a, hd, e->st) != cudaSuccess) return -1;
             n++;
         }
         auto tap = [&](float* dst, const float* src, int width) {

@@ -55,8 +55,8 @@ __device__ __forceinline__ float gdn_conv_value(const GdnArgs& a, int c, int cha
     return acc / (1.f + expf(-acc));
 }
 
-// Inside a token the kernel before this one is the layer's projection, which writes neither the state nor the conv history
-// and starts this kernel only when what ran before it is complete: the state (64 KB a head) and all that does not come from the
+// Inside a token (st) the kernel before this one is the layer's projection, which writes neither the state nor the conv history
+// and starts this kernel only behind its own wait, when what ran before it is complete (WaitsFirst): the state (64 KB a head) and all that does not come from the
 // projection is asked for before the dependency wait and arrives under it (64 tokens in and 32 out on the hybrid 4B shape, with the
 // same in k_qk_norm_rope_store: 46.33 -> 44.57 ms).  A stand-alone call may follow another one on the same state and waits first.
 __global__ void __launch_bounds__(GDN_THREADS, 1) k_gdn_step(GdnArgs a, const TokenState* st) {
@@ -367,7 +367,7 @@ struct QkNormArgs {
 };
 
 __global__ void __launch_bounds__(256) k_qk_norm_rope_store(QkNormArgs a, const TokenState* st) {
-    // the state's words together and before the wait, as in k_gdn_step: the kernel before this one does not write them
+    // the state's words together and before the wait, as in k_gdn_step: the kernel before this one (WaitsFirst) does not write them
     int done = 0, pos0 = a.pos;
     if (st) {
         done = st->done, pos0 = st->pos;

@@ -481,6 +481,8 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     prof_mark(3, pa.prof_id);
     // Only now may the next kernel start its prologue: its bulk weight requests then queue behind this
     // kernel's own latency-critical loads instead of in front of them, and never run two kernels ahead.
+    // Results depend on it, too: k_gdn_step, k_qk_norm_rope_store and k_attn_decode read ahead of their wait what kernels before
+    // this one wrote (WaitsFirst below).
     griddep_launch_dependents();
     const int done = st ? st->done : 0;
     // residual values of this CTA's rows (pair-ordered epilogues only), one per thread
@@ -745,8 +747,16 @@ inline cudaError_t launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// The launch of a kernel that lets the next one start only behind its own dependency wait: all that ran before it is complete by
+// then.  Kernels that read such results ahead of their own wait (the decode state, the recurrent state, cache rows) are launched
+// directly behind one and take its WaitsFirst; k_gemm_tc, which lets the next kernel start at its entry, makes none.
+struct WaitsFirst {
+    cudaError_t err;
+    operator cudaError_t() const { return err; }
+};
+
 template <class BLK, class Epi>
-inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa, const RowJob& ja, const RowJob& jb,
+inline WaitsFirst launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa, const RowJob& ja, const RowJob& jb,
                                const F32Seg& fseg, const Epi& epi, int K, TokenState* st) {
     const int nb = K / 256;
     constexpr int TB = BLK::TILE_BYTES;
@@ -764,7 +774,7 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     // tiles a CTA can need: where row groups are no whole tiles, a matrix's share may straddle an extra one
     const int straddle = (ROW_GROUP * nb) % 32 ? 1 : 0;
     const int need = (ra * nb + 31) / 32 + straddle + (rb ? (rb * nb + 31) / 32 + straddle : 0);
-    if (fixed + 256 + 1024 + TB > GEMV_SMEM_MAX) return cudaErrorInvalidValue;
+    if (fixed + 256 + 1024 + TB > GEMV_SMEM_MAX) return WaitsFirst{cudaErrorInvalidValue};
     int slots = (int)((GEMV_SMEM_MAX - fixed - 256 - 1024) / (TB + 8));
     const bool resident = slots >= need;
     if (resident) slots = need;
@@ -773,7 +783,7 @@ inline cudaError_t launch_gemv(cudaStream_t stream, int grid, const PrepArgs& pa
     const size_t smem = fixed + (size_t)slots * 8 + 256 + (size_t)slots * TB;
     auto launch = [&](auto threads, auto whole) {
         constexpr int T = decltype(threads)::value;
-        return launch_pdl(k_gemv<BLK, Epi, T, decltype(whole)::value>, dim3(grid), dim3(T), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st);
+        return WaitsFirst{launch_pdl(k_gemv<BLK, Epi, T, decltype(whole)::value>, dim3(grid), dim3(T), smem, stream, pa, ja, jb, fseg, epi, K, pf, slots, st)};
     };
     auto by_rows = [&](auto threads) {
         // (Q8_0: no gain, 2 048 x 8 192 and 2 048 x 2 048 residual rows in turn 9.15 us without and 9.14 with such an instance)
