@@ -218,7 +218,7 @@ __device__ __forceinline__ void tc_st(unsigned addr, const float* v) {
                      : "memory");
 }
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 16, 24 or 32 columns.
+// 16 or 24 columns.
 template <int N>
 __device__ __forceinline__ void tc_ldn(float* v, unsigned addr) {
 #pragma unroll
@@ -234,12 +234,8 @@ __device__ __forceinline__ void tc_stn(unsigned addr, const float* v) {
 // Waits for this warp's loads.  Uses of the values stay behind it if they are volatile assembly (fma_pair and the like); other uses
 // take the second form, which costs moves.
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-template <int W>
-__device__ __forceinline__ void tc_ld_wait(float* v) {
-    if constexpr (W == 8)
-        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])::"memory");
-    else
-        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])::"memory");
+__device__ __forceinline__ void tc_ld_wait8(float* v) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])::"memory");
 }
 __device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
     float2 d;
@@ -526,12 +522,13 @@ struct TcGeom {
     static constexpr int T_BYTES = TC_LANES * 128, W_PLANE = ROWS * 128, STAGE = T_BYTES + (Q4 ? 1 : 2) * W_PLANE;
     static constexpr int SUM_STRIDE = ROWS / 2 + 1;         // float2 of a token's sums when k parts meet; odd, so that 16 tokens' pairs lie in 32 banks
     static constexpr int OUT_PAIRS = 4;               // pairs of columns a warp turns from tokens to columns at a time
-    static constexpr int WARP_BYTES = 32 * (OUT_PAIRS + 1) * 8 + NC * 4;  // a draining warp's own: that, and its columns' d and dmin
+    static constexpr int WARP_BYTES = 32 * (OUT_PAIRS + 1) * 8 + (Q4 ? 0 : NC * 4);  // a draining warp's own: that, and on Q6_K its columns' d
     static constexpr int ONES_BYTES = Q4 ? TC_LANES * 32 : 0;  // a tf32 operand whose first column is ones, the others zero
     static constexpr int NST_MAX = (int)((TC_SMEM_MAX - 1024 - TC_D_WARPS * WARP_BYTES - ONES_BYTES) / STAGE);
     static constexpr int NST = NST_MAX < TC_MAX_STAGES ? NST_MAX : TC_MAX_STAGES;
     static constexpr size_t SMEM = (size_t)NST * STAGE + TC_D_WARPS * WARP_BYTES + ONES_BYTES + 1024;
-    static_assert(NC % CH == 0 && WARP_BYTES % 16 == 0 && (TC_ACCS + 1) * ROWS <= 512 && NC % 8 == 0 && TC_LANES * SUM_STRIDE * 8 <= NST * STAGE, "");
+    static_assert(ROWS % 32 == 0 && NC <= 32 && NC % CH == 0 && NC / 2 % OUT_PAIRS == 0, "whole warps of rows, a lane for every column, whole steps");
+    static_assert(WARP_BYTES % 16 == 0 && (TC_ACCS + 1) * ROWS <= 512 && TC_LANES * SUM_STRIDE * 8 <= NST * STAGE, "");
 };
 constexpr size_t TC_PARK_BYTES = TC_LANES * 96 * 4;
 // Scratch for matrices of nb blocks a row: three CTAs' sums for every SM, where a chain can be cut at all.
@@ -557,7 +554,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
     unsigned char* smem = tc_smem_raw + (-smem_u32(tc_smem_raw) & 1023u);
     if (tid == 0) {
         for (int i = 0; i < nst; i++) {
-            mbar_init(bars + i, (ROWS + 31) / 32 + 1);  // the warps that unpack a half and the tokens (with the bytes)
+            mbar_init(bars + i, ROWS / 32 + 1);  // the warps that unpack a half and the tokens (with the bytes)
             mbar_init(bars + TC_MAX_STAGES + i, 2);
         }
         for (int i = 0; i < 2; i++) {
@@ -678,17 +675,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
         tc_regs<TC_REGS_A>();
         const int ta = tid - 32 * TC_C_WARPS, g = ta >> 7, row_l = ta & 127;  // half of the blocks; row of the tile
         griddep_launch_dependents();
-        if (row_l < ((ROWS + 31) & ~31)) {
-            const int r = min(row_l, ROWS - 1);
-            const bool on = row_l < ROWS;
-            const unsigned tile = smem_u32(smem) + T_BYTES + tc_row_at(r);  // the row in slot 0
+        if (row_l < ROWS) {
+            const unsigned tile = smem_u32(smem) + T_BYTES + tc_row_at(row_l);  // the row in slot 0
             int slot = 0;  // of the block's first stage
             unsigned lap = 0;
             bool again = false;  // the ring has been round
             for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
                 const TcItem<ROWS> it(a, item);
                 int f0;
-                const uint8_t* wdata = it.row(a, r, f0);
+                const uint8_t* wdata = it.row(a, row_l, f0);
                 RAW raw;
                 raw.load_stage(0, wdata, f0 + ROW_GROUP * b0, g);  // weights do not depend on earlier kernels
                 raw.load_stage(1, wdata, f0 + ROW_GROUP * b0, g);
@@ -710,7 +705,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
                     const bool wrap = slot + s >= nst;
                     const int at = slot + s - (wrap ? nst : 0);
                     if (again || wrap) tc_wait_idle(empty + 8 * at, (lap ^ (wrap ? 1u : 0u)) ^ 1u, dead);
-                    if (on) fill(tile + at * STAGE);
+                    fill(tile + at * STAGE);
                     __syncwarp();
                     if (lane == 0) tc_arrive(full + 8 * at);
                 };
@@ -745,26 +740,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
     const int pieces = (b1 - b0 + TC_CHAIN - 1) / TC_CHAIN;
     unsigned par = 0;  // of the buffers' first uses in a block; Q4_K uses them three times
     for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
-        // Q6_K: lanes hold two columns' d, a block ahead: column lane and, where there is one, 32 further
-        int df, dmore;  // flat index of the one; from there to the other
+        // Q6_K: the lanes hold the columns' d, a block ahead
+        int df;
         const uint8_t* dp;
         unsigned d8_at;
         {
             const TcItem<ROWS> it(a, item);
-            int f;
-            dp = (a.zip && (lane & 1)) || it.second ? a.A2.data : a.A1.data;
             d8_at = (unsigned)(4 * b0) * a.Mp + min(it.n0 + tok, a.Mp - 1);
-            it.row(a, cg * NC + min(lane, NC - 1), df);
-            it.row(a, cg * NC + (NC > 32 ? min(lane + 32, NC - 1) : 0), f);  // 32 is even: the same matrix, unless it repeats the last column
-            dmore = lane + 32 < NC ? f - df : 0;
+            dp = it.row(a, cg * NC + min(lane, NC - 1), df);
         }
-        float dnext[2];
+        float dnext;
         auto load_d = [&](int b) {
-#pragma unroll
-            for (int h = 0; h < (NC > 32 ? 2 : 1); h++) {
-                const int f = df + ROW_GROUP * b + (h ? dmore : 0);
-                dnext[h] = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(dp + (size_t)(f >> 5) * Q6_TILE_BYTES + Q6_PIECES * 512 + (f & 31) * 2)));
-            }
+            const int f = df + ROW_GROUP * b;
+            dnext = f16_to_f32(__ldg(reinterpret_cast<const unsigned short*>(dp + (size_t)(f >> 5) * Q6_TILE_BYTES + Q6_PIECES * 512 + (f & 31) * 2)));
         };
         if (!Q4) load_d(b0);
         // d8 of the token's groups, two stages ahead
@@ -787,8 +775,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
         clear();
         for (int b = b0; b < b1; b++) {
             if (!Q4) {
-                if (lane < NC) colscale[lane] = dnext[0];
-                if (NC > 32 && lane + 32 < NC) colscale[lane + 32] = dnext[1];
+                if (lane < NC) colscale[lane] = dnext;
                 if (b + 1 < b1) load_d(b + 1);
             }
             // use k of the block of buffer `buf`
@@ -914,7 +901,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
         for (int c = 0; c < NC / 8; c++) {
             float v[8];
             tc_ld<8>(v, lanes_tot + 8 * c);
-            tc_ld_wait<8>(v);
+            tc_ld_wait8(v);
 #pragma unroll
             for (int i = 0; i < 4; i++) tot[4 * c + i] = make_float2(v[2 * i], v[2 * i + 1]);
         }
@@ -943,7 +930,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
             continue;
         }
         constexpr int OP = G::OUT_PAIRS;
-        static_assert((NC / 2) % 4 == 0, "");
         const bool res = a.epi.kind == CEPI_STORE && a.epi.use_res == 2;
         ChunkEpi epi = a.epi;
         epi.use_res = 0;
@@ -952,11 +938,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < OP; i++)
-                if (c + i < NC / 2) turn[lane * (OP + 1) + i] = tot[c + i];
+                turn[lane * (OP + 1) + i] = tot[c + i];
             __syncwarp();
             const int pl = lane & (OP - 1), pair = cg * (NC / 2) + c + pl;
             const int row = it.row0 + (a.zip ? pair : 2 * pair);
-            const bool on = c + pl < NC / 2 && row < it.N;
+            const bool on = row < it.N;
             const int id = it.id_base + (a.zip ? row : row >> 1);
             float2 r[OP];
 #pragma unroll
