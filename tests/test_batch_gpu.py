@@ -213,6 +213,58 @@ def test_larger_batches_beyond_one_tile_a_cta(E, wtype, K, N, M):
     w.free()
 
 
+@pytest.mark.parametrize("wtype", [S.Q4_K, S.Q6_K], ids=["q4", "q6"])
+@pytest.mark.parametrize("K,N,M", [(20736, 888, 1792), (27648, 885, 1790)])
+def test_larger_batches_whose_chains_have_middle_pieces(E, wtype, K, N, M):
+    """81 and 108 blocks a row on 10 x 14 tiles of 96 rows x 128 tokens, which is one round of CTAs with the k range in one part: chains of
+    additions in three and four pieces, whose middle ones read parked sums and park again.  Error against float64, against dp4a's."""
+    rng = np.random.default_rng(K)
+    w, exact = _matrix(E, wtype, K, N, rng)
+    x = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).cuda()
+    dp4a, tc = _errors(E, w, exact, x, (DP4A, TC))
+    assert tc < PRECISION * dp4a, (dp4a, tc)
+    w.free()
+
+
+@pytest.mark.parametrize("K,N,M", [(512, 11008, 300), (512, 5003, 300), (256, 3600, 640)])
+def test_gate_up_pairs_beyond_one_tile_a_cta(E, K, N, M):
+    """Interleaved pairs where a CTA works on several tiles: whole tiles that leave from the registers, a last tile with rows that do not
+    exist, outputs that are no multiple of four.  All values against dp4a on the same int8 activations.  The bound of the sums holds
+    for their product: an error e of both branches moves it by at most (1.1 |up| + |gate|) e, which at the largest value, a few rms in
+    either branch, is below e times that value."""
+    from taraference_b200 import synth_gpu as G
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K + N)
+    w, b = (E.GpuMat(S.Q4_K, K, N, G.quantized_matrix(S.Q4_K, K, N, gen, 0.04)) for _ in range(2))
+    x, outs = torch.randn((M, K), generator=gen, device="cuda"), []
+    for route in (DP4A, TC):
+        outs.append(torch.full((M, N), float("nan"), device="cuda"))
+        E.op_project_rows(w, x, outs[-1], M, route=route, b=b)
+    assert _rel(outs[1].cpu().numpy(), outs[0].cpu().numpy()) < SAME_INT8
+    w.free()
+    b.free()
+
+
+def test_q_and_k_rows_beyond_one_tile_a_cta(E, monkeypatch):
+    """A matrix that follows another in one launch (K rows behind Q rows) where a CTA works on several tiles of both: 43 + 6 row tiles x 5
+    token tiles.  K rows of all tokens against the dp4a route's, up to f16 steps; the second layer's, which depend on the first
+    one's Q rows of every token, up to what a flipped rounding moves."""
+    cfg = dict(ODD, n_layer=2, n_embd=512, n_head=32, n_kv=4, n_ff=1024, n_vocab=2000)
+    m, n = E.CudaModel.load_with(cfg, S.make_dense_model(cfg, seed=37)), 640
+    prompt = [int(t) for t in np.random.default_rng(3).integers(0, cfg["n_vocab"], n)]
+    out = []
+    for dp4a in (True, False):
+        (monkeypatch.setenv if dp4a else monkeypatch.delenv)(*(("TFR_GEMM_DP4A", "1") if dp4a else ("TFR_GEMM_DP4A",)))
+        kv = m.alloc_kv(n + 8)
+        m.forward_greedy(prompt, kv)
+        out.append([m.debug_read("k", n * 512, np.uint16, kv=kv, layer=i).view(np.float16).astype(np.float32) for i in range(2)])
+        kv.free()
+    (a0, a1), (b0, b1) = out
+    assert _rel(b0, a0) < 5e-4
+    assert _rel(b1, a1) < 2 * TF_WORST
+    m.destroy()
+
+
 @pytest.mark.parametrize("chunk,n", [(2, 7), (16, 16), (16, 45), (64, 19), (2048, 41)])
 def test_hybrid_prompt_in_batches_equals_step_by_step(E, chunk, n):
     """Batches of a hybrid model: conv history across batches (shorter ones than the kernel, too), scan tiles of 16 tokens,
