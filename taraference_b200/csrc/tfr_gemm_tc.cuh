@@ -531,8 +531,13 @@ struct TcGeom {
     static_assert(WARP_BYTES % 16 == 0 && (TC_ACCS + 1) * ROWS <= 512 && TC_LANES * SUM_STRIDE * 8 <= NST * STAGE, "");
 };
 constexpr size_t TC_PARK_BYTES = TC_LANES * 96 * 4;
-// Scratch for matrices of nb blocks a row: three CTAs' sums for every SM, where a chain can be cut at all.
-__host__ __device__ inline size_t tc_park_bytes(int nb, int sms) { return nb > TC_CHAIN ? (size_t)3 * sms * TC_PARK_BYTES : 0; }
+// Most CTAs of a launch that cut chains: one an SM where the k range is in one part, three where parts of it are cut once more.
+__host__ __device__ inline int tc_park_ctas(int parts, int sms) { return (parts > 1 ? 3 : 1) * sms; }
+// Scratch for matrices of up to nb blocks a row, the sums of those CTAs (7.3 MB on 148 SMs for rows of 7 168 to 13 824 inputs, 21.8 MB
+// for longer ones): rows short of two chains are whole ones or cut once, by the parts.
+__host__ __device__ inline size_t tc_park_bytes(int nb, int sms) {
+    return nb > 2 * TC_CHAIN ? tc_park_ctas(2, sms) * TC_PARK_BYTES : nb > TC_CHAIN ? tc_park_ctas(1, sms) * TC_PARK_BYTES : 0;
+}
 
 template <class RAW, int ROWS>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant__ TcArgs a) {
@@ -1231,7 +1236,7 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
             int first;
             const int ctas = tiles(r, first) * a.groups * s, at_once = cluster_ctas(k_gemm_tc<RawQ4, 96>, TC_THREADS, s, sms);
             const int blocks = (ja.m.nb + s - 1) / s;
-            if (s > 1 && blocks > TC_CHAIN && ctas > 3 * sms) continue;  // parked sums have no room
+            if (s > 1 && blocks > TC_CHAIN && ctas > tc_park_ctas(s, sms)) continue;  // parked sums have no room
             const double t = (double)((ctas + at_once - 1) / at_once) * ((r == 96 ? 0.75 : 0.62) * blocks + 1 + (s > 1 ? 1 : 0));
             if (t < best) best = t, S = s, rows = r;
         }
