@@ -77,6 +77,12 @@ def test_projections_of_batches_at_tile_edges(E, oracle, cfg, n, monkeypatch):
     m.destroy()
 
 
+@pytest.mark.parametrize("n", [64, 65, 72, 80, 81])
+def test_projections_of_a_batch_on_both_tensor_core_kernels(E, oracle, n, monkeypatch):
+    """The same where gate and up rows are on tcgen05 beside Q, K and output rows on mma.sync: 65 to 80 tokens, more than 4 096 rows."""
+    test_projections_of_batches_at_tile_edges(E, oracle, dict(ODD, n_ff=5120), n, monkeypatch)
+
+
 def _q4_k_exact(raw, K, N):
     """GGUF bytes -> float64 weights, exactly (kernels/common.cu:40-84)."""
     b = raw.reshape(N, K // 256, 144)
@@ -153,6 +159,25 @@ def test_projection_routes_agree_on_equal_int8(E, wtype, K, N):
         assert _rel(outs[1], outs[0]) < SAME_INT8 and _rel(outs[2], outs[0]) < SAME_INT8, kw.keys()
     w.free()
     w2.free()
+
+
+@pytest.mark.parametrize("wtype,N,M,pair,route", [
+    (S.Q4_K, 512, 4, False, DP4A), (S.Q4_K, 512, 5, False, MMA), (S.Q4_K, 4097, 64, False, MMA), (S.Q4_K, 4097, 65, False, TC), (S.Q4_K, 4096, 65, False, MMA),
+    (S.Q4_K, 4096, 80, False, MMA), (S.Q4_K, 4096, 81, False, TC), (S.Q4_K, 4096, 65, True, MMA), (S.Q4_K, 4100, 65, True, TC),
+    (S.Q6_K, 512, 32, False, MMA), (S.Q6_K, 512, 33, False, TC)])
+def test_route_of_a_batch(E, wtype, N, M, pair, route):
+    """The engine's own choice on both sides of every line is the kernel whose bits it leaves; all kernels agree up to the order of sums."""
+    rng = np.random.default_rng(N + M)
+    w, b = (_matrix(E, wtype, 1024, N, rng)[0] for _ in range(2))
+    x, out = torch.from_numpy(rng.standard_normal((M, 1024)).astype(np.float32)).cuda(), {}
+    for r in (-1, DP4A, TC) + ((MMA,) if M <= (80 if wtype == S.Q4_K else 32) else ()):
+        out[r] = torch.full((M, N), float("nan"), device="cuda")
+        E.op_project_rows(w, x, out[r], M, route=r, b=b if pair else None)
+    for r in out:
+        assert torch.equal(out[r], out[-1]) == (r in (-1, route)), r
+        assert _rel(out[r].cpu().numpy(), out[DP4A].cpu().numpy()) < SAME_INT8
+    w.free()
+    b.free()
 
 
 # Rounding errors of fp32 sums of exact products grow with the kernel's order of additions alone: dp4a adds a row's blocks as a
