@@ -1790,9 +1790,12 @@ static int chunk_buffers(tfr_engine* e, int M) {
 
 // The kernel of a batch's projections.  Fewer than five tokens leave the tensor cores idle and keep the dp4a kernel, as Q8_0
 // matrices do (TFR_GEMM_DP4A=1 in the environment keeps everything there, a test aid).  mma.sync where it is the faster one.
-// Launches by themselves, us, mma.sync against tcgen05: Q4_K, 11 008 gate and up rows of 2 048, 48 tokens 31 : 47, 64 tokens 50 : 48,
-// 65 tokens 60 : 47; 27 648 rows of 5 120, 48 tokens 170 : 203, 64 211 : 204, 65 367 : 204; few rows (2 048 of 2 048) 64 tokens
-// 10.5 : 14.8, 80 tokens 14.0 : 14.9.  Q6_K, whose MMAs are half as deep, 2 048 rows of 11 008: 32 tokens 26 : 35.
+// Launches by themselves (cold caches), us, mma.sync : tcgen05.  Q4_K at 64 and at 65 tokens, where mma.sync needs another pass of tokens:
+// 12 288 rows of 2 048 26.5 : 28.3 and 38.4 : 28.7, of 5 120 55.7 : 55.8 and 106 : 57; gate and up rows, 11 008 of 2 048 each, 48.6 : 49.1
+// and 59.8 : 49.2; 6 144 rows of 2 048 17.8 : 21.7 and 21.9 : 20.9.  The line of 4 096 rows (of the first matrix) is where rows of 2 048
+// inputs break even at 65 to 80 tokens: 2 048 rows 13.2 : 14.6, 4 096 rows 18.8 : 18.8, pairs of 2 048 and 3 072 rows 17.8 : 18.8 and
+// 20.4 : 20.4.  Longer rows cross earlier (4 096 rows of 5 120 at 65 tokens 44.8 : 31.3, 2 048 of 11 008 49.3 : 32.7): the line costs
+// them that much.  Q6_K, whose MMAs are half as deep, 2 048 rows of 11 008: 32 tokens 26 : 35.
 enum { GEMM_DP4A, GEMM_MMA, GEMM_TC };
 static int gemm_route(const Mat& m, int M) {
     const int type = m.type, nb = m.nb;

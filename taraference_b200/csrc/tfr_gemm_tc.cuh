@@ -19,14 +19,18 @@
 // The min term of Q4_K, sum over a block's groups of m * (d8 * sum q8), is a tf32 product of 8 terms: m is exact, the group sums
 // are two rounded terms whose products stay in accumulators of their own.
 //
-//   What bounds it: instructions, and the waits between the roles.  The schedulers issue in two thirds of the cycles; a block of 256
-//   weights x 96 rows x 128 tokens takes 4 300 cycles, of which the tensor pipe works a fifth.  Gate and up rows of 2 048 inputs,
+//   What bounds it: instructions, and the waits between the roles.  A block of 256 weights x 96 rows x 128 tokens takes 4 300
+//   cycles; the schedulers issue in 57 % of them, the tensor pipe works in 21 (768 tokens).  Gate and up rows of 2 048 inputs,
 //   2 048 tokens: 477 us (before: 744), without the unpacking 433, without the MMAs 385, without the multiply-adds 433, with none of
 //   them and without the blocks' ends 212.  11 008 inputs to 2 048 rows: 281 us (before: 326).
 //   What made the difference: waits looked at before their loop (tc_wait), one hand-over for both groups of a stage (532 us with one
 //   for each), d and dmin from TMEM (tc_mma of ones), a CTA that goes on with the next tile, no register spills (local memory is an
 //   L2 round trip where shared memory takes all of L1).  Tried on the way: eight draining warps with 48 or 64 columns each (532 us),
-//   one issuing warp (534), pairs of CTAs on one tile of rows (an arrival at the other CTA takes 1 000 cycles).
+//   one issuing warp (534), pairs of CTAs on one tile of rows (an arrival at the other CTA takes 1 000 cycles).  A CTA's first rows
+//   into L2 at its entry, as the ones that follow: launches of several token tiles up to 7 % faster, of one tile on Q4_K up to 5 %
+//   slower, prompts as before (77 tokens 5 251 and 5 228 us, 2 048 tokens 45 098 and 45 123).
+//   Fixed costs are higher than with one tile a CTA: launches of a few blocks a CTA on Q6_K take 0.7 to 1 us more (512 inputs to 2 048
+//   rows, 40 tokens, 11.1 -> 12.0 us).
 #pragma once
 #include "tfr_chunk.cuh"
 
@@ -1221,9 +1225,10 @@ inline cudaError_t launch_gemm_tc(cudaStream_t stream, int sms, const unsigned c
     a.epi = epi, a.st = st, a.park = park;
     a.groups = (M + TC_LANES - 1) / TC_LANES;
     // Tile and number of k parts with the shortest longest chain: waves of CTAs x (blocks x what a block takes + the ends), in units of
-    // 3.2 us.  Measured: 96 rows 2.4 us a block, 64 rows 1.95; ends 3 us, cut k ranges 3 more.  Down rows of 11 008 inputs: 77 tokens
-    // 29.7 us (64 rows, four parts; 96 rows 32.8, one part 99.8), 300 tokens 58.6 (96 rows, two parts; one 103, four 66.6), 2 048
-    // tokens 284 (two parts; one 319).
+    // 3.2 us.  Measured on Q6_K rows: 96 rows 2.4 us a block, 64 rows 1.95; ends 3 us, cut k ranges 3 more.  Q4_K has other stages and takes
+    // what Q6_K takes (2 048 rows of 11 008 inputs, 500 and 2 048 tokens: 99.7 and 295 us, Q6_K 104 and 298).  All eight choices timed on
+    // 14 matrices and pairs of both types, 2 048 to 27 648 inputs, at 66 to 2 048 tokens: the one taken is the fastest or within 7 % of it,
+    // in 109 of 112 within 4 % (2 048 rows of 11 008 at 1 000 tokens 191 us in tiles of 64 rows, 179 in 96 and two parts).
     int S = 1, rows = 96;
     double best = 1e30;
     auto tiles = [&](int r, int& first) {

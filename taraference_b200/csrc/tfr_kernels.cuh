@@ -383,7 +383,8 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     const int nb = K >> 8;
     constexpr int TB = BLK::TILE_BYTES;
     // aligned as an offset, not as an address: the compiler then knows that tiles lie in shared memory and reads them as such
-    // (a token of the 3B shape 1 286 -> 1 264 us, 32 tokens on eight layers of the 32B shape 28.42 -> 27.72 ms)
+    // (with the early request of the plain vector below: a token of the 3B shape 1 297 -> 1 273 us, 32 tokens on eight layers of the 32B
+    // shape 28.44 -> 27.56 ms, a feed-forward block 15.69 -> 15.32 us)
     const unsigned ring_at = ((unsigned)act_bytes + ((unsigned)pbuf_floats + 272) * 4 + 8 * (unsigned)slots + 127) & ~127u;
     unsigned char* ring = smem + ring_at;
 
@@ -495,7 +496,7 @@ k_gemv(PrepArgs pa, RowJob ja, RowJob jb, F32Seg fseg, Epi epi_in, int K, int pb
     float scale = 1.f;
     if (!embed && !with_xf) {
         // plain vector: quantise pass by pass straight from the registers that fetched it.  The vector is asked for beside `done`, not
-        // behind it: that would be a second trip to L2 in a row (64 tokens of the 3B shape 70.91 -> 70.53 ms)
+        // behind it: that would be a second trip to L2 in a row (64 tokens of the 3B shape 70.91 -> 70.53 ms, the two together 71.05 -> 70.72)
         for (int base = 0; base < n4; base += STAGE_REGS * T) {
             float4 sx[STAGE_REGS];
 #pragma unroll
