@@ -305,3 +305,31 @@ def test_hybrid_with_q5_k_and_q8_0_tensors(E, oracle):
     assert np.median(le) < 2e-5 and le.max() < TF_WORST and he.max() < TF_WORST, (le, he)
     kv.free()
     m.destroy()
+
+
+def test_stopped_burst_leaves_the_recurrent_state_of_its_last_token(E):
+    """Tokens that are already enqueued when a burst stops pass by without touching the recurrent state or the conv history: a stopped burst
+    and one that was asked for no more leave the same bits, and continue alike."""
+    cfg = S.TINY_HYBRID
+    m = E.CudaModel.load_with(cfg, S.make_model(cfg, seed=12))
+    channels = (2 * cfg["ssm_n_k"] + cfg["ssm_n_v"]) * 128
+    linear = [i for i in range(cfg["n_layer"]) if S.is_linear_layer(cfg, i)]
+
+    def burst(n, **kw):
+        kv = m.alloc_kv(64)
+        toks = list(m.decode_burst(m.forward_greedy([5, 6, 7], kv), n, kv, **kw))
+        state = [m.debug_read("ssm_state", cfg["ssm_n_v"] * 128 * 128, kv=kv, layer=i) for i in linear]
+        state += [m.debug_read("conv_state", (cfg["conv_kernel"] - 1) * channels, kv=kv, layer=i) for i in linear]
+        m.forward_greedy([9], kv)
+        state.append(m.current_logits())
+        kv.free()
+        return toks, state
+
+    free, _ = burst(24)
+    at = max(free.index(t) for t in set(free))  # the latest first appearance of a token
+    assert at < 23
+    cut, a = burst(24, stop_ids=[free[at]])
+    whole, b = burst(at + 1)
+    assert cut == whole == free[:at + 1]
+    assert all(np.array_equal(x, y) for x, y in zip(a, b))
+    m.destroy()
